@@ -27,6 +27,7 @@
 
 #include "aig_b200.h"
 #include "aig_host.h"
+#include "cnn_stream.h"
 
 namespace {
 
@@ -90,6 +91,7 @@ struct aig_cnn {
   uint8_t* frames_slot[2] = {nullptr, nullptr};
   cudaEvent_t ev_h2d[2] = {nullptr, nullptr}, ev_used[2] = {nullptr, nullptr}, ev_done[2] = {nullptr, nullptr};
   bool slot_used[2] = {false, false};
+  CnnStaging staging;                  // host memory of the offline inference over recordings, from its first call on
   int launches_per_forward = 0;
   // optional per-launch timing (eager forward only): one CUDA event between consecutive launches
   struct Site {
@@ -102,6 +104,8 @@ struct aig_cnn {
   int prof_cap = 0, prof_steps = 0;
   bool prof_on = false;
 };
+
+static void cnn_staging_free(CnnStaging& st);
 
 namespace {
 
@@ -328,6 +332,7 @@ int aig_cnn_destroy(aig_cnn* m) {
       if (m->ev_done[i]) cudaEventDestroy(m->ev_done[i]);
     }
   }
+  cnn_staging_free(m->staging);
   aig_conv0_plan_destroy(m->conv0);
   for (auto& b : m->blocks) {
     aig_conv_plan_destroy(b.c0);
@@ -575,16 +580,15 @@ int aig_cnn_forward_graph_rgb(aig_cnn* m, const uint8_t* rgb_planar_dev) { retur
 // forward of step i.  Host buffers should be pinned.
 }  // extern "C"
 
-static int cnn_submit_host_impl(aig_cnn* m, int slot, const uint8_t* bgra_host, float* out_host, bool planar) {
-  if (!m || !bgra_host || !out_host || slot < 0 || slot > 1) return AIG_ERR_INVALID;
-  const aig_cnn_config& c = m->cfg;
-  const size_t fb = (size_t)c.batch * c.height * c.width * 4;             // slot buffers hold either format
-  const size_t copy_bytes = (size_t)c.batch * c.height * c.width * (planar ? 3 : 4);
-  cudaStream_t s = (cudaStream_t)aig_ctx_stream(m->ctx);
+static size_t cnn_slot_bytes(const aig_cnn* m) { return (size_t)m->cfg.batch * m->cfg.height * m->cfg.width * 4; }  // either frame format
+
+const aig_cnn_config& cnn_config(const aig_cnn* m) { return m->cfg; }
+
+int cnn_stream_begin(aig_cnn* m, int slot) {
   if (!m->copy_stream) {
     CNN_CUDA(m, cudaStreamCreateWithFlags(&m->copy_stream, cudaStreamNonBlocking));
     for (int i = 0; i < 2; ++i) {
-      CNN_CUDA(m, cudaMalloc(reinterpret_cast<void**>(&m->frames_slot[i]), fb));
+      CNN_CUDA(m, cudaMalloc(reinterpret_cast<void**>(&m->frames_slot[i]), cnn_slot_bytes(m)));
       CNN_CUDA(m, cudaEventCreateWithFlags(&m->ev_h2d[i], cudaEventDisableTiming));
       CNN_CUDA(m, cudaEventCreateWithFlags(&m->ev_used[i], cudaEventDisableTiming));
       CNN_CUDA(m, cudaEventCreateWithFlags(&m->ev_done[i], cudaEventDisableTiming));
@@ -592,16 +596,69 @@ static int cnn_submit_host_impl(aig_cnn* m, int slot, const uint8_t* bgra_host, 
   }
   // the slot's frame buffer is free once the forward that last read it has run
   if (m->slot_used[slot]) CNN_CUDA(m, cudaStreamWaitEvent(m->copy_stream, m->ev_used[slot], 0));
-  CNN_CUDA(m, cudaMemcpyAsync(m->frames_slot[slot], bgra_host, copy_bytes, cudaMemcpyHostToDevice, m->copy_stream));
+  return AIG_OK;
+}
+
+int cnn_stream_copy(aig_cnn* m, int slot, size_t offset, const void* host, size_t bytes, cudaEvent_t copied) {
+  if (offset + bytes > cnn_slot_bytes(m)) return fail(m, AIG_ERR_INVALID, "frames beyond the slot's batch");
+  CNN_CUDA(m, cudaMemcpyAsync(m->frames_slot[slot] + offset, host, bytes, cudaMemcpyHostToDevice, m->copy_stream));
+  if (copied) CNN_CUDA(m, cudaEventRecord(copied, m->copy_stream));
+  return AIG_OK;
+}
+
+int cnn_stream_submit(aig_cnn* m, int slot, float* out_host, bool planar) {
+  cudaStream_t s = (cudaStream_t)aig_ctx_stream(m->ctx);
   CNN_CUDA(m, cudaEventRecord(m->ev_h2d[slot], m->copy_stream));
   CNN_CUDA(m, cudaStreamWaitEvent(s, m->ev_h2d[slot], 0));
   const int rc = cnn_forward_graph_impl(m, m->frames_slot[slot], planar);
   if (rc != AIG_OK) return rc;
   CNN_CUDA(m, cudaEventRecord(m->ev_used[slot], s));
   m->slot_used[slot] = true;
-  CNN_CUDA(m, cudaMemcpyAsync(out_host, m->out_f32, (size_t)c.batch * c.n_out * sizeof(float), cudaMemcpyDeviceToHost, s));
+  CNN_CUDA(m, cudaMemcpyAsync(out_host, m->out_f32, (size_t)m->cfg.batch * m->cfg.n_out * sizeof(float), cudaMemcpyDeviceToHost, s));
   CNN_CUDA(m, cudaEventRecord(m->ev_done[slot], s));
   return AIG_OK;
+}
+
+int cnn_stream_drain(aig_cnn* m) {
+  if (m->copy_stream) CNN_CUDA(m, cudaStreamSynchronize(m->copy_stream));
+  CNN_CUDA(m, cudaStreamSynchronize((cudaStream_t)aig_ctx_stream(m->ctx)));
+  return AIG_OK;
+}
+
+static void cnn_staging_free(CnnStaging& st) {
+  cudaFreeHost(st.ring);
+  for (cudaEvent_t& e : st.copied)
+    if (e) cudaEventDestroy(e);
+  for (float* o : st.out) cudaFreeHost(o);
+  st = CnnStaging();
+}
+
+int cnn_staging(aig_cnn* m, size_t piece_bytes, int slots, CnnStaging** out) {
+  CnnStaging& st = m->staging;
+  if (st.piece_bytes < piece_bytes || st.slots < slots) {
+    cnn_staging_free(st);
+    const size_t ob = (size_t)m->cfg.batch * m->cfg.n_out * sizeof(float);
+    cudaError_t e = cudaMallocHost(reinterpret_cast<void**>(&st.ring), piece_bytes * slots);
+    for (int i = 0; i < 2 && e == cudaSuccess; ++i) e = cudaMallocHost(reinterpret_cast<void**>(&st.out[i]), ob);
+    for (int i = 0; i < slots && e == cudaSuccess; ++i) e = cudaEventCreateWithFlags(&st.copied[i], cudaEventDisableTiming);
+    if (e != cudaSuccess) {
+      cnn_staging_free(st);
+      return fail(m, AIG_ERR_CUDA, "pinned staging allocation failed");
+    }
+    st.piece_bytes = piece_bytes;
+    st.slots = slots;
+  }
+  *out = &st;
+  return AIG_OK;
+}
+
+static int cnn_submit_host_impl(aig_cnn* m, int slot, const uint8_t* frames_host, float* out_host, bool planar) {
+  if (!m || !frames_host || !out_host || slot < 0 || slot > 1) return AIG_ERR_INVALID;
+  const aig_cnn_config& c = m->cfg;
+  int rc = cnn_stream_begin(m, slot);
+  if (rc == AIG_OK) rc = cnn_stream_copy(m, slot, 0, frames_host, (size_t)c.batch * c.height * c.width * (planar ? 3 : 4), nullptr);
+  if (rc == AIG_OK) rc = cnn_stream_submit(m, slot, out_host, planar);
+  return rc;
 }
 
 extern "C" {

@@ -220,3 +220,32 @@ def test_recording_file_to_batched_inference(env, tmp_path):
     assert np.array_equal(t[:, :14], ((keys[:, None] >> np.arange(14)) & 1).astype(np.float32))
     enc.close()
     rec.close()
+
+
+@gpu
+@pytest.mark.parametrize("n", [1, 64, 65, 64 * 9 + 5])
+def test_recording_pieces(env, tmp_path, n):
+    """Recordings read in pieces by several threads: one frame, one batch, a batch and one frame, and more pieces than
+    the pinned ring has slots (56 + 8 frames a batch), against the same frames given to the encoder batch by batch."""
+    U = env
+    c, pk = U.ctx(), U.pkg()
+    B, H, W, widths = 64, 64, 96, (32, 64)
+    enc = pk.CnnEncoder(c, B, H, W, widths=widths)
+    enc.load_bytes(PL.serialize_cnn_checkpoint(PL.make_cnn_params(7, widths=widths, trivial=False), W, H))
+    frames = np.random.default_rng(n).integers(0, 256, (n, 3, H, W), dtype=np.uint8)
+    path = tmp_path / "r.bin"
+    with open(path, "wb") as f:
+        f.write(np.array([W, H], np.int32).tobytes())
+        for fr in frames:
+            f.write(b"\0" * 10 + fr.tobytes())
+    rec = pk.Recording(path)
+    got = rec.infer(enc, 0, n)
+    for lo in range(0, n, B):
+        chunk = np.zeros((B, 3, H, W), np.uint8)
+        chunk[: min(B, n - lo)] = frames[lo:lo + B]
+        enc.forward_rgb(U.dev(chunk))
+        c.sync()
+        assert np.array_equal(got[lo:lo + B], U.host(enc.outputs_f32())[: min(B, n - lo)])
+    assert np.array_equal(rec.infer(enc, 0, n), got)
+    rec.close()
+    enc.close()
