@@ -75,6 +75,22 @@ static inline long long ceil_div_ll(long long a, long long b) { return (a + b - 
 // Device helpers
 #ifdef __CUDACC__
 
+// Launch that may start under its predecessor's tail (the kernel calls griddep_wait before it touches what others write)
+template <class... P, class... A>
+static inline cudaError_t launch_pdl(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, A&&... args) {
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = grid;
+  cfg.blockDim = block;
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = stream;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
+}
+
 __device__ __forceinline__ float act_apply(float v, int act, float slope) {
   switch (act) {
     case AIG_ACT_RELU: return v > 0.f ? v : 0.f;

@@ -581,7 +581,7 @@ __global__ void fc_head_kernel(const __half* __restrict__ x, const __half* __res
 // x*m), global average pool, FC with the reference's two roundings (FCLayer.cpp:50-51), sigmoid on the
 // first n_sig outputs / tanh on the rest (Sigmoid.cpp:8-12), fp16 and fp32 results.  Same arithmetic
 // and rounding points as the stand-alone kernels above; x is read once from HBM.
-__global__ void cnn_head_kernel(const __half* __restrict__ x, const __half* __restrict__ w1, float b1,
+__global__ void cnn_head_kernel(const __half* x, const __half* __restrict__ w1, float b1,
                                 const __half* __restrict__ fcw, const __half* __restrict__ fcb, __half* __restrict__ feat,
                                 __half* __restrict__ out_h, float* __restrict__ out_f, int HW, int C, int n_out, int n_sig) {
   extern __shared__ uint8_t head_smem[];
@@ -591,6 +591,8 @@ __global__ void cnn_head_kernel(const __half* __restrict__ x, const __half* __re
   const int b = blockIdx.x, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, nwarps = blockDim.x >> 5;
   const __half* xb = x + (size_t)b * HW * C;
   const int nvec = HW * C / 8;
+  griddep_launch_dependents();  // the streaming agent's next launch loads its weights under this one
+  griddep_wait();
   for (int i = tid; i < nvec; i += blockDim.x) reinterpret_cast<uint4*>(sx)[i] = reinterpret_cast<const uint4*>(xb)[i];
   __syncthreads();
   for (int p = warp; p < HW; p += nwarps) {
@@ -874,10 +876,8 @@ int aig_cnn_head_forward(aig_ctx* ctx, const aig_half* x_nhwc, const aig_half* m
   if (smem > 200 * 1024) return aig_fail(ctx, AIG_ERR_UNSUPPORTED, "aig_cnn_head_forward: %d x %d feature map does not fit shared memory", hw, c);
   if (batch == 0) return AIG_OK;
   AIG_CUDA_OK(ctx, cudaFuncSetAttribute(cnn_head_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
-  cnn_head_kernel<<<batch, 256, smem, ctx->stream>>>((const __half*)x_nhwc, (const __half*)mask_w, mask_b, (const __half*)fc_w,
-                                                     (const __half*)fc_b, (__half*)feat, (__half*)out_half, out_f32, hw, c, n_out,
-                                                     n_sigmoid);
-  AIG_LAUNCH_OK(ctx);
+  AIG_CUDA_OK(ctx, launch_pdl(cnn_head_kernel, dim3(batch), dim3(256), smem, ctx->stream, (const __half*)x_nhwc, (const __half*)mask_w, mask_b,
+                              (const __half*)fc_w, (const __half*)fc_b, (__half*)feat, (__half*)out_half, out_f32, hw, c, n_out, n_sigmoid));
   return AIG_OK;
 }
 

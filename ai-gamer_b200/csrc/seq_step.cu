@@ -1,15 +1,22 @@
-// seq_step.cu -- the streaming step of the sequence head (LSTM layers -> attention over the ring cache
-// -> LayerNorm -> FC -> sigmoid/tanh) as ONE cooperative kernel for small batches.
+// seq_step.cu -- the streaming step of the sequence head ([bridge FC ->] LSTM layers -> attention over the ring cache
+// -> LayerNorm -> FC -> sigmoid/tanh) as ONE cooperative kernel for up to 128 sequences.
 //
-// At batch 1 every matrix of the head is a matrix-vector product: 10.5 MB of fp16 weights against a
-// handful of 512-element vectors, no tensor-core shape, and as separate launches (projection GEMM +
-// recurrent kernel per LSTM layer, three projections, attention, output projection, LayerNorm, FC,
-// activations) the step is ~18 launches of ~10 us each.  Here all SMs stream the weights with 16-byte
-// loads, one warp per output row (row-dot with a shuffle reduction), and the dependent stages are
-// separated by grid-wide barriers on a global counter (bounded spin, cooperative launch):
-//   LSTM layer 0 | LSTM layer 1 | ... | q,k,v | attention per (sequence, head) | output projection | tail
-// Arithmetic follows the multi-launch path: fp32 accumulation, fp16 where that path stores fp16
-// (h, c, q, k, v, context, attention output, LayerNorm output, FC output before and after the bias).
+// A step multiplies 10.5 MB of fp16 weights (two layers of 512) with one column per sequence.  What bounds it is the
+// chain of dependent stages, not bandwidth: as launches it was 15 of them at 9 to 19 us (a GEMM of one M tile walks its
+// K extent in 4 to 32 CTAs), and as one kernel that streamed the weights from L2 after each stage's barrier 57 us.  Here
+//  - the weights of a CTA (4 hidden units: their 16 gate rows of every layer's W and R, 4 rows each of Wq, Wk, Wv, Wo,
+//    the FC: 95 KB at 512) go to shared memory by bulk copies that are issued at once, before the kernel waits for its
+//    predecessor (programmatic launch), so they arrive under the last kernels of the frame encoder;
+//  - R.h of every layer needs the previous step only and is done while the first weights are the only ones there;
+//  - a stage is a [16 rows x K] x [K x batch] product on mma.sync m16n8k16: with 16 weight rows per CTA the stage is
+//    bound by latency and by L2 (every CTA reads all activations), which tcgen05's 128-row tiles would only worsen.
+//    The eight warps split the sequences in tiles of eight and, where there are fewer tiles than warps, K;
+//  - stages are separated by grid barriers on a global counter (bounded spin, cooperative launch):
+//    [bridge] | LSTM 0 | LSTM 1 | ... | q,k,v | attention per (sequence, head) | output projection | LayerNorm, FC.
+// The step's position and the barrier's epoch live in device memory, so that a captured graph replays the step.
+//
+// Arithmetic: fp32 accumulation, fp16 where the per-operator launches store fp16 (embedding before and after the bias,
+// h, c, q, k, v, context, attention output, LayerNorm output, FC output before and after the bias).
 #include <math.h>
 
 #include "aig_common.cuh"
@@ -22,25 +29,41 @@ constexpr int kWarps = kThreads / 32;
 constexpr int kMaxLayers = 4;
 constexpr int kMaxWindow = 128;
 constexpr int kHeadDim = 64;
+constexpr int kUnits = 4;         // hidden units (and rows of every other matrix) per CTA
+constexpr int kRows = 16;         // rows of an mma tile: four gates of kUnits units
+constexpr int kMaxBatch = 128;
+constexpr int kMaxBars = 2 + kMaxLayers + 3;
+constexpr size_t kMaxSmem = 220 * 1024;
+
+enum { kCount0 = 0, kCount1 = 1, kEpoch = 2, kPosition = 3, kWords = 4 };
 
 struct StepParams {
-  int B, in_c, H, layers, heads, window, n_out, n_sig;
-  int position, n_valid, double_bias;
+  int B, nt, kw;                  // sequences, tiles of eight of them, warps along K
+  int in_c, H, layers, heads, window, n_out, n_sig, feat, bridge_rows;
   float rope_base, scale, clip;
+  const __half* features;         // [B][feat], or null: emb is the input
+  const __half *bw_t, *bb;        // bridge [in_c][feat], bias
+  __half* emb_out;
   const __half* emb;
   const __half* lstm;
   unsigned long long w_off[kMaxLayers], r_off[kMaxLayers], bw_off[kMaxLayers], br_off[kMaxLayers];
+  int double_bias;
   const __half *wq_t, *wk_t, *wv_t, *wo_t, *fcw_t, *fcb;  // [out][in]
   const float *ln_g, *ln_b;
   __half *h_state, *c_state, *h_new;
-  __half *q, *k, *v, *ctx, *a, *n;
+  __half *q, *k, *v, *ctx, *a;
   __half *kcache, *vcache;
   __half *y, *logits;
   float* out_f32;
-  unsigned int* counter;       // this launch's barrier counter: zero when the launch starts
-  unsigned int* counter_next;  // the next launch's counter, zeroed by this launch
+  unsigned int* words;
   int* gerr;
+  // shared memory, bytes from the start
+  int o_r[kMaxLayers], o_w[kMaxLayers], o_bridge, o_qkv, o_wo, o_fc, o_pre, o_red, o_cell, o_hid, o_bias, o_attn;
 };
+
+// rows of `k` halfs in shared memory: whole 64-byte blocks, and an odd number of them, so that the eight rows a warp
+// reads at once (16 bytes a lane) fall on different banks
+__host__ __device__ constexpr int row_stride(int k) { return (((k * 2 + 63) / 64) | 1) * 64; }
 
 __device__ __forceinline__ unsigned int ld_acquire_gpu(const unsigned int* p) {
   unsigned int v;
@@ -50,214 +73,416 @@ __device__ __forceinline__ unsigned int ld_acquire_gpu(const unsigned int* p) {
 __device__ __forceinline__ void red_release_gpu_add(unsigned int* p, unsigned int v) {
   asm volatile("red.release.gpu.global.add.u32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
 }
-
-// Grid-wide barrier number `idx` of this launch.  Every CTA arrives once; the wait is bounded.
-__device__ bool grid_barrier(const StepParams& p, int idx, int* s_flag) {
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    __threadfence();
-    red_release_gpu_add(p.counter, 1u);
-    const unsigned int target = (unsigned int)(idx + 1) * gridDim.x;
-    const long long t0 = clock64();
-    int ok = 1;
-    while ((int)(ld_acquire_gpu(p.counter) - target) < 0) {
-      if (clock64() - t0 > AIG_WAIT_CYCLES) {
-        atomicCAS(p.gerr, 0, 701 + idx);
-        ok = 0;
-        break;
-      }
-    }
-    *s_flag = ok;
-  }
-  __syncthreads();
-  return *s_flag != 0;
+__device__ __forceinline__ void bulk_load(uint32_t dst, const void* src, uint32_t bytes, uint32_t bar) {
+  asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(dst), "l"(src), "r"(bytes), "r"(bar)
+               : "memory");
 }
-
-// sum_k w[k] * x[k] over n halfs (n % 8 == 0), lanes stride the 16-byte chunks; every lane gets the sum
-__device__ __forceinline__ float row_dot(const __half* __restrict__ w, const __half* __restrict__ x, int n, int lane) {
-  float acc = 0.f;
-  const uint4* w4 = reinterpret_cast<const uint4*>(w);
-  const uint4* x4 = reinterpret_cast<const uint4*>(x);
-  for (int c = lane; c < n / 8; c += 32) {
-    const uint4 a = __ldg(w4 + c), b = x4[c];
-    const __half2* ah = reinterpret_cast<const __half2*>(&a);
-    const __half2* bh = reinterpret_cast<const __half2*>(&b);
-#pragma unroll
-    for (int e = 0; e < 4; ++e) {
-      const float2 fa = __half22float2(ah[e]), fb = __half22float2(bh[e]);
-      acc = fmaf(fa.x, fb.x, acc);
-      acc = fmaf(fa.y, fb.y, acc);
-    }
-  }
-  for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
-  return acc;
+__device__ __forceinline__ void prefetch_l2(const void* p) { asm volatile("prefetch.global.L2 [%0];" ::"l"(p)); }
+__device__ __forceinline__ void mma_16816(float (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
+  asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+               : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
+               : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
 }
-
 __device__ __forceinline__ float sigmoidf_(float x) { return 1.0f / (1.0f + expf(-x)); }
 
-__global__ void __launch_bounds__(kThreads, 1) seq_step_kernel(const StepParams p) {
-  __shared__ int s_flag;
-  __shared__ float s_attn[kWarps * (kHeadDim + kMaxWindow)];
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int gw = blockIdx.x * kWarps + warp, tw = gridDim.x * kWarps;
-  const int H = p.H, B = p.B;
-  int bar = 0;
-  // Two counters alternate between launches.  Each launch clears the one its successor will use (its last
-  // user, the launch before this one, has finished), so a launch always starts from zero even when an
-  // earlier launch gave up on a barrier and left its own counter short.
-  if (blockIdx.x == 0 && threadIdx.x == 0) *p.counter_next = 0u;
+struct StepCta {
+  const StepParams& p;
+  uint8_t* sm;
+  uint32_t bars;
+  volatile int* abort_flag;
+  int* s_flag;
+  unsigned int* counter;
+  unsigned int arrived;
 
-  // ---- LSTM layers: one warp per (sequence, hidden unit): the four gate rows of W and of R
-  for (int l = 0; l < p.layers; ++l) {
-    const int in_l = l == 0 ? p.in_c : H;
-    const __half* W = p.lstm + p.w_off[l];
-    const __half* R = p.lstm + p.r_off[l];
-    const __half* bW = p.lstm + p.bw_off[l];
-    const __half* bR = p.double_bias ? p.lstm + p.br_off[l] : nullptr;
-    for (int i = gw; i < B * H; i += tw) {
-      const int b = i / H, u = i - b * H;
-      const __half* x = l == 0 ? p.emb + (size_t)b * p.in_c : p.h_new + ((size_t)(l - 1) * B + b) * H;
-      const __half* hp = p.h_state + ((size_t)l * B + b) * H;
+  // Grid-wide barrier.  Every CTA arrives once; the wait is bounded.
+  __device__ bool barrier(int code) {
+    __syncthreads();
+    arrived += gridDim.x;
+    if (threadIdx.x == 0) {
+      __threadfence();
+      red_release_gpu_add(counter, 1u);
+      const long long t0 = clock64();
+      int ok = 1;
+      while ((int)(ld_acquire_gpu(counter) - arrived) < 0) {
+        if (clock64() - t0 > AIG_WAIT_CYCLES) {
+          atomicCAS(p.gerr, 0, code);
+          ok = 0;
+          break;
+        }
+      }
+      *s_flag = ok;
+    }
+    __syncthreads();
+    return *s_flag != 0;
+  }
+  // the same answer for every thread
+  __device__ bool weights(int i) { return __syncthreads_and(mbar_wait_bounded(bars + 8 * i, 0, abort_flag, p.gerr, 720 + i)) != 0; }
+  __device__ float* red() const { return reinterpret_cast<float*>(sm + p.o_red); }
+  // element (row, b) of the product that `multiply` left behind, its parts along K added up
+  __device__ float value(int row, int b) const {
+    const float* r = red() + ((b >> 3) * kRows + row) * 8 + (b & 7);
+    float s = r[0];
+    for (int w = 1; w < p.kw; ++w) s += r[(size_t)w * p.nt * kRows * 8];
+    return s;
+  }
+  // [16 rows of `a` in shared memory] x [K x B], x [b][K] in global memory.  A lane takes 16 bytes of a row and of a
+  // column at the same place, which the two mma steps of a 32-deep block use as their k: the order of k is free.
+  template <int TPW>
+  __device__ void multiply(const uint8_t* a, const __half* x, int x_stride, int K) {
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, q = lane & 3;
+    const int wk = warp % p.kw, wn = warp / p.kw, groups = kWarps / p.kw;
+    const int nkb = (K + 31) >> 5, stride = row_stride(K);
+    const uint8_t* a0 = a + g * stride + q * 16;
+    const uint8_t* a1 = a0 + 8 * stride;
+    constexpr int U = 8;  // blocks in flight
+    float acc[TPW][4];
+    const __half* xr[TPW];
+    bool on[TPW];
+#pragma unroll
+    for (int j = 0; j < TPW; ++j) {
+      const int b = (wn + j * groups) * 8 + g;
+      on[j] = b < p.B;
+      xr[j] = x + (size_t)(on[j] ? b : 0) * x_stride + q * 8;
+      acc[j][0] = acc[j][1] = acc[j][2] = acc[j][3] = 0.f;
+    }
+    for (int kb0 = wk; kb0 < nkb; kb0 += p.kw * U) {
+      uint4 xv[U][TPW];
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        const int kb = kb0 + u * p.kw;
+#pragma unroll
+        for (int j = 0; j < TPW; ++j)
+          xv[u][j] = on[j] && kb * 32 + q * 8 < K ? __ldcg(reinterpret_cast<const uint4*>(xr[j] + kb * 32)) : make_uint4(0, 0, 0, 0);
+      }
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        const int kb = kb0 + u * p.kw;
+        if (kb >= nkb) break;
+        const uint4 w0 = *reinterpret_cast<const uint4*>(a0 + kb * 64), w1 = *reinterpret_cast<const uint4*>(a1 + kb * 64);
+#pragma unroll
+        for (int j = 0; j < TPW; ++j) {
+          mma_16816(acc[j], w0.x, w1.x, w0.y, w1.y, xv[u][j].x, xv[u][j].y);
+          mma_16816(acc[j], w0.z, w1.z, w0.w, w1.w, xv[u][j].z, xv[u][j].w);
+        }
+      }
+    }
+    float* r = red();
+#pragma unroll
+    for (int j = 0; j < TPW; ++j) {
+      const int t = wn + j * groups;
+      if (t < p.nt) {
+        float* d = r + ((size_t)(wk * p.nt + t) * kRows + g) * 8 + 2 * q;
+        *reinterpret_cast<float2*>(d) = make_float2(acc[j][0], acc[j][1]);
+        *reinterpret_cast<float2*>(d + 8 * 8) = make_float2(acc[j][2], acc[j][3]);
+      }
+    }
+    __syncthreads();
+  }
+};
+
+// attention of one (sequence, head) by one warp: rotate q and k at `position`, append k and v to the ring, attend
+__device__ void attend(const StepParams& p, int item, int position, int n_valid, float cs, float sn, float* sq, int lane) {
+  const int b = item / p.heads, h = item - b * p.heads, E = p.H, d = kHeadDim, half_d = d / 2, window = p.window;
+  float* sp = sq + d;
+  const size_t row = (size_t)b * E + (size_t)h * d, ring = (size_t)b * window * E + (size_t)h * d;
+  const int slot = position % window;
+  {
+    __half* kslot = p.kcache + ring + (size_t)slot * E;
+    __half* vslot = p.vcache + ring + (size_t)slot * E;
+    const int j = lane;  // half_d == 32
+    const float qa = __half2float(__ldcg(p.q + row + j)), qb = __half2float(__ldcg(p.q + row + j + half_d));
+    const float ka = __half2float(__ldcg(p.k + row + j)), kb = __half2float(__ldcg(p.k + row + j + half_d));
+    sq[j] = __half2float(__float2half(qa * cs - qb * sn));
+    sq[j + half_d] = __half2float(__float2half(qb * cs + qa * sn));
+    kslot[j] = __float2half(ka * cs - kb * sn);
+    kslot[j + half_d] = __float2half(kb * cs + ka * sn);
+    vslot[j] = __ldcg(p.v + row + j);
+    vslot[j + half_d] = __ldcg(p.v + row + j + half_d);
+  }
+  __syncwarp();
+  // scores: a lane per earlier step (slot order, not time order: the softmax does not mind), 128 bytes of k each
+  float mx = -INFINITY;
+  for (int i = lane; i < n_valid; i += 32) {
+    const uint4* kr = reinterpret_cast<const uint4*>(p.kcache + ring + (size_t)i * E);
+    uint4 kv[d / 8];
+#pragma unroll
+    for (int c = 0; c < d / 8; ++c) kv[c] = kr[c];
+    float acc = 0.f;
+#pragma unroll
+    for (int c = 0; c < d / 8; ++c) {
+      const __half2* kh = reinterpret_cast<const __half2*>(&kv[c]);
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        const float2 f = __half22float2(kh[e]);
+        acc = fmaf(sq[c * 8 + 2 * e], f.x, acc);
+        acc = fmaf(sq[c * 8 + 2 * e + 1], f.y, acc);
+      }
+    }
+    sp[i] = acc * p.scale;
+    mx = fmaxf(mx, sp[i]);
+  }
+  for (int o = 16; o > 0; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+  float sum = 0.f;
+  for (int i = lane; i < n_valid; i += 32) {
+    const float e = expf(sp[i] - mx);
+    sp[i] = e;
+    sum += e;
+  }
+  for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
+  __syncwarp();
+  // context: a lane takes eight dimensions of every fourth step
+  const int grp = lane >> 3, dim = (lane & 7) * 8;
+  float acc[8];
+#pragma unroll
+  for (int e = 0; e < 8; ++e) acc[e] = 0.f;
+#pragma unroll 8
+  for (int i = grp; i < n_valid; i += 4) {
+    const uint4 vv = *reinterpret_cast<const uint4*>(p.vcache + ring + (size_t)i * E + dim);
+    const float w = sp[i];
+    const __half2* vh = reinterpret_cast<const __half2*>(&vv);
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      const float2 f = __half22float2(vh[e]);
+      acc[2 * e] = fmaf(w, f.x, acc[2 * e]);
+      acc[2 * e + 1] = fmaf(w, f.y, acc[2 * e + 1]);
+    }
+  }
+  const float inv = 1.0f / sum;
+#pragma unroll
+  for (int e = 0; e < 8; ++e) {
+    acc[e] += __shfl_xor_sync(0xffffffffu, acc[e], 8);
+    acc[e] += __shfl_xor_sync(0xffffffffu, acc[e], 16);
+  }
+  if (grp == 0) {
+    __align__(16) __half out[8];
+#pragma unroll
+    for (int e = 0; e < 8; ++e) out[e] = __float2half(acc[e] * inv);
+    *reinterpret_cast<uint4*>(p.ctx + row + dim) = *reinterpret_cast<const uint4*>(out);
+  }
+  __syncwarp();
+}
+
+// TPW = tiles of eight sequences per warp: 1 up to 64 sequences, 2 up to 128
+template <int TPW>
+__global__ void __launch_bounds__(kThreads, 1) seq_step_kernel(const StepParams p) {
+  extern __shared__ __align__(128) uint8_t sm[];
+  __shared__ uint64_t s_bars[kMaxBars];
+  __shared__ int s_flag;
+  __shared__ int s_abort;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int H = p.H, B = p.B, L = p.layers, unit0 = blockIdx.x * kUnits, n_bars = 2 + L + 3;
+  const uint32_t base = smem_u32(sm), bars = smem_u32(s_bars);
+  const int b_bridge = 1, b_qkv = 2 + L, b_wo = 3 + L, b_fc = 4 + L;
+  const int bridge0 = blockIdx.x * p.bridge_rows, n_bridge = p.features ? max(0, min(p.bridge_rows, p.in_c - bridge0)) : 0;
+
+  // ---- weights to shared memory, in the order of their use
+  if (warp == 0) {
+    if (lane == 0) {
+      for (int i = 0; i < n_bars; ++i) mbar_init(bars + 8 * i, 1);
+      s_abort = 0;
+      fence_mbar_init();
+      mbar_expect_tx(bars, (uint32_t)(L * kRows * H * 2));
+      mbar_expect_tx(bars + 8 * b_bridge, (uint32_t)(n_bridge * p.feat * 2));
+      for (int l = 0; l < L; ++l) mbar_expect_tx(bars + 8 * (2 + l), (uint32_t)(kRows * (l == 0 ? p.in_c : H) * 2));
+      mbar_expect_tx(bars + 8 * b_qkv, (uint32_t)(3 * kUnits * H * 2));
+      mbar_expect_tx(bars + 8 * b_wo, (uint32_t)(kUnits * H * 2));
+      mbar_expect_tx(bars + 8 * b_fc, (uint32_t)(p.n_out * H * 2));
+    }
+    __syncwarp();
+    const uint32_t hb = (uint32_t)H * 2;
+    const int hs = row_stride(H);
+    for (int i = lane; i < L * kRows; i += 32) {
+      const int l = i / kRows, r = i % kRows;
+      bulk_load(base + p.o_r[l] + r * hs, p.lstm + p.r_off[l] + ((size_t)(r >> 2) * H + unit0 + (r & 3)) * H, hb, bars);
+    }
+    for (int r = lane; r < n_bridge; r += 32)
+      bulk_load(base + p.o_bridge + r * row_stride(p.feat), p.bw_t + (size_t)(bridge0 + r) * p.feat, (uint32_t)p.feat * 2, bars + 8 * b_bridge);
+    for (int i = lane; i < L * kRows; i += 32) {
+      const int l = i / kRows, r = i % kRows, in = l == 0 ? p.in_c : H;
+      bulk_load(base + p.o_w[l] + r * row_stride(in), p.lstm + p.w_off[l] + ((size_t)(r >> 2) * H + unit0 + (r & 3)) * in, (uint32_t)in * 2,
+                bars + 8 * (2 + l));
+    }
+    for (int r = lane; r < 3 * kUnits; r += 32) {
+      const __half* m = (r >> 2) == 0 ? p.wq_t : ((r >> 2) == 1 ? p.wk_t : p.wv_t);
+      bulk_load(base + p.o_qkv + r * hs, m + (size_t)(unit0 + (r & 3)) * H, hb, bars + 8 * b_qkv);
+    }
+    for (int r = lane; r < kUnits; r += 32) bulk_load(base + p.o_wo + r * hs, p.wo_t + (size_t)(unit0 + r) * H, hb, bars + 8 * b_wo);
+    for (int r = lane; r < p.n_out; r += 32) bulk_load(base + p.o_fc + r * hb, p.fcw_t + (size_t)r * H, hb, bars + 8 * b_fc);
+  }
+  // a K that is an odd multiple of 16 leaves half a block per row: zero, not whatever was there
+  if (p.in_c % 32 != 0)
+    for (int i = tid; i < kRows * 8; i += kThreads)
+      *reinterpret_cast<uint32_t*>(sm + p.o_w[0] + (i >> 3) * row_stride(p.in_c) + p.in_c * 2 + (i & 7) * 4) = 0u;
+  if (n_bridge && p.feat % 32 != 0)
+    for (int i = tid; i < n_bridge * 8; i += kThreads)
+      *reinterpret_cast<uint32_t*>(sm + p.o_bridge + (i >> 3) * row_stride(p.feat) + p.feat * 2 + (i & 7) * 4) = 0u;
+  float* s_bias = reinterpret_cast<float*>(sm + p.o_bias);  // [L][16]
+  for (int i = tid; i < L * kRows; i += kThreads) {
+    const int l = i / kRows, r = i % kRows;
+    const size_t at = (size_t)(r >> 2) * H + unit0 + (r & 3);
+    s_bias[i] = __half2float(p.lstm[p.bw_off[l] + at]) + (p.double_bias ? __half2float(p.lstm[p.br_off[l] + at]) : 0.f);
+  }
+
+  // ---- carried state.  Its last writer is the step before, which had finished before the first kernel of this step's
+  // encoder started (that one is an ordinary launch), so it need not wait for this kernel's direct predecessor.
+  const unsigned int epoch = p.words[kEpoch];
+  const int position = (int)p.words[kPosition], n_valid = min(position + 1, p.window);
+  float* s_cell = reinterpret_cast<float*>(sm + p.o_cell);    // [L][B][4]
+  __half* s_hid = reinterpret_cast<__half*>(sm + p.o_hid);    // [L][B][4], this step's
+  for (int i = tid; i < L * B * kUnits; i += kThreads) {
+    const int l = i / (B * kUnits), b = i / kUnits % B, u = i % kUnits;
+    s_cell[i] = __half2float(p.c_state[((size_t)l * B + b) * H + unit0 + u]);
+  }
+  float cs = 1.f, sn = 0.f;
+  if (p.rope_base > 0.f) {
+    const float ang = (float)position * powf(p.rope_base, -2.0f * (float)lane / (float)kHeadDim);
+    cs = cosf(ang);
+    sn = sinf(ang);
+  }
+  for (int item = blockIdx.x * kWarps + warp; item < B * p.heads; item += gridDim.x * kWarps) {
+    const size_t ring = (size_t)(item / p.heads) * p.window * H + (size_t)(item % p.heads) * kHeadDim;
+    for (int i = lane; i < n_valid; i += 32) {
+      prefetch_l2(p.kcache + ring + (size_t)i * H);
+      prefetch_l2(p.vcache + ring + (size_t)i * H);
+    }
+  }
+  __syncthreads();
+  StepCta c{p, sm, bars, &s_abort, &s_flag, p.words + (epoch & 1u), 0u};
+  float* s_pre = reinterpret_cast<float*>(sm + p.o_pre);      // [L][16][nt*8]: R.h
+  const int pre_n = p.nt * 8;
+  bool ok = c.weights(0);
+  for (int l = 0; l < L && ok; ++l) {
+    c.template multiply<TPW>(sm + p.o_r[l], p.h_state + (size_t)l * B * H, H, H);
+    for (int i = tid; i < kRows * B; i += kThreads) s_pre[((size_t)l * kRows + i / B) * pre_n + i % B] = c.value(i / B, i % B);
+    __syncthreads();
+  }
+  griddep_wait();
+  // Two counters alternate between launches: each launch clears the one that its successor will use, whose last user,
+  // the launch before this one, has finished; so a launch starts from zero even after one that gave up on a barrier.
+  if (blockIdx.x == 0 && tid == 0) p.words[(epoch + 1u) & 1u] = 0u;
+
+  // ---- bridge FC: features -> embedding, rounded before and after the bias
+  if (p.features && ok) {
+    ok = c.weights(b_bridge);
+    for (int r0 = 0; r0 < n_bridge && ok; r0 += kRows) {
+      c.template multiply<TPW>(sm + p.o_bridge + r0 * row_stride(p.feat), p.features, p.feat, p.feat);
+      const int n = min(kRows, n_bridge - r0);
+      for (int i = tid; i < n * B; i += kThreads) {
+        const int r = i % n, b = i / n, o = bridge0 + r0 + r;
+        const float t = __half2float(__float2half(c.value(r, b)));
+        p.emb_out[(size_t)b * p.in_c + o] = __float2half(t + __half2float(p.bb[o]));
+      }
+      __syncthreads();
+    }
+    ok = ok && c.barrier(701);
+  }
+
+  // ---- LSTM layers
+  for (int l = 0; l < L && ok; ++l) {
+    ok = c.weights(2 + l);
+    if (!ok) break;
+    if (l == 0) c.template multiply<TPW>(sm + p.o_w[0], p.features ? p.emb_out : p.emb, p.in_c, p.in_c);
+    else c.template multiply<TPW>(sm + p.o_w[l], p.h_new + (size_t)(l - 1) * B * H, H, H);
+    for (int i = tid; i < B * kUnits; i += kThreads) {
+      const int b = i / kUnits, u = i % kUnits;
       float pre[4];
 #pragma unroll
       for (int g = 0; g < 4; ++g) {
-        const size_t row = (size_t)g * H + u;
-        const float gx = row_dot(W + row * in_l, x, in_l, lane) + __half2float(bW[row]) + (bR ? __half2float(bR[row]) : 0.f);
-        pre[g] = row_dot(R + row * H, hp, H, lane) + gx;
+        const int r = g * kUnits + u;
+        pre[g] = s_pre[((size_t)l * kRows + r) * pre_n + b] + (c.value(r, b) + s_bias[l * kRows + r]);
       }
-      if (lane == 0) {
-        const size_t si = ((size_t)l * B + b) * H + u;
-        const float ig = sigmoidf_(pre[0]), fg = sigmoidf_(pre[1]), gg = tanhf(pre[2]), og = sigmoidf_(pre[3]);
-        float cn = fg * __half2float(p.c_state[si]) + ig * gg;
-        if (p.clip > 0.f) cn = fminf(p.clip, fmaxf(-p.clip, cn));
-        const __half ch = __float2half(cn);
-        p.c_state[si] = ch;
-        const __half hn = __float2half(og * tanhf(__half2float(ch)));
-        p.h_new[si] = hn;
-        if (l == p.layers - 1) p.y[(size_t)b * H + u] = hn;
-      }
+      const float ig = sigmoidf_(pre[0]), fg = sigmoidf_(pre[1]), gg = tanhf(pre[2]), og = sigmoidf_(pre[3]);
+      float cn = fg * s_cell[l * B * kUnits + i] + ig * gg;
+      if (p.clip > 0.f) cn = fminf(p.clip, fmaxf(-p.clip, cn));
+      const __half ch = __float2half(cn), hn = __float2half(og * tanhf(__half2float(ch)));
+      const size_t si = ((size_t)l * B + b) * H + unit0 + u;
+      p.c_state[si] = ch;
+      p.h_new[si] = hn;
+      s_hid[l * B * kUnits + i] = hn;
+      if (l == L - 1) p.y[(size_t)b * H + unit0 + u] = hn;
     }
-    if (!grid_barrier(p, bar++, &s_flag)) return;
+    ok = c.barrier(702 + l);
   }
-  const __half* top = p.h_new + (size_t)(p.layers - 1) * B * H;
 
-  // ---- q, k, v projections: one warp per output row
-  for (int i = gw; i < 3 * H; i += tw) {
-    const int m = i / H, j = i - m * H;
-    const __half* Wt = (m == 0 ? p.wq_t : (m == 1 ? p.wk_t : p.wv_t)) + (size_t)j * H;
-    __half* dst = m == 0 ? p.q : (m == 1 ? p.k : p.v);
-    for (int b = 0; b < B; ++b) {
-      const float acc = row_dot(Wt, top + (size_t)b * H, H, lane);
-      if (lane == 0) dst[(size_t)b * H + j] = __float2half(acc);
+  // ---- q, k, v
+  if (ok && (ok = c.weights(b_qkv))) {
+    c.template multiply<TPW>(sm + p.o_qkv, p.h_new + (size_t)(L - 1) * B * H, H, H);
+    for (int i = tid; i < 3 * B * kUnits; i += kThreads) {
+      const int m = i / (B * kUnits), b = i / kUnits % B, u = i % kUnits;
+      (m == 0 ? p.q : (m == 1 ? p.k : p.v))[(size_t)b * H + unit0 + u] = __float2half(c.value(m * kUnits + u, b));
     }
+    // every CTA has read the previous hidden state by now: publish the new one
+    for (int i = tid; i < L * B * kUnits; i += kThreads) {
+      const int l = i / (B * kUnits), b = i / kUnits % B, u = i % kUnits;
+      p.h_state[((size_t)l * B + b) * H + unit0 + u] = s_hid[i];
+    }
+    ok = c.barrier(707);
   }
-  // the carried hidden state is no longer read by anyone: publish the new one
-  for (int i = blockIdx.x * kThreads + threadIdx.x; i < p.layers * B * H; i += gridDim.x * kThreads) p.h_state[i] = p.h_new[i];
-  if (!grid_barrier(p, bar++, &s_flag)) return;
-
-  // ---- attention: one warp per (sequence, head); rotate q and k at `position`, append k, v to the ring
-  for (int item = gw; item < B * p.heads; item += tw) {
-    const int b = item / p.heads, h = item - b * p.heads;
-    const int d = kHeadDim, half_d = d / 2, E = H, window = p.window, position = p.position;
-    float* sq = s_attn + warp * (kHeadDim + kMaxWindow);
-    float* sp = sq + d;
-    const size_t row = (size_t)b * E + (size_t)h * d;
-    const int slot = position % window;
-    __half* kslot = p.kcache + ((size_t)b * window + slot) * E + (size_t)h * d;
-    __half* vslot = p.vcache + ((size_t)b * window + slot) * E + (size_t)h * d;
-    for (int j = lane; j < half_d; j += 32) {
-      float cs = 1.f, sn = 0.f;
-      if (p.rope_base > 0.f) {
-        const float inv = powf(p.rope_base, -2.0f * (float)j / (float)d);
-        const float ang = (float)position * inv;
-        cs = cosf(ang);
-        sn = sinf(ang);
-      }
-      const float qa = __half2float(p.q[row + j]), qb = __half2float(p.q[row + j + half_d]);
-      const float ka = __half2float(p.k[row + j]), kb = __half2float(p.k[row + j + half_d]);
-      sq[j] = __half2float(__float2half(qa * cs - qb * sn));
-      sq[j + half_d] = __half2float(__float2half(qb * cs + qa * sn));
-      kslot[j] = __float2half(ka * cs - kb * sn);
-      kslot[j + half_d] = __float2half(kb * cs + ka * sn);
-      vslot[j] = p.v[row + j];
-      vslot[j + half_d] = p.v[row + j + half_d];
-    }
-    __syncwarp();
-    float mx = -INFINITY;
-    for (int i = lane; i < p.n_valid; i += 32) {
-      const int pos = position - i;
-      const __half* kr = p.kcache + ((size_t)b * window + (pos % window)) * E + (size_t)h * d;
-      float acc = 0.f;
-      for (int c = 0; c < d; c += 8) {
-        const uint4 kv = *reinterpret_cast<const uint4*>(kr + c);
-        const __half* kh = reinterpret_cast<const __half*>(&kv);
-#pragma unroll
-        for (int e = 0; e < 8; ++e) acc = fmaf(sq[c + e], __half2float(kh[e]), acc);
-      }
-      sp[i] = acc * p.scale;
-      mx = fmaxf(mx, sp[i]);
-    }
-    for (int o = 16; o > 0; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
-    float sum = 0.f;
-    for (int i = lane; i < p.n_valid; i += 32) {
-      const float e = expf(sp[i] - mx);
-      sp[i] = e;
-      sum += e;
-    }
-    for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
-    __syncwarp();
-    const float inv = 1.0f / sum;
-    for (int c = lane; c < d; c += 32) {
-      float acc = 0.f;
-      for (int i = 0; i < p.n_valid; ++i) {
-        const int pos = position - i;
-        acc = fmaf(sp[i], __half2float(p.vcache[((size_t)b * window + (pos % window)) * E + (size_t)h * d + c]), acc);
-      }
-      p.ctx[row + c] = __float2half(acc * inv);
-    }
-    __syncwarp();
+  // ---- attention
+  if (ok) {
+    float* sq = reinterpret_cast<float*>(sm + p.o_attn) + warp * (kHeadDim + kMaxWindow);
+    for (int item = blockIdx.x * kWarps + warp; item < B * p.heads; item += gridDim.x * kWarps) attend(p, item, position, n_valid, cs, sn, sq, lane);
+    ok = c.barrier(708);
   }
-  if (!grid_barrier(p, bar++, &s_flag)) return;
-
   // ---- output projection
-  for (int j = gw; j < H; j += tw) {
-    for (int b = 0; b < B; ++b) {
-      const float acc = row_dot(p.wo_t + (size_t)j * H, p.ctx + (size_t)b * H, H, lane);
-      if (lane == 0) p.a[(size_t)b * H + j] = __float2half(acc);
+  if (ok && (ok = c.weights(b_wo))) {
+    c.template multiply<TPW>(sm + p.o_wo, p.ctx, H, H);
+    for (int i = tid; i < B * kUnits; i += kThreads) p.a[(size_t)(i / kUnits) * H + unit0 + i % kUnits] = __float2half(c.value(i % kUnits, i / kUnits));
+    ok = c.barrier(709);
+  }
+  // ---- per sequence: row LayerNorm (eps 1e-5; every warp for itself), FC with the two-step rounding, sigmoid / tanh
+  if (ok && (ok = c.weights(b_fc))) {
+    constexpr int kPairs = 512 / 64;  // half2 a lane holds at most
+    for (int b = blockIdx.x; b < B; b += gridDim.x) {
+      const __half2* src = reinterpret_cast<const __half2*>(p.a + (size_t)b * H);
+      float2 v[kPairs];
+      float s = 0.f, ss = 0.f;
+#pragma unroll
+      for (int j = 0; j < kPairs; ++j) {
+        v[j] = j * 64 < H ? __half22float2(__ldcg(src + lane + 32 * j)) : make_float2(0.f, 0.f);
+        s += v[j].x + v[j].y;
+      }
+      for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+      const float mu = s / (float)H;
+#pragma unroll
+      for (int j = 0; j < kPairs; ++j)
+        if (j * 64 < H) ss += (v[j].x - mu) * (v[j].x - mu) + (v[j].y - mu) * (v[j].y - mu);
+      for (int o = 16; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
+      const float rstd = rsqrtf(ss / (float)H + 1e-5f);
+#pragma unroll
+      for (int j = 0; j < kPairs; ++j)
+        if (j * 64 < H) {
+          const float2 gm = reinterpret_cast<const float2*>(p.ln_g)[lane + 32 * j], bt = reinterpret_cast<const float2*>(p.ln_b)[lane + 32 * j];
+          v[j] = __half22float2(__floats2half2_rn((v[j].x - mu) * rstd * gm.x + bt.x, (v[j].y - mu) * rstd * gm.y + bt.y));
+        }
+      for (int o = warp; o < p.n_out; o += kWarps) {
+        const __half2* w = reinterpret_cast<const __half2*>(sm + p.o_fc + (size_t)o * H * 2);
+        float acc = 0.f;
+#pragma unroll
+        for (int j = 0; j < kPairs; ++j)
+          if (j * 64 < H) {
+            const float2 f = __half22float2(w[lane + 32 * j]);
+            acc = fmaf(f.x, v[j].x, acc);
+            acc = fmaf(f.y, v[j].y, acc);
+          }
+        for (int k = 16; k > 0; k >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, k);
+        if (lane == 0) {
+          const float t = __half2float(__float2half(acc));                           // FCLayer: GEMM result stored as half,
+          float r = __half2float(__float2half(t + __half2float(p.fcb[o])));          // then bias added and stored again
+          r = o < p.n_sig ? sigmoidf_(r) : tanhf(r);
+          const __half hv = __float2half(r);
+          p.logits[(size_t)b * p.n_out + o] = hv;
+          p.out_f32[(size_t)b * p.n_out + o] = __half2float(hv);
+        }
+      }
     }
   }
-  if (!grid_barrier(p, bar++, &s_flag)) return;
-
-  // ---- tail on CTA 0: row LayerNorm (eps 1e-5), FC with the two-step rounding, sigmoid / tanh, fp32 copy
-  if (blockIdx.x != 0) return;
-  for (int b = warp; b < B; b += kWarps) {
-    const __half* src = p.a + (size_t)b * H;
-    float s = 0.f;
-    for (int c = lane; c < H; c += 32) s += __half2float(src[c]);
-    for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-    const float mu = s / (float)H;
-    float ss = 0.f;
-    for (int c = lane; c < H; c += 32) {
-      const float dlt = __half2float(src[c]) - mu;
-      ss += dlt * dlt;
-    }
-    for (int o = 16; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
-    const float rstd = rsqrtf(ss / (float)H + 1e-5f);
-    for (int c = lane; c < H; c += 32)
-      p.n[(size_t)b * H + c] = __float2half((__half2float(src[c]) - mu) * rstd * p.ln_g[c] + p.ln_b[c]);
-  }
-  __syncthreads();
-  for (int i = warp; i < B * p.n_out; i += kWarps) {
-    const int b = i / p.n_out, o = i - b * p.n_out;
-    const float acc = row_dot(p.fcw_t + (size_t)o * H, p.n + (size_t)b * H, H, lane);
-    if (lane == 0) {
-      const float t = __half2float(__float2half(acc));                           // FCLayer: GEMM result stored as half,
-      float v = __half2float(__float2half(t + __half2float(p.fcb[o])));          // then bias added and stored again
-      v = o < p.n_sig ? 1.0f / (1.0f + expf(-v)) : tanhf(v);
-      const __half hv = __float2half(v);
-      p.logits[i] = hv;
-      p.out_f32[i] = __half2float(hv);
-    }
+  // no CTA leaves with copies into its shared memory still under way
+  if (!ok)
+    for (int i = 0; i < n_bars; ++i) c.weights(i);
+  if (blockIdx.x == 0 && tid == 0) {
+    p.words[kEpoch] = epoch + 1u;
+    if (ok) p.words[kPosition] = (unsigned int)position + 1u;
   }
 }
 
@@ -276,16 +501,69 @@ struct SeqStepFused {
   SeqStepConfig cfg{};
   StepParams prm{};
   __half* buf = nullptr;        // transposed weights + scratch
-  unsigned int* counter = nullptr;  // two counters, used by alternate launches
-  unsigned int launches = 0;
+  unsigned int* words = nullptr;
   int grid = 1;
-  int stream_start = -1;
+  size_t smem = 0;
   bool weights_set = false;
 };
 
+namespace {
+
+using StepKernel = void (*)(const StepParams);
+StepKernel step_kernel(int batch) { return batch <= 64 ? seq_step_kernel<1> : seq_step_kernel<2>; }
+
+// shared memory of one CTA; sets the offsets
+size_t lay_out(StepParams& p) {
+  size_t off = 0;
+  auto take = [&](size_t bytes) {
+    const size_t at = off;
+    off = (off + bytes + 127) & ~(size_t)127;
+    return (int)at;
+  };
+  const size_t hs = row_stride(p.H);
+  size_t tile_end = 0;  // a multiply reads 16 rows, also where fewer are kept
+  auto tile = [&](size_t rows, size_t stride) {
+    const int at = take(rows * stride);
+    const size_t last = (rows + kRows - 1) / kRows * kRows;
+    tile_end = tile_end > at + last * stride ? tile_end : at + last * stride;
+    return at;
+  };
+  for (int l = 0; l < p.layers; ++l) p.o_r[l] = tile(kRows, hs);
+  p.o_bridge = p.bridge_rows ? tile(p.bridge_rows, row_stride(p.feat)) : 0;
+  for (int l = 0; l < p.layers; ++l) p.o_w[l] = tile(kRows, l == 0 ? row_stride(p.in_c) : hs);
+  p.o_qkv = tile(3 * kUnits, hs);
+  p.o_wo = tile(kUnits, hs);
+  p.o_fc = take((size_t)p.n_out * p.H * 2);
+  p.o_pre = take((size_t)p.layers * kRows * p.nt * 8 * 4);
+  p.o_red = take((size_t)p.kw * p.nt * kRows * 8 * 4);
+  p.o_cell = take((size_t)p.layers * p.B * kUnits * 4);
+  p.o_hid = take((size_t)p.layers * p.B * kUnits * 2);
+  p.o_bias = take((size_t)p.layers * kRows * 4);
+  p.o_attn = take((size_t)kWarps * (kHeadDim + kMaxWindow) * 4);
+  return off > tile_end ? off : tile_end;
+}
+
+StepParams step_shape(const SeqStepConfig& c) {
+  StepParams p{};
+  p.B = c.batch; p.in_c = c.in_c; p.H = c.hidden; p.layers = c.layers; p.heads = c.heads; p.window = c.window;
+  p.n_out = c.n_out; p.n_sig = c.n_sigmoid; p.double_bias = c.double_bias; p.rope_base = c.rope_base;
+  p.scale = 1.0f / sqrtf((float)kHeadDim); p.clip = c.clip;
+  p.nt = (c.batch + 7) / 8;
+  p.kw = p.nt == 1 ? 8 : (p.nt == 2 ? 4 : (p.nt <= 4 ? 2 : 1));  // as many warps along K as the tiles leave free
+  p.feat = c.features;
+  if (c.features) p.bridge_rows = (c.in_c + c.hidden / kUnits - 1) / (c.hidden / kUnits);
+  return p;
+}
+
+}  // namespace
+
 bool seq_step_fused_supported(const SeqStepConfig& c) {
-  return c.batch >= 1 && c.batch <= 4 && c.layers >= 1 && c.layers <= kMaxLayers && c.hidden % 8 == 0 && c.in_c % 8 == 0 &&
-         c.heads * kHeadDim == c.hidden && c.window >= 1 && c.window <= kMaxWindow && c.n_out >= 1 && c.n_out <= 64;
+  if (!(c.batch >= 1 && c.batch <= kMaxBatch && c.layers >= 1 && c.layers <= kMaxLayers && c.hidden % 64 == 0 && c.hidden <= 512 &&
+        c.in_c % 16 == 0 && c.features % 16 == 0 && c.heads * kHeadDim == c.hidden && c.window >= 1 && c.window <= kMaxWindow && c.n_out >= 1 &&
+        c.n_out <= 64))
+    return false;
+  StepParams p = step_shape(c);
+  return lay_out(p) <= kMaxSmem;
 }
 
 int seq_step_fused_create(aig_ctx* ctx, const SeqStepConfig& c, SeqStepFused** out) {
@@ -295,28 +573,37 @@ int seq_step_fused_create(aig_ctx* ctx, const SeqStepConfig& c, SeqStepFused** o
   SeqStepFused* s = new SeqStepFused();
   s->ctx = ctx;
   s->cfg = c;
+  StepParams& p = s->prm;
+  p = step_shape(c);
+  s->smem = lay_out(p);
+  s->grid = c.hidden / kUnits;
   const size_t E = c.hidden, BE = (size_t)c.batch * E;
-  // layout of buf (halfs): wq_t wk_t wv_t wo_t fcw_t | h_new q k v ctx a n | kcache vcache
-  const size_t n_w = 4 * E * E + (size_t)c.n_out * E;
-  const size_t n_s = (size_t)c.layers * BE + 6 * BE;
+  // layout of buf (halfs): wq_t wk_t wv_t wo_t fcw_t bw_t | h_new q k v ctx a emb | kcache vcache
+  const size_t n_w = 4 * E * E + (size_t)c.n_out * E + (size_t)c.features * c.in_c;
+  const size_t n_s = (size_t)c.layers * BE + 5 * BE + (size_t)c.batch * c.in_c;
   const size_t n_c = 2 * (size_t)c.batch * c.window * E;
-  if (cudaMalloc(&s->buf, (n_w + n_s + n_c) * sizeof(__half)) != cudaSuccess || cudaMalloc(&s->counter, 2 * sizeof(unsigned int)) != cudaSuccess) {
+  int per_sm = 0;
+  if (cudaMalloc(&s->buf, (n_w + n_s + n_c) * sizeof(__half)) != cudaSuccess || cudaMalloc(&s->words, kWords * sizeof(unsigned int)) != cudaSuccess ||
+      cudaMemsetAsync(s->buf, 0, (n_w + n_s + n_c) * sizeof(__half), ctx->stream) != cudaSuccess ||
+      cudaMemsetAsync(s->words, 0, kWords * sizeof(unsigned int), ctx->stream) != cudaSuccess ||
+      cudaFuncSetAttribute(step_kernel(c.batch), cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMaxSmem) != cudaSuccess ||
+      cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, step_kernel(c.batch), kThreads, s->smem) != cudaSuccess) {
     seq_step_fused_destroy(s);
     return aig_fail(ctx, AIG_ERR_CUDA, "fused sequence step: allocation failed");
   }
-  cudaMemsetAsync(s->buf, 0, (n_w + n_s + n_c) * sizeof(__half), ctx->stream);
-  cudaMemsetAsync(s->counter, 0, 2 * sizeof(unsigned int), ctx->stream);
-  StepParams& p = s->prm;
-  p.B = c.batch; p.in_c = c.in_c; p.H = c.hidden; p.layers = c.layers; p.heads = c.heads; p.window = c.window;
-  p.n_out = c.n_out; p.n_sig = c.n_sigmoid; p.double_bias = c.double_bias; p.rope_base = c.rope_base;
-  p.scale = 1.0f / sqrtf((float)kHeadDim); p.clip = c.clip;
+  if (per_sm * ctx->sm_count < s->grid) {
+    seq_step_fused_destroy(s);
+    return aig_fail(ctx, AIG_ERR_UNSUPPORTED, "fused sequence step: %d CTAs cannot be co-resident", s->grid);
+  }
   __half* w = s->buf;
   p.wq_t = w; p.wk_t = w + E * E; p.wv_t = w + 2 * E * E; p.wo_t = w + 3 * E * E; p.fcw_t = w + 4 * E * E;
+  p.bw_t = p.fcw_t + (size_t)c.n_out * E;
   __half* sc = s->buf + n_w;
   p.h_new = sc; sc += (size_t)c.layers * BE;
-  p.q = sc; p.k = sc + BE; p.v = sc + 2 * BE; p.ctx = sc + 3 * BE; p.a = sc + 4 * BE; p.n = sc + 5 * BE;
+  p.q = sc; p.k = sc + BE; p.v = sc + 2 * BE; p.ctx = sc + 3 * BE; p.a = sc + 4 * BE; p.emb_out = sc + 5 * BE;
   p.kcache = s->buf + n_w + n_s;
   p.vcache = p.kcache + (size_t)c.batch * c.window * E;
+  p.words = s->words;
   p.gerr = ctx->d_err;
   // blob offsets (halfs): per layer W then R, then per layer bW [and bR]
   size_t off = 0;
@@ -329,16 +616,6 @@ int seq_step_fused_create(aig_ctx* ctx, const SeqStepConfig& c, SeqStepFused** o
     p.bw_off[l] = off; off += 4 * E;
     if (c.double_bias) { p.br_off[l] = off; off += 4 * E; }
   }
-  // one CTA per SM at most, and no more CTAs than there are rows to give every warp one
-  int per_sm = 0;
-  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, seq_step_kernel, kThreads, 0);
-  int grid = (int)((BE + kWarps - 1) / kWarps);
-  if (grid > ctx->sm_count) grid = ctx->sm_count;
-  if (per_sm < 1) {
-    seq_step_fused_destroy(s);
-    return aig_fail(ctx, AIG_ERR_UNSUPPORTED, "fused sequence step: kernel cannot be resident");
-  }
-  s->grid = grid < 1 ? 1 : grid;
   *out = s;
   return AIG_OK;
 }
@@ -346,7 +623,7 @@ int seq_step_fused_create(aig_ctx* ctx, const SeqStepConfig& c, SeqStepFused** o
 void seq_step_fused_destroy(SeqStepFused* s) {
   if (!s) return;
   cudaFree(s->buf);
-  cudaFree(s->counter);
+  cudaFree(s->words);
   delete s;
 }
 
@@ -373,33 +650,48 @@ int seq_step_fused_set_weights(SeqStepFused* s, const aig_half* lstm_blob, const
   return AIG_OK;
 }
 
-int seq_step_fused_reset(SeqStepFused* s) {
-  s->stream_start = -1;
-  cudaMemsetAsync(s->counter, 0, 2 * sizeof(unsigned int), s->ctx->stream);
+int seq_step_fused_set_bridge(SeqStepFused* s, const aig_half* w_in_out, const aig_half* bias) {
+  aig_ctx* ctx = s->ctx;
+  DeviceGuard g(ctx->device);
+  AIG_REQUIRE(ctx, s->cfg.features > 0 && w_in_out && bias, "fused sequence step: no bridge in this configuration");
+  transpose_kernel<<<ctx->sm_count, 256, 0, ctx->stream>>>((const __half*)w_in_out, (__half*)s->prm.bw_t, s->cfg.features, s->cfg.in_c);
+  AIG_LAUNCH_OK(ctx);
+  s->prm.bb = (const __half*)bias;
   return AIG_OK;
 }
 
-int seq_step_fused_run(SeqStepFused* s, const aig_half* emb, aig_half* h_state, aig_half* c_state, aig_half* y, aig_half* logits,
-                       float* out_f32, int position) {
+int seq_step_fused_reset(SeqStepFused* s) {
+  aig_ctx* ctx = s->ctx;
+  AIG_CUDA_OK(ctx, cudaMemsetAsync(s->words, 0, kWords * sizeof(unsigned int), ctx->stream));
+  return AIG_OK;
+}
+
+int seq_step_fused_run(SeqStepFused* s, const aig_half* emb, const aig_half* features, aig_half* h_state, aig_half* c_state, aig_half* y,
+                       aig_half* logits, float* out_f32, bool after_encoder) {
   aig_ctx* ctx = s->ctx;
   DeviceGuard g(ctx->device);
-  AIG_REQUIRE(ctx, s->weights_set && emb && h_state && c_state && y && logits && out_f32 && position >= 0, "fused sequence step: bad arguments");
-  if (s->stream_start < 0) s->stream_start = position;
-  AIG_REQUIRE(ctx, position >= s->stream_start, "fused sequence step: positions must not go backwards without a reset");
-  StepParams& p = s->prm;
+  AIG_REQUIRE(ctx, s->weights_set && (emb || (features && s->prm.bb)) && h_state && c_state && y && logits && out_f32,
+              "fused sequence step: bad arguments");
+  StepParams p = s->prm;
   p.emb = (const __half*)emb;
+  p.features = (const __half*)features;
   p.h_state = (__half*)h_state;
   p.c_state = (__half*)c_state;
   p.y = (__half*)y;
   p.logits = (__half*)logits;
   p.out_f32 = out_f32;
-  p.position = position;
-  int n_valid = position - s->stream_start + 1;
-  p.n_valid = n_valid > s->cfg.window ? s->cfg.window : n_valid;
-  p.counter = s->counter + (s->launches & 1u);
-  p.counter_next = s->counter + ((s->launches + 1u) & 1u);
-  ++s->launches;
-  void* args[] = {(void*)&p};
-  AIG_CUDA_OK(ctx, cudaLaunchCooperativeKernel((const void*)seq_step_kernel, dim3(s->grid), dim3(kThreads), args, 0, ctx->stream));
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3(s->grid);
+  cfg.blockDim = dim3(kThreads);
+  cfg.dynamicSmemBytes = s->smem;
+  cfg.stream = ctx->stream;
+  cudaLaunchAttribute attr[2];
+  attr[0].id = cudaLaunchAttributeCooperative;
+  attr[0].val.cooperative = 1;
+  attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[1].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = after_encoder ? 2 : 1;
+  AIG_CUDA_OK(ctx, cudaLaunchKernelEx(&cfg, step_kernel(s->cfg.batch), p));
   return AIG_OK;
 }

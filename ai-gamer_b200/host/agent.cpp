@@ -11,6 +11,7 @@
 
 #include "aig_b200.h"
 #include "aig_host.h"
+#include "seq_step.h"
 
 struct aig_agent {
   aig_ctx* ctx = nullptr;
@@ -22,6 +23,10 @@ struct aig_agent {
   int feat = 0;
   aig_half *bw = nullptr, *bb = nullptr, *emb = nullptr;
   uint8_t* frames_dev = nullptr;
+  static constexpr int kGraphs = 8;    // captured steps, keyed by input pointer (where the head has its fused step)
+  aig_graph* graphs[kGraphs] = {};
+  const uint8_t* graph_ins[kGraphs] = {};
+  int graph_next = 0;
   std::string err;
 };
 
@@ -50,8 +55,8 @@ int aig_agent_create(aig_ctx* ctx, const aig_cnn_config* ccfg, const aig_seq_con
   a->scfg = *scfg;
   a->feat = ccfg->widths[ccfg->n_blocks];
   int rc = aig_cnn_create(ctx, ccfg, &a->cnn);
-  if (rc == AIG_OK) rc = aig_seq_create(ctx, scfg, &a->seq);
-  if (rc == AIG_OK) rc = aig_fc_plan_create(ctx, ccfg->batch, a->feat, scfg->in_c, AIG_ACT_NONE, 0.f, 1, &a->bridge);
+  if (rc == AIG_OK) rc = seq_create_with_bridge(ctx, scfg, a->feat, &a->seq);
+  if (rc == AIG_OK && !seq_has_fused_step(a->seq)) rc = aig_fc_plan_create(ctx, ccfg->batch, a->feat, scfg->in_c, AIG_ACT_NONE, 0.f, 1, &a->bridge);
   if (rc == AIG_OK && (cudaMalloc(&a->bw, (size_t)a->feat * scfg->in_c * 2) != cudaSuccess ||
                        cudaMalloc(&a->bb, (size_t)scfg->in_c * 2) != cudaSuccess ||
                        cudaMalloc(&a->emb, (size_t)ccfg->batch * scfg->in_c * 2) != cudaSuccess ||
@@ -68,6 +73,7 @@ int aig_agent_create(aig_ctx* ctx, const aig_cnn_config* ccfg, const aig_seq_con
 int aig_agent_destroy(aig_agent* a) {
   if (!a) return AIG_OK;
   if (a->ctx) aig_ctx_sync(a->ctx);
+  for (aig_graph* g : a->graphs) aig_graph_destroy(g);
   aig_cnn_destroy(a->cnn);
   aig_seq_destroy(a->seq);
   aig_conv_plan_destroy(a->bridge);
@@ -91,18 +97,60 @@ int aig_agent_load_memory(aig_agent* a, const void* blob, size_t bytes) {
   if ((rc = aig_memcpy(a->ctx, a->bw, p + n_cnn, n_w)) != AIG_OK || (rc = aig_memcpy(a->ctx, a->bb, p + n_cnn + n_w, n_b)) != AIG_OK ||
       (rc = aig_ctx_sync(a->ctx)) != AIG_OK)
     return afail(a, rc, aig_last_error(a->ctx));
-  if ((rc = aig_fc_plan_set_weights(a->bridge, a->bw, a->bb, nullptr, nullptr, nullptr, nullptr, 0.f)) != AIG_OK)
+  if (a->bridge && (rc = aig_fc_plan_set_weights(a->bridge, a->bw, a->bb, nullptr, nullptr, nullptr, nullptr, 0.f)) != AIG_OK)
     return afail(a, rc, aig_last_error(a->ctx));
   rc = aig_seq_load_memory(a->seq, p + n_cnn + n_w + n_b, bytes - n_cnn - n_w - n_b);
+  if (rc == AIG_OK && !a->bridge) rc = seq_set_bridge(a->seq, a->bw, a->bb);
   if (rc != AIG_OK) return afail(a, rc, aig_seq_last_error(a->seq));
   return AIG_OK;
 }
 
+}  // extern "C"
+
+// The encoder's launches and the head's one launch, captured as one graph per input buffer: the head's kernel starts
+// (and loads its weights) under the encoder's last kernels, and a step costs the host one launch.
+static int agent_graph(aig_agent* a, const uint8_t* bgra_dev, aig_graph** out) {
+  for (int i = 0; i < aig_agent::kGraphs; ++i)
+    if (a->graphs[i] && a->graph_ins[i] == bgra_dev) {
+      *out = a->graphs[i];
+      return AIG_OK;
+    }
+  // one eager pass of the encoder first (the head's step would advance its state): every plan encodes its tensor maps
+  int rc = aig_cnn_forward(a->cnn, bgra_dev);
+  if (rc != AIG_OK) return afail(a, rc, aig_cnn_last_error(a->cnn));
+  if ((rc = aig_graph_begin(a->ctx)) != AIG_OK) return afail(a, rc, aig_last_error(a->ctx));
+  rc = aig_cnn_forward(a->cnn, bgra_dev);
+  if (rc != AIG_OK) a->err = aig_cnn_last_error(a->cnn);
+  else if ((rc = seq_step_from_features(a->seq, aig_cnn_features(a->cnn))) != AIG_OK) a->err = aig_seq_last_error(a->seq);
+  aig_graph* g = nullptr;
+  const int rc2 = aig_graph_end(a->ctx, &g);  // always ends the capture, also after a failed call
+  if (rc != AIG_OK) {
+    aig_graph_destroy(g);
+    return rc;
+  }
+  if (rc2 != AIG_OK) return afail(a, rc2, aig_last_error(a->ctx));
+  const int slot = a->graph_next;
+  a->graph_next = (a->graph_next + 1) % aig_agent::kGraphs;
+  if (a->graphs[slot]) aig_graph_destroy(a->graphs[slot]);
+  a->graphs[slot] = *out = g;
+  a->graph_ins[slot] = bgra_dev;
+  return AIG_OK;
+}
+
+extern "C" {
+
 // One frame per sequence (device BGRA [B][H][W][4]) -> outputs [B][n_out] (aig_agent_outputs_f32).
 int aig_agent_step(aig_agent* a, const uint8_t* bgra_dev) {
   if (!a || !bgra_dev) return AIG_ERR_INVALID;
+  int rc;
+  if (!a->bridge) {
+    aig_graph* g = nullptr;
+    if ((rc = agent_graph(a, bgra_dev, &g)) != AIG_OK) return rc;
+    if ((rc = aig_graph_launch(a->ctx, g)) != AIG_OK) return afail(a, rc, aig_last_error(a->ctx));
+    return AIG_OK;
+  }
   // the encoder's launches replay from a CUDA graph (captured per input buffer on first use)
-  int rc = aig_cnn_forward_graph(a->cnn, bgra_dev);
+  rc = aig_cnn_forward_graph(a->cnn, bgra_dev);
   if (rc != AIG_OK) return afail(a, rc, aig_cnn_last_error(a->cnn));
   if ((rc = aig_conv_forward(a->bridge, aig_cnn_features(a->cnn), nullptr, a->emb)) != AIG_OK) return afail(a, rc, aig_last_error(a->ctx));
   if ((rc = aig_seq_step(a->seq, a->emb)) != AIG_OK) return afail(a, rc, aig_seq_last_error(a->seq));

@@ -34,8 +34,8 @@ struct aig_seq {
   aig_half *h_state = nullptr, *c_state = nullptr;                        // [layers][B][hid]
   float* out_f32 = nullptr;
   bool loaded = false;
-  int position = 0;
-  SeqStepFused* fused = nullptr;  // one-kernel streaming step for small batches (replaces the launches of aig_seq_step)
+  int position = 0;               // steps of the per-operator launches (the fused step counts its own on the device)
+  SeqStepFused* fused = nullptr;  // one-kernel streaming step for up to 128 sequences (replaces the launches of aig_seq_step)
 };
 
 namespace {
@@ -62,7 +62,9 @@ size_t aig_seq_param_bytes(const aig_seq_config* c) {
   return aig_lstm_weight_count(c->in_c, c->hidden, c->layers, 1) * 2 + 4 * E * E * 2 + 2 * E * 4 + (E * c->n_out + c->n_out) * 2;
 }
 
-int aig_seq_create(aig_ctx* ctx, const aig_seq_config* cfg, aig_seq** out) {
+}  // extern "C"
+
+int seq_create_with_bridge(aig_ctx* ctx, const aig_seq_config* cfg, int features, aig_seq** out) {
   if (!ctx || !cfg || !out) return AIG_ERR_INVALID;
   *out = nullptr;
   if (cfg->batch <= 0 || cfg->seq_len <= 0 || cfg->in_c <= 0 || cfg->hidden <= 0 || cfg->layers <= 0 || cfg->heads <= 0 ||
@@ -72,11 +74,14 @@ int aig_seq_create(aig_ctx* ctx, const aig_seq_config* cfg, aig_seq** out) {
   m->ctx = ctx;
   m->cfg = *cfg;
   const aig_seq_config& c = m->cfg;
+  const SeqStepConfig sc{c.batch, c.in_c, c.hidden, c.layers, c.heads, c.window > 0 ? c.window : c.seq_len, c.n_out, c.n_sigmoid, c.rope_base, 5.0f, 1, features};
+  const char* off = getenv("AIG_SEQ_NO_FUSED_STEP");
+  const bool fused = seq_step_fused_supported(sc) && !(off && atoi(off));
   int rc = aig_lstm_plan_create(ctx, c.seq_len, c.layers, c.hidden, c.batch, c.in_c, 5.0f, 1, /*batch_major*/ 1, &m->lstm_full);
-  if (rc == AIG_OK) rc = aig_lstm_plan_create(ctx, 1, c.layers, c.hidden, c.batch, c.in_c, 5.0f, 1, 1, &m->lstm_step);
+  if (rc == AIG_OK && !fused) rc = aig_lstm_plan_create(ctx, 1, c.layers, c.hidden, c.batch, c.in_c, 5.0f, 1, 1, &m->lstm_step);
   if (rc == AIG_OK) rc = aig_mha_plan_create(ctx, c.batch, c.seq_len, c.hidden, c.heads, c.rope_base, c.window, &m->mha);
   if (rc == AIG_OK) rc = aig_fc_plan_create(ctx, c.batch * c.seq_len, c.hidden, c.n_out, AIG_ACT_NONE, 0.f, 1, &m->fc_full);
-  if (rc == AIG_OK) rc = aig_fc_plan_create(ctx, c.batch, c.hidden, c.n_out, AIG_ACT_NONE, 0.f, 1, &m->fc_step);
+  if (rc == AIG_OK && !fused) rc = aig_fc_plan_create(ctx, c.batch, c.hidden, c.n_out, AIG_ACT_NONE, 0.f, 1, &m->fc_step);
   const size_t rows = (size_t)c.batch * c.seq_len, E = c.hidden;
   const size_t state = (size_t)c.layers * c.batch * E;
   if (rc == AIG_OK &&
@@ -87,12 +92,7 @@ int aig_seq_create(aig_ctx* ctx, const aig_seq_config* cfg, aig_seq** out) {
        cudaMemset(m->c_state, 0, state * 2) != cudaSuccess ||
        cudaMalloc(&m->params, aig_seq_param_bytes(&c) + 16 * 256) != cudaSuccess))
     rc = AIG_ERR_CUDA;
-  if (rc == AIG_OK) {
-    const int window = c.window > 0 ? c.window : c.seq_len;
-    const SeqStepConfig sc{c.batch, c.in_c, c.hidden, c.layers, c.heads, window, c.n_out, c.n_sigmoid, c.rope_base, 5.0f, 1};
-    const char* off = getenv("AIG_SEQ_NO_FUSED_STEP");
-    if (seq_step_fused_supported(sc) && !(off && atoi(off))) rc = seq_step_fused_create(ctx, sc, &m->fused);
-  }
+  if (rc == AIG_OK && fused) rc = seq_step_fused_create(ctx, sc, &m->fused);
   if (rc != AIG_OK) {
     aig_seq_destroy(m);
     return rc;
@@ -100,6 +100,20 @@ int aig_seq_create(aig_ctx* ctx, const aig_seq_config* cfg, aig_seq** out) {
   *out = m;
   return AIG_OK;
 }
+bool seq_has_fused_step(const aig_seq* m) { return m->fused != nullptr; }
+int seq_set_bridge(aig_seq* m, const aig_half* w_in_out, const aig_half* bias) {
+  SEQ_OK(m, seq_step_fused_set_bridge(m->fused, w_in_out, bias));
+  return AIG_OK;
+}
+int seq_step_from_features(aig_seq* m, const aig_half* features) {
+  if (!m->loaded) return sfail(m, AIG_ERR_INVALID, "parameters not loaded");
+  SEQ_OK(m, seq_step_fused_run(m->fused, nullptr, features, m->h_state, m->c_state, m->y, m->logits, m->out_f32, true));
+  return AIG_OK;
+}
+
+extern "C" {
+
+int aig_seq_create(aig_ctx* ctx, const aig_seq_config* cfg, aig_seq** out) { return seq_create_with_bridge(ctx, cfg, 0, out); }
 
 int aig_seq_destroy(aig_seq* m) {
   if (!m) return AIG_OK;
@@ -136,10 +150,10 @@ int aig_seq_load_memory(aig_seq* m, const void* blob, size_t bytes) {
   }
   SEQ_OK(m, aig_ctx_sync(m->ctx));  // the caller may free the blob now
   SEQ_OK(m, aig_lstm_plan_set_weights(m->lstm_full, m->lstm_w));
-  SEQ_OK(m, aig_lstm_plan_set_weights(m->lstm_step, m->lstm_w));
+  if (!m->fused) SEQ_OK(m, aig_lstm_plan_set_weights(m->lstm_step, m->lstm_w));
   SEQ_OK(m, aig_mha_plan_set_weights(m->mha, m->wq, m->wk, m->wv, m->wo));
   SEQ_OK(m, aig_fc_plan_set_weights(m->fc_full, m->fcw, m->fcb, nullptr, nullptr, nullptr, nullptr, 0.f));
-  SEQ_OK(m, aig_fc_plan_set_weights(m->fc_step, m->fcw, m->fcb, nullptr, nullptr, nullptr, nullptr, 0.f));
+  if (!m->fused) SEQ_OK(m, aig_fc_plan_set_weights(m->fc_step, m->fcw, m->fcb, nullptr, nullptr, nullptr, nullptr, 0.f));
   if (m->fused) SEQ_OK(m, seq_step_fused_set_weights(m->fused, m->lstm_w, m->wq, m->wk, m->wv, m->wo, m->ln_g, m->ln_b, m->fcw, m->fcb));
   m->loaded = true;
   return AIG_OK;
@@ -171,8 +185,7 @@ int aig_seq_step(aig_seq* m, const aig_half* emb_t) {
   if (!m->loaded) return sfail(m, AIG_ERR_INVALID, "parameters not loaded");
   const aig_seq_config& c = m->cfg;
   if (m->fused) {
-    SEQ_OK(m, seq_step_fused_run(m->fused, emb_t, m->h_state, m->c_state, m->y, m->logits, m->out_f32, m->position));
-    ++m->position;
+    SEQ_OK(m, seq_step_fused_run(m->fused, emb_t, nullptr, m->h_state, m->c_state, m->y, m->logits, m->out_f32, false));
     return AIG_OK;
   }
   SEQ_OK(m, aig_lstm_forward(m->lstm_step, emb_t, m->y, m->h_state, m->c_state, 1));
@@ -188,7 +201,7 @@ int aig_seq_reset(aig_seq* m) {
   if (cudaMemsetAsync(m->h_state, 0, state, s) != cudaSuccess || cudaMemsetAsync(m->c_state, 0, state, s) != cudaSuccess)
     return sfail(m, AIG_ERR_CUDA, "state reset failed");
   m->position = 0;
-  if (m->fused) seq_step_fused_reset(m->fused);
+  if (m->fused) SEQ_OK(m, seq_step_fused_reset(m->fused));
   return aig_mha_reset(m->mha);
 }
 

@@ -148,3 +148,31 @@ def test_fc_layernorm_swish_twin(env, rows):
     got = U.host(z).astype(np.float32)
     assert np.abs(got - want.astype(np.float32)).max() < 6e-3
     assert U.rel_err(got, want.astype(np.float32), 0.05).max() < TOL
+
+
+@gpu
+@pytest.mark.parametrize("B,in_c,d,heads,window,layers", [
+    (1, 16, 64, 1, 1, 1), (8, 48, 64, 1, 3, 1), (9, 272, 128, 2, 4, 2), (16, 128, 64, 1, 5, 3), (17, 64, 192, 3, 2, 2), (33, 80, 64, 1, 128, 2),
+    (64, 32, 64, 1, 4, 4), (65, 64, 128, 2, 3, 1), (128, 48, 64, 1, 4, 2), (4, 512, 512, 8, 64, 2)])
+def test_streaming_step_shapes(env, B, in_c, d, heads, window, layers):
+    """The one-kernel step over its range: one sequence to 128 (full and ragged tiles of eight, one and two tiles a warp,
+    one to eight warps along K), input widths that leave half a block of K, windows that wrap, one to four layers."""
+    U = env
+    U.pkg()
+    from ai_gamer_b200 import runners as R
+
+    T = 6
+    p = PL.make_seq_params(B + d, d=in_c, hid=d, layers=layers, heads=heads)
+    emb = PL.make_embeddings(3, T, B, in_c)
+    _, _, _, want = PL.seq_forward(p, emb, rope_base=10000.0, window=window)
+    head = R.SeqHead(U.ctx(), B, 16, in_c=in_c, hidden=d, layers=layers, heads=heads, rope_base=10000.0, window=window)
+    head.load_bytes(PL.serialize_seq_params(p))
+    for run in range(2):
+        outs = []
+        for t in range(T):
+            head.step(U.dev(np.ascontiguousarray(emb[t])))
+            outs.append(U.host(head.outputs_f32(step=True)))
+        got = np.stack(outs, axis=1)
+        assert U.rel_err(got, want.astype(np.float32), 0.2).max() < TOL   # an output near zero: 4e-3 absolute
+        head.reset()
+    head.close()
