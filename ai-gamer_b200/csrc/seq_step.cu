@@ -30,6 +30,7 @@ constexpr int kMaxLayers = 4;
 constexpr int kMaxWindow = 128;
 constexpr int kHeadDim = 64;
 constexpr int kUnits = 4;         // hidden units (and rows of every other matrix) per CTA
+constexpr int kAttnFloats = 3 * kHeadDim + 16;  // a warp's q, k, v and partial context
 constexpr int kRows = 16;         // rows of an mma tile: four gates of kUnits units
 constexpr int kMaxBatch = 128;
 constexpr int kMaxBars = 2 + kMaxLayers + 3;
@@ -99,8 +100,7 @@ struct StepCta {
     __syncthreads();
     arrived += gridDim.x;
     if (threadIdx.x == 0) {
-      __threadfence();
-      red_release_gpu_add(counter, 1u);
+      red_release_gpu_add(counter, 1u);  // (releases what the block wrote before the __syncthreads)
       const long long t0 = clock64();
       int ok = 1;
       while ((int)(ld_acquire_gpu(counter) - arrived) < 0) {
@@ -180,86 +180,115 @@ struct StepCta {
   }
 };
 
-// attention of one (sequence, head) by one warp: rotate q and k at `position`, append k and v to the ring, attend
-__device__ void attend(const StepParams& p, int item, int position, int n_valid, float cs, float sn, float* sq, int lane) {
-  const int b = item / p.heads, h = item - b * p.heads, E = p.H, d = kHeadDim, half_d = d / 2, window = p.window;
-  float* sp = sq + d;
-  const size_t row = (size_t)b * E + (size_t)h * d, ring = (size_t)b * window * E + (size_t)h * d;
-  const int slot = position % window;
+// Attention of one (sequence, head) by `warps` warps of a CTA, this one being number `sub`: rotate q and k at `position`,
+// append k and v to the ring (warp 0), attend to the slots of this warp's share.  A lane takes eight dimensions of every
+// fourth slot; all of a block's k and v rows are in flight together, because the stage is bound by that latency.  The
+// share's running maximum, sum and context go to `part` where an item has several warps, else to the context itself.
+__device__ void attend(const StepParams& p, int item, int position, int n_valid, float cs, float sn, float* sq, float* part, int warps, int sub,
+                       int lane) {
+  constexpr int d = kHeadDim, half_d = d / 2, kBlock = 8;  // slots a lane has in flight (32 per warp)
+  const int b = item / p.heads, h = item - b * p.heads, E = p.H, slot = position % p.window;
+  const size_t row = (size_t)b * E + (size_t)h * d, ring = (size_t)b * p.window * E + (size_t)h * d;
+  const int grp = lane >> 3, dim = (lane & 7) * 8;
+  const int share = ((n_valid + warps - 1) / warps + 3) & ~3, lo = sub * share, hi = min(n_valid, lo + share);
+  __half* sk = reinterpret_cast<__half*>(sq + d);  // this step's k and v
+  __half* sv = sk + d;
   {
-    __half* kslot = p.kcache + ring + (size_t)slot * E;
-    __half* vslot = p.vcache + ring + (size_t)slot * E;
     const int j = lane;  // half_d == 32
     const float qa = __half2float(__ldcg(p.q + row + j)), qb = __half2float(__ldcg(p.q + row + j + half_d));
     const float ka = __half2float(__ldcg(p.k + row + j)), kb = __half2float(__ldcg(p.k + row + j + half_d));
+    const __half va = __ldcg(p.v + row + j), vb = __ldcg(p.v + row + j + half_d);
+    const __half k0 = __float2half(ka * cs - kb * sn), k1 = __float2half(kb * cs + ka * sn);
     sq[j] = __half2float(__float2half(qa * cs - qb * sn));
     sq[j + half_d] = __half2float(__float2half(qb * cs + qa * sn));
-    kslot[j] = __float2half(ka * cs - kb * sn);
-    kslot[j + half_d] = __float2half(kb * cs + ka * sn);
-    vslot[j] = __ldcg(p.v + row + j);
-    vslot[j + half_d] = __ldcg(p.v + row + j + half_d);
+    sk[j] = k0; sk[j + half_d] = k1;
+    sv[j] = va; sv[j + half_d] = vb;
+    if (sub == 0) {
+      __half* kslot = p.kcache + ring + (size_t)slot * E;
+      __half* vslot = p.vcache + ring + (size_t)slot * E;
+      kslot[j] = k0; kslot[j + half_d] = k1;
+      vslot[j] = va; vslot[j + half_d] = vb;
+    }
   }
   __syncwarp();
-  // scores: a lane per earlier step (slot order, not time order: the softmax does not mind), 128 bytes of k each
-  float mx = -INFINITY;
-  for (int i = lane; i < n_valid; i += 32) {
-    const uint4* kr = reinterpret_cast<const uint4*>(p.kcache + ring + (size_t)i * E);
-    uint4 kv[d / 8];
+  float q[8], acc[8], mx = -INFINITY, sum = 0.f;
 #pragma unroll
-    for (int c = 0; c < d / 8; ++c) kv[c] = kr[c];
-    float acc = 0.f;
+  for (int e = 0; e < 8; ++e) {
+    q[e] = sq[dim + e] * p.scale;
+    acc[e] = 0.f;
+  }
+  for (int i0 = lo; i0 < hi; i0 += 4 * kBlock) {
+    uint4 kv[kBlock], vv[kBlock];
 #pragma unroll
-    for (int c = 0; c < d / 8; ++c) {
-      const __half2* kh = reinterpret_cast<const __half2*>(&kv[c]);
+    for (int u = 0; u < kBlock; ++u) {
+      const int i = i0 + 4 * u + grp;
+      kv[u] = vv[u] = make_uint4(0, 0, 0, 0);
+      if (i < hi && i != slot) {
+        kv[u] = *reinterpret_cast<const uint4*>(p.kcache + ring + (size_t)i * E + dim);
+        vv[u] = *reinterpret_cast<const uint4*>(p.vcache + ring + (size_t)i * E + dim);
+      } else if (i < hi) {
+        kv[u] = *reinterpret_cast<const uint4*>(sk + dim);
+        vv[u] = *reinterpret_cast<const uint4*>(sv + dim);
+      }
+    }
+    float s[kBlock], top = mx;
+#pragma unroll
+    for (int u = 0; u < kBlock; ++u) {
+      const __half2* kh = reinterpret_cast<const __half2*>(&kv[u]);
+      float t = 0.f;
 #pragma unroll
       for (int e = 0; e < 4; ++e) {
         const float2 f = __half22float2(kh[e]);
-        acc = fmaf(sq[c * 8 + 2 * e], f.x, acc);
-        acc = fmaf(sq[c * 8 + 2 * e + 1], f.y, acc);
+        t = fmaf(q[2 * e], f.x, t);
+        t = fmaf(q[2 * e + 1], f.y, t);
+      }
+      t += __shfl_xor_sync(0xffffffffu, t, 1);
+      t += __shfl_xor_sync(0xffffffffu, t, 2);
+      t += __shfl_xor_sync(0xffffffffu, t, 4);
+      s[u] = i0 + 4 * u + grp < hi ? t : -INFINITY;
+      top = fmaxf(top, s[u]);
+    }
+    top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, 8));
+    top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, 16));
+    const float keep = expf(mx - top);  // (0 in the first block)
+    mx = top;
+    sum *= keep;
+#pragma unroll
+    for (int e = 0; e < 8; ++e) acc[e] *= keep;
+#pragma unroll
+    for (int u = 0; u < kBlock; ++u) {
+      const float w = expf(s[u] - mx);
+      const __half2* vh = reinterpret_cast<const __half2*>(&vv[u]);
+      sum += w;
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        const float2 f = __half22float2(vh[e]);
+        acc[2 * e] = fmaf(w, f.x, acc[2 * e]);
+        acc[2 * e + 1] = fmaf(w, f.y, acc[2 * e + 1]);
       }
     }
-    sp[i] = acc * p.scale;
-    mx = fmaxf(mx, sp[i]);
   }
-  for (int o = 16; o > 0; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
-  float sum = 0.f;
-  for (int i = lane; i < n_valid; i += 32) {
-    const float e = expf(sp[i] - mx);
-    sp[i] = e;
-    sum += e;
-  }
-  for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
-  __syncwarp();
-  // context: a lane takes eight dimensions of every fourth step
-  const int grp = lane >> 3, dim = (lane & 7) * 8;
-  float acc[8];
-#pragma unroll
-  for (int e = 0; e < 8; ++e) acc[e] = 0.f;
-#pragma unroll 8
-  for (int i = grp; i < n_valid; i += 4) {
-    const uint4 vv = *reinterpret_cast<const uint4*>(p.vcache + ring + (size_t)i * E + dim);
-    const float w = sp[i];
-    const __half2* vh = reinterpret_cast<const __half2*>(&vv);
-#pragma unroll
-    for (int e = 0; e < 4; ++e) {
-      const float2 f = __half22float2(vh[e]);
-      acc[2 * e] = fmaf(w, f.x, acc[2 * e]);
-      acc[2 * e + 1] = fmaf(w, f.y, acc[2 * e + 1]);
-    }
-  }
-  const float inv = 1.0f / sum;
+  sum += __shfl_xor_sync(0xffffffffu, sum, 8);
+  sum += __shfl_xor_sync(0xffffffffu, sum, 16);
 #pragma unroll
   for (int e = 0; e < 8; ++e) {
     acc[e] += __shfl_xor_sync(0xffffffffu, acc[e], 8);
     acc[e] += __shfl_xor_sync(0xffffffffu, acc[e], 16);
   }
-  if (grp == 0) {
+  if (grp != 0) return;
+  if (warps == 1) {
     __align__(16) __half out[8];
 #pragma unroll
-    for (int e = 0; e < 8; ++e) out[e] = __float2half(acc[e] * inv);
+    for (int e = 0; e < 8; ++e) out[e] = __float2half(acc[e] / sum);
     *reinterpret_cast<uint4*>(p.ctx + row + dim) = *reinterpret_cast<const uint4*>(out);
+  } else {
+#pragma unroll
+    for (int e = 0; e < 8; ++e) part[dim + e] = acc[e];
+    if (dim == 0) {
+      part[d] = mx;
+      part[d + 1] = sum;
+    }
   }
-  __syncwarp();
 }
 
 // TPW = tiles of eight sequences per warp: 1 up to 64 sequences, 2 up to 128
@@ -339,9 +368,10 @@ __global__ void __launch_bounds__(kThreads, 1) seq_step_kernel(const StepParams 
     cs = cosf(ang);
     sn = sinf(ang);
   }
-  for (int item = blockIdx.x * kWarps + warp; item < B * p.heads; item += gridDim.x * kWarps) {
+  const bool item_per_cta = B * p.heads <= (int)gridDim.x;
+  for (int item = item_per_cta ? blockIdx.x : blockIdx.x * kWarps + warp; item < B * p.heads; item += item_per_cta ? gridDim.x : gridDim.x * kWarps) {
     const size_t ring = (size_t)(item / p.heads) * p.window * H + (size_t)(item % p.heads) * kHeadDim;
-    for (int i = lane; i < n_valid; i += 32) {
+    for (int i = item_per_cta ? tid : lane; i < n_valid; i += item_per_cta ? kThreads : 32) {
       prefetch_l2(p.kcache + ring + (size_t)i * H);
       prefetch_l2(p.vcache + ring + (size_t)i * H);
     }
@@ -383,23 +413,27 @@ __global__ void __launch_bounds__(kThreads, 1) seq_step_kernel(const StepParams 
     if (!ok) break;
     if (l == 0) c.template multiply<TPW>(sm + p.o_w[0], p.features ? p.emb_out : p.emb, p.in_c, p.in_c);
     else c.template multiply<TPW>(sm + p.o_w[l], p.h_new + (size_t)(l - 1) * B * H, H, H);
-    for (int i = tid; i < B * kUnits; i += kThreads) {
-      const int b = i / kUnits, u = i % kUnits;
-      float pre[4];
-#pragma unroll
-      for (int g = 0; g < 4; ++g) {
-        const int r = g * kUnits + u;
-        pre[g] = s_pre[((size_t)l * kRows + r) * pre_n + b] + (c.value(r, b) + s_bias[l * kRows + r]);
+    // a lane per gate, four lanes per (unit, sequence)
+    for (int i = tid; i < (B * kRows + 31) / 32 * 32; i += kThreads) {
+      const int g = i & 3, cell = i >> 2, u = cell & 3, b = cell >> 2, r = g * kUnits + u;
+      const bool on = b < B;
+      float act = 0.f;
+      if (on) {
+        const float pre = s_pre[((size_t)l * kRows + r) * pre_n + b] + (c.value(r, b) + s_bias[l * kRows + r]);
+        act = sigmoidf_(g == 2 ? 2.0f * pre : pre);
+        if (g == 2) act = 2.0f * act - 1.0f;
       }
-      const float ig = sigmoidf_(pre[0]), fg = sigmoidf_(pre[1]), gg = tanhf(pre[2]), og = sigmoidf_(pre[3]);
-      float cn = fg * s_cell[l * B * kUnits + i] + ig * gg;
-      if (p.clip > 0.f) cn = fminf(p.clip, fmaxf(-p.clip, cn));
-      const __half ch = __float2half(cn), hn = __float2half(og * tanhf(__half2float(ch)));
-      const size_t si = ((size_t)l * B + b) * H + unit0 + u;
-      p.c_state[si] = ch;
-      p.h_new[si] = hn;
-      s_hid[l * B * kUnits + i] = hn;
-      if (l == L - 1) p.y[(size_t)b * H + unit0 + u] = hn;
+      const float fg = __shfl_down_sync(0xffffffffu, act, 1), gg = __shfl_down_sync(0xffffffffu, act, 2), og = __shfl_down_sync(0xffffffffu, act, 3);
+      if (on && g == 0) {
+        float cn = fg * s_cell[l * B * kUnits + cell] + act * gg;
+        if (p.clip > 0.f) cn = fminf(p.clip, fmaxf(-p.clip, cn));
+        const __half ch = __float2half(cn), hn = __float2half(og * tanhf(__half2float(ch)));
+        const size_t si = ((size_t)l * B + b) * H + unit0 + u;
+        p.c_state[si] = ch;
+        p.h_new[si] = hn;
+        s_hid[l * B * kUnits + cell] = hn;
+        if (l == L - 1) p.y[(size_t)b * H + unit0 + u] = hn;
+      }
     }
     ok = c.barrier(702 + l);
   }
@@ -420,8 +454,28 @@ __global__ void __launch_bounds__(kThreads, 1) seq_step_kernel(const StepParams 
   }
   // ---- attention
   if (ok) {
-    float* sq = reinterpret_cast<float*>(sm + p.o_attn) + warp * (kHeadDim + kMaxWindow);
-    for (int item = blockIdx.x * kWarps + warp; item < B * p.heads; item += gridDim.x * kWarps) attend(p, item, position, n_valid, cs, sn, sq, lane);
+    // an item per warp, or per CTA where every item can have one of its own
+    float* sq = reinterpret_cast<float*>(sm + p.o_attn) + warp * kAttnFloats;
+    const int items = B * p.heads;
+    if (!item_per_cta) {
+      for (int item = blockIdx.x * kWarps + warp; item < items; item += gridDim.x * kWarps)
+        attend(p, item, position, n_valid, cs, sn, sq, nullptr, 1, 0, lane);
+    } else if ((int)blockIdx.x < items) {
+      float* part = sq + 2 * kHeadDim;
+      attend(p, blockIdx.x, position, n_valid, cs, sn, sq, part, kWarps, warp, lane);
+      __syncthreads();
+      if (tid < kHeadDim) {
+        const float* all = reinterpret_cast<float*>(sm + p.o_attn) + 2 * kHeadDim;
+        float mx = -INFINITY, sum = 0.f, acc = 0.f;
+        for (int w = 0; w < kWarps; ++w) mx = fmaxf(mx, all[w * kAttnFloats + kHeadDim]);
+        for (int w = 0; w < kWarps; ++w) {
+          const float f = expf(all[w * kAttnFloats + kHeadDim] - mx);  // (0 for a warp without a share)
+          sum = fmaf(f, all[w * kAttnFloats + kHeadDim + 1], sum);
+          acc = fmaf(f, all[w * kAttnFloats + tid], acc);
+        }
+        p.ctx[(size_t)(blockIdx.x / p.heads) * H + (size_t)(blockIdx.x % p.heads) * kHeadDim + tid] = __float2half(acc / sum);
+      }
+    }
     ok = c.barrier(708);
   }
   // ---- output projection
@@ -539,7 +593,7 @@ size_t lay_out(StepParams& p) {
   p.o_cell = take((size_t)p.layers * p.B * kUnits * 4);
   p.o_hid = take((size_t)p.layers * p.B * kUnits * 2);
   p.o_bias = take((size_t)p.layers * kRows * 4);
-  p.o_attn = take((size_t)kWarps * (kHeadDim + kMaxWindow) * 4);
+  p.o_attn = take((size_t)kWarps * kAttnFloats * 4);
   return off > tile_end ? off : tile_end;
 }
 
