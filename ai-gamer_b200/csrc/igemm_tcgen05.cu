@@ -24,6 +24,7 @@
 #include <vector>
 
 #include "aig_common.cuh"
+#include "res_chain.h"
 
 namespace {
 
@@ -2325,6 +2326,20 @@ int aig_fc_plan_set_weights_out_in(aig_conv_plan* pl, const aig_half* w_out_in, 
 // K-major weight operand [out_c][in_c] in place, once the identity epilogue (scale 1, shift 0) has been folded, and
 // the fp32 per-column shift (= the bias of a plain FC layer) of a plan whose weights were set.
 extern "C++" {
+bool conv_plan_view(const aig_conv_plan* pl, ConvPlanView* v) {
+  const PconvParams& q = pl->pp;
+  if (!pl->use_pconv || !q.flat || pl->out_f32 || (pl->is_down && !q.seg[0].padded)) return false;
+  *v = ConvPlanView{};
+  v->is_down = pl->is_down;
+  v->batch = q.batch; v->in_c = pl->pc_in_c; v->out_c = pl->d.out_c; v->Ho = q.Ho; v->Wo = q.Wo;
+  v->P = q.P; v->RP = q.RP; v->pad = q.pad; v->kw = q.kw; v->kh = q.taps / q.kw; v->taps = q.taps;
+  v->cblocks = q.cblocks; v->sub_cblocks = pl->is_down && pl->d.in_c % 64 == 0 ? q.sub_cblocks : 0;
+  v->act = pl->d.act; v->slope = pl->d.slope;
+  v->s2d = q.seg[0].s2d; v->Hb = q.seg[0].Hb; v->Wb = q.seg[0].Wb;
+  v->w = pl->w_packed; v->w_rows = pl->Kpad; v->w_k = pl->Ktot;
+  v->scale = pl->scale; v->shift = pl->shift;
+  return true;
+}
 __half* fc_plan_weight_buffer(aig_conv_plan* pl) { return pl && pl->is_fc ? pl->w_packed : nullptr; }
 float* fc_plan_shift_buffer(aig_conv_plan* pl) { return pl && pl->is_fc && pl->weights_set ? pl->shift : nullptr; }
 int fc_plan_identity_affine(aig_conv_plan* pl) {

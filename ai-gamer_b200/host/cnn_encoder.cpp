@@ -28,6 +28,7 @@
 #include "aig_b200.h"
 #include "aig_host.h"
 #include "cnn_stream.h"
+#include "res_chain.h"
 
 namespace {
 
@@ -71,6 +72,7 @@ struct aig_cnn {
   aig_half* stage_scratch = nullptr;  // channels-last copy of a space-to-depth stage, made on request
   size_t stage_scratch_elems = 0;
   std::vector<Block> blocks;
+  ResChain* chain = nullptr;          // the blocks and the head as one launch (small batches)
   aig_conv_plan* fc = nullptr;
   aig_half *act0 = nullptr, *sa = nullptr, *feat = nullptr, *logits = nullptr;
   float* out_f32 = nullptr;
@@ -312,6 +314,18 @@ int aig_cnn_create(aig_ctx* ctx, const aig_cnn_config* cfg, aig_cnn** out) {
     m->sites.push_back({"fc_head", 2.0 * c.batch * cl * c.n_out, (double)c.batch * cl * 2 + (double)cl * c.n_out * 2});
     m->sites.push_back({"sigmoid_tanh_tofloat", 0.0, (double)c.batch * c.n_out * 8});
   }
+  if (m->fused_head) {
+    std::vector<ResChainBlock> rb;
+    const aig_half* in = m->act0;
+    bool ok = true;
+    for (auto& b : m->blocks) {
+      ok = ok && b.down;
+      rb.push_back(ResChainBlock{b.down, b.c1, (aig_half*)in, b.t, b.r, b.y});
+      in = b.y;
+    }
+    if (ok && (rc = res_chain_create(ctx, rb, h * w, cl, c.n_out, &m->chain)) != AIG_OK) return bail(rc);
+    if (m->chain) m->launches_per_forward = 2;
+  }
   m->params.cap = aig_cnn_checkpoint_bytes(&c) + 256 * (16 + 32 * (size_t)c.n_blocks);
   if (cudaMalloc(reinterpret_cast<void**>(&m->params.base), m->params.cap) != cudaSuccess) return bail(AIG_ERR_CUDA);
   *out = m;
@@ -333,6 +347,7 @@ int aig_cnn_destroy(aig_cnn* m) {
     }
   }
   cnn_staging_free(m->staging);
+  res_chain_destroy(m->chain);
   aig_conv0_plan_destroy(m->conv0);
   for (auto& b : m->blocks) {
     aig_conv_plan_destroy(b.c0);
@@ -440,6 +455,12 @@ static int cnn_forward_impl(aig_cnn* m, const uint8_t* bgra_dev, bool planar) {
   if (planar) CNN_OK(m, aig_conv0_forward_rgb_planar(m->conv0, bgra_dev, m->act0));
   else CNN_OK(m, aig_conv0_forward_bgra(m->conv0, bgra_dev, m->act0));
   tick();
+  if (m->chain && !prof) {
+    const int hw = m->bh.back() * m->bw.back();
+    CNN_OK(m, res_chain_forward(m->chain, ResChainHead{m->sa_w, m->fcw, m->fcb, m->sa_b, m->feat, m->logits, m->out_f32, hw, c.widths[c.n_blocks],
+                                                       c.n_out, c.n_sigmoid}));
+    return AIG_OK;
+  }
   const aig_half* x = m->act0;
   for (auto& b : m->blocks) {
     if (b.down) {

@@ -249,3 +249,35 @@ def test_recording_pieces(env, tmp_path, n):
     assert np.array_equal(rec.infer(enc, 0, n), got)
     rec.close()
     enc.close()
+
+
+@gpu
+@pytest.mark.parametrize("B,H,W,widths,act", [
+    (1, 32, 32, (32, 64), "ACT_SWISH"), (1, 144, 256, (32, 64, 128, 256, 256), "ACT_SWISH"), (3, 67, 131, (32, 64, 128), "ACT_RELU"),
+    (6, 120, 200, (32, 64, 128, 256, 256), "ACT_LEAKY"), (19, 107, 189, (32, 64, 128, 256, 256), "ACT_SWISH"), (5, 50, 322, (64, 64, 192), "ACT_SWISH"),
+    (150, 20, 20, (32, 64, 128), "ACT_SWISH")])
+def test_small_batches_in_one_launch(env, monkeypatch, B, H, W, widths, act):
+    """Residual blocks and head as one launch against the per-layer launches: one tile to several rounds of tiles per
+    CTA, jobs split over one, two and four CTAs, rows of an image and whole images ending inside a tile, more frames
+    than CTAs for the head."""
+    U = env
+    c, pk = U.ctx(), U.pkg()
+    params = PL.make_cnn_params(B + H, widths=widths, trivial=False)
+    blob = PL.serialize_cnn_checkpoint(params, W, H)
+    frames = U.dev(PL.make_frames(B, B, H, W))
+    got = []
+    for off in ("1", "0"):
+        monkeypatch.setenv("AIG_CNN_NO_CHAIN", off)
+        enc = pk.CnnEncoder(c, B, H, W, widths=widths, act=getattr(pk, act))
+        enc.load_bytes(blob)
+        assert (enc.kernel_launches == 2) == (off == "0")
+        runs = []
+        for _ in range(3):
+            enc.forward(frames)
+            c.sync()
+            runs.append([U.host(enc.features()), U.host(enc.outputs_f32())] + [U.host(enc.stage_output(i)) for i in range(len(widths))])
+        assert all(np.array_equal(x, y) for r in runs[1:] for x, y in zip(runs[0], r))
+        got.append([x.astype(np.float32) for x in runs[0]])
+        enc.close()
+    for i, (a, b) in enumerate(zip(*got)):
+        assert U.scaled_err(b, a) < 6e-3, "result %d: %.4f" % (i, U.scaled_err(b, a))   # other summation orders, then a few fp16 roundings
