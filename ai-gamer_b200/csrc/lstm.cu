@@ -3,7 +3,7 @@
 // Per layer:  (1) the input projection W.x + bW + bR for all time steps is hoisted into one
 // tcgen05 GEMM (rows = T*B, fp32 output);  (2) the recurrence.  Sequences are independent, so a cluster of CTAs takes
 // 16 or 32 of them through all steps: each of its H/32 CTAs keeps the 4 gate rows of 32 hidden units of R (128 rows x H
-// fp16) in shared memory and every step
+// fp16) in TMEM and every step
 //    - waits until all h_{t-1} of the cluster's sequences has arrived in its own shared memory,
 //    - issues tcgen05.mma  R-slice [128 x H] x h_{t-1} [H x sequences]  into TMEM (gates are the M side, so that few
 //      sequences waste nothing but columns),
@@ -11,9 +11,13 @@
 //      within each quad of lanes, keep the cell state in registers (rounded to fp16 every step, like the library's cy
 //      tensor) and write h_t as fp16, and
 //    - one bulk copy per CTA of the cluster delivers its 32 units of h_t, already in the operand's layout.
+// With so few columns an MMA instruction costs what its issue costs: 41 to 48 clk with R in shared memory, 33 in TMEM.
 // What bounds a step is this chain's latency.  Sharing the sequences' h through global memory, with a step barrier over
 // all CTAs on a global counter, took 4.06 us a step at H = 512 and 128 sequences (3.66 at 3 sequences, H = 256); this
-// takes RESULT.
+// takes 1.7 us up to 112 sequences (1.2 at H = 256).  Of a step's 3300 clk the 32 MMAs take 1400, the gate functions 560,
+// issue and delivery of the copies 1070 (about 20 B/clk of distributed shared memory).  Above 112 sequences (16 in each
+// of the seven clusters of 16 CTAs that fit the device) a cluster takes two groups of 16, each with its own epilogue
+// warps, so that one group's MMAs run under the other's gates and delivery.
 // Gate order i,f,g,o; blob layout: per layer W then R, then per layer bW [and bR]  (the library's
 // blob is opaque in the reference: LSTMLayer.cpp:29-35,139-146; this layout is this library's
 // definition, stated in the header).
@@ -25,12 +29,14 @@ namespace {
 
 constexpr int kUnits = 32;        // hidden units per CTA: 128 gate rows, UMMA's M
 constexpr int kGateRows = 4 * kUnits;
-constexpr int kThreads = 160;     // MMA warp, four epilogue warps
-constexpr int kKB = 64;           // K block of R (128-byte swizzle span of fp16)
+constexpr int kSeqs = 16;         // sequences of a group: UMMA's N
+__host__ __device__ constexpr int lstm_threads(int groups) { return 32 + 128 * groups; }  // MMA warp, four epilogue warps per group
+constexpr int kColR = 64;         // first TMEM column of R (two values of K each); the accumulator is below
 
 struct LstmParams {
   int T, B, H, ctas;              // ctas: CTAs of the cluster that have units (the rest of a power of two only wait)
   float clip;
+  const __half* R;                // [4][H][H]
   const float* gx;                // hoisted projection, element (t,b,j) at t*gx_sT + b*gx_sB + j, j < 4H
   long long gx_sT, gx_sB;
   __half* y;                      // output sequence, element (t,b,j) at t*y_sT + b*y_sB + j
@@ -40,20 +46,32 @@ struct LstmParams {
   int* gerr;
 };
 
-__device__ __forceinline__ void tma_load_3d(uint32_t dst, const void* desc, uint32_t bar, int c0, int c1, int c2) {
-  asm volatile(
-      "cp.async.bulk.tensor.3d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5}], [%2];"
-      ::"r"(dst), "l"(reinterpret_cast<uint64_t>(desc)), "r"(bar), "r"(c0), "r"(c1), "r"(c2)
-      : "memory");
-}
 // own shared memory -> a cluster CTA's, the bytes counted on that CTA's barrier
 __device__ __forceinline__ void bulk_to_cluster(uint32_t dst, uint32_t src, uint32_t bytes, uint32_t bar) {
   asm volatile("cp.async.bulk.shared::cluster.shared::cta.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(dst), "r"(src), "r"(bytes), "r"(bar)
                : "memory");
 }
-// K-major operand without swizzle: 8-row x 16-byte core matrices, `lbo` between neighbours along K, `sbo` along N
-__device__ __forceinline__ uint64_t desc_plain(uint32_t saddr, uint32_t lbo, uint32_t sbo) {
-  return (uint64_t)((saddr & 0x3FFFFu) >> 4) | (uint64_t)(lbo >> 4) << 16 | (uint64_t)(sbo >> 4) << 32 | (uint64_t)1 << 46;
+// D[tmem] (+)= A[tmem] * B[smem].  B: K-major without swizzle, 8-row x 16-byte core matrices, `lbo` bytes between
+// neighbours along K, 128 along N; b_lo = plain_lo(address, lbo).
+__device__ __forceinline__ uint32_t plain_lo(uint32_t saddr, uint32_t lbo) { return ((saddr & 0x3FFFFu) >> 4) | (lbo >> 4) << 16; }
+__device__ __forceinline__ void umma_f16_ts(uint32_t d_tmem, uint32_t a_tmem, uint32_t b_lo, uint32_t idesc, uint32_t accumulate) {
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t.reg .b64 db;\n\t"
+      "mov.b64 db, {%2, %3};\n\t"
+      "setp.ne.b32 p, %5, 0;\n\t"
+      "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], db, %4, p;\n\t}"
+      ::"r"(d_tmem), "r"(a_tmem), "r"(b_lo), "r"((128u >> 4) | (1u << 14)), "r"(idesc), "r"(accumulate)
+      : "memory");
+}
+__device__ __forceinline__ void tmem_st_32x32(uint32_t taddr, const uint32_t (&r)[32]) {
+  asm volatile(
+      "tcgen05.st.sync.aligned.32x32b.x32.b32 [%0], "
+      "{%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16, "
+      "%17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31, %32};" ::"r"(taddr),
+      "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]), "r"(r[8]), "r"(r[9]), "r"(r[10]), "r"(r[11]), "r"(r[12]),
+      "r"(r[13]), "r"(r[14]), "r"(r[15]), "r"(r[16]), "r"(r[17]), "r"(r[18]), "r"(r[19]), "r"(r[20]), "r"(r[21]), "r"(r[22]), "r"(r[23]), "r"(r[24]),
+      "r"(r[25]), "r"(r[26]), "r"(r[27]), "r"(r[28]), "r"(r[29]), "r"(r[30]), "r"(r[31])
+      : "memory");
 }
 // Gate non-linearities through the special-function unit (ex2 and rcp approximations, relative error ~2^-22, far
 // below the fp16 rounding of h and c): an exact expf, IEEE division and tanhf per gate made the 128-thread
@@ -67,16 +85,16 @@ __device__ __forceinline__ float sigmoid_fast(float x) {
 __device__ __forceinline__ float tanh_fast(float x) {  // 2*sigmoid(2x) - 1
   return fmaf(2.0f, sigmoid_fast(2.0f * x), -1.0f);
 }
-// the four epilogue warps meet; true if all of them say so
-__device__ __forceinline__ bool epilogue_and(bool v) {
+// the four epilogue warps of a group meet; true if all of them say so
+__device__ __forceinline__ bool epilogue_and(int group, bool v) {
   uint32_t r;
   asm volatile(
       "{\n\t.reg .pred p, q;\n\t"
       "setp.ne.u32 q, %1, 0;\n\t"
-      "bar.red.and.pred p, 1, 128, q;\n\t"
+      "bar.red.and.pred p, %2, 128, q;\n\t"
       "selp.u32 %0, 1, 0, p;\n\t}"
       : "=r"(r)
-      : "r"(v ? 1u : 0u)
+      : "r"(v ? 1u : 0u), "r"(1 + group)
       : "memory");
   return r != 0;
 }
@@ -97,89 +115,98 @@ __device__ __forceinline__ void transpose_quad(float (&x)[4], int lane) {
   }
 }
 
-// NB = sequences per cluster: 16 or 32.
-template <int NB>
-__global__ void __launch_bounds__(kThreads, 1) lstm_recurrent_kernel(const __grid_constant__ CUtensorMap tmapR, const LstmParams p) {
-  constexpr int kBlock = NB * kUnits * 2;      // one CTA's units of all sequences: 4 chunks of 8 units, each NB rows x 16 bytes
-  constexpr uint32_t kTmemCols = 32;
+// G = groups of 16 sequences per cluster: 1 or 2.
+template <int G>
+__global__ void __launch_bounds__(lstm_threads(G), 1) lstm_recurrent_kernel(const LstmParams p) {
+  constexpr int NB = kSeqs, kThreads = lstm_threads(G);
+  constexpr int kBlock = NB * kUnits * 2;      // one CTA's units of a group: 4 chunks of 8 units, each NB rows x 16 bytes
   extern __shared__ uint8_t smem_raw[];
   const uint32_t raw = smem_u32(smem_raw), base = (raw + 1023u) & ~1023u;
   uint8_t* sm = smem_raw + (base - raw);
-  const int nkb = p.H / kKB, h_bytes = NB * p.H * 2;
-  const uint32_t sR = base;                                  // nkb slabs of 128 rows x 128 B (row = unit * 4 + gate)
-  uint8_t* hbuf = sm + nkb * kGateRows * 128;                // [2] h of all units: chunks of 8 units, each NB rows x 16 bytes
-  const uint32_t sH = base + nkb * kGateRows * 128;
-  uint8_t* stage = hbuf + 2 * h_bytes;                       // [2] this CTA's part of h_t
-  uint64_t* bars = reinterpret_cast<uint64_t*>(stage + 2 * kBlock);
-  const uint32_t bar_r = smem_u32(bars), bar_h = bar_r + 8, bar_tfull = bar_r + 24, bar_tempty = bar_r + 32;
-  uint32_t* s_tmem = reinterpret_cast<uint32_t*>(bars + 5);
+  const int h_bytes = NB * p.H * 2;
+  const uint32_t tmem_cols = p.H > 384 ? 512u : 256u;        // accumulators, R
+  // per group: h of all units [2] (chunks of 8 units, each NB rows x 16 bytes), then this CTA's part of h_t [2]
+  const int group_bytes = 2 * (h_bytes + kBlock);
+  uint64_t* bars = reinterpret_cast<uint64_t*>(sm + G * group_bytes);
+  const uint32_t bar0 = smem_u32(bars);                      // per group: h arrived [2], accumulator ready, accumulator drained
+  uint32_t* s_tmem = reinterpret_cast<uint32_t*>(bars + 4 * G);
   volatile int* s_abort = reinterpret_cast<volatile int*>(s_tmem + 1);
 
   const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;  // (uniform for the compiler)
   const int rank = (int)cluster_ctarank();
   uint32_t n_ctarank;
   asm volatile("mov.u32 %0, %%cluster_nctarank;" : "=r"(n_ctarank));
-  const int row0 = (int)(blockIdx.x / n_ctarank) * NB, unit0 = rank * kUnits;
+  const int row0 = (int)(blockIdx.x / n_ctarank) * (G * NB), unit0 = rank * kUnits;
   const bool working = rank < p.ctas;
 
   if (threadIdx.x == 0) {
-    mbar_init(bar_r, 1);
-    mbar_init(bar_h, 1);
-    mbar_init(bar_h + 8, 1);
-    mbar_init(bar_tfull, 1);
-    mbar_init(bar_tempty, 4);
+    for (int i = 0; i < 4 * G; ++i) mbar_init(bar0 + 8 * i, i % 4 == 3 ? 4 : 1);
     *s_abort = 0;
     fence_mbar_init();
-    if (working) {
-      mbar_expect_tx(bar_r, (uint32_t)(nkb * kGateRows * 128));
-      for (int kb = 0; kb < nkb; ++kb) tma_load_3d(sR + kb * kGateRows * 128, &tmapR, bar_r, kb * kKB, 0, unit0);
-    }
   }
   if (warp == 0) {
-    tmem_alloc(smem_u32(s_tmem), kTmemCols);
+    tmem_alloc(smem_u32(s_tmem), tmem_cols);
     tmem_relinquish();
   }
   if (working) {
     // h_{-1}, as step -1 would have delivered it (buffer 1)
-    for (int i = threadIdx.x; i < h_bytes / 16; i += kThreads) {
-      const int chunk = i / NB, b = row0 + i % NB;
+    for (int i = threadIdx.x; i < G * h_bytes / 16; i += kThreads) {
+      const int g = i / (h_bytes / 16), k = i - g * (h_bytes / 16), chunk = k / NB, b = row0 + g * NB + k % NB;
       uint4 v = make_uint4(0, 0, 0, 0);
       if (p.h0 && b < p.B) v = *reinterpret_cast<const uint4*>(p.h0 + (size_t)b * p.H + chunk * 8);
-      reinterpret_cast<uint4*>(hbuf + h_bytes)[i] = v;
+      reinterpret_cast<uint4*>(sm + g * group_bytes + h_bytes)[k] = v;
     }
   }
   fence_proxy_async_smem();
   tc_fence_before();
   __syncthreads();
-  cluster_sync_all();  // barriers are there before anything crosses, and every CTA has read the initial h
   tc_fence_after();
   const uint32_t tmem_base = *s_tmem;
+  if (working && warp >= 1 && warp <= 4) {
+    // R to TMEM: lane = row = unit * 4 + gate
+    const int q = warp & 3;
+    const uint4* src = reinterpret_cast<const uint4*>(p.R + ((size_t)(lane & 3) * p.H + unit0 + q * 8 + (lane >> 2)) * p.H);
+    for (int k = 0; k < p.H / 64; ++k) {
+      uint4 v[8];
+#pragma unroll
+      for (int i = 0; i < 8; ++i) v[i] = __ldg(src + k * 8 + i);
+      tmem_st_32x32(tmem_base + kColR + k * 32 + ((uint32_t)(q * 32) << 16), reinterpret_cast<const uint32_t (&)[32]>(v));
+    }
+    asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+  }
+  tc_fence_before();
+  cluster_sync_all();  // barriers and R are there, and every CTA has read the initial h
+  tc_fence_after();
 
   if (working && warp == 0) {
     // ------------------------------------------------------------------ MMA issuer
     // (all lanes run the loop with identical values, one elected lane issues: see elect_one)
     constexpr uint32_t idesc = umma_idesc_f16(kGateRows, NB);
     const bool leader = elect_one();
-    bool ok = mbar_wait_bounded(bar_r, 0, s_abort, p.gerr, 402);
+    bool ok = true;
     for (int t = 0; t < p.T && ok; ++t) {
       const uint32_t prev = (uint32_t)(t + 1) & 1u;  // buffer of h_{t-1}
-      if (leader && t + 1 < p.T) mbar_expect_tx(bar_h + 8 * (t & 1), (uint32_t)h_bytes);
-      if (t > 0) ok = mbar_wait_bounded_cl(bar_h + 8 * prev, (uint32_t)((t - 1) >> 1) & 1u, s_abort, p.gerr, 404) &&
-                      mbar_wait_bounded(bar_tempty, (uint32_t)(t - 1) & 1u, s_abort, p.gerr, 403);
-      if (!ok) break;
-      tc_fence_after();
-      const uint32_t h = sH + prev * h_bytes;
-      for (int kb = 0; kb < nkb; ++kb) {
-        const uint32_t a = sR + kb * kGateRows * 128, b = h + kb * (kKB / 8) * NB * 16;
 #pragma unroll
-        for (int k = 0; k < kKB / 16; ++k)
-          if (leader) umma_f16_ss(tmem_base, umma_smem_desc(a + k * 32, 128), desc_plain(b + k * 2 * NB * 16, NB * 16, 128), idesc, (kb | k) != 0 ? 1u : 0u);
+      for (int g = 0; g < G; ++g) {
+        const uint32_t bar_h = bar0 + 32 * g;
+        if (row0 + g * NB >= p.B) break;  // (no sequence in this group)
+        if (leader && t + 1 < p.T) mbar_expect_tx(bar_h + 8 * (t & 1), (uint32_t)h_bytes);
+        if (t > 0) ok = ok && mbar_wait_bounded_cl(bar_h + 8 * prev, (uint32_t)((t - 1) >> 1) & 1u, s_abort, p.gerr, 404) &&
+                        mbar_wait_bounded(bar_h + 24, (uint32_t)(t - 1) & 1u, s_abort, p.gerr, 403);
+        if (!ok) break;
+        tc_fence_after();
+        const uint32_t h = plain_lo(base + g * group_bytes + prev * h_bytes, NB * 16);
+#pragma unroll 4
+        for (int k = 0; k < p.H / 16; ++k)
+          if (leader) umma_f16_ts(tmem_base + g * NB, tmem_base + kColR + k * 8, h + (uint32_t)(k * 2 * NB), idesc, k != 0 ? 1u : 0u);
+        if (leader) umma_commit(bar_h + 16);
       }
-      if (leader) umma_commit(bar_tfull);
     }
-  } else if (working) {
+  } else if (working && row0 + ((warp - 1) >> 2) * NB < p.B) {
     // ------------------------------------------------------------------ gates: one thread per gate row
-    const int q = warp & 3, tid = (warp - 1) * 32 + lane;
+    const int group = (warp - 1) >> 2, w4 = (warp - 1) & 3, q = warp & 3, tid = w4 * 32 + lane, seq0 = row0 + group * NB;
+    const uint32_t sH = base + group * group_bytes, bar_h = bar0 + 32 * group;
+    uint8_t* stage = sm + group * group_bytes + 2 * h_bytes;
     const int gate = lane & 3, unit = q * 8 + (lane >> 2);
     // sigmoid(x), or 2*sigmoid(2x) - 1 on the lanes of the g gate
     const float in_scale = gate == 2 ? 2.0f : 1.0f, out_scale = in_scale, out_shift = gate == 2 ? -1.0f : 0.0f;
@@ -187,23 +214,22 @@ __global__ void __launch_bounds__(kThreads, 1) lstm_recurrent_kernel(const __gri
     float c[NB / 4], gx[NB];
 #pragma unroll
     for (int j = 0; j < NB / 4; ++j) {  // this lane's cells: its unit of sequences gate, gate + 4, ...
-      const int b = row0 + 4 * j + gate;
+      const int b = seq0 + 4 * j + gate;
       c[j] = p.c0 && b < p.B ? __half2float(p.c0[(size_t)b * p.H + unit0 + unit]) : 0.f;
     }
 #pragma unroll
-    for (int n = 0; n < NB; ++n) gx[n] = row0 + n < p.B ? __ldg(gsrc + (size_t)(row0 + n) * p.gx_sB) : 0.f;
-    const uint32_t t_addr = tmem_base + ((uint32_t)(q * 32) << 16);
+    for (int n = 0; n < NB; ++n) gx[n] = seq0 + n < p.B ? __ldg(gsrc + (size_t)(seq0 + n) * p.gx_sB) : 0.f;
+    const uint32_t t_addr = tmem_base + group * NB + ((uint32_t)(q * 32) << 16);
     bool ok = true;
     for (int t = 0; t < p.T && ok; ++t) {
-      ok = mbar_wait_bounded(bar_tfull, (uint32_t)t & 1u, s_abort, p.gerr, 405);
+      ok = mbar_wait_bounded(bar_h + 16, (uint32_t)t & 1u, s_abort, p.gerr, 405);
       tc_fence_after();
       uint32_t r[NB];
-      if constexpr (NB == 32) tmem_ld_32x32(t_addr, r);
-      else tmem_ld_32x16(t_addr, r);
+      tmem_ld_32x16(t_addr, r);
       tmem_ld_wait();
       tc_fence_before();
       __syncwarp();
-      if (lane == 0) mbar_arrive(bar_tempty);
+      if (lane == 0) mbar_arrive(bar_h + 24);
       __half* st = reinterpret_cast<__half*>(stage + (t & 1) * kBlock);
 #pragma unroll
       for (int j = 0; j < NB / 4; ++j) {
@@ -218,20 +244,22 @@ __global__ void __launch_bounds__(kThreads, 1) lstm_recurrent_kernel(const __gri
         st[(q * NB + n) * 8 + (lane >> 2)] = __float2half(x[3] * tanh_fast(c[j]));
       }
       fence_proxy_async_smem();
-      ok = epilogue_and(ok);
+      ok = epilogue_and(group, ok);
       if (!ok) break;
-      if (t + 1 < p.T && tid < p.ctas)
-        bulk_to_cluster(mapa_shared(sH + (uint32_t)((t & 1) * h_bytes + rank * kBlock), (uint32_t)tid), smem_u32(st), kBlock,
-                        mapa_shared(bar_h + 8 * (t & 1), (uint32_t)tid));
+      // (four warps issue: the copies of one warp's lanes go out one after another)
+      const int dst = (lane << 2) | w4;
+      if (t + 1 < p.T && dst < p.ctas)
+        bulk_to_cluster(mapa_shared(sH + (uint32_t)((t & 1) * h_bytes + rank * kBlock), (uint32_t)dst), smem_u32(st), kBlock,
+                        mapa_shared(bar_h + 8 * (t & 1), (uint32_t)dst));
       // under the delivery: this step's h to memory (16 bytes of a sequence per thread), the next step's projection
       if (t + 1 < p.T) {
         const float* g1 = gsrc + (size_t)(t + 1) * p.gx_sT;
 #pragma unroll
         for (int n = 0; n < NB; ++n)
-          if (row0 + n < p.B) gx[n] = __ldg(g1 + (size_t)(row0 + n) * p.gx_sB);
+          if (seq0 + n < p.B) gx[n] = __ldg(g1 + (size_t)(seq0 + n) * p.gx_sB);
       }
       if (tid < 4 * NB) {
-        const int chunk = tid / NB, b = row0 + tid % NB;
+        const int chunk = tid / NB, b = seq0 + tid % NB;
         if (b < p.B) {
           const uint4 v = reinterpret_cast<const uint4*>(st)[tid];
           *reinterpret_cast<uint4*>(p.y + (size_t)t * p.y_sT + (size_t)b * p.y_sB + unit0 + chunk * 8) = v;
@@ -242,7 +270,7 @@ __global__ void __launch_bounds__(kThreads, 1) lstm_recurrent_kernel(const __gri
     if (ok && p.cT)
 #pragma unroll
       for (int j = 0; j < NB / 4; ++j) {
-        const int b = row0 + 4 * j + gate;
+        const int b = seq0 + 4 * j + gate;
         if (b < p.B) p.cT[(size_t)b * p.H + unit0 + unit] = __float2half(c[j]);
       }
   }
@@ -255,95 +283,67 @@ __global__ void __launch_bounds__(kThreads, 1) lstm_recurrent_kernel(const __gri
   cluster_sync_all();  // no CTA leaves while another may still write to it
   if (warp == 0) {
     tc_fence_after();
-    tmem_dealloc(tmem_base, kTmemCols);
+    tmem_dealloc(tmem_base, tmem_cols);
   }
-}
-
-typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
-                                  const cuuint64_t*, const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave,
-                                  CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
-EncodeTiledFn encode_fn() {
-  static EncodeTiledFn fn = nullptr;
-  if (!fn) {
-    void* p = nullptr;
-    cudaDriverEntryPointQueryResult qres;
-    if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &p, cudaEnableDefault, &qres) == cudaSuccess &&
-        qres == cudaDriverEntryPointSuccess)
-      fn = reinterpret_cast<EncodeTiledFn>(p);
-  }
-  return fn;
-}
-
-// R of one layer [4][H][H] as (K, gate, unit): a box of 64 x 4 x 32 is a slab of 128 rows in the order unit * 4 + gate
-int encode_R(aig_ctx* ctx, CUtensorMap* m, const void* r, int H) {
-  EncodeTiledFn enc = encode_fn();
-  if (!enc) return aig_fail(ctx, AIG_ERR_CUDA, "cuTensorMapEncodeTiled entry point not available");
-  cuuint64_t dims[3] = {(cuuint64_t)H, 4, (cuuint64_t)H};
-  cuuint64_t strides[2] = {(cuuint64_t)H * H * 2, (cuuint64_t)H * 2};
-  cuuint32_t box[3] = {kKB, 4, kUnits}, es[3] = {1, 1, 1};
-  CUresult rc = enc(m, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 3, const_cast<void*>(r), dims, strides, box, es, CU_TENSOR_MAP_INTERLEAVE_NONE,
-                    CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-  if (rc != CUDA_SUCCESS) return aig_fail(ctx, AIG_ERR_CUDA, "cuTensorMapEncodeTiled(R) failed: %d", (int)rc);
-  return AIG_OK;
 }
 
 // Shape of a recurrence launch.
 struct LstmLaunch {
-  int nb = 16, ctas = 0, cluster = 0;
+  int groups = 1, ctas = 0, cluster = 0;
   size_t smem = 0;
 };
-size_t recurrent_smem(int H, int nb) { return (size_t)H / kKB * kGateRows * 128 + 2 * (size_t)nb * H * 2 + 2 * (size_t)nb * kUnits * 2 + 64 + 1024; }
+size_t recurrent_smem(int H, int groups) { return (size_t)groups * (2 * kSeqs * (H + kUnits) * 2 + 32) + 64 + 1024; }
 
-template <int NB>
+template <int G>
 int recurrent_config(aig_ctx* ctx, const LstmLaunch& l, int batch, cudaLaunchConfig_t* cfg, cudaLaunchAttribute* attr) {
   attr->id = cudaLaunchAttributeClusterDimension;
   attr->val.clusterDim.x = l.cluster;
   attr->val.clusterDim.y = attr->val.clusterDim.z = 1;
   *cfg = cudaLaunchConfig_t{};
-  cfg->gridDim = dim3(ceil_div(batch, NB) * l.cluster);
-  cfg->blockDim = dim3(kThreads);
+  cfg->gridDim = dim3(ceil_div(batch, G * kSeqs) * l.cluster);
+  cfg->blockDim = dim3(lstm_threads(G));
   cfg->dynamicSmemBytes = l.smem;
   cfg->stream = ctx->stream;
   cfg->attrs = attr;
   cfg->numAttrs = 1;
-  AIG_CUDA_OK(ctx, cudaFuncSetAttribute(lstm_recurrent_kernel<NB>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)l.smem));
-  AIG_CUDA_OK(ctx, cudaFuncSetAttribute(lstm_recurrent_kernel<NB>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+  AIG_CUDA_OK(ctx, cudaFuncSetAttribute(lstm_recurrent_kernel<G>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)l.smem));
+  AIG_CUDA_OK(ctx, cudaFuncSetAttribute(lstm_recurrent_kernel<G>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
   return AIG_OK;
 }
 
-// Sequences per cluster: 16, or 32 where clusters of 16 sequences would not all run at once.
+// One group of sequences per cluster, or two where the clusters of one group would not all run at once.
 int recurrent_shape(aig_ctx* ctx, int H, int batch, LstmLaunch* l) {
   l->ctas = H / kUnits;
   l->cluster = 1;
   while (l->cluster < l->ctas) l->cluster *= 2;
-  l->nb = 16;
-  l->smem = recurrent_smem(H, 16);
+  l->groups = 1;
+  l->smem = recurrent_smem(H, 1);
   cudaLaunchConfig_t cfg;
   cudaLaunchAttribute attr;
-  int rc = recurrent_config<16>(ctx, *l, batch, &cfg, &attr), n = 0;
+  int rc = recurrent_config<1>(ctx, *l, batch, &cfg, &attr), n = 0;
   if (rc != AIG_OK) return rc;
-  AIG_CUDA_OK(ctx, cudaOccupancyMaxActiveClusters(&n, lstm_recurrent_kernel<16>, &cfg));
+  AIG_CUDA_OK(ctx, cudaOccupancyMaxActiveClusters(&n, lstm_recurrent_kernel<1>, &cfg));
   if (n < 1) return aig_fail(ctx, AIG_ERR_UNSUPPORTED, "lstm: no cluster of %d CTAs fits this device", l->cluster);
-  if (ceil_div(batch, 16) > n) {
-    l->nb = 32;
-    l->smem = recurrent_smem(H, 32);
+  if (ceil_div(batch, kSeqs) > n) {
+    l->groups = 2;
+    l->smem = recurrent_smem(H, 2);
   }
   return AIG_OK;
 }
 
-template <int NB>
-int launch_recurrent(aig_ctx* ctx, const LstmLaunch& l, const CUtensorMap& mR, const LstmParams& prm) {
+template <int G>
+int launch_recurrent(aig_ctx* ctx, const LstmLaunch& l, const LstmParams& prm) {
   cudaLaunchConfig_t cfg;
   cudaLaunchAttribute attr;
-  const int rc = recurrent_config<NB>(ctx, l, prm.B, &cfg, &attr);
+  const int rc = recurrent_config<G>(ctx, l, prm.B, &cfg, &attr);
   if (rc != AIG_OK) return rc;
-  AIG_CUDA_OK(ctx, cudaLaunchKernelEx(&cfg, lstm_recurrent_kernel<NB>, mR, prm));
+  AIG_CUDA_OK(ctx, cudaLaunchKernelEx(&cfg, lstm_recurrent_kernel<G>, prm));
   return AIG_OK;
 }
-int run_recurrent(aig_ctx* ctx, const LstmLaunch& l, const CUtensorMap& mR, LstmParams prm) {
+int run_recurrent(aig_ctx* ctx, const LstmLaunch& l, LstmParams prm) {
   prm.ctas = l.ctas;
   prm.gerr = ctx->d_err;
-  return l.nb == 16 ? launch_recurrent<16>(ctx, l, mR, prm) : launch_recurrent<32>(ctx, l, mR, prm);
+  return l.groups == 1 ? launch_recurrent<1>(ctx, l, prm) : launch_recurrent<2>(ctx, l, prm);
 }
 
 }  // namespace
@@ -359,7 +359,6 @@ struct aig_lstm_plan {
   std::vector<aig_conv_plan*> proj;     // hoisted input projection per layer
   float* gx = nullptr;                  // [T*B][4H] fp32 scratch
   __half* mid = nullptr;                // intermediate layer outputs (same layout as y)
-  std::vector<CUtensorMap> mapR;
 };
 
 extern "C" {
@@ -417,7 +416,6 @@ int aig_lstm_plan_create(aig_ctx* ctx, int seq_len, int layers, int hidden, int 
     aig_lstm_plan_destroy(pl);
     return rc;
   }
-  pl->mapR.resize(layers);
   *out = pl;
   return AIG_OK;
 }
@@ -443,8 +441,6 @@ int aig_lstm_plan_set_weights(aig_lstm_plan* pl, const aig_half* blob) {
     int rc = aig_fc_plan_set_weights_out_in(pl->proj[l], blob + pl->w_off[l], blob + pl->bw_off[l]);
     if (rc != AIG_OK) return rc;
     if (pl->double_bias && (rc = aig_fc_plan_add_bias(pl->proj[l], blob + pl->br_off[l])) != AIG_OK) return rc;
-    rc = encode_R(ctx, &pl->mapR[l], blob + pl->r_off[l], pl->H);
-    if (rc != AIG_OK) return rc;
   }
   return AIG_OK;
 }
@@ -471,6 +467,7 @@ int aig_lstm_forward(aig_lstm_plan* pl, const aig_half* x, aig_half* y, aig_half
     LstmParams prm{};
     prm.T = T; prm.B = B; prm.H = H;
     prm.clip = pl->clip;
+    prm.R = pl->blob + pl->r_off[l];
     prm.gx = pl->gx;
     // the projection's rows follow x's memory order
     prm.gx_sT = pl->batch_major ? (long long)4 * H : (long long)B * 4 * H;
@@ -480,7 +477,7 @@ int aig_lstm_forward(aig_lstm_plan* pl, const aig_half* x, aig_half* y, aig_half
     prm.c0 = use_state ? (const __half*)c_state + (size_t)l * B * H : nullptr;
     prm.hT = h_state ? (__half*)h_state + (size_t)l * B * H : nullptr;
     prm.cT = c_state ? (__half*)c_state + (size_t)l * B * H : nullptr;
-    if ((rc = run_recurrent(ctx, pl->shape, pl->mapR[l], prm)) != AIG_OK) return rc;
+    if ((rc = run_recurrent(ctx, pl->shape, prm)) != AIG_OK) return rc;
     in = out;
   }
   return AIG_OK;
@@ -595,18 +592,17 @@ int aig_lstm_forward_noalloc(aig_ctx* ctx, const aig_half* x, const aig_half* bl
       (const __half*)x, hb + w_off, hb + bw_off, double_bias ? hb + br_off : nullptr, gx, rows, in_c, 4 * hidden);
   AIG_LAUNCH_OK(ctx);
   // ---- recurrence
-  CUtensorMap mR;
-  if ((rc = encode_R(ctx, &mR, hb + r_off, hidden)) != AIG_OK) return rc;
   LstmParams prm{};
   prm.T = seq_len; prm.B = batch; prm.H = hidden;
   prm.clip = clip;
+  prm.R = hb + r_off;
   prm.gx = gx;
   prm.gx_sT = (long long)batch * 4 * hidden;
   prm.gx_sB = (long long)4 * hidden;
   prm.y = (__half*)y;
   prm.y_sT = (long long)batch * hidden;
   prm.y_sB = hidden;
-  return run_recurrent(ctx, shape, mR, prm);
+  return run_recurrent(ctx, shape, prm);
 }
 
 }  // extern "C"
