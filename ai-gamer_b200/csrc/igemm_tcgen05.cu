@@ -25,6 +25,7 @@
 
 #include "aig_common.cuh"
 #include "res_chain.h"
+#include "skinny_fc.h"
 
 namespace {
 
@@ -1344,6 +1345,13 @@ __global__ void repack_fc_kernel(const __half* __restrict__ w_in_out, __half* __
     packed[i] = w_in_out[(size_t)k * outC + o];
   }
 }
+__global__ void repack_fc_nhwc_kernel(const __half* __restrict__ w_in_out, __half* __restrict__ packed, int c, int hw, int outC) {
+  const long long inC = (long long)c * hw, total = inC * outC;
+  for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (long long)gridDim.x * blockDim.x) {
+    const long long k = i % inC, o = i / inC;  // k = position * c + channel
+    packed[i] = w_in_out[(size_t)((k % c) * hw + k / c) * outC + o];
+  }
+}
 __global__ void fold_affine_kernel(float* scale, float* shift, const __half* bias, const float* gamma, const float* beta,
                                    const float* mean, const float* var, float eps, int K, int Kpad) {
   for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < Kpad; k += gridDim.x * blockDim.x) {
@@ -1429,6 +1437,7 @@ struct aig_conv_plan {
   aig_conv_desc d{};
   int Do = 1, Ho = 1, Wo = 1;
   bool is_fc = false;
+  bool skinny = false;                         // FC plans of few rows: see skinny_fc.cu
   int BK = 64, NT = 64, MS = 1, Kpad = 0, taps = 1, Ktot = 0;
   IgemmParams prm{};
   __half* w_packed = nullptr;
@@ -2144,6 +2153,20 @@ int pconv_try_plain(aig_ctx* ctx, aig_conv_plan* pl) {
 }
 }  // namespace
 
+namespace {
+int run_skinny(aig_conv_plan* pl, const void* x, void* y, const FcTail& tail) {
+  SkinnyFc s{};
+  s.rows = pl->d.in_w; s.in_c = pl->d.in_c; s.out_c = pl->d.out_c;
+  s.w = pl->w_packed; s.x = (const __half*)x;
+  s.scale = pl->scale; s.shift = pl->shift;
+  s.two_step = pl->d.two_step; s.act = pl->d.act; s.slope = pl->d.slope;
+  s.y = pl->out_f32 ? nullptr : (__half*)y;
+  s.y32 = pl->out_f32 ? (float*)y : nullptr;
+  s.tail = tail;
+  return skinny_fc_forward(pl->ctx, s);
+}
+}  // namespace
+
 extern "C" {
 
 int aig_conv_plan_create(aig_ctx* ctx, const aig_conv_desc* desc, aig_conv_plan** out) {
@@ -2248,6 +2271,7 @@ int aig_conv_forward(aig_conv_plan* pl, const aig_half* x, const aig_half* resid
     }
     return dispatch_pconv(pl);
   }
+  if (pl->skinny && !residual) return run_skinny(pl, x, y, FcTail{});
   if (pl->tmapA_ptr != x) {
     const int rc = encode_A(pl, x);
     if (rc != AIG_OK) return rc;
@@ -2272,6 +2296,7 @@ int aig_fc_plan_create(aig_ctx* ctx, int rows, int in_c, int out_c, int act, flo
   d.act = act; d.slope = slope; d.two_step = two_step;
   pl->d = d;
   pl->Do = 1; pl->Ho = 1; pl->Wo = rows;
+  pl->skinny = rows <= kSkinnyRows;
   const int rc = plan_finish(ctx, pl);
   if (rc != AIG_OK) {
     aig_conv_plan_destroy(pl);
@@ -2346,6 +2371,31 @@ int fc_plan_identity_affine(aig_conv_plan* pl) {
   if (!pl || !pl->is_fc) return AIG_ERR_INVALID;
   DeviceGuard g(pl->ctx->device);
   return set_affine(pl, nullptr, nullptr, nullptr, nullptr, nullptr, 0.f);
+}
+void fc_plan_use_skinny(aig_conv_plan* pl, bool enable) { pl->skinny = enable; }
+int fc_plan_forward_tail(aig_conv_plan* pl, const aig_half* x, aig_half* y, const FcTail& tail) {
+  aig_ctx* ctx = pl->ctx;
+  DeviceGuard g(ctx->device);
+  AIG_REQUIRE(ctx, x && y && pl->is_fc && pl->weights_set && pl->d.two_step && !pl->out_f32 && pl->skinny, "fc forward with tail: not such a plan");
+  return run_skinny(pl, x, y, tail);
+}
+int fc_plan_pack_columns(aig_conv_plan* pl, const aig_half* w_in_out, int n, int first) {
+  aig_ctx* ctx = pl->ctx;
+  DeviceGuard g(ctx->device);
+  AIG_REQUIRE(ctx, pl->is_fc && w_in_out && n > 0 && first >= 0 && first + n <= pl->d.out_c, "fc pack: columns outside the plan");
+  const long long blocks = ceil_div_ll((long long)n * pl->d.in_c, 256);
+  repack_fc_kernel<<<(int)(blocks > ctx->sm_count * 8 ? ctx->sm_count * 8 : blocks), 256, 0, ctx->stream>>>(
+      (const __half*)w_in_out, pl->w_packed + (size_t)first * pl->d.in_c, pl->d.in_c, n);
+  AIG_LAUNCH_OK(ctx);
+  return AIG_OK;
+}
+int fc_plan_set_weights_nhwc(aig_conv_plan* pl, const aig_half* w_in_out, const aig_half* bias, int c, int hw) {
+  aig_ctx* ctx = pl->ctx;
+  DeviceGuard g(ctx->device);
+  AIG_REQUIRE(ctx, pl->is_fc && w_in_out && c * hw == pl->d.in_c, "fc set_weights: channels and positions do not match the plan");
+  repack_fc_nhwc_kernel<<<ctx->sm_count * 8, 256, 0, ctx->stream>>>((const __half*)w_in_out, pl->w_packed, c, hw, pl->d.out_c);
+  AIG_LAUNCH_OK(ctx);
+  return set_affine(pl, bias, nullptr, nullptr, nullptr, nullptr, 0.f);
 }
 }  // extern "C++"
 

@@ -24,6 +24,7 @@
 #include <vector>
 
 #include "aig_common.cuh"
+#include "skinny_fc.h"
 
 namespace {
 
@@ -406,6 +407,7 @@ int aig_lstm_plan_create(aig_ctx* ctx, int seq_len, int layers, int hidden, int 
     rc = aig_fc_plan_create(ctx, seq_len * batch, l == 0 ? in_c : hidden, 4 * hidden, AIG_ACT_NONE, 0.f, 0, &fp);
     if (rc == AIG_OK) {
       aig_fc_plan_set_output_f32(fp, 1);
+      fc_plan_use_skinny(fp, false);  // a sequence in pieces gives the bits of the whole
       pl->proj.push_back(fp);
     }
   }

@@ -435,3 +435,33 @@ def test_fused_downsampling_refuses_unsupported_channel_counts(env):
         pk.ResDownPlan(U.ctx(), 1, 24, 10, 12, 64)
     with pytest.raises(pk.AigError, match="out_c"):
         pk.ResDownPlan(U.ctx(), 1, 32, 10, 12, 48)
+
+
+@gpu
+@pytest.mark.parametrize("rows,inC,outC", [(1, 16, 1), (1, 8208, 1024), (7, 48, 15), (8, 272, 17), (9, 1024, 512), (16, 4096, 40), (17, 512, 1024),
+                                           (33, 144, 100), (64, 2048, 33), (65, 256, 16), (128, 1040, 18), (129, 512, 64)])
+@pytest.mark.parametrize("f32", [False, True])
+def test_fc_few_rows(env, rows, inC, outC, f32):
+    """The product for few rows: tiles of eight rows and of sixteen outputs that are not full, half a block of K at the
+    end, one CTA and clusters of two to eight along K, one row more than it takes; fp16 with an activation, and fp32."""
+    U = env
+    import torch
+
+    c, pk = U.ctx(), U.pkg()
+    rng = np.random.default_rng(rows * 7 + outC)
+    x, W = h(rng.standard_normal((rows, inC))), h(rng.standard_normal((inC, outC)) / np.sqrt(inC))
+    b = h(rng.uniform(-0.5, 0.5, outC))
+    want = x.astype(np.float64) @ W.astype(np.float64) + b.astype(np.float64)
+    plan = pk.FcPlan(c, rows, inC, outC, act=pk.ACT_NONE if f32 else pk.ACT_LEAKY, slope=0.25)
+    if f32:
+        pk.lib().aig_fc_plan_set_output_f32(plan.handle, 1)
+    else:
+        want = np.where(want < 0, 0.25 * want, want)
+    plan.set_weights(U.dev(W), U.dev(b))
+    dy = torch.zeros(rows * outC, dtype=torch.float32 if f32 else torch.float16, device="cuda")
+    dx = U.dev(x)
+    for _ in range(2):
+        plan.forward(dx, dy)
+    c.sync()
+    assert np.abs(U.host(dy).reshape(rows, outC) - want).max() < (2e-4 if f32 else 4e-3)
+    plan.close()
