@@ -2,8 +2,9 @@
 // sm_100a, with rotary embedding applied while the Q/K tiles are staged and a ring key/value cache
 // for step-by-step use.
 //
-// Full sequence:  Q,K,V = x.Wq, x.Wk, x.Wv (three tcgen05 GEMM launches), then one attention kernel:
-//   per (sequence, head) work item a CTA
+// Full sequence:  Q,K,V = x.[Wq Wk Wv] (one GEMM launch), then one attention kernel:
+//   per (sequence, head) work item a CTA (two or three resident on an SM: an item is a chain of loads, rotation, two
+//   MMAs and a softmax, none of which fills the SM)
 //     - TMA-loads the Q tile (128 query rows, rows >= T zero-filled), K and V tiles (NK key rows),
 //     - its 128 row threads rotate Q and K in shared memory (RoPE), transpose V to K-major,
 //     - tcgen05.mma  S = Q.K^T  into TMEM, row threads do the masked softmax from TMEM and write
@@ -15,6 +16,7 @@
 #include <vector>
 
 #include "aig_common.cuh"
+#include "skinny_fc.h"
 
 namespace {
 
@@ -60,13 +62,17 @@ __device__ __forceinline__ void rope_row(uint8_t* tile, int r, const float2* cs)
   }
 }
 
+// CTAs per SM: bounded by TMEM (128 or 256 columns each) and registers (a row of scores per thread)
+template <int NK>
+constexpr int kAttnCtas = NK == 64 ? 3 : 2;
+
 // NK = key slots per tile (64 or 128); T <= NK, T <= 128.
 template <int NK>
-__global__ void __launch_bounds__(kThreads, 1)
+__global__ void __launch_bounds__(kThreads, kAttnCtas<NK>)
 attention_tile_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constant__ CUtensorMap mapK,
                       const __grid_constant__ CUtensorMap mapV, const AttnParams p) {
   constexpr int kKB = NK / 64;                 // 64-key blocks
-  constexpr int kTmemCols = 256;               // S: NK columns at 0, O: 64 columns at NK
+  constexpr int kTmemCols = NK == 64 ? 128 : 256;  // S: NK columns at 0, O: 64 columns at NK
   constexpr uint32_t kLoadBytes = kQRows * 128 + 2 * NK * 128;
   extern __shared__ uint8_t smem_raw[];
   const uint32_t raw = smem_u32(smem_raw);
@@ -354,15 +360,16 @@ struct aig_mha_plan {
   aig_ctx* ctx = nullptr;
   int B = 0, T = 0, E = 0, heads = 0, d = 0, window = 0;
   float rope_base = 0.f;
-  aig_conv_plan *pq = nullptr, *pk = nullptr, *pv = nullptr, *po = nullptr;       // full sequence (rows B*T)
+  aig_conv_plan *pqkv = nullptr, *po = nullptr;                                    // full sequence (rows B*T)
   aig_conv_plan *sq = nullptr, *sk = nullptr, *sv = nullptr, *so = nullptr;       // streaming (rows B)
-  __half *q = nullptr, *k = nullptr, *v = nullptr, *ctxbuf = nullptr;              // [B][T][E]
+  __half *qkv = nullptr, *ctxbuf = nullptr;                                        // [B][T][3E], [B][T][E]; a step's q, k, v are [B][E] each in qkv
   __half *kcache = nullptr, *vcache = nullptr;                                     // [B][window][E]
   float2* rope = nullptr;
   CUtensorMap mq{}, mk{}, mv{};
   bool weights_set = false;
   int stream_start = -1;  // first position appended since the last reset
   int ring = 0;           // slots in the ring cache
+  int rope_pos0 = -1;     // first position of the table in `rope` (-1: none)
 };
 
 namespace {
@@ -371,7 +378,7 @@ int encode_qkv(aig_mha_plan* pl, CUtensorMap* m, const void* ptr, int box_rows) 
   EncodeTiledFn enc = encode_fn();
   if (!enc) return aig_fail(pl->ctx, AIG_ERR_CUDA, "cuTensorMapEncodeTiled entry point not available");
   cuuint64_t dims[3] = {(cuuint64_t)pl->E, (cuuint64_t)pl->T, (cuuint64_t)pl->B};
-  cuuint64_t strides[2] = {(cuuint64_t)pl->E * 2, (cuuint64_t)pl->T * pl->E * 2};
+  cuuint64_t strides[2] = {(cuuint64_t)pl->E * 6, (cuuint64_t)pl->T * pl->E * 6};
   cuuint32_t box[3] = {64, (cuuint32_t)box_rows, 1};
   cuuint32_t es[3] = {1, 1, 1};
   CUresult r = enc(m, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 3, const_cast<void*>(ptr), dims, strides, box, es, CU_TENSOR_MAP_INTERLEAVE_NONE,
@@ -387,7 +394,7 @@ int launch_attention(aig_mha_plan* pl, const AttnParams& prm) {
   const size_t smem = (size_t)kQRows * 128 + 2 * NK * 128 + kKB * 64 * 128 + kKB * kQRows * 128 + 1024 + 128;
   AIG_CUDA_OK(ctx, cudaFuncSetAttribute(attention_tile_kernel<NK>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   const int items = pl->B * pl->heads;
-  const int grid = items < ctx->sm_count ? items : ctx->sm_count;
+  const int grid = items < kAttnCtas<NK> * ctx->sm_count ? items : kAttnCtas<NK> * ctx->sm_count;
   attention_tile_kernel<NK><<<grid, kThreads, smem, ctx->stream>>>(pl->mq, pl->mk, pl->mv, prm);
   AIG_LAUNCH_OK(ctx);
   return AIG_OK;
@@ -409,21 +416,20 @@ int aig_mha_plan_create(aig_ctx* ctx, int batch, int seq_len, int embed, int hea
   pl->B = batch; pl->T = seq_len; pl->E = embed; pl->heads = heads; pl->d = kD; pl->window = window; pl->rope_base = rope_base;
   pl->ring = window > 0 ? window : seq_len;
   int rc = AIG_OK;
-  aig_conv_plan** full[4] = {&pl->pq, &pl->pk, &pl->pv, &pl->po};
   aig_conv_plan** step[4] = {&pl->sq, &pl->sk, &pl->sv, &pl->so};
-  for (int i = 0; i < 4 && rc == AIG_OK; ++i) rc = aig_fc_plan_create(ctx, batch * seq_len, embed, embed, AIG_ACT_NONE, 0.f, 1, full[i]);
+  rc = aig_fc_plan_create(ctx, batch * seq_len, embed, 3 * embed, AIG_ACT_NONE, 0.f, 1, &pl->pqkv);
+  if (rc == AIG_OK) rc = aig_fc_plan_create(ctx, batch * seq_len, embed, embed, AIG_ACT_NONE, 0.f, 1, &pl->po);
   for (int i = 0; i < 4 && rc == AIG_OK; ++i) rc = aig_fc_plan_create(ctx, batch, embed, embed, AIG_ACT_NONE, 0.f, 1, step[i]);
   const size_t n = (size_t)batch * seq_len * embed;
-  if (rc == AIG_OK && (cudaMalloc(&pl->q, n * 2) != cudaSuccess || cudaMalloc(&pl->k, n * 2) != cudaSuccess ||
-                       cudaMalloc(&pl->v, n * 2) != cudaSuccess || cudaMalloc(&pl->ctxbuf, n * 2) != cudaSuccess ||
+  if (rc == AIG_OK && (cudaMalloc(&pl->qkv, 3 * n * 2) != cudaSuccess || cudaMalloc(&pl->ctxbuf, n * 2) != cudaSuccess ||
                        cudaMalloc(&pl->kcache, (size_t)batch * pl->ring * embed * 2) != cudaSuccess ||
                        cudaMalloc(&pl->vcache, (size_t)batch * pl->ring * embed * 2) != cudaSuccess ||
                        cudaMalloc(&pl->rope, (size_t)seq_len * (kD / 2) * sizeof(float2)) != cudaSuccess))
     rc = aig_fail(ctx, AIG_ERR_CUDA, "mha plan: device allocation failed");
   const int nk = seq_len <= 64 ? 64 : 128;
-  if (rc == AIG_OK) rc = encode_qkv(pl, &pl->mq, pl->q, kQRows);
-  if (rc == AIG_OK) rc = encode_qkv(pl, &pl->mk, pl->k, nk);
-  if (rc == AIG_OK) rc = encode_qkv(pl, &pl->mv, pl->v, nk);
+  if (rc == AIG_OK) rc = encode_qkv(pl, &pl->mq, pl->qkv, kQRows);
+  if (rc == AIG_OK) rc = encode_qkv(pl, &pl->mk, pl->qkv + embed, nk);
+  if (rc == AIG_OK) rc = encode_qkv(pl, &pl->mv, pl->qkv + 2 * embed, nk);
   if (rc != AIG_OK) {
     aig_mha_plan_destroy(pl);
     return rc;
@@ -436,11 +442,9 @@ int aig_mha_plan_destroy(aig_mha_plan* pl) {
   if (!pl) return AIG_OK;
   DeviceGuard g(pl->ctx->device);
   cudaStreamSynchronize(pl->ctx->stream);
-  aig_conv_plan* plans[8] = {pl->pq, pl->pk, pl->pv, pl->po, pl->sq, pl->sk, pl->sv, pl->so};
+  aig_conv_plan* plans[6] = {pl->pqkv, pl->po, pl->sq, pl->sk, pl->sv, pl->so};
   for (aig_conv_plan* p : plans) aig_conv_plan_destroy(p);
-  cudaFree(pl->q);
-  cudaFree(pl->k);
-  cudaFree(pl->v);
+  cudaFree(pl->qkv);
   cudaFree(pl->ctxbuf);
   cudaFree(pl->kcache);
   cudaFree(pl->vcache);
@@ -454,13 +458,15 @@ int aig_mha_plan_set_weights(aig_mha_plan* pl, const aig_half* wq, const aig_hal
   aig_ctx* ctx = pl->ctx;
   AIG_REQUIRE(ctx, wq && wk && wv && wo, "mha set_weights: null pointer");
   const aig_half* w[4] = {wq, wk, wv, wo};
-  aig_conv_plan* full[4] = {pl->pq, pl->pk, pl->pv, pl->po};
   aig_conv_plan* step[4] = {pl->sq, pl->sk, pl->sv, pl->so};
   for (int i = 0; i < 4; ++i) {
-    int rc = aig_fc_plan_set_weights(full[i], w[i], nullptr, nullptr, nullptr, nullptr, nullptr, 0.f);
+    int rc = i < 3 ? fc_plan_pack_columns(pl->pqkv, w[i], pl->E, i * pl->E)
+                   : aig_fc_plan_set_weights(pl->po, w[i], nullptr, nullptr, nullptr, nullptr, nullptr, 0.f);
     if (rc == AIG_OK) rc = aig_fc_plan_set_weights(step[i], w[i], nullptr, nullptr, nullptr, nullptr, nullptr, 0.f);
     if (rc != AIG_OK) return rc;
   }
+  const int rc = fc_plan_identity_affine(pl->pqkv);
+  if (rc != AIG_OK) return rc;
   pl->weights_set = true;
   return AIG_OK;
 }
@@ -471,9 +477,7 @@ int aig_mha_forward(aig_mha_plan* pl, const aig_half* x, aig_half* y, int pos0) 
   DeviceGuard g(ctx->device);
   AIG_REQUIRE(ctx, x && y && pl->weights_set, "mha forward: null pointer or weights not set");
   int rc;
-  if ((rc = aig_conv_forward(pl->pq, x, nullptr, (aig_half*)pl->q)) != AIG_OK) return rc;
-  if ((rc = aig_conv_forward(pl->pk, x, nullptr, (aig_half*)pl->k)) != AIG_OK) return rc;
-  if ((rc = aig_conv_forward(pl->pv, x, nullptr, (aig_half*)pl->v)) != AIG_OK) return rc;
+  if ((rc = aig_conv_forward(pl->pqkv, x, nullptr, (aig_half*)pl->qkv)) != AIG_OK) return rc;
   AttnParams prm{};
   prm.B = pl->B; prm.T = pl->T; prm.E = pl->E; prm.heads = pl->heads; prm.window = pl->window;
   prm.scale = 1.0f / sqrtf((float)pl->d);
@@ -481,9 +485,15 @@ int aig_mha_forward(aig_mha_plan* pl, const aig_half* x, aig_half* y, int pos0) 
   prm.gerr = ctx->d_err;
   prm.rope = nullptr;
   if (pl->rope_base > 0.f) {
+    // the table of these positions is kept (a capture records its making: the graph may run before anything else does)
+    cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;
+    AIG_CUDA_OK(ctx, cudaStreamIsCapturing(ctx->stream, &capturing));
     const int n = pl->T * (kD / 2);
-    rope_table_kernel<<<ceil_div(n, 128), 128, 0, ctx->stream>>>(pl->rope, pl->T, kD / 2, kD, pl->rope_base, pos0);
-    AIG_LAUNCH_OK(ctx);
+    if (pl->rope_pos0 != pos0 || capturing != cudaStreamCaptureStatusNone) {
+      pl->rope_pos0 = capturing == cudaStreamCaptureStatusNone ? pos0 : -1;
+      rope_table_kernel<<<ceil_div(n, 128), 128, 0, ctx->stream>>>(pl->rope, pl->T, kD / 2, kD, pl->rope_base, pos0);
+      AIG_LAUNCH_OK(ctx);
+    }
     prm.rope = pl->rope;
   }
   rc = pl->T <= 64 ? launch_attention<64>(pl, prm) : launch_attention<128>(pl, prm);
@@ -507,15 +517,16 @@ int aig_mha_step(aig_mha_plan* pl, const aig_half* x, aig_half* y, int position)
   int n_valid = position - pl->stream_start + 1;
   if (n_valid > pl->ring) n_valid = pl->ring;
   int rc;
-  // the per-step projections reuse the head of the sequence buffers: [B][E]
-  if ((rc = aig_conv_forward(pl->sq, x, nullptr, (aig_half*)pl->q)) != AIG_OK) return rc;
-  if ((rc = aig_conv_forward(pl->sk, x, nullptr, (aig_half*)pl->k)) != AIG_OK) return rc;
-  if ((rc = aig_conv_forward(pl->sv, x, nullptr, (aig_half*)pl->v)) != AIG_OK) return rc;
+  // the per-step projections reuse the head of the sequence buffer: [B][E] each
+  __half *q = pl->qkv, *k = q + (size_t)pl->B * pl->E, *v = k + (size_t)pl->B * pl->E;
+  if ((rc = aig_conv_forward(pl->sq, x, nullptr, (aig_half*)q)) != AIG_OK) return rc;
+  if ((rc = aig_conv_forward(pl->sk, x, nullptr, (aig_half*)k)) != AIG_OK) return rc;
+  if ((rc = aig_conv_forward(pl->sv, x, nullptr, (aig_half*)v)) != AIG_OK) return rc;
   const int warps = 4;
   const int items = pl->B * pl->heads;
   const size_t smem = (size_t)warps * (pl->d + pl->ring) * sizeof(float);
   attention_step_kernel<<<ceil_div(items, warps), warps * 32, smem, ctx->stream>>>(
-      pl->q, pl->k, pl->v, pl->kcache, pl->vcache, pl->ctxbuf, pl->B, pl->E, pl->heads, pl->d, pl->ring, position, n_valid,
+      q, k, v, pl->kcache, pl->vcache, pl->ctxbuf, pl->B, pl->E, pl->heads, pl->d, pl->ring, position, n_valid,
       pl->rope_base, 1.0f / sqrtf((float)pl->d));
   AIG_LAUNCH_OK(ctx);
   return aig_conv_forward(pl->so, (const aig_half*)pl->ctxbuf, nullptr, y);
