@@ -3,6 +3,9 @@
 // attention (reference mode and mask mode), pooling.  All are 128-bit vectorised where the
 // pointer/extent alignment allows and sized as grid-stride loops over a multiple of the SM count.
 #include "aig_common.cuh"
+#include "seq_step.h"
+
+#include <algorithm>
 
 namespace {
 
@@ -624,7 +627,136 @@ __global__ void cnn_head_kernel(const __half* x, const __half* __restrict__ w1, 
   }
 }
 
+// Row LayerNorm, FC, sigmoid / tanh of the sequence head.  As separate launches (row LayerNorm, a GEMM of one 32-wide
+// column tile, two in-place activations, a conversion) 8192 rows of 512 took 28 us, three times through memory, and 111
+// rows of 256 took 22 us, all launches.  A warp takes 16 rows: they stay in registers in the layout of mma.sync's A operand
+// (a lane has 16-byte pieces of two rows), the row sums are two shuffles, the product with the few output columns is
+// three to four mma tiles.  Bound by the one read of x.
+constexpr int kTailBlocks = 16, kTailTiles = 4, kTailWarps = 4;
+__global__ void __launch_bounds__(kTailWarps * 32) seq_tail_kernel(const __half* x, const float* __restrict__ gamma, const float* __restrict__ beta,
+                                                                   const __half* __restrict__ fcw, const __half* __restrict__ fcb, __half* out_h, float* out_f,
+                                                                   int rows, int C, int n_out, int n_sig, float eps) {
+  extern __shared__ __align__(16) uint8_t tail_smem[];
+  const int stride = C + 8;                                       // halfs: rows of the weights on different banks
+  float* s_g = reinterpret_cast<float*>(tail_smem);               // gamma, beta
+  float* s_b = s_g + C;
+  __half* s_w = reinterpret_cast<__half*>(s_b + C);               // [tiles * 8][C]
+  const int tid = threadIdx.x, lane = tid & 31, g = lane >> 2, q = lane & 3, nb = C / 32, tiles = (n_out + 7) / 8;
+  for (int i = tid; i < C; i += blockDim.x) {
+    s_g[i] = gamma[i];
+    s_b[i] = beta[i];
+  }
+#pragma unroll 4
+  for (int i = tid * 8; i < n_out * C; i += blockDim.x * 8) {  // [C][n_out], eight at a time
+    const uint4 w8 = *reinterpret_cast<const uint4*>(fcw + i);
+    int k = i / n_out, o = i - k * n_out;
+#pragma unroll
+    for (int e = 0; e < 8; ++e) {
+      s_w[o * stride + k] = reinterpret_cast<const __half*>(&w8)[e];
+      if (++o == n_out) { o = 0; ++k; }
+    }
+  }
+  for (int i = tid; i < (tiles * 8 - n_out) * C; i += blockDim.x) s_w[(n_out + i / C) * stride + i % C] = __float2half(0.f);
+  griddep_launch_dependents();
+  griddep_wait();
+  __syncthreads();
+  for (int r0 = (blockIdx.x * kTailWarps + (tid >> 5)) * 16; r0 < rows; r0 += gridDim.x * kTailWarps * 16) {
+    uint4 v[2][kTailBlocks];
+    float mu[2], rstd[2];
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      const int r = min(r0 + g + 8 * h, rows - 1);
+      const uint4* src = reinterpret_cast<const uint4*>(x + (size_t)r * C) + q;
+#pragma unroll
+      for (int kb = 0; kb < kTailBlocks; ++kb) v[h][kb] = kb < nb ? src[kb * 4] : make_uint4(0, 0, 0, 0);
+    }
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      float s = 0.f, ss = 0.f;
+#pragma unroll
+      for (int kb = 0; kb < kTailBlocks; ++kb)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          const float2 f = __half22float2(reinterpret_cast<const __half2*>(&v[h][kb])[e]);
+          s += f.x + f.y;
+        }
+      s += __shfl_xor_sync(0xffffffffu, s, 1);
+      s += __shfl_xor_sync(0xffffffffu, s, 2);
+      mu[h] = s / (float)C;
+#pragma unroll
+      for (int kb = 0; kb < kTailBlocks; ++kb)
+        if (kb < nb)
+#pragma unroll
+          for (int e = 0; e < 4; ++e) {
+            const float2 f = __half22float2(reinterpret_cast<const __half2*>(&v[h][kb])[e]);
+            ss += (f.x - mu[h]) * (f.x - mu[h]) + (f.y - mu[h]) * (f.y - mu[h]);
+          }
+      ss += __shfl_xor_sync(0xffffffffu, ss, 1);
+      ss += __shfl_xor_sync(0xffffffffu, ss, 2);
+      rstd[h] = rsqrtf(ss / (float)C + eps);
+    }
+    float acc[kTailTiles][4];
+#pragma unroll
+    for (int t = 0; t < kTailTiles; ++t) acc[t][0] = acc[t][1] = acc[t][2] = acc[t][3] = 0.f;
+#pragma unroll
+    for (int kb = 0; kb < kTailBlocks; ++kb) {
+      if (kb >= nb) break;
+      const int k0 = kb * 32 + q * 8;
+      float gm[8], bt[8];
+#pragma unroll
+      for (int e = 0; e < 8; e += 4) {
+        *reinterpret_cast<float4*>(gm + e) = *reinterpret_cast<const float4*>(s_g + k0 + e);
+        *reinterpret_cast<float4*>(bt + e) = *reinterpret_cast<const float4*>(s_b + k0 + e);
+      }
+      uint32_t a[2][4];
+#pragma unroll
+      for (int h = 0; h < 2; ++h)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          const float2 f = __half22float2(reinterpret_cast<const __half2*>(&v[h][kb])[e]);
+          const __half2 n = __floats2half2_rn((f.x - mu[h]) * rstd[h] * gm[2 * e] + bt[2 * e], (f.y - mu[h]) * rstd[h] * gm[2 * e + 1] + bt[2 * e + 1]);
+          a[h][e] = *reinterpret_cast<const uint32_t*>(&n);
+        }
+#pragma unroll
+      for (int t = 0; t < kTailTiles; ++t) {
+        if (t >= tiles) break;
+        const uint4 w = *reinterpret_cast<const uint4*>(s_w + (t * 8 + g) * stride + k0);
+        // (the two steps of a 32-deep block take a lane's 16 bytes as their k: the order of k is free)
+        asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+                     : "+f"(acc[t][0]), "+f"(acc[t][1]), "+f"(acc[t][2]), "+f"(acc[t][3])
+                     : "r"(a[0][0]), "r"(a[1][0]), "r"(a[0][1]), "r"(a[1][1]), "r"(w.x), "r"(w.y));
+        asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+                     : "+f"(acc[t][0]), "+f"(acc[t][1]), "+f"(acc[t][2]), "+f"(acc[t][3])
+                     : "r"(a[0][2]), "r"(a[1][2]), "r"(a[0][3]), "r"(a[1][3]), "r"(w.z), "r"(w.w));
+      }
+    }
+#pragma unroll
+    for (int t = 0; t < kTailTiles; ++t)
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        const int r = r0 + g + 8 * (e >> 1), o = t * 8 + 2 * q + (e & 1);
+        if (t >= tiles || r >= rows || o >= n_out) continue;
+        const float s = __half2float(__float2half(acc[t][e]));                  // FCLayer: GEMM result stored as half,
+        const float y = __half2float(__float2half(s + __half2float(fcb[o])));   // then bias added and stored again
+        const __half hv = __float2half(o < n_sig ? 1.0f / (1.0f + expf(-y)) : tanhf(y));
+        out_h[(size_t)r * n_out + o] = hv;
+        out_f[(size_t)r * n_out + o] = __half2float(hv);
+      }
+  }
+}
+
 }  // namespace
+
+bool seq_tail_supported(int c, int n_out) { return c % 32 == 0 && c <= 32 * kTailBlocks && n_out >= 1 && n_out <= 8 * kTailTiles; }
+int seq_tail_forward(aig_ctx* ctx, const aig_half* x, const float* gamma, const float* beta, const aig_half* fc_w, const aig_half* fc_b, aig_half* out_half,
+                     float* out_f32, int rows, int c, int n_out, int n_sigmoid, float eps) {
+  DeviceGuard guard(ctx->device);
+  const size_t smem = (size_t)c * 8 + (size_t)(n_out + 7) / 8 * 8 * (c + 8) * 2;
+  const int grid = std::min((rows + 16 * kTailWarps - 1) / (16 * kTailWarps), 2 * ctx->sm_count);
+  AIG_CUDA_OK(ctx, launch_pdl(seq_tail_kernel, dim3(grid), dim3(kTailWarps * 32), smem, ctx->stream, (const __half*)x, gamma, beta, (const __half*)fc_w,
+                              (const __half*)fc_b, (__half*)out_half, out_f32, rows, c, n_out, n_sigmoid, eps));
+  return AIG_OK;
+}
 
 // ============================================================================================
 extern "C" {

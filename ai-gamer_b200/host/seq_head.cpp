@@ -161,6 +161,10 @@ int aig_seq_load_memory(aig_seq* m, const void* blob, size_t bytes) {
 
 static int seq_tail(aig_seq* m, aig_conv_plan* fc, int rows) {
   const aig_seq_config& c = m->cfg;
+  if (seq_tail_supported(c.hidden, c.n_out)) {
+    SEQ_OK(m, seq_tail_forward(m->ctx, m->a, m->ln_g, m->ln_b, m->fcw, m->fcb, m->logits, m->out_f32, rows, c.hidden, c.n_out, c.n_sigmoid, 1e-5f));
+    return AIG_OK;
+  }
   SEQ_OK(m, aig_layernorm_rows_forward(m->ctx, m->n, m->a, m->ln_g, m->ln_b, rows, c.hidden, 1e-5f));
   SEQ_OK(m, aig_conv_forward(fc, m->n, nullptr, m->logits));
   SEQ_OK(m, aig_sigmoid_forward(m->ctx, m->logits, c.n_out, c.n_sigmoid, rows * c.n_out));
