@@ -501,7 +501,8 @@ __global__ void __launch_bounds__(kThreads, 1) res_chain_kernel(const __grid_con
     int acc = 0, split_jobs = 0, free_jobs[2] = {0, 0}, jobs = 0;
     uint32_t aph = 0;
     bool ok = true;
-    if ((int)blockIdx.x < p.batch) {
+    const bool with_head = p.head.hw > 0;
+    if (with_head && (int)blockIdx.x < p.batch) {
       const int n_fc = p.head.c * p.head.n_out;
       for (int i = tid; i < n_fc / 8; i += 128) reinterpret_cast<uint4*>(s_head)[i] = __ldg(reinterpret_cast<const uint4*>(p.head.fc_w) + i);
       for (int i = tid; i < p.head.c; i += 128) s_head[n_fc + i] = reinterpret_cast<const __half*>(p.head.mask_w)[i];
@@ -591,7 +592,7 @@ __global__ void __launch_bounds__(kThreads, 1) res_chain_kernel(const __grid_con
       named_bar_sync(1, 128);
       if (tid == 0) red_release_gpu_add(counters + si, 1u);
     }
-    if (ok && (int)blockIdx.x < p.batch) {
+    if (ok && with_head && (int)blockIdx.x < p.batch) {
       // ---------------------------------------------------------------- head (patches and ring are free by now)
       const int last = p.n_stages - 1;
       __half* sx = reinterpret_cast<__half*>(sm);

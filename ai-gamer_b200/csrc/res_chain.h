@@ -27,7 +27,7 @@ struct ResChainBlock {
   aig_conv_plan *down, *conv1;
   aig_half *in, *t, *r, *y;  // block input (space-to-depth), the pair's outputs (padded layout), block output
 };
-struct ResChainHead {        // as aig_cnn_head_forward
+struct ResChainHead {        // as aig_cnn_head_forward; hw = 0: no head
   const aig_half *mask_w, *fc_w, *fc_b;
   float mask_b;
   aig_half *feat, *out_half;
@@ -36,7 +36,7 @@ struct ResChainHead {        // as aig_cnn_head_forward
 };
 struct ResChain;
 // *out stays null (and the call succeeds) where the per-layer launches are the better or the only choice.
-// hw, c_last, n_out: positions and channels of the last block's output, outputs of the head.
+// hw, c_last, n_out: positions and channels of the last block's output, outputs of the head (0: none).
 int res_chain_create(aig_ctx* ctx, const std::vector<ResChainBlock>& blocks, int hw, int c_last, int n_out, ResChain** out);
 void res_chain_destroy(ResChain* c);
 int res_chain_forward(ResChain* c, const ResChainHead& head);

@@ -4,6 +4,8 @@
 #include "Layers.h"
 
 #include "aig_compat.h"
+#include "res_chain.h"
+#include "skinny_fc.h"
 
 #include <string.h>
 
@@ -97,6 +99,7 @@ ConvLayer::~ConvLayer() {
   cudaFree(weights_); cudaFree(bias_); cudaFree(outData_); cudaFree(nhwcIn_); cudaFree(nhwcOut_);
 }
 void ConvLayer::SyncWeights() {
+  ++paramVersion_;
   if (plan0_) check(ctx_, aig_conv0_plan_set_weights(plan0_, H(weights_), H(bias_), nullptr, nullptr, nullptr, nullptr, 0.f), layerName_);
   else check(ctx_, aig_conv_plan_set_weights(plan_, H(weights_), H(bias_), nullptr, nullptr, nullptr, nullptr, 0.f), layerName_);
 }
@@ -209,6 +212,7 @@ __half* BatchNorm::Forward(__half* data) {
 void BatchNorm::LoadParameters(std::ifstream& file, unsigned char* buffer) {
   float* arrays[6] = {bnScale_, bnBias_, bnRunningMean_, bnRunningVar_, bnSavedMean_, bnSavedInvVariance_};
   for (float* a : arrays) loadArray(file, buffer, a, paramCount_ * sizeof(float));
+  SyncWeights();
 }
 void BatchNorm::SaveParameters(std::ofstream& file, unsigned char* buffer) {
   float* arrays[6] = {bnScale_, bnBias_, bnRunningMean_, bnRunningVar_, bnSavedMean_, bnSavedInvVariance_};
@@ -294,6 +298,7 @@ FCLayer::~FCLayer() {
   cudaFree(m_Weights_); cudaFree(v_Weights_); cudaFree(m_Bias_); cudaFree(v_Bias_);
 }
 void FCLayer::SyncWeights() {
+  ++paramVersion_;
   check(ctx_, aig_fc_plan_set_weights(plan_, H(weights_), H(bias_), nullptr, nullptr, nullptr, nullptr, 0.f), layerName_);
 }
 __half* FCLayer::Forward(__half* data) {
@@ -537,6 +542,134 @@ void MultiHeadAttentionLayer::SaveParameters(std::ofstream& file, unsigned char*
 }
 
 // ------------------------------------------------------------------------------------------ NN
+// The network's inference as six launches: first convolution with BatchNorm and ReLU, the three residual blocks as one
+// chain, and the four FC layers with what follows them.  The layers one after another are 59 launches of 3 to 20 us with
+// a change of layout around every convolution (a 144x256 frame: 672 us, of them 318 in the first FC layer; 118 now).
+// BatchNorm is folded into the convolutions (one rounding where the layers make three); the FC layers round as the layers do.
+struct NN::Inference {
+  struct Block {
+    aig_conv_plan *down = nullptr, *conv1 = nullptr;
+    __half *t = nullptr, *r = nullptr, *y = nullptr;
+  };
+  aig_ctx* ctx;
+  std::vector<Layer*> layers;
+  aig_conv0_plan* conv0 = nullptr;
+  std::vector<Block> blocks;
+  ResChain* chain = nullptr;
+  aig_conv_plan* fc0 = nullptr;  // reads the last block's output as it is: (position, channel)
+  __half *act0 = nullptr, *hidden[3] = {nullptr, nullptr, nullptr};
+  int hw = 0;
+  unsigned version = 0;
+
+  explicit Inference(aig_ctx* c, const std::vector<Layer*>& l) : ctx(c), layers(l) {}
+  ~Inference() {
+    aig_ctx_sync(ctx);
+    aig_conv0_plan_destroy(conv0);
+    res_chain_destroy(chain);
+    for (Block& b : blocks) {
+      aig_conv_plan_destroy(b.down);
+      aig_conv_plan_destroy(b.conv1);
+      cudaFree(b.t); cudaFree(b.r); cudaFree(b.y);
+    }
+    aig_conv_plan_destroy(fc0);
+    cudaFree(act0);
+    for (__half* h : hidden) cudaFree(h);
+  }
+  template <class T>
+  T* layer(int i) const { return static_cast<T*>(layers[i]); }
+  ResConvLayer* res(int i) const { return layer<ResConvLayer>(3 + i); }
+
+  unsigned currentVersion() const {
+    unsigned v = 0;
+    for (Layer* l : layers) v += l->paramVersion_;
+    for (int i = 0; i < 3; ++i) {
+      for (Layer* l : res(i)->layers_) v += l->paramVersion_;
+      v += res(i)->residue_->paramVersion_;
+    }
+    return v;
+  }
+  // false: some part does not cover this frame size
+  bool create(int width, int height) {
+    const int widths[4] = {32, 64, 128, 256};
+    if (aig_conv0_plan_create(ctx, 1, height, width, widths[0], 2, 2, 0, AIG_ACT_RELU, 0.f, &conv0) != AIG_OK) return false;
+    int h, w;
+    aig_conv0_plan_out_dims(conv0, nullptr, &h, &w);
+    if (h < 2 || w < 2 || aig_conv0_plan_set_output_s2d(conv0, 1) != AIG_OK) return false;
+    mallocZero(&act0, aig_s2d_elems(1, h, w, widths[0]));
+    std::vector<ResChainBlock> chained;
+    __half* in = act0;
+    for (int i = 0; i < 3; ++i) {
+      blocks.emplace_back();
+      Block& b = blocks.back();
+      const int ci = widths[i], co = widths[i + 1];
+      int oh, ow;
+      if (h < 2 || w < 2 || aig_resdown_plan_create(ctx, 1, ci, h, w, co, AIG_ACT_RELU, 0.f, &b.down) != AIG_OK) return false;
+      aig_conv_plan_out_dims(b.down, nullptr, &oh, &ow);
+      aig_conv_desc d{};
+      d.batch = 1; d.in_c = co; d.in_d = 1; d.in_h = oh; d.in_w = ow; d.out_c = co;
+      d.kd = 1; d.kh = d.kw = 3; d.sd = d.sh = d.sw = 1; d.pd = 0; d.ph = d.pw = 1; d.act = AIG_ACT_RELU;
+      const bool last = i == 2;
+      if (aig_conv_plan_create(ctx, &d, &b.conv1) != AIG_OK || aig_resdown_plan_set_output_padded(b.down, 1) != AIG_OK ||
+          aig_conv_plan_set_input_padded(b.conv1, 1) != AIG_OK || (!last && aig_conv_plan_set_output_s2d(b.conv1, 1) != AIG_OK))
+        return false;
+      const size_t rows = (size_t)aig_conv_padded_rows(1, oh, ow, 1);
+      mallocZero(&b.t, rows * co);
+      mallocZero(&b.r, rows * co);
+      mallocZero(&b.y, last ? (size_t)oh * ow * co : aig_s2d_elems(1, oh, ow, co));
+      chained.push_back(ResChainBlock{b.down, b.conv1, H(in), H(b.t), H(b.r), H(b.y)});
+      in = b.y;
+      h = oh;
+      w = ow;
+    }
+    hw = h * w;
+    if (res_chain_create(ctx, chained, 0, 0, 0, &chain) != AIG_OK || !chain) return false;
+    if (aig_fc_plan_create(ctx, 1, widths[3] * hw, layer<FCLayer>(6)->outC_, AIG_ACT_NONE, 0.f, 1, &fc0) != AIG_OK) return false;
+    for (int i = 0; i < 3; ++i) mallocZero(&hidden[i], (size_t)layer<FCLayer>(6 + 3 * i)->outC_);
+    return true;
+  }
+  void takeParameters() {
+    const float eps = 1e-6f;  // BatchNorm.cpp:5
+    ConvLayer* c0 = layer<ConvLayer>(0);
+    BatchNorm* n0 = layer<BatchNorm>(1);
+    check(ctx, aig_conv0_plan_set_weights(conv0, H(c0->weights_), H(c0->bias_), n0->bnScale_, n0->bnBias_, n0->bnRunningMean_, n0->bnRunningVar_, eps), "NN");
+    for (int i = 0; i < 3; ++i) {
+      ResConvLayer* r = res(i);
+      ConvLayer *a = static_cast<ConvLayer*>(r->layers_[0]), *b = static_cast<ConvLayer*>(r->layers_[3]), *s = r->residue_;
+      BatchNorm *na = static_cast<BatchNorm*>(r->layers_[1]), *nb = static_cast<BatchNorm*>(r->layers_[4]);
+      check(ctx, aig_resdown_plan_set_weights(blocks[i].down, H(a->weights_), H(a->bias_), na->bnScale_, na->bnBias_, na->bnRunningMean_,
+                                              na->bnRunningVar_, eps, H(s->weights_), H(s->bias_)), "NN");
+      check(ctx, aig_conv_plan_set_weights(blocks[i].conv1, H(b->weights_), H(b->bias_), nb->bnScale_, nb->bnBias_, nb->bnRunningMean_,
+                                           nb->bnRunningVar_, eps), "NN");
+    }
+    FCLayer* f = layer<FCLayer>(6);
+    check(ctx, fc_plan_set_weights_nhwc(fc0, H(f->weights_), H(f->bias_), 256, hw), "NN");
+    version = currentVersion();
+  }
+  __half* forward(__half* data) {
+    if (version != currentVersion()) takeParameters();
+    check(ctx, aig_conv0_forward_nchw(conv0, H(data), H(act0)), "NN");
+    check(ctx, res_chain_forward(chain, ResChainHead{}), "NN");
+    const __half* x = blocks.back().y;
+    for (int i = 0; i < 4; ++i) {
+      FCLayer* f = layer<FCLayer>(6 + 3 * i);
+      FcTail tail;
+      __half* y = f->outData_;
+      if (i < 3) {
+        BatchNorm* n = layer<BatchNorm>(7 + 3 * i);
+        tail.gamma = n->bnScale_; tail.beta = n->bnBias_; tail.mean = n->bnRunningMean_; tail.var = n->bnRunningVar_;
+        tail.eps = 1e-6f;
+        tail.relu = 1;
+        y = hidden[i];
+      } else {
+        tail.n_sigmoid = numButs_;  // in place on the FC's output, as Sigmoid.cpp:8-12
+      }
+      check(ctx, fc_plan_forward_tail(i == 0 ? fc0 : f->plan(), H(x), H(y), tail), "NN");
+      x = y;
+    }
+    return layer<FCLayer>(15)->outData_;
+  }
+};
+
 NN::NN(cudnnHandle_t cudnnHandle, cublasHandle_t cublasHandle, int w, int h, bool train, const std::string& ckptFileName)
     : cudnn_(cudnnHandle), cublas_(cublasHandle), batchSize_(40), seqLength_(1), inWidth_(0), inHeight_(0), maxBufferSize_(0) {
   if (!train) batchSize_ = 1;  // NN.cpp:12
@@ -584,11 +717,23 @@ NN::NN(cudnnHandle_t cudnnHandle, cublasHandle_t cublasHandle, int w, int h, boo
     }
     cudaFreeHost(buffer);
   }
+  if (!train) {
+    fused_ = new Inference(cudnn_, layers_);
+    if (fused_->create(inWidth_, inHeight_)) {
+      fused_->takeParameters();
+    } else {
+      cudaGetLastError();
+      delete fused_;
+      fused_ = nullptr;
+    }
+  }
 }
 NN::~NN() {
+  delete fused_;
   for (Layer* l : layers_) delete l;
 }
 __half* NN::Forward(__half* data) {  // NN.cpp:93-100
+  if (fused_) return fused_->forward(data);
   for (Layer* layer : layers_) data = layer->Forward(data);
   return data;
 }

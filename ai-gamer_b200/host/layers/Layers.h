@@ -42,6 +42,7 @@ class Layer {
   const char* layerName_ = "";
   bool train_ = false;
   size_t weightCount_ = 0;
+  unsigned paramVersion_ = 0;  // counts what LoadParameters (and SyncWeights) brought: NN keeps a fused copy of its layers' parameters
 };
 
 // ConvLayer.h:8 / ConvLayer.cpp:4-50,74-79
@@ -97,6 +98,7 @@ class BatchNorm final : public Layer {
   void LoadParameters(std::ifstream& file, unsigned char* buffer) override;
   void SaveParameters(std::ofstream& file, unsigned char* buffer) override;
   size_t GetParameterSize() override { return 6 * paramCount_ * sizeof(float); }
+  void SyncWeights() { ++paramVersion_; }
   float *bnScale_ = nullptr, *bnBias_ = nullptr, *bnRunningMean_ = nullptr, *bnRunningVar_ = nullptr, *bnSavedMean_ = nullptr,
         *bnSavedInvVariance_ = nullptr;
   __half* outData_ = nullptr;
@@ -159,6 +161,7 @@ class FCLayer final : public Layer {
   void LoadOptimizerState(std::ifstream& file, unsigned char* buffer) override;
   size_t GetOptimizerStateSize() override { return weightCount_ * sizeof(__half); }
   void SyncWeights();
+  aig_conv_plan* plan() const { return plan_; }
   __half *weights_ = nullptr, *bias_ = nullptr, *outData_ = nullptr;
   __half *gradOut_ = nullptr, *gradWeights_ = nullptr, *gradBias_ = nullptr;
   __half *m_Weights_ = nullptr, *v_Weights_ = nullptr, *m_Bias_ = nullptr, *v_Bias_ = nullptr;
@@ -288,6 +291,9 @@ class Dropout final : public Layer {
 
 // NN.h / NN.cpp:11-100: the network the reference builds (Conv k2 s2 + BN + ReLU, three ResConv blocks, three
 // FC+BN+ReLU, FC(16), Sigmoid(14)).  The checkpoint path is an argument instead of a fixed drive letter.
+// At inference (train = false) Forward runs the network as six fused launches made from the layers' parameters instead of
+// the 59 of the layers one after another; the layers stay and can be called one by one.  Parameters that change through
+// LoadParameters or SyncWeights are noticed; a caller that writes a BatchNorm's device arrays itself calls its SyncWeights.
 class NN {
  public:
   NN(cudnnHandle_t cudnnHandle, cublasHandle_t cublasHandle, int w, int h, bool train, const std::string& ckptFile);
@@ -298,6 +304,10 @@ class NN {
   std::vector<Layer*> layers_;
   int batchSize_, seqLength_, inWidth_, inHeight_;
   size_t maxBufferSize_;
+
+ private:
+  struct Inference;
+  Inference* fused_ = nullptr;  // null where the fused launches do not cover the frame size
 };
 
 // The context used by layers whose reference constructors take no handle (Swish, LeakyReLU, Sigmoid, LayerNorm):
