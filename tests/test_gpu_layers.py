@@ -277,3 +277,32 @@ def test_infer_loop_body_through_the_reference_names_without_synchronisation(env
         assert U.rel_err(out_host, want, 0.05).max() < 5e-3, "frame %d" % i
     lib.aig_refnn_destroy(nn)
     lib.aig_ctx_destroy(handle)
+
+
+@gpu
+@pytest.mark.parametrize("H,W", [(16, 16), (48, 64), (67, 131), (144, 256)])
+def test_reference_network_sizes(env, H, W):
+    """The reference's network in its fused launches against the oracle, from one position in the last block to 144."""
+    U = env
+    import torch
+
+    c, pk = U.ctx(), U.pkg()
+    lib = pk.lib()
+    p = PL.make_refnn_params(H, W, H)
+    x = O.preprocess_frames(np.random.default_rng(W).integers(0, 256, (1, H, W, 4), dtype=np.uint8))
+    want = PL.refnn_forward(p, x)[0].astype(np.float32)
+    with tempfile.TemporaryDirectory() as d:
+        path = os.path.join(d, "n.ckpt")
+        with open(path, "wb") as f:
+            f.write(PL.serialize_refnn_checkpoint(p))
+        nn = ctypes.c_void_p()
+        assert lib.aig_refnn_create(c.handle, 0, 0, path.encode(), ctypes.byref(nn)) == 0, lib.aig_layers_last_error().decode()
+    dx, out = U.dev(x), ctypes.c_void_p()
+    got = torch.empty(16, dtype=torch.float16, device="cuda")
+    for _ in range(2):
+        assert lib.aig_refnn_forward(nn, pk.ptr(dx), ctypes.byref(out)) == 0
+    c.call("aig_memcpy", pk.ptr(got), out, 32)
+    c.sync()
+    lib.aig_refnn_destroy(nn)
+    # BatchNorm is folded into the convolutions: one rounding where the layers one after another make three
+    assert U.rel_err(U.host(got).astype(np.float32), want, 0.2).max() < 1e-2

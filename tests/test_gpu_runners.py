@@ -176,3 +176,28 @@ def test_streaming_step_shapes(env, B, in_c, d, heads, window, layers):
         assert U.rel_err(got, want.astype(np.float32), 0.2).max() < TOL   # an output near zero: 4e-3 absolute
         head.reset()
     head.close()
+
+
+@gpu
+@pytest.mark.parametrize("B,T,d,heads,n_out", [(1, 3, 64, 1, 1), (2, 7, 192, 3, 31), (1, 65, 512, 8, 32), (3, 128, 128, 2, 18), (3, 5, 128, 2, 40)])
+def test_whole_sequences_tail_shapes(env, B, T, d, heads, n_out):
+    """LayerNorm, FC and activations in one launch: ragged groups of 16 rows, one column tile to four, more outputs than
+    it takes; widths of two to sixteen blocks of 32; attention tiles of 64 and 128 keys."""
+    U = env
+    U.pkg()
+    from ai_gamer_b200 import runners as R
+
+    p = PL.make_seq_params(B + n_out, d=d, hid=d, layers=1, heads=heads, n_out=n_out)
+    emb = PL.make_embeddings(9, T, B, d)
+    n_sig = n_out - n_out // 3
+    _, _, _, want = PL.seq_forward(p, emb, rope_base=10000.0, n_sigmoid=n_sig)
+    head = R.SeqHead(U.ctx(), B, T, in_c=d, hidden=d, layers=1, heads=heads, n_out=n_out, n_sigmoid=n_sig, rope_base=10000.0)
+    head.load_bytes(PL.serialize_seq_params(p))
+    dev = U.dev(np.ascontiguousarray(emb.transpose(1, 0, 2)))
+    head.forward(dev, 5)
+    other = U.host(head.outputs_f32())
+    head.forward(dev)
+    got = U.host(head.outputs_f32())
+    assert U.rel_err(got, want.astype(np.float32), 0.2).max() < TOL
+    assert np.abs(other - got).max() < 8e-3   # rotary attention depends on distances only; the angles round differently
+    head.close()
