@@ -304,5 +304,7 @@ def test_reference_network_sizes(env, H, W):
     c.call("aig_memcpy", pk.ptr(got), out, 32)
     c.sync()
     lib.aig_refnn_destroy(nn)
-    # BatchNorm is folded into the convolutions: one rounding where the layers one after another make three
-    assert U.rel_err(U.host(got).astype(np.float32), want, 0.2).max() < 1e-2
+    # BatchNorm is folded into the convolutions: one rounding where the layers one after another make three; those put
+    # the oracle itself up to 4e-3 from exact arithmetic at these sizes
+    got = U.host(got).astype(np.float32)
+    assert (np.abs(got - want) / np.maximum(1.0, np.abs(want))).max() < 8e-3
