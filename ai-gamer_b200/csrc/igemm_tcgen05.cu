@@ -483,12 +483,7 @@ igemm_kernel(const __grid_constant__ CUtensorMap tmapA, const __grid_constant__ 
 
   const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;  // (uniform for the compiler)
 
-  if (p.n_tiles == 1) {
-    for (int i = threadIdx.x; i < NT; i += kNumThreads) {
-      s_scale[i] = p.scale[i];
-      s_shift[i] = p.shift[i];
-    }
-  }
+  griddep_launch_dependents();
   if (threadIdx.x == 0) {
     for (int s = 0; s < kStages; ++s) {
       mbar_init(bar_full + 8 * s, 1);
@@ -506,6 +501,13 @@ igemm_kernel(const __grid_constant__ CUtensorMap tmapA, const __grid_constant__ 
   if (warp == 1) {
     tmem_alloc(smem_u32(s_tmem), Cfg::kTmemCols);
     tmem_relinquish();
+  }
+  griddep_wait();  // weights and affine may be new as well as the activations (a training step's update)
+  if (p.n_tiles == 1) {
+    for (int i = threadIdx.x; i < NT; i += kNumThreads) {
+      s_scale[i] = p.scale[i];
+      s_shift[i] = p.shift[i];
+    }
   }
   tc_fence_before();
   __syncthreads();
@@ -1478,8 +1480,7 @@ int launch_igemm(aig_conv_plan* pl) {
     AIG_CUDA_OK(ctx, cudaFuncSetAttribute(igemm_kernel<NT, BK, MS>, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::kSmemBytes));
     attr_set[ctx->device & 63] = true;
   }
-  igemm_kernel<NT, BK, MS><<<pl->grid, kNumThreads, Cfg::kSmemBytes, ctx->stream>>>(pl->tmapA, pl->tmapB, pl->prm);
-  AIG_LAUNCH_OK(ctx);
+  AIG_CUDA_OK(ctx, launch_pdl(igemm_kernel<NT, BK, MS>, dim3(pl->grid), dim3(kNumThreads), Cfg::kSmemBytes, ctx->stream, pl->tmapA, pl->tmapB, pl->prm));
   return AIG_OK;
 }
 

@@ -149,16 +149,7 @@ __global__ void __launch_bounds__(lstm_threads(G), 1) lstm_recurrent_kernel(cons
     tmem_alloc(smem_u32(s_tmem), tmem_cols);
     tmem_relinquish();
   }
-  if (working) {
-    // h_{-1}, as step -1 would have delivered it (buffer 1)
-    for (int i = threadIdx.x; i < G * h_bytes / 16; i += kThreads) {
-      const int g = i / (h_bytes / 16), k = i - g * (h_bytes / 16), chunk = k / NB, b = row0 + g * NB + k % NB;
-      uint4 v = make_uint4(0, 0, 0, 0);
-      if (p.h0 && b < p.B) v = *reinterpret_cast<const uint4*>(p.h0 + (size_t)b * p.H + chunk * 8);
-      reinterpret_cast<uint4*>(sm + g * group_bytes + h_bytes)[k] = v;
-    }
-  }
-  fence_proxy_async_smem();
+  griddep_launch_dependents();
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
@@ -175,6 +166,17 @@ __global__ void __launch_bounds__(lstm_threads(G), 1) lstm_recurrent_kernel(cons
     }
     asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
   }
+  griddep_wait();  // (R is what the plan was given at load time; the rest comes from the launches before this one)
+  if (working) {
+    // h_{-1}, as step -1 would have delivered it (buffer 1)
+    for (int i = threadIdx.x; i < G * h_bytes / 16; i += kThreads) {
+      const int g = i / (h_bytes / 16), k = i - g * (h_bytes / 16), chunk = k / NB, b = row0 + g * NB + k % NB;
+      uint4 v = make_uint4(0, 0, 0, 0);
+      if (p.h0 && b < p.B) v = *reinterpret_cast<const uint4*>(p.h0 + (size_t)b * p.H + chunk * 8);
+      reinterpret_cast<uint4*>(sm + g * group_bytes + h_bytes)[k] = v;
+    }
+  }
+  fence_proxy_async_smem();
   tc_fence_before();
   cluster_sync_all();  // barriers and R are there, and every CTA has read the initial h
   tc_fence_after();
@@ -296,17 +298,19 @@ struct LstmLaunch {
 size_t recurrent_smem(int H, int groups) { return (size_t)groups * (2 * kSeqs * (H + kUnits) * 2 + 32) + 64 + 1024; }
 
 template <int G>
-int recurrent_config(aig_ctx* ctx, const LstmLaunch& l, int batch, cudaLaunchConfig_t* cfg, cudaLaunchAttribute* attr) {
-  attr->id = cudaLaunchAttributeClusterDimension;
-  attr->val.clusterDim.x = l.cluster;
-  attr->val.clusterDim.y = attr->val.clusterDim.z = 1;
+int recurrent_config(aig_ctx* ctx, const LstmLaunch& l, int batch, cudaLaunchConfig_t* cfg, cudaLaunchAttribute (&attr)[2]) {
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = l.cluster;
+  attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+  attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[1].val.programmaticStreamSerializationAllowed = 1;
   *cfg = cudaLaunchConfig_t{};
   cfg->gridDim = dim3(ceil_div(batch, G * kSeqs) * l.cluster);
   cfg->blockDim = dim3(lstm_threads(G));
   cfg->dynamicSmemBytes = l.smem;
   cfg->stream = ctx->stream;
   cfg->attrs = attr;
-  cfg->numAttrs = 1;
+  cfg->numAttrs = 2;
   AIG_CUDA_OK(ctx, cudaFuncSetAttribute(lstm_recurrent_kernel<G>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)l.smem));
   AIG_CUDA_OK(ctx, cudaFuncSetAttribute(lstm_recurrent_kernel<G>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
   return AIG_OK;
@@ -320,8 +324,8 @@ int recurrent_shape(aig_ctx* ctx, int H, int batch, LstmLaunch* l) {
   l->groups = 1;
   l->smem = recurrent_smem(H, 1);
   cudaLaunchConfig_t cfg;
-  cudaLaunchAttribute attr;
-  int rc = recurrent_config<1>(ctx, *l, batch, &cfg, &attr), n = 0;
+  cudaLaunchAttribute attr[2];
+  int rc = recurrent_config<1>(ctx, *l, batch, &cfg, attr), n = 0;
   if (rc != AIG_OK) return rc;
   AIG_CUDA_OK(ctx, cudaOccupancyMaxActiveClusters(&n, lstm_recurrent_kernel<1>, &cfg));
   if (n < 1) return aig_fail(ctx, AIG_ERR_UNSUPPORTED, "lstm: no cluster of %d CTAs fits this device", l->cluster);
@@ -335,8 +339,8 @@ int recurrent_shape(aig_ctx* ctx, int H, int batch, LstmLaunch* l) {
 template <int G>
 int launch_recurrent(aig_ctx* ctx, const LstmLaunch& l, const LstmParams& prm) {
   cudaLaunchConfig_t cfg;
-  cudaLaunchAttribute attr;
-  const int rc = recurrent_config<G>(ctx, l, prm.B, &cfg, &attr);
+  cudaLaunchAttribute attr[2];
+  const int rc = recurrent_config<G>(ctx, l, prm.B, &cfg, attr);
   if (rc != AIG_OK) return rc;
   AIG_CUDA_OK(ctx, cudaLaunchKernelEx(&cfg, lstm_recurrent_kernel<G>, prm));
   return AIG_OK;

@@ -107,6 +107,8 @@ attention_tile_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_con
     tmem_alloc(smem_u32(s_tmem), kTmemCols);
     tmem_relinquish();
   }
+  griddep_launch_dependents();
+  griddep_wait();
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
@@ -395,8 +397,7 @@ int launch_attention(aig_mha_plan* pl, const AttnParams& prm) {
   AIG_CUDA_OK(ctx, cudaFuncSetAttribute(attention_tile_kernel<NK>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   const int items = pl->B * pl->heads;
   const int grid = items < kAttnCtas<NK> * ctx->sm_count ? items : kAttnCtas<NK> * ctx->sm_count;
-  attention_tile_kernel<NK><<<grid, kThreads, smem, ctx->stream>>>(pl->mq, pl->mk, pl->mv, prm);
-  AIG_LAUNCH_OK(ctx);
+  AIG_CUDA_OK(ctx, launch_pdl(attention_tile_kernel<NK>, dim3(grid), dim3(kThreads), smem, ctx->stream, pl->mq, pl->mk, pl->mv, prm));
   return AIG_OK;
 }
 
