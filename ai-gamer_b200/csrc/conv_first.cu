@@ -169,7 +169,7 @@ struct aig_conv0_plan {
   size_t smem = 0;
   dim3 grid;
   ConvFirstTc* tc = nullptr;  // tensor-core path when the filter geometry has an instantiation
-  ConvFirstRows* rows = nullptr;  // row-resident tensor-core path for uint8 frames (5x5, stride 2, 32 channels)
+  ConvFirstRows* rows = nullptr;  // row-resident tensor-core path: uint8 frames (5x5, stride 2, 32 channels), clips (3x3x3)
   __half* planar_scratch = nullptr;  // planar uint8 frames converted to fp16, for geometries without the row kernel
 };
 
@@ -337,6 +337,7 @@ int aig_conv0_forward_nchw(aig_conv0_plan* pl, const aig_half* x, aig_half* y) {
   DeviceGuard g(ctx->device);
   AIG_REQUIRE(ctx, x && y && pl->weights_set, "conv0 forward: null pointer or weights not set");
   AIG_REQUIRE(ctx, ((uintptr_t)y & 15) == 0, "conv0 forward: misaligned output");
+  if (pl->rows && pl->p.kd > 1 && ((uintptr_t)x & 15) == 0) return conv_first_rows_forward_clips(pl->rows, (const __half*)x, (__half*)y);
   if (pl->tc) return conv_first_tc_forward(pl->tc, x, false, (__half*)y);
   conv_first_kernel<false><<<pl->grid, kTH * kTW, pl->smem, ctx->stream>>>(x, (__half*)y, pl->p);
   AIG_LAUNCH_OK(ctx);

@@ -19,6 +19,13 @@
 // every input row is read and converted once per CTA (twice at range borders).
 // Conversion: half(float(u8) / 255.0f) as the reference computes it; float(u8) * fl(1/255) rounds to the same
 // half for all 256 byte values, so the division is a multiplication here.
+// Frames whose rows are not whole 16-byte pieces are loaded by aligned 32-bit words, four pixels at a time.
+//
+// CLIP: the first layer of the clip encoder (ConvLayer3D, 3 -> 32 channels, 3x3x3, stride 1x2x2, pad 1) from planar fp16
+// clips in the same way: pixel x lies at half-unit x + 1, so output pixel x reads units x, x+1 (pixels 2x-1 .. 2x+2, the
+// last with zero weights) and each of the nine (depth, row) pairs is one instruction.  Tiles run along the depth first: a
+// column of three input rows joins the ring per tile, so every input row is loaded once or, at odd rows, twice.  Bound by
+// HBM (16 clips of 8x144x256: 28 MB in, 75 MB out); the per-tap gather that this replaces took 69 us there.
 #include "conv_first_rows.h"
 
 #include "aig_common.cuh"
@@ -26,32 +33,36 @@
 namespace {
 
 constexpr int kThreads = 9 * 32;
-constexpr int kRing = 16;             // input row buffers
+constexpr int kRing = 16;             // input row buffers (clips: eight columns of three)
 constexpr int kLead = 4;              // tiles the loaders may run ahead of completed MMAs
 constexpr int kPitch = 130 * 16;      // bytes per row buffer: (256 / 2 + 2) units; also what 128 MMA rows x 3 units span
 constexpr int kN = 32;                // output channels
-constexpr int kMmas = 10;             // 5 filter rows x 2
 constexpr int kOutSlots = 130;
 constexpr int kOutBytes = 9216;       // one output staging buffer (130 slots x 64 B, 1024-aligned)
-constexpr int kSmemRing = kRing * kPitch;
 constexpr int kSmemZero = kPitch + 64;                    // the all-zero row (+ what the last instruction over-reads)
-constexpr int kSmemB = kMmas * 2 * kN * 16;               // weights: [mma][chunk][n][8 halves]
 constexpr int kOffOut = 0;
 constexpr int kOffRing = 2 * kOutBytes;
-constexpr int kOffZero = kOffRing + kSmemRing;
-constexpr int kOffB = kOffZero + ((kSmemZero + 127) & ~127);
-constexpr int kOffBars = kOffB + kSmemB;
-constexpr int kSmemBytes = kOffBars + 256 + 1024;
+constexpr int kColumns = 8, kColRows = 3;
+template <bool CLIP>
+struct RowsCfg {
+  static constexpr int kMmas = CLIP ? 9 : 10;             // 3 x 3 filter rows, or 5 filter rows x 2
+  static constexpr int kSmemB = kMmas * 2 * kN * 16;      // weights: [mma][chunk][n][8 halves]
+  static constexpr int kOffZero = kOffRing + (CLIP ? kColumns * kColRows : kRing) * kPitch;
+  static constexpr int kOffB = kOffZero + ((kSmemZero + 127) & ~127);
+  static constexpr int kOffBars = kOffB + kSmemB;
+  static constexpr int kSmemBytes = kOffBars + 256 + 1024;
+  static constexpr int kCtas = CLIP ? 2 : 3;              // per SM
+};
 
 struct RowsParams {
-  int batch, H, W, Ho, Wo;
-  int tiles;               // batch * Ho
+  int batch, D, H, W, Ho, Wo;
+  int tiles;               // batch * Ho (* D)
   int s2d, Hb;             // output in space-to-depth blocks; block rows per image
   int planar;              // 1: frames are three uint8 planes R, G, B; 0: BGRA pixels
   float slope;
   float scale[kN], shift[kN];
-  const uint8_t* frames;
-  const uint4* wimg;       // kSmemB bytes, the shared-memory image of the weights
+  const uint8_t* frames;   // clips: planar fp16
+  const uint4* wimg;       // RowsCfg::kSmemB bytes, the shared-memory image of the weights
   int* gerr;
 };
 
@@ -99,9 +110,40 @@ __device__ __forceinline__ float act_rows(float v, float slope) {
   return v;
 }
 
-template <int ACT>
-__global__ void __launch_bounds__(kThreads, 3)
+// eight halves of a row starting at any element, `n` of them in the row (zero beyond), by aligned 32-bit words; a word
+// that holds a needed half may hold one past the tensor's end as well
+__device__ __forceinline__ uint4 load_halfs8(const __half* src, int n) {
+  const uintptr_t a = reinterpret_cast<uintptr_t>(src);
+  const uint32_t* w = reinterpret_cast<const uint32_t*>(a & ~(uintptr_t)3);
+  const int odd = (int)(a >> 1) & 1;
+  uint32_t v[5];
+#pragma unroll
+  for (int k = 0; k < 5; ++k) v[k] = 2 * k - odd < n && (k < 4 || odd) ? __ldg(w + k) : 0u;
+  uint4 o;
+  uint32_t* p = reinterpret_cast<uint32_t*>(&o);
+#pragma unroll
+  for (int k = 0; k < 4; ++k) {
+    p[k] = odd ? __funnelshift_r(v[k], v[k + 1], 16) : v[k];
+    if (2 * k >= n) p[k] = 0u;
+    else if (2 * k + 1 >= n) p[k] &= 0xFFFFu;
+  }
+  return o;
+}
+// four bytes likewise
+__device__ __forceinline__ uint32_t load_bytes4(const uint8_t* src, int n) {
+  const uintptr_t a = reinterpret_cast<uintptr_t>(src);
+  const uint32_t* w = reinterpret_cast<const uint32_t*>(a & ~(uintptr_t)3);
+  const int off = (int)(a & 3);
+  const uint32_t lo = __ldg(w), hi = off + n > 4 ? __ldg(w + 1) : 0u;
+  const uint32_t v = __funnelshift_r(lo, hi, off * 8);
+  return n < 4 ? v & ((1u << (8 * n)) - 1u) : v;
+}
+
+template <int ACT, bool CLIP>
+__global__ void __launch_bounds__(kThreads, RowsCfg<CLIP>::kCtas)
 conv_first_rows_kernel(const __grid_constant__ CUtensorMap tmapY, const __grid_constant__ RowsParams p) {
+  using Cfg = RowsCfg<CLIP>;
+  constexpr int kOffZero = Cfg::kOffZero, kOffB = Cfg::kOffB, kOffBars = Cfg::kOffBars, kSmemB = Cfg::kSmemB;
   extern __shared__ uint8_t smem_raw[];
   const uint32_t raw = smem_u32(smem_raw);
   const uint32_t base = (raw + 1023u) & ~1023u;
@@ -144,7 +186,7 @@ conv_first_rows_kernel(const __grid_constant__ CUtensorMap tmapY, const __grid_c
   tc_fence_after();
   const uint32_t tmem_base = *s_tmem;
 
-  // contiguous range of (frame, output row) tiles of this CTA
+  // contiguous range of (frame, output row) or (clip, output row, depth) tiles of this CTA
   const int t_begin = (int)((long long)p.tiles * blockIdx.x / gridDim.x), t_end = (int)((long long)p.tiles * (blockIdx.x + 1) / gridDim.x);
 
   if (warp == 0) {
@@ -154,17 +196,32 @@ conv_first_rows_kernel(const __grid_constant__ CUtensorMap tmapY, const __grid_c
       constexpr uint32_t idesc = umma_idesc_f16(128, kN);
       const bool leader = elect_one();
       bool ok = true;
-      int y = t_begin % p.Ho;
+      int z = CLIP ? t_begin % p.D : 0, y = (CLIP ? t_begin / p.D : t_begin) % p.Ho;
+      int ring_off = 0;  // input rows take ring slots in the order of their loading, also from one frame to the next
+      int col = 0;  // CLIP: number, since this CTA's start, of the column that holds depth z - 1 (the first: depth max(z - 1, 0))
       for (int i = 0; i < t_end - t_begin && ok; ++i) {
         const int acc = i & 3;
         if (!mbar_wait_bounded_sleepy(bar_tempty + 8 * acc, (((uint32_t)i >> 2) & 1u) ^ 1u, s_abort, p.gerr, 811)) { ok = false; break; }
         if (!mbar_wait_bounded_sleepy(bar_ready + 8 * (i & 7), ((uint32_t)i >> 3) & 1u, s_abort, p.gerr, 812)) { ok = false; break; }
         tc_fence_after();
         const uint32_t d_tmem = tmem_base + (uint32_t)(acc * kN);
+        if constexpr (CLIP) {
+          const bool first_of_range = i == 0;
+          if (first_of_range) col = z > 0 ? 0 : -1;
+#pragma unroll
+          for (int m = 0; m < 9; ++m) {
+            const int d = z - 1 + m / 3, row = 2 * y - 1 + m % 3;
+            const uint32_t a_row = (d < 0 || d >= p.D || row < 0 || row >= p.H)
+                                       ? sZero : sRing + (uint32_t)(((col + m / 3) & (kColumns - 1)) * kColRows + m % 3) * kPitch;
+            const uint64_t adesc = desc_noswizzle(a_row, 16u, 128u);
+            const uint64_t bdesc = desc_noswizzle(sB + (uint32_t)(m * 2 * kN * 16), (uint32_t)(kN * 16), 128u);
+            if (leader) umma_f16_ss(d_tmem, adesc, bdesc, idesc, m != 0 ? 1u : 0u);
+          }
+        } else {
 #pragma unroll
         for (int r = 0; r < 5; ++r) {
           const int row = 2 * y - 2 + r;
-          const uint32_t a_row = (row < 0 || row >= p.H) ? sZero : sRing + (uint32_t)(row & (kRing - 1)) * kPitch;
+          const uint32_t a_row = (row < 0 || row >= p.H) ? sZero : sRing + (uint32_t)((row + ring_off) & (kRing - 1)) * kPitch;
 #pragma unroll
           for (int h = 0; h < 2; ++h) {
             const uint64_t adesc = desc_noswizzle(a_row + 32u * h, 16u, 128u);
@@ -172,11 +229,21 @@ conv_first_rows_kernel(const __grid_constant__ CUtensorMap tmapY, const __grid_c
             if (leader) umma_f16_ss(d_tmem, adesc, bdesc, idesc, (r | h) != 0 ? 1u : 0u);
           }
         }
+        }
         if (leader) {
           umma_commit(bar_tfull + 8 * acc);
           umma_commit(bar_done + 8 * (i & 7));
         }
-        if (++y == p.Ho) y = 0;
+        if constexpr (CLIP) {
+          ++col;
+          if (++z == p.D) {
+            z = 0;          // the next tile's depth 0 is the column after this group's last one (depth D - 1 = col + 0 now)
+            if (++y == p.Ho) y = 0;
+          }
+        } else if (++y == p.Ho) {
+          y = 0;
+          ring_off += p.H;
+        }
       }
     }
   } else if (warp <= 4) {
@@ -186,7 +253,7 @@ conv_first_rows_kernel(const __grid_constant__ CUtensorMap tmapY, const __grid_c
     const int tid_e = threadIdx.x - 32;
     const int slot = x + (p.s2d ? 1 : 0);
     const uint32_t swz = (uint32_t)((slot >> 1) & 3);
-    int n = t_begin / p.Ho, y = t_begin - n * p.Ho;
+    int z = CLIP ? t_begin % p.D : 0, n = (CLIP ? t_begin / p.D : t_begin) / p.Ho, y = (CLIP ? t_begin / p.D : t_begin) - n * p.Ho;
     griddep_wait();                               // the output buffer may still be read by an earlier launch
     for (int i = 0; i < t_end - t_begin; ++i) {
       const int acc = i & 3, buf = i & 1;
@@ -224,9 +291,11 @@ conv_first_rows_kernel(const __grid_constant__ CUtensorMap tmapY, const __grid_c
       if (tid_e == 0) {
         const uint32_t src = sOut + (uint32_t)buf * kOutBytes;
         if (p.s2d) tma_store_5d(&tmapY, src, 0, 0, 0, (y + 1) & 1, n * p.Hb + ((y + 1) >> 1));
-        else tma_store_4d(&tmapY, src, 0, 0, y, n);
+        else tma_store_4d(&tmapY, src, 0, 0, y, CLIP ? n * p.D + z : n);
         bulk_commit();
       }
+      if (CLIP && ++z < p.D) continue;
+      z = 0;
       if (++y == p.Ho) {
         y = 0;
         ++n;
@@ -238,13 +307,73 @@ conv_first_rows_kernel(const __grid_constant__ CUtensorMap tmapY, const __grid_c
     // Every tile needs the input rows not yet in the ring (two in steady state, three at the top of a frame, five
     // at the start of the CTA's range), cut into 16-byte items; thread t takes items t, t+128, ...
     const int tid_l = threadIdx.x - 5 * 32;
+    if constexpr (CLIP) {
+      const int segs = (p.W + 7) / 8;                     // eight pixels each
+      const size_t plane = (size_t)p.D * p.H * p.W;
+      const bool whole = p.W % 8 == 0;
+      int z = t_begin % p.D, n = t_begin / p.D / p.Ho, y = t_begin / p.D - n * p.Ho, col = 0, loaded = 0;
+      bool ok = true;
+      griddep_wait();
+      for (int i = 0; i < t_end - t_begin && ok; ++i) {
+        // columns of this tile that are not there yet: depth d0 .. d1
+        const int d1 = min(z + 1, p.D - 1), d0 = i == 0 ? max(z - 1, 0) : (z == 0 ? 0 : loaded + 1);
+        if (i >= kLead && !mbar_wait_bounded_sleepy(bar_done + 8 * ((i - kLead) & 7), ((uint32_t)(i - kLead) >> 3) & 1u, s_abort, p.gerr, 831)) { ok = false; break; }
+        const int items = (d1 - d0 + 1) * kColRows * segs;
+        for (int idx = tid_l; idx < items; idx += 128) {
+          const int rr = idx / segs, seg = idx - rr * segs, c = rr / kColRows, r = rr - c * kColRows, row = 2 * y - 1 + r;
+          if (row < 0 || row >= p.H) continue;
+          const __half* src = reinterpret_cast<const __half*>(p.frames) + (size_t)n * 3 * plane + ((size_t)(d0 + c) * p.H + row) * p.W + 8 * seg;
+          uint4 v[3];
+#pragma unroll
+          for (int ch = 0; ch < 3; ++ch) v[ch] = whole ? __ldg(reinterpret_cast<const uint4*>(src + ch * plane)) : load_halfs8(src + ch * plane, p.W - 8 * seg);
+          const uint32_t *pr = reinterpret_cast<const uint32_t*>(&v[0]), *pg = reinterpret_cast<const uint32_t*>(&v[1]), *pb = reinterpret_cast<const uint32_t*>(&v[2]);
+          uint2* d = reinterpret_cast<uint2*>(sm + kOffRing + (size_t)(((col + c) & (kColumns - 1)) * kColRows + r) * kPitch) + 8 * seg + 1;
+#pragma unroll
+          for (int k = 0; k < 4; ++k) {
+            d[2 * k] = make_uint2(__byte_perm(pr[k], pg[k], 0x5410u), pb[k] & 0xFFFFu);
+            d[2 * k + 1] = make_uint2(__byte_perm(pr[k], pg[k], 0x7632u), pb[k] >> 16);
+          }
+        }
+        fence_proxy_async_smem();
+        mbar_arrive(bar_ready + 8 * (i & 7));
+        col += d1 - d0 + 1;
+        loaded = d1;
+        if (++z == p.D) {
+          z = 0;
+          if (++y == p.Ho) {
+            y = 0;
+            ++n;
+          }
+        }
+      }
+    } else {
     const size_t frame_bytes = (size_t)p.H * p.W * (p.planar ? 3 : 4);
     const size_t plane = (size_t)p.H * p.W;
-    const int segs = p.planar ? p.W / 16 : p.W / 4;   // 16-byte loads per input row (per plane when planar)
+    const bool vec = p.W % (p.planar ? 16 : 4) == 0;  // rows of whole 16-byte pieces
+    const int segs = !vec ? (p.W + 3) / 4 : (p.planar ? p.W / 16 : p.W / 4);   // items per input row
     const int rr0 = tid_l / segs, seg0 = tid_l - rr0 * segs;  // this thread's first item of any tile
+    int ring_off = 0;                                 // as the MMA warp's
     auto convert_item = [&](const uint8_t* frame, int row, int seg) {
-      uint8_t* dst_row = sm + kOffRing + (size_t)(row & (kRing - 1)) * kPitch;
-      if (!p.planar) {
+      uint8_t* dst_row = sm + kOffRing + (size_t)((row + ring_off) & (kRing - 1)) * kPitch;
+      if (!vec) {                                       // four pixels, those past the row's end zero
+        const int left = p.W - 4 * seg;
+        const size_t off = (size_t)row * p.W + 4 * seg;
+        uint2 px[4];
+        if (!p.planar) {
+          const uint32_t* s = reinterpret_cast<const uint32_t*>(frame) + off;
+#pragma unroll
+          for (int k = 0; k < 4; ++k) px[k] = k < left ? pixel_bgra(__ldg(s + k)) : make_uint2(0, 0);
+        } else {
+          const uint32_t r = load_bytes4(frame + off, left), g = load_bytes4(frame + plane + off, left), b = load_bytes4(frame + 2 * plane + off, left);
+          px[0] = pixel_rgb(r, g, b, 0x7540u);
+          px[1] = pixel_rgb(r, g, b, 0x7541u);
+          px[2] = pixel_rgb(r, g, b, 0x7542u);
+          px[3] = pixel_rgb(r, g, b, 0x7543u);
+        }
+        uint4* d = reinterpret_cast<uint4*>(dst_row + (2 * seg + 1) * 16);
+        d[0] = make_uint4(px[0].x, px[0].y, px[1].x, px[1].y);
+        d[1] = make_uint4(px[2].x, px[2].y, px[3].x, px[3].y);
+      } else if (!p.planar) {
         const uint4 v = __ldg(reinterpret_cast<const uint4*>(frame + ((size_t)row * p.W + 4 * seg) * 4));
         const uint2 p0 = pixel_bgra(v.x), p1 = pixel_bgra(v.y), p2 = pixel_bgra(v.z), p3 = pixel_bgra(v.w);
         uint4* d = reinterpret_cast<uint4*>(dst_row + (2 * seg + 1) * 16);  // pixels 4seg .. 4seg+3 = units 2seg+1, 2seg+2
@@ -287,8 +416,10 @@ conv_first_rows_kernel(const __grid_constant__ CUtensorMap tmapY, const __grid_c
         y = 0;
         ++n;
         frame += frame_bytes;
+        ring_off += p.H;
         loaded_hi = -1;
       }
+    }
     }
   }
 
@@ -307,13 +438,21 @@ conv_first_rows_kernel(const __grid_constant__ CUtensorMap tmapY, const __grid_c
 // eight halves e = 4*s + ch covering tap column t = 4h + 2c + s of filter row r, channel ch (zero for t >= 5 or ch == 3)
 __global__ void pack_rows_weights_kernel(const __half* __restrict__ w, __half* __restrict__ img) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= kMmas * 2 * kN * 8) return;
+  if (i >= RowsCfg<false>::kMmas * 2 * kN * 8) return;
   const int e = i & 7, n = (i >> 3) % kN, j = i / (8 * kN);  // j = m*2 + c
   const int m = j >> 1, c = j & 1, r = m >> 1, h = m & 1;
   const int s = e >> 2, ch = e & 3, t = 4 * h + 2 * c + s;
   __half v = __ushort_as_half((unsigned short)0);
   if (t < 5 && ch < 3) v = w[((n * 3 + ch) * 5 + r) * 5 + t];
   img[i] = v;
+}
+
+// w [32][3][3][3][3] likewise: MMA m = fd*3 + fr, chunk c, e = 4*s + ch covering tap column t = 2c + s (zero for t == 3)
+__global__ void pack_clip_weights_kernel(const __half* __restrict__ w, __half* __restrict__ img) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= RowsCfg<true>::kMmas * 2 * kN * 8) return;
+  const int e = i & 7, n = (i >> 3) % kN, j = i / (8 * kN), m = j >> 1, ch = e & 3, t = 2 * (j & 1) + (e >> 2);
+  img[i] = t < 3 && ch < 3 ? w[((n * 3 + ch) * 9 + m) * 3 + t] : __ushort_as_half((unsigned short)0);
 }
 
 typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*, const cuuint32_t*,
@@ -344,9 +483,11 @@ struct ConvFirstRows {
   int grid = 1;
 };
 
+static bool is_clip(const ConvFirstGeom& g) { return g.kd == 3; }
 bool conv_first_rows_supported(const ConvFirstGeom& g) {
-  return g.D == 1 && g.kd == 1 && g.k == 5 && g.s == 2 && g.pad == 2 && g.K == kN && g.W % 16 == 0 && g.W >= 16 && g.W <= 256 && g.H >= 2 &&
-         g.Wo <= 128 && g.Wo >= 2 && g.Ho >= 2;
+  if (g.s != 2 || g.K != kN || g.W > 256 || g.Wo > 128) return false;
+  if (is_clip(g)) return g.k == 3 && g.sd == 1 && g.pd == 1 && g.pad == 1;
+  return g.D == 1 && g.kd == 1 && g.k == 5 && g.pad == 2 && g.W >= 4 && g.H >= 2 && g.Wo >= 2 && g.Ho >= 2;
 }
 
 int conv_first_rows_create(aig_ctx* ctx, const ConvFirstGeom& g, const float* scale, const float* shift, ConvFirstRows** out) {
@@ -358,16 +499,17 @@ int conv_first_rows_create(aig_ctx* ctx, const ConvFirstGeom& g, const float* sc
   t->scale_dev = scale;
   t->shift_dev = shift;
   RowsParams& p = t->prm;
-  p.batch = g.batch; p.H = g.H; p.W = g.W; p.Ho = g.Ho; p.Wo = g.Wo;
-  p.tiles = g.batch * g.Ho;
+  p.batch = g.batch; p.D = g.D; p.H = g.H; p.W = g.W; p.Ho = g.Ho; p.Wo = g.Wo;
+  p.tiles = g.batch * g.Ho * g.D;
   p.slope = g.slope;
   p.gerr = ctx->d_err;
-  if (cudaMalloc(&t->wimg, kSmemB) != cudaSuccess) {
+  if (cudaMalloc(&t->wimg, RowsCfg<false>::kSmemB) != cudaSuccess) {  // (the larger of the two)
     delete t;
     return aig_fail(ctx, AIG_ERR_CUDA, "first-layer row kernel: allocation failed");
   }
   p.wimg = reinterpret_cast<const uint4*>(t->wimg);
-  t->grid = 3 * ctx->sm_count < p.tiles ? 3 * ctx->sm_count : p.tiles;
+  const int ctas = (is_clip(g) ? RowsCfg<true>::kCtas : RowsCfg<false>::kCtas) * ctx->sm_count;
+  t->grid = ctas < p.tiles ? ctas : p.tiles;
   *out = t;
   return AIG_OK;
 }
@@ -382,7 +524,8 @@ void conv_first_rows_destroy(ConvFirstRows* t) {
 // travel to the kernel as launch parameters (constant bank), so they are read back here once.
 int conv_first_rows_set_weights(ConvFirstRows* t, const __half* w) {
   aig_ctx* ctx = t->ctx;
-  pack_rows_weights_kernel<<<ceil_div(kMmas * 2 * kN * 8, 256), 256, 0, ctx->stream>>>(w, t->wimg);
+  if (is_clip(t->g)) pack_clip_weights_kernel<<<ceil_div(RowsCfg<true>::kMmas * 2 * kN * 8, 256), 256, 0, ctx->stream>>>(w, t->wimg);
+  else pack_rows_weights_kernel<<<ceil_div(RowsCfg<false>::kMmas * 2 * kN * 8, 256), 256, 0, ctx->stream>>>(w, t->wimg);
   AIG_LAUNCH_OK(ctx);
   AIG_CUDA_OK(ctx, cudaMemcpyAsync(t->prm.scale, t->scale_dev, kN * sizeof(float), cudaMemcpyDeviceToHost, ctx->stream));
   AIG_CUDA_OK(ctx, cudaMemcpyAsync(t->prm.shift, t->shift_dev, kN * sizeof(float), cudaMemcpyDeviceToHost, ctx->stream));
@@ -414,7 +557,7 @@ static int rows_encode_output(ConvFirstRows* t, __half* y) {
     r = enc(&t->tmapY, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 5, y, dims, strides, box, es, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_64B,
             CU_TENSOR_MAP_L2_PROMOTION_NONE, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   } else {
-    cuuint64_t dims[4] = {(cuuint64_t)kN, (cuuint64_t)g.Wo, (cuuint64_t)g.Ho, (cuuint64_t)g.batch};
+    cuuint64_t dims[4] = {(cuuint64_t)kN, (cuuint64_t)g.Wo, (cuuint64_t)g.Ho, (cuuint64_t)g.batch * g.D};
     cuuint64_t strides[3] = {(cuuint64_t)kN * 2, (cuuint64_t)g.Wo * kN * 2, (cuuint64_t)g.Ho * g.Wo * kN * 2};
     cuuint32_t box[4] = {(cuuint32_t)kN, (cuuint32_t)g.Wo, 1, 1};
     cuuint32_t es[4] = {1, 1, 1, 1};
@@ -427,32 +570,38 @@ static int rows_encode_output(ConvFirstRows* t, __half* y) {
   return AIG_OK;
 }
 
-template <int ACT>
+template <int ACT, bool CLIP>
 static int rows_launch(ConvFirstRows* t) {
   static bool attr_set[64] = {};
   aig_ctx* ctx = t->ctx;
+  constexpr int smem = RowsCfg<CLIP>::kSmemBytes;
   if (!attr_set[ctx->device & 63]) {
-    AIG_CUDA_OK(ctx, cudaFuncSetAttribute(conv_first_rows_kernel<ACT>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBytes));
+    AIG_CUDA_OK(ctx, cudaFuncSetAttribute(conv_first_rows_kernel<ACT, CLIP>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
     attr_set[ctx->device & 63] = true;
   }
-  conv_first_rows_kernel<ACT><<<t->grid, kThreads, kSmemBytes, ctx->stream>>>(t->tmapY, t->prm);
+  conv_first_rows_kernel<ACT, CLIP><<<t->grid, kThreads, smem, ctx->stream>>>(t->tmapY, t->prm);
   AIG_LAUNCH_OK(ctx);
   return AIG_OK;
 }
-
-int conv_first_rows_forward(ConvFirstRows* t, const uint8_t* frames, int planar_rgb, __half* y) {
+template <bool CLIP>
+static int rows_forward(ConvFirstRows* t, const void* x, __half* y) {
   aig_ctx* ctx = t->ctx;
-  if (((uintptr_t)frames & 15) != 0 || ((uintptr_t)y & 15) != 0) return aig_fail(ctx, AIG_ERR_INVALID, "first-layer row kernel: frames and output must be 16-byte aligned");
+  if (((uintptr_t)x & 15) != 0 || ((uintptr_t)y & 15) != 0) return aig_fail(ctx, AIG_ERR_INVALID, "first-layer row kernel: input and output must be 16-byte aligned");
   if (t->tmap_ptr != y || t->tmap_s2d != t->prm.s2d) {
     const int rc = rows_encode_output(t, y);
     if (rc != AIG_OK) return rc;
   }
-  t->prm.frames = frames;
-  t->prm.planar = planar_rgb ? 1 : 0;
+  t->prm.frames = static_cast<const uint8_t*>(x);
   switch (t->g.act) {
-    case AIG_ACT_RELU: return rows_launch<AIG_ACT_RELU>(t);
-    case AIG_ACT_SWISH: return rows_launch<AIG_ACT_SWISH>(t);
-    case AIG_ACT_LEAKY: return rows_launch<AIG_ACT_LEAKY>(t);
-    default: return rows_launch<AIG_ACT_NONE>(t);
+    case AIG_ACT_RELU: return rows_launch<AIG_ACT_RELU, CLIP>(t);
+    case AIG_ACT_SWISH: return rows_launch<AIG_ACT_SWISH, CLIP>(t);
+    case AIG_ACT_LEAKY: return rows_launch<AIG_ACT_LEAKY, CLIP>(t);
+    default: return rows_launch<AIG_ACT_NONE, CLIP>(t);
   }
 }
+
+int conv_first_rows_forward(ConvFirstRows* t, const uint8_t* frames, int planar_rgb, __half* y) {
+  t->prm.planar = planar_rgb ? 1 : 0;
+  return rows_forward<false>(t, frames, y);
+}
+int conv_first_rows_forward_clips(ConvFirstRows* t, const __half* clips, __half* y) { return rows_forward<true>(t, clips, y); }

@@ -465,3 +465,56 @@ def test_fc_few_rows(env, rows, inC, outC, f32):
     c.sync()
     assert np.abs(U.host(dy).reshape(rows, outC) - want).max() < (2e-4 if f32 else 4e-3)
     plan.close()
+
+
+@gpu
+@pytest.mark.parametrize("B,H,W", [(200, 18, 4), (150, 25, 35), (90, 24, 50), (40, 41, 129), (3, 33, 255), (60, 17, 256), (2, 2, 101)])
+def test_first_layer_row_kernel_any_width(env, B, H, W):
+    """Rows that are not whole 16-byte pieces (one to three pixels left over, odd widths up to the widest) and frame
+    heights at which consecutive frames meet anywhere in the ring of rows, many frames per CTA; BGRA and planar."""
+    U = env
+    import torch
+
+    c, pk = U.ctx(), U.pkg()
+    rng = np.random.default_rng(W)
+    w, b = h(rng.standard_normal((32, 3, 5, 5)) * 0.2), h(rng.uniform(-0.2, 0.2, 32))
+    frames = PL.make_frames(W, B, H, W)
+    x = torch.from_numpy(O.preprocess_frames(frames).astype(np.float32))
+    want = torch.nn.functional.conv2d(x, torch.from_numpy(w.astype(np.float32)), torch.from_numpy(b.astype(np.float32)), 2, 2).numpy()
+    plan = pk.Conv0Plan(c, B, H, W, 32, 5, 2, 2)
+    plan.set_weights(U.dev(w), U.dev(b))
+    _, Ho, Wo = plan.out_dims()
+    for planar in (False, True):
+        y = torch.full((B, Ho, Wo, 32), 7.0, dtype=torch.float16, device="cuda")
+        src = U.dev(np.ascontiguousarray(frames[..., [2, 1, 0]].transpose(0, 3, 1, 2)) if planar else frames)
+        (plan.forward_rgb_planar if planar else plan.forward_bgra)(src, y)
+        c.sync()
+        assert np.abs(U.nchw(U.host(y)).astype(np.float32) - want).max() < 4e-3
+    plan.close()
+
+
+@gpu
+@pytest.mark.parametrize("B,D,H,W", [(1, 1, 1, 1), (30, 1, 19, 7), (20, 2, 18, 40), (9, 3, 33, 255), (12, 5, 20, 256), (4, 8, 36, 130), (3, 12, 30, 101)])
+def test_first_clip_layer(env, B, D, H, W):
+    """First layer of the clip encoder: depths shorter than the filter to longer than the ring, widths of whole and
+    broken 16-byte pieces in even and odd positions, ranges of tiles that begin anywhere in a clip."""
+    U = env
+    import torch
+
+    c, pk = U.ctx(), U.pkg()
+    rng = np.random.default_rng(W + D)
+    w, b = h(rng.standard_normal((32, 3, 3, 3, 3)) * 0.2), h(rng.uniform(-0.2, 0.2, 32))
+    x = h(rng.random((B, 3, D, H, W)))
+    want = torch.nn.functional.conv3d(torch.from_numpy(x.astype(np.float32)), torch.from_numpy(w.astype(np.float32)),
+                                      torch.from_numpy(b.astype(np.float32)), (1, 2, 2), 1)
+    want = torch.nn.functional.leaky_relu(want, 0.01).numpy()
+    plan = pk.Conv0Plan(c, B, H, W, 32, 3, 2, 1, act=pk.ACT_LEAKY, slope=0.01, in_d=D, kd=3, sd=1, pd=1)
+    plan.set_weights(U.dev(w), U.dev(b))
+    _, Ho, Wo = plan.out_dims()
+    y = torch.full((B, D, Ho, Wo, 32), 7.0, dtype=torch.float16, device="cuda")
+    dx = U.dev(x)
+    for _ in range(2):
+        plan.forward_nchw(dx, y)
+    c.sync()
+    assert np.abs(U.host(y).astype(np.float32).transpose(0, 4, 1, 2, 3) - want).max() < 6e-3
+    plan.close()
