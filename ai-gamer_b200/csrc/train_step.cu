@@ -62,7 +62,9 @@ __global__ void sq_err_final_kernel(const double* __restrict__ partial, int bloc
 }
 
 // ---- loss gradient of the squared error as the reference takes it: prediction - target, in half arithmetic
-__global__ void loss_gradient_kernel(__half* __restrict__ g, const __half* __restrict__ pred, const __half* __restrict__ target, long long n) {
+__global__ void loss_gradient_kernel(__half* g, const __half* pred, const __half* target, long long n) {
+  griddep_launch_dependents();
+  griddep_wait();
   for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) g[i] = __hsub(pred[i], target[i]);
 }
 
@@ -172,45 +174,111 @@ __global__ void adamw_f16_kernel(__half* __restrict__ p, const __half* __restric
     v[i] = r.v;
   }
 }
-// The same update on an FC layer's weights [rows = in_c][cols = out_c], which also writes the new weights transposed
-// ([out_c][in_c], the K-major operand of the forward GEMM) through a shared-memory tile: one launch instead of the
-// update and a repacking pass.  Block (32, 8), tile 32 x 32.
-__global__ void adamw_f16_fc_weights_kernel(__half* __restrict__ p, const __half* __restrict__ g, __half* __restrict__ m, __half* __restrict__ v,
-                                            __half* __restrict__ p_t, int rows, int cols, float lr, int t, float wd) {
-  __shared__ __half tile[32][34];
-  __shared__ double s_c[2];
-  adamw_block_corrections(t, s_c);
-  const double c1 = s_c[0], c2 = s_c[1];
-  const int c0 = blockIdx.x * 32, r0 = blockIdx.y * 32;
-  for (int i = threadIdx.y; i < 32; i += blockDim.y) {
-    const int r = r0 + i, c = c0 + threadIdx.x;
-    if (r < rows && c < cols) {
-      const size_t at = (size_t)r * cols + c;
-      const AdamHalf u = adamw_f16_element(p[at], g[at], m[at], v[at], lr, c1, c2, wd);
-      p[at] = u.p;
-      m[at] = u.m;
-      v[at] = u.v;
-      tile[i][threadIdx.x] = u.p;
+// The same update on an FC layer's weights [rows = in_c][cols = out_c] and bias, which also writes the new weights
+// transposed ([out_c][in_c], the K-major operand of the forward GEMM) and the fp32 bias that the forward reads.  As two
+// launches of scalar accesses with three double-precision divisions and a root per element it took 18 us for 1 M weights;
+// what it cannot do without is 16 MB of traffic, mostly in L2.  So: 16-byte accesses, tiles of 64 x 64, and the step in
+// single precision with a bound on its error: where both ends of the bound round to the same half, that is the double
+// computation's result too, else (one element in thousands) the double computation decides.
+constexpr int kAdamTile = 64;
+__device__ __forceinline__ AdamHalf adamw_f16_element_fast(__half p, __half g, __half m, __half v, float lr, double c1, double c2, float r1, float r2, float wd) {
+  const float gc = fmaxf(fminf(__half2float(g), kGradClip), -kGradClip);
+  const float mi = kBeta1 * __half2float(m) + (1.0f - kBeta1) * gc;
+  const float vi = kBeta2 * __half2float(v) + (1.0f - kBeta2) * gc * gc;
+  const float w = __half2float(p) * (1.0f - wd);
+  const float u = mi * r1 / (sqrtf(vi * r2) + (float)kAdamEps);  // seven roundings of 2^-24 at most; the bound allows sixteen
+  AdamHalf r;
+  r.m = __float2half(mi);
+  r.v = __float2half(vi);
+  r.p = __float2half(w - lr * (u * (1.0f - 9.5367e-7f)));
+  const __half hi = __float2half(w - lr * (u * (1.0f + 9.5367e-7f)));
+  if (__half_as_ushort(r.p) != __half_as_ushort(hi) || __hisnan(hi)) r.p = __float2half(w - lr * static_cast<float>(mi / c1 / (sqrt(vi / c2) + kAdamEps)));
+  return r;
+}
+struct AdamwFc {
+  __half *p, *m, *v, *p_t, *bias, *m_b, *v_b;
+  const __half *g, *g_b;
+  float* shift;
+  int rows, cols;
+  float lr, wd, r1, r2;
+  double c1, c2;   // 1 - beta^t; r1, r2 their reciprocals
+};
+template <bool VEC>   // rows of whole 16-byte pieces
+__global__ void __launch_bounds__(256) adamw_f16_fc_kernel(const AdamwFc a) {
+  __shared__ __half tile[kAdamTile][kAdamTile + 2];
+  griddep_launch_dependents();
+  griddep_wait();
+  const int c0 = blockIdx.x * kAdamTile, r0 = blockIdx.y * kAdamTile, tid = threadIdx.x;
+  if (r0 >= a.rows) {  // the last row of blocks: the bias
+    const int i = c0 + tid;
+    if (tid < kAdamTile && i < a.cols) {
+      const AdamHalf u = adamw_f16_element_fast(a.bias[i], a.g_b[i], a.m_b[i], a.v_b[i], a.lr, a.c1, a.c2, a.r1, a.r2, a.wd);
+      a.bias[i] = u.p;
+      a.m_b[i] = u.m;
+      a.v_b[i] = u.v;
+      a.shift[i] = __half2float(u.p);
+    }
+    return;
+  }
+#pragma unroll
+  for (int k = 0; k < 2; ++k) {
+    const int i = tid / 8 + 32 * k, r = r0 + i, c = c0 + tid % 8 * 8;
+    if (r >= a.rows || c >= a.cols) continue;
+    const size_t at = (size_t)r * a.cols + c;
+    __align__(16) __half p8[8], g8[8], m8[8], v8[8];
+    if constexpr (VEC) {
+      *reinterpret_cast<uint4*>(p8) = *reinterpret_cast<const uint4*>(a.p + at);
+      *reinterpret_cast<uint4*>(g8) = *reinterpret_cast<const uint4*>(a.g + at);
+      *reinterpret_cast<uint4*>(m8) = *reinterpret_cast<const uint4*>(a.m + at);
+      *reinterpret_cast<uint4*>(v8) = *reinterpret_cast<const uint4*>(a.v + at);
+    } else {
+#pragma unroll
+      for (int e = 0; e < 8; ++e) {
+        const bool in = c + e < a.cols;
+        p8[e] = in ? a.p[at + e] : __float2half(0.f);
+        g8[e] = in ? a.g[at + e] : __float2half(0.f);
+        m8[e] = in ? a.m[at + e] : __float2half(0.f);
+        v8[e] = in ? a.v[at + e] : __float2half(0.f);
+      }
+    }
+#pragma unroll
+    for (int e = 0; e < 8; ++e) {
+      const AdamHalf u = adamw_f16_element_fast(p8[e], g8[e], m8[e], v8[e], a.lr, a.c1, a.c2, a.r1, a.r2, a.wd);
+      p8[e] = u.p;
+      m8[e] = u.m;
+      v8[e] = u.v;
+      tile[i][c - c0 + e] = u.p;
+    }
+    if constexpr (VEC) {
+      *reinterpret_cast<uint4*>(a.p + at) = *reinterpret_cast<const uint4*>(p8);
+      *reinterpret_cast<uint4*>(a.m + at) = *reinterpret_cast<const uint4*>(m8);
+      *reinterpret_cast<uint4*>(a.v + at) = *reinterpret_cast<const uint4*>(v8);
+    } else {
+#pragma unroll
+      for (int e = 0; e < 8; ++e)
+        if (c + e < a.cols) {
+          a.p[at + e] = p8[e];
+          a.m[at + e] = m8[e];
+          a.v[at + e] = v8[e];
+        }
     }
   }
   __syncthreads();
-  for (int i = threadIdx.y; i < 32; i += blockDim.y) {
-    const int c = c0 + i, r = r0 + threadIdx.x;
-    if (c < cols && r < rows) p_t[(size_t)c * rows + r] = tile[threadIdx.x][i];
-  }
-}
-// The same update on the bias, which also refreshes the forward plan's fp32 shift
-__global__ void adamw_f16_fc_bias_kernel(__half* __restrict__ p, const __half* __restrict__ g, __half* __restrict__ m, __half* __restrict__ v,
-                                         float* __restrict__ shift, int n, float lr, int t, float wd) {
-  __shared__ double s_c[2];
-  adamw_block_corrections(t, s_c);
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < n) {
-    const AdamHalf u = adamw_f16_element(p[i], g[i], m[i], v[i], lr, s_c[0], s_c[1], wd);
-    p[i] = u.p;
-    m[i] = u.m;
-    v[i] = u.v;
-    shift[i] = __half2float(u.p);
+#pragma unroll
+  for (int k = 0; k < 2; ++k) {
+    const int i = tid / 8 + 32 * k, c = c0 + i, j = tid % 8 * 8, r = r0 + j;
+    if (c >= a.cols || r >= a.rows) continue;
+    __align__(16) __half t8[8];
+#pragma unroll
+    for (int e = 0; e < 8; ++e) t8[e] = tile[j + e][i];
+    __half* dst = a.p_t + (size_t)c * a.rows + r;
+    if (a.rows % 8 == 0) {
+      *reinterpret_cast<uint4*>(dst) = *reinterpret_cast<const uint4*>(t8);
+    } else {
+#pragma unroll
+      for (int e = 0; e < 8; ++e)
+        if (r + e < a.rows) dst[e] = t8[e];
+    }
   }
 }
 
@@ -248,8 +316,8 @@ int aig_loss_gradient(aig_ctx* ctx, aig_half* grad, const aig_half* pred, const 
   AIG_ENTER(ctx);
   AIG_REQUIRE(ctx, grad && pred && targets && n >= 0, "aig_loss_gradient: bad arguments");
   if (n == 0) return AIG_OK;
-  loss_gradient_kernel<<<blocks_for(ctx, n), kThreads, 0, ctx->stream>>>((__half*)grad, (const __half*)pred, (const __half*)targets, n);
-  AIG_LAUNCH_OK(ctx);
+  AIG_CUDA_OK(ctx, launch_pdl(loss_gradient_kernel, dim3(blocks_for(ctx, n)), dim3(kThreads), 0, ctx->stream, (__half*)grad, (const __half*)pred,
+                              (const __half*)targets, n));
   return AIG_OK;
 }
 
@@ -347,8 +415,8 @@ int aig_adamw_step_f16(aig_ctx* ctx, aig_half* params, const aig_half* grads, ai
 // W [in_c][out_c] (fp16, fp32 accumulation, one rounding to fp16 each, as the reference's cublasGemmEx calls):
 //   grad_w [in_c][out_c] = x^T . g        grad_b [out_c] = sum over the batch of g        grad_x [batch][in_c] = g . W^T
 // Both products run on the tcgen05 GEMM of the forward path (an FC plan computes rows . weights^T with both
-// operands K-major).  grad_x has that form as it stands (rows = g, weights = W, K = out_c); grad_w needs the batch
-// as the K dimension, so x and g are transposed first (one launch, which also forms grad_b).  K extents that are not a multiple of 16
+// operands K-major), or, in small batches, on kernels of their own (skinny_fc.cu, fc_wgrad_small_kernel).  grad_x has that
+// form as it stands (rows = g, weights = W, K = out_c); grad_w needs the batch as the K dimension, so x and g are transposed first (one launch, which also forms grad_b).  K extents that are not a multiple of 16
 // (an 18-wide head, odd batches) are padded with zeros, which adds exact zeros to the fp32 sums.
 namespace {
 
@@ -397,6 +465,90 @@ __global__ void pad_cols_kernel(const __half* __restrict__ src, __half* __restri
   }
 }
 
+// grad_w = x^T . g and grad_b for small batches straight from the row-major x [batch][in_c] and g [batch][out_c]: with
+// few rows the product is a write of grad_w with little before it, and transposing the operands for the K-major GEMM cost
+// a launch as long as the product (6.8 + 7.7 us at 64 x 1024 x 1024).  A CTA makes a 64 x 64 tile; ldmatrix.trans
+// turns both operands on their way from shared memory to mma.sync.  grad_b: sums in batch order, as bias_gradient_kernel.
+constexpr int kWgTile = 64, kWgPitch = kWgTile + 8, kWgMaxBatch = 256;
+__device__ __forceinline__ void ldmatrix_x4_trans(uint32_t (&r)[4], uint32_t addr) {
+  asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(addr) : "memory");
+}
+// rows k0 .. k0 + 63, columns c0 .. c0 + 63 of [rows][cols], zero outside
+__device__ __forceinline__ void wgrad_load(__half (*dst)[kWgPitch], const __half* src, int rows, int cols, int k0, int c0, bool vec) {
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const int item = threadIdx.x + 128 * i, k = k0 + item / 8, c = c0 + item % 8 * 8;
+    uint4 v = make_uint4(0, 0, 0, 0);
+    if (k < rows && c < cols) {
+      const __half* s = src + (size_t)k * cols + c;
+      if (vec) {
+        v = *reinterpret_cast<const uint4*>(s);
+      } else {
+        __half* h = reinterpret_cast<__half*>(&v);
+#pragma unroll
+        for (int e = 0; e < 8; ++e)
+          if (c + e < cols) h[e] = s[e];
+      }
+    }
+    *reinterpret_cast<uint4*>(&dst[item / 8][item % 8 * 8]) = v;
+  }
+}
+__global__ void __launch_bounds__(128) fc_wgrad_small_kernel(const __half* x, const __half* g, __half* grad_w, __half* grad_b, int batch, int in_c, int out_c,
+                                                             int vec_x, int vec_g) {
+  __shared__ __align__(16) __half sx[kWgTile][kWgPitch], sg[kWgTile][kWgPitch];
+  griddep_launch_dependents();
+  griddep_wait();
+  const int n0 = blockIdx.x * kWgTile, m0 = blockIdx.y * kWgTile, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int wm = (warp >> 1) * 32, wn = (warp & 1) * 32;
+  float acc[2][4][4] = {};
+  float bias = 0.f;
+  for (int k0 = 0; k0 < batch; k0 += kWgTile) {
+    if (k0) __syncthreads();
+    wgrad_load(sx, x, batch, in_c, k0, m0, vec_x);
+    wgrad_load(sg, g, batch, out_c, k0, n0, vec_g);
+    __syncthreads();
+#pragma unroll
+    for (int kk = 0; kk < kWgTile; kk += 16) {
+      if (k0 + kk >= batch) break;
+      uint32_t a[2][4], b[2][4];
+#pragma unroll
+      for (int i = 0; i < 2; ++i) {
+        // x: (k 0-7, m 0-7), (k 0-7, m 8-15), (k 8-15, m 0-7), (k 8-15, m 8-15); g: (k 0-7, n 0-7), (k 8-15, n 0-7), then n 8-15
+        ldmatrix_x4_trans(a[i], smem_u32(&sx[kk + (lane & 7) + (lane >> 4) * 8][wm + 16 * i + ((lane >> 3) & 1) * 8]));
+        ldmatrix_x4_trans(b[i], smem_u32(&sg[kk + (lane & 7) + ((lane >> 3) & 1) * 8][wn + 16 * i + (lane >> 4) * 8]));
+      }
+#pragma unroll
+      for (int i = 0; i < 2; ++i)
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+          asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+                       : "+f"(acc[i][j][0]), "+f"(acc[i][j][1]), "+f"(acc[i][j][2]), "+f"(acc[i][j][3])
+                       : "r"(a[i][0]), "r"(a[i][1]), "r"(a[i][2]), "r"(a[i][3]), "r"(b[j >> 1][(j & 1) * 2]), "r"(b[j >> 1][(j & 1) * 2 + 1]));
+    }
+    if (grad_b && blockIdx.y == 0 && threadIdx.x < kWgTile) {
+      const int n = min(kWgTile, batch - k0);
+      for (int k = 0; k < n; ++k) bias += __half2float(sg[k][threadIdx.x]);
+    }
+  }
+  if (grad_b && blockIdx.y == 0 && threadIdx.x < kWgTile && n0 + threadIdx.x < out_c) grad_b[n0 + threadIdx.x] = __float2half(bias);
+#pragma unroll
+  for (int i = 0; i < 2; ++i)
+#pragma unroll
+    for (int j = 0; j < 4; ++j)
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        const int m = m0 + wm + 16 * i + (lane >> 2) + 8 * h, n = n0 + wn + 8 * j + 2 * (lane & 3);
+        if (m >= in_c || n >= out_c) continue;
+        __half* dst = grad_w + (size_t)m * out_c + n;
+        if (vec_g) {
+          *reinterpret_cast<__half2*>(dst) = __floats2half2_rn(acc[i][j][2 * h], acc[i][j][2 * h + 1]);
+        } else {
+          dst[0] = __float2half(acc[i][j][2 * h]);
+          if (n + 1 < out_c) dst[1] = __float2half(acc[i][j][2 * h + 1]);
+        }
+      }
+}
+
 inline int round_up16(int v) { return (v + 15) / 16 * 16; }
 
 }  // namespace
@@ -435,7 +587,8 @@ int aig_fc_backward_plan_create(aig_ctx* ctx, int batch, int in_c, int out_c, ai
   pl->kd = round_up16(out_c);
   pl->kw = round_up16(batch);
   int rc = aig_fc_plan_create(ctx, batch, pl->kd, in_c, AIG_ACT_NONE, 0.f, /*two_step*/ 0, &pl->dgrad);
-  if (rc == AIG_OK) rc = aig_fc_plan_create(ctx, in_c, pl->kw, out_c, AIG_ACT_NONE, 0.f, 0, &pl->wgrad);
+  const bool small = batch <= kWgMaxBatch;   // fc_wgrad_small_kernel: no operands to keep
+  if (rc == AIG_OK && !small) rc = aig_fc_plan_create(ctx, in_c, pl->kw, out_c, AIG_ACT_NONE, 0.f, 0, &pl->wgrad);
   auto alloc = [&](__half** p, size_t elems) {
     if (rc != AIG_OK) return;
     if (cudaMalloc(reinterpret_cast<void**>(p), elems * sizeof(__half)) != cudaSuccess) {
@@ -444,8 +597,8 @@ int aig_fc_backward_plan_create(aig_ctx* ctx, int batch, int in_c, int out_c, ai
     }
   };
   if (rc == AIG_OK) rc = fc_plan_identity_affine(pl->dgrad);
-  if (rc == AIG_OK) rc = fc_plan_identity_affine(pl->wgrad);
-  alloc(&pl->x_t, (size_t)in_c * pl->kw);
+  if (rc == AIG_OK && !small) rc = fc_plan_identity_affine(pl->wgrad);
+  if (!small) alloc(&pl->x_t, (size_t)in_c * pl->kw);
   if (pl->kd != out_c) alloc(&pl->g_pad, (size_t)batch * pl->kd);
   if (rc != AIG_OK) {
     aig_fc_backward_plan_destroy(pl);
@@ -467,12 +620,19 @@ int aig_fc_adamw_update(aig_ctx* ctx, aig_conv_plan* forward_plan, int in_c, int
   float* shift = fc_plan_shift_buffer(forward_plan);
   AIG_REQUIRE(ctx, w_t && shift && in_c > 0 && out_c > 0 && weights && grad_w && m_w && v_w && bias && grad_b && m_b && v_b && t >= 1,
               "aig_fc_adamw_update: needs an FC plan with its weights set, all parameter arrays and t >= 1");
-  adamw_f16_fc_weights_kernel<<<dim3((out_c + 31) / 32, (in_c + 31) / 32), dim3(32, 8), 0, ctx->stream>>>(
-      (__half*)weights, (const __half*)grad_w, (__half*)m_w, (__half*)v_w, w_t, in_c, out_c, lr, t, weight_decay);
-  AIG_LAUNCH_OK(ctx);
-  adamw_f16_fc_bias_kernel<<<(out_c + kThreads - 1) / kThreads, kThreads, 0, ctx->stream>>>((__half*)bias, (const __half*)grad_b, (__half*)m_b,
-                                                                                            (__half*)v_b, shift, out_c, lr, t, weight_decay);
-  AIG_LAUNCH_OK(ctx);
+  AdamwFc a{};
+  a.p = (__half*)weights; a.m = (__half*)m_w; a.v = (__half*)v_w; a.p_t = w_t; a.bias = (__half*)bias; a.m_b = (__half*)m_b; a.v_b = (__half*)v_b;
+  a.g = (const __half*)grad_w; a.g_b = (const __half*)grad_b;
+  a.shift = shift;
+  a.rows = in_c; a.cols = out_c;
+  a.lr = lr; a.wd = weight_decay;
+  a.c1 = 1.0 - pow((double)kBeta1, t);
+  a.c2 = 1.0 - pow((double)kBeta2, t);
+  a.r1 = (float)(1.0 / a.c1);
+  a.r2 = (float)(1.0 / a.c2);
+  const bool vec = out_c % 8 == 0 && (((uintptr_t)weights | (uintptr_t)grad_w | (uintptr_t)m_w | (uintptr_t)v_w) & 15) == 0;
+  const dim3 grid((out_c + kAdamTile - 1) / kAdamTile, (in_c + kAdamTile - 1) / kAdamTile + 1);
+  AIG_CUDA_OK(ctx, launch_pdl(vec ? adamw_f16_fc_kernel<true> : adamw_f16_fc_kernel<false>, grid, dim3(256), 0, ctx->stream, a));
   return AIG_OK;
 }
 
@@ -489,7 +649,12 @@ int aig_fc_backward(aig_fc_backward_plan* pl, const aig_half* x, const aig_half*
               "aig_fc_backward: the weight gradient needs x, the input gradient needs the weights");
   const dim3 tb(kTrTile, 8);
   int rc = AIG_OK;
-  if (grad_w) {
+  if (grad_w && pl->batch <= kWgMaxBatch) {
+    const bool aligned = (((uintptr_t)x | (uintptr_t)grad | (uintptr_t)grad_w) & 15) == 0;
+    AIG_CUDA_OK(ctx, launch_pdl(fc_wgrad_small_kernel, dim3((pl->out_c + kWgTile - 1) / kWgTile, (pl->in_c + kWgTile - 1) / kWgTile), dim3(128), 0, ctx->stream,
+                                (const __half*)x, (const __half*)grad, (__half*)grad_w, (__half*)grad_b, pl->batch, pl->in_c, pl->out_c,
+                                aligned && pl->in_c % 8 == 0 ? 1 : 0, aligned && pl->out_c % 8 == 0 ? 1 : 0));
+  } else if (grad_w) {
     const int widest = pl->in_c > pl->out_c ? pl->in_c : pl->out_c;
     fc_backward_operands_kernel<<<dim3((widest + kTrTile - 1) / kTrTile, 2), tb, 0, ctx->stream>>>(
         (const __half*)x, pl->x_t, pl->in_c, (const __half*)grad, fc_plan_weight_buffer(pl->wgrad), pl->out_c, (__half*)grad_b, pl->batch, pl->kw);

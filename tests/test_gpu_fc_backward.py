@@ -190,3 +190,48 @@ def test_fc_training_steps_against_the_reference_class(env, B, I, N):
         plan.close()
         ref.ref_layer_destroy(rl)
         lib.aig_layer_destroy(ol)
+
+
+@gpu
+@pytest.mark.parametrize("B,I,N", [(1, 8, 2), (64, 64, 64), (65, 72, 70), (256, 136, 18), (257, 64, 48), (16, 200, 130)])
+def test_fc_gradients_and_update_at_tile_edges(env, B, I, N):
+    """Weight gradient straight from the row-major operands (one row to the most it takes, one more; tiles that are not
+    full; columns that are not whole 16-byte pieces), and the layer's AdamW step against the stand-alone kernel's bits."""
+    U = env
+    import torch
+
+    c, pk, lib = U.ctx(), U.pkg(), U.pkg().lib()
+    x, g, W = _case(B + N, B, I, N)
+    want_w, want_b, want_x = O.fc_backward(x, g, W)
+    plan = pk.FcBackwardPlan(c, B, I, N)
+    z = lambda *s: torch.zeros(s, dtype=torch.float16, device="cuda")  # noqa: E731
+    dw, db, dx = z(I, N), z(N), z(B, I)
+    dX, dG, dW = U.dev(x), U.dev(g), U.dev(W)
+    plan.backward(dX, dG, dW, dw, db, dx)
+    c.sync()
+    _check(U.host(dw), want_w, "grad_w")
+    _check(U.host(dx), want_x, "grad_x")
+    U.assert_close16(U.host(db), want_b, max_ulp=1, what="grad_b", atol=1e-4)
+    plan.close()
+    if I % 16:
+        return                                             # no forward plan of that width
+    fwd = pk.FcPlan(c, B, I, N, two_step=True)
+    bias = U.dev(np.linspace(-1, 1, N).astype(f16))
+    fwd.set_weights(dW, bias)
+    mine = [dW.clone(), z(I, N), z(I, N), bias.clone(), z(N), z(N)]
+    other = [t.clone() for t in mine]
+    for step in range(1, 4):
+        gw, gb = (dw * step).contiguous(), (db * step).contiguous()
+        torch.cuda.synchronize()
+        c.call("aig_fc_adamw_update", fwd.handle, I, N, pk.ptr(mine[0]), pk.ptr(gw), pk.ptr(mine[1]), pk.ptr(mine[2]), pk.ptr(mine[3]), pk.ptr(gb),
+               pk.ptr(mine[4]), pk.ptr(mine[5]), 1e-3, step, 1e-6)
+        c.call("aig_adamw_step_f16", pk.ptr(other[0]), pk.ptr(gw), pk.ptr(other[1]), pk.ptr(other[2]), I * N, 1e-3, step, 1e-6)
+        c.call("aig_adamw_step_f16", pk.ptr(other[3]), pk.ptr(gb), pk.ptr(other[4]), pk.ptr(other[5]), N, 1e-3, step, 1e-6)
+        c.sync()
+        for i, (a, b) in enumerate(zip(mine, other)):
+            assert torch.equal(a, b), "step %d, array %d: %d differ" % (step, i, int((a != b).sum()))
+    y = z(B, N)
+    fwd.forward(dX, y)
+    c.sync()
+    U.assert_two_step(U.host(y), O.fc(x, U.host(mine[0]), U.host(mine[3])), U.host(mine[3]).reshape(1, N), what="forward after the update", frac_exact=0.95)
+    fwd.close()
