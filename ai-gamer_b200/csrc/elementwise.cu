@@ -652,7 +652,8 @@ __global__ void cnn_head_kernel(const __half* x, const __half* __restrict__ w1, 
 // column tile, two in-place activations, a conversion) 8192 rows of 512 took 28 us, three times through memory, and 111
 // rows of 256 took 22 us, all launches.  A warp takes 16 rows: they stay in registers in the layout of mma.sync's A operand
 // (a lane has 16-byte pieces of two rows), the row sums are two shuffles, the product with the few output columns is
-// three to four mma tiles.  Bound by the one read of x.
+// three to four mma tiles.  Bound by the one read of x; the weights come K-major from the head's own copy (turning them
+// here, per CTA, was 12 of 20 us).
 constexpr int kTailBlocks = 16, kTailTiles = 4, kTailWarps = 4;
 __global__ void __launch_bounds__(kTailWarps * 32) seq_tail_kernel(const __half* x, const float* __restrict__ gamma, const float* __restrict__ beta,
                                                                    const __half* __restrict__ fcw, const __half* __restrict__ fcb, __half* out_h, float* out_f,
@@ -667,15 +668,10 @@ __global__ void __launch_bounds__(kTailWarps * 32) seq_tail_kernel(const __half*
     s_g[i] = gamma[i];
     s_b[i] = beta[i];
   }
-#pragma unroll 4
-  for (int i = tid * 8; i < n_out * C; i += blockDim.x * 8) {  // [C][n_out], eight at a time
-    const uint4 w8 = *reinterpret_cast<const uint4*>(fcw + i);
-    int k = i / n_out, o = i - k * n_out;
-#pragma unroll
-    for (int e = 0; e < 8; ++e) {
-      s_w[o * stride + k] = reinterpret_cast<const __half*>(&w8)[e];
-      if (++o == n_out) { o = 0; ++k; }
-    }
+#pragma unroll 8
+  for (int i = tid; i < n_out * (C / 8); i += blockDim.x) {  // [n_out][C]
+    const int o = i / (C / 8), k = i - o * (C / 8);
+    *reinterpret_cast<uint4*>(s_w + o * stride + k * 8) = __ldg(reinterpret_cast<const uint4*>(fcw) + i);
   }
   for (int i = tid; i < (tiles * 8 - n_out) * C; i += blockDim.x) s_w[(n_out + i / C) * stride + i % C] = __float2half(0.f);
   griddep_launch_dependents();

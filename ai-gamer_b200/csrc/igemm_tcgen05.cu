@@ -53,16 +53,22 @@ struct IgemmParams {
   int* gerr;
 };
 
-template <int NT, int BK, int MS>
+// Tiled outputs of FC plans (STAGED): the epilogue passes 128 rows x 32 columns at a time through a staging tile per team of
+// four warps, from where one TMA store takes them.  A TMEM lane is a row of the output, so per-lane stores touched 32 rows
+// with 16 bytes each, and with the scalar affine loads the epilogue was three times as long as the tile's loads and MMAs:
+// 8192 x 512 -> 2048 in fp32 (67 MB) took 49 us.
+constexpr int kFcStage = 128 * 128;
+template <int NT, int BK, int MS, bool STAGED = false>
 struct IgemmCfg {
   static constexpr int kSubBytes = kTileM * BK * 2;
   static constexpr int kABytes = MS * kSubBytes;
   static constexpr int kBBytes = NT * BK * 2;
   static constexpr int kStageBytes = kABytes + kBBytes;
-  static constexpr int kStagesRaw = kSmemBudget / kStageBytes;
+  static constexpr int kStaging = STAGED ? 2 * kFcStage : 0;
+  static constexpr int kStagesRaw = (STAGED ? 227 * 1024 - 4096 - kStaging : kSmemBudget) / kStageBytes;
   static constexpr int kStages = kStagesRaw > 8 ? 8 : kStagesRaw;
   static constexpr int kTmemCols = 2 * MS * NT < 32 ? 32 : 2 * MS * NT;
-  static constexpr int kSmemBytes = kStages * kStageBytes + 1024 + 2048 + 256;
+  static constexpr int kSmemBytes = kStages * kStageBytes + kStaging + 1024 + 2048 + 256;
   static_assert(kStages >= 2, "tile too large for a two-stage pipeline");
   static_assert(kTmemCols <= 512, "accumulators exceed TMEM");
 };
@@ -460,10 +466,38 @@ __device__ __forceinline__ void epi_generic_cols(uint32_t t_addr, int col_lo, in
   }
 }
 
-template <int NT, int BK, int MS>
+// One 32-column step of a staged tile: affine (or the two roundings of an FC layer), activation, fp16 or fp32.
+__device__ __forceinline__ void fc_stage_step(uint32_t t_addr, const IgemmParams& p, int n0, uint32_t stage, int row) {
+  uint32_t r[32];
+  tmem_ld_32x32(t_addr, r);
+  tmem_ld_wait();
+#pragma unroll
+  for (int c4 = 0; c4 < 8; ++c4) {  // four columns
+    // (scale and shift are padded to whole tiles)
+    const float4 sc = __ldg(reinterpret_cast<const float4*>(p.scale + n0) + c4), sf = __ldg(reinterpret_cast<const float4*>(p.shift + n0) + c4);
+    const float s4[4] = {sc.x, sc.y, sc.z, sc.w}, f4[4] = {sf.x, sf.y, sf.z, sf.w};
+    float v[4];
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      const float a = __uint_as_float(r[c4 * 4 + e]);
+      v[e] = p.two_step ? __half2float(__float2half(__half2float(__float2half(a)) + f4[e])) : a * s4[e] + f4[e];
+    }
+    if (p.y32) {
+      asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(stage + (uint32_t)row * 128u + (uint32_t)((c4 ^ (row & 7)) << 4)), "r"(__float_as_uint(v[0])),
+                   "r"(__float_as_uint(v[1])), "r"(__float_as_uint(v[2])), "r"(__float_as_uint(v[3])) : "memory");
+    } else {
+      const __half2 lo = __floats2half2_rn(act_apply_fast(v[0], p.act, p.slope), act_apply_fast(v[1], p.act, p.slope));
+      const __half2 hi = __floats2half2_rn(act_apply_fast(v[2], p.act, p.slope), act_apply_fast(v[3], p.act, p.slope));
+      asm volatile("st.shared.v2.b32 [%0], {%1, %2};" ::"r"(stage + (uint32_t)row * 64u + (uint32_t)((((c4 >> 1) ^ ((row >> 1) & 3)) << 4) + (c4 & 1) * 8)),
+                   "r"(*reinterpret_cast<const uint32_t*>(&lo)), "r"(*reinterpret_cast<const uint32_t*>(&hi)) : "memory");
+    }
+  }
+}
+
+template <int NT, int BK, int MS, bool STAGED>
 __global__ void __launch_bounds__(kNumThreads, 1)
-igemm_kernel(const __grid_constant__ CUtensorMap tmapA, const __grid_constant__ CUtensorMap tmapB, const IgemmParams p) {
-  using Cfg = IgemmCfg<NT, BK, MS>;
+igemm_kernel(const __grid_constant__ CUtensorMap tmapA, const __grid_constant__ CUtensorMap tmapB, const __grid_constant__ CUtensorMap tmapY, const IgemmParams p) {
+  using Cfg = IgemmCfg<NT, BK, MS, STAGED>;
   constexpr int kStages = Cfg::kStages;
   extern __shared__ uint8_t smem_raw[];
   const uint32_t raw = smem_u32(smem_raw);
@@ -471,9 +505,9 @@ igemm_kernel(const __grid_constant__ CUtensorMap tmapA, const __grid_constant__ 
   uint8_t* sm = smem_raw + (base - raw);
   const uint32_t sA = base;
   const uint32_t sB = base + kStages * Cfg::kABytes;
-  float* s_scale = reinterpret_cast<float*>(sm + kStages * Cfg::kStageBytes);
+  float* s_scale = reinterpret_cast<float*>(sm + kStages * Cfg::kStageBytes + Cfg::kStaging);
   float* s_shift = s_scale + 256;
-  uint64_t* bars = reinterpret_cast<uint64_t*>(sm + kStages * Cfg::kStageBytes + 2048);
+  uint64_t* bars = reinterpret_cast<uint64_t*>(sm + kStages * Cfg::kStageBytes + Cfg::kStaging + 2048);
   const uint32_t bar_full = smem_u32(bars);                    // [kStages]
   const uint32_t bar_empty = bar_full + 8 * kStages;           // [kStages]
   const uint32_t bar_tfull = bar_empty + 8 * kStages;          // [2]
@@ -651,6 +685,31 @@ igemm_kernel(const __grid_constant__ CUtensorMap tmapA, const __grid_constant__ 
       const float* sc = p.n_tiles == 1 ? s_scale : p.scale + n_tile * NT;
       const float* sf = p.n_tiles == 1 ? s_shift : p.shift + n_tile * NT;
       const int nb = n_tile * NT;
+      if constexpr (STAGED) {
+        // the four warps of a team go on together: their steps meet at named barriers
+        const int team = (warp - 2) >> 2;
+        ok = named_bar_and(1 + team, 128, mbar_wait_bounded(bar_tfull + 8 * acc, acc_phase, s_abort, p.gerr, 301));
+        if (!ok) break;
+        tc_fence_after();
+        const uint32_t stage = base + kStages * Cfg::kStageBytes + (uint32_t)(team * kFcStage);
+        const bool issuer = ((warp - 2) & 3) == 0 && lane == 0;
+#pragma unroll 1
+        for (int c0 = col_lo; c0 < col_hi; c0 += 32) {
+          if (issuer) bulk_wait_group_read0();  // the store before this one has left the tile
+          named_bar_sync(1 + team, 128);
+          fc_stage_step(tmem_base + (uint32_t)(acc * NT + c0) + ((uint32_t)(q * 32) << 16), p, nb + c0, stage, row_in_tile);
+          fence_proxy_async_smem();
+          named_bar_sync(1 + team, 128);
+          if (issuer) {
+            tma_store_2d(&tmapY, stage, nb + c0, m_sup * kTileM);
+            bulk_commit_group();
+          }
+        }
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(bar_tempty + 8 * acc);
+        continue;
+      }
       if (!mbar_wait_bounded(bar_tfull + 8 * acc, acc_phase, s_abort, p.gerr, 301)) { ok = false; break; }
       tc_fence_after();
 #pragma unroll 1
@@ -687,6 +746,7 @@ igemm_kernel(const __grid_constant__ CUtensorMap tmapA, const __grid_constant__ 
       __syncwarp();
       if (lane == 0) mbar_arrive(bar_tempty + 8 * acc);
     }
+    if (STAGED && ((warp - 2) & 3) == 0 && lane == 0) bulk_wait_group0();
   }
 
   // ------------------------------------------------------------------ common exit
@@ -1439,6 +1499,10 @@ struct aig_conv_plan {
   aig_conv_desc d{};
   int Do = 1, Ho = 1, Wo = 1;
   bool is_fc = false;
+  bool staged = false;                         // this forward's output tiles leave by TMA (FC plans; see kFcStage)
+  CUtensorMap tmapFc{};                        // the output for that
+  const void* tmapFc_ptr = nullptr;
+  bool tmapFc_f32 = false;
   bool skinny = false;                         // FC plans of few rows: see skinny_fc.cu
   int BK = 64, NT = 64, MS = 1, Kpad = 0, taps = 1, Ktot = 0;
   IgemmParams prm{};
@@ -1471,16 +1535,16 @@ struct aig_conv_plan {
 
 namespace {
 
-template <int NT, int BK, int MS>
+template <int NT, int BK, int MS, bool STAGED = false>
 int launch_igemm(aig_conv_plan* pl) {
-  using Cfg = IgemmCfg<NT, BK, MS>;
+  using Cfg = IgemmCfg<NT, BK, MS, STAGED>;
   static bool attr_set[64] = {};
   aig_ctx* ctx = pl->ctx;
   if (!attr_set[ctx->device & 63]) {
-    AIG_CUDA_OK(ctx, cudaFuncSetAttribute(igemm_kernel<NT, BK, MS>, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::kSmemBytes));
+    AIG_CUDA_OK(ctx, cudaFuncSetAttribute(igemm_kernel<NT, BK, MS, STAGED>, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::kSmemBytes));
     attr_set[ctx->device & 63] = true;
   }
-  AIG_CUDA_OK(ctx, launch_pdl(igemm_kernel<NT, BK, MS>, dim3(pl->grid), dim3(kNumThreads), Cfg::kSmemBytes, ctx->stream, pl->tmapA, pl->tmapB, pl->prm));
+  AIG_CUDA_OK(ctx, launch_pdl(igemm_kernel<NT, BK, MS, STAGED>, dim3(pl->grid), dim3(kNumThreads), Cfg::kSmemBytes, ctx->stream, pl->tmapA, pl->tmapB, pl->tmapFc, pl->prm));
   return AIG_OK;
 }
 
@@ -1495,6 +1559,13 @@ int dispatch_bk(aig_conv_plan* pl) {
 }
 
 int dispatch(aig_conv_plan* pl) {
+  if (pl->staged) {
+    switch (pl->NT) {
+      case 64: return launch_igemm<64, 64, 1, true>(pl);
+      case 128: return launch_igemm<128, 64, 1, true>(pl);
+      case 256: return launch_igemm<256, 64, 1, true>(pl);
+    }
+  }
   const int key = pl->NT * 10 + pl->MS;
   switch (key) {
     case 321: return dispatch_bk<32, 1>(pl);
@@ -1546,10 +1617,28 @@ int encode_A(aig_conv_plan* pl, const void* x) {
   return AIG_OK;
 }
 
+// Output of an FC plan as a 2-D tensor, box 32 columns x 128 rows.
+int encode_fc_output(aig_conv_plan* pl, const void* y) {
+  EncodeTiledFn enc = get_encode_fn();
+  if (!enc) return aig_fail(pl->ctx, AIG_ERR_CUDA, "cuTensorMapEncodeTiled entry point not available");
+  const cuuint64_t es = pl->out_f32 ? 4 : 2;
+  cuuint64_t dims[2] = {(cuuint64_t)pl->d.out_c, (cuuint64_t)pl->d.in_w};
+  cuuint64_t strides[1] = {dims[0] * es};
+  cuuint32_t box[2] = {32u, 128u}, estr[2] = {1, 1};
+  const CUresult r = enc(&pl->tmapFc, pl->out_f32 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT32 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, const_cast<void*>(y), dims, strides, box,
+                         estr, CU_TENSOR_MAP_INTERLEAVE_NONE, pl->out_f32 ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_64B,
+                         CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  if (r != CUDA_SUCCESS) return aig_fail(pl->ctx, AIG_ERR_CUDA, "cuTensorMapEncodeTiled(fc output) failed: %d", (int)r);
+  pl->tmapFc_ptr = y;
+  pl->tmapFc_f32 = pl->out_f32;
+  return AIG_OK;
+}
+
 int plan_finish(aig_ctx* ctx, aig_conv_plan* pl) {
   const aig_conv_desc& d = pl->d;
   // K blocking: the largest of 64/32/16 channels that divides in_c
-  if (d.in_c % 64 == 0) pl->BK = 64;
+  // (an FC's last block may reach past K: the TMA unit fills both operands with zeros there)
+  if (d.in_c % 64 == 0 || (pl->is_fc && d.in_c % 16 == 0 && d.in_c > 64)) pl->BK = 64;
   else if (d.in_c % 32 == 0) pl->BK = 32;
   else if (d.in_c % 16 == 0) pl->BK = 16;
   else return aig_fail(ctx, AIG_ERR_UNSUPPORTED, "igemm needs in_c %% 16 == 0 (got %d); 3-channel inputs use the conv0 plans", d.in_c);
@@ -1572,6 +1661,7 @@ int plan_finish(aig_ctx* ctx, aig_conv_plan* pl) {
       best_tw = tw;
     }
   }
+  if (pl->is_fc) best_tw = kTileM;  // rows of one matrix: one box a tile, rows past the end read as zeros
   IgemmParams& p = pl->prm;
   p.tw = best_tw;
   p.segs = kTileM / best_tw;
@@ -1598,7 +1688,7 @@ int plan_finish(aig_ctx* ctx, aig_conv_plan* pl) {
   while (ms > 1 && (long long)ceil_div(m_tiles, ms) * p.n_tiles < 2LL * ctx->sm_count) ms /= 2;
   pl->MS = ms;
   p.m_super = ceil_div(m_tiles, ms);
-  p.cblocks = d.in_c / pl->BK;
+  p.cblocks = ceil_div(d.in_c, pl->BK);
   p.num_kb = pl->taps * p.cblocks;
   p.taps_hw = d.kh * d.kw;
   p.kw = d.kw;
@@ -2275,6 +2365,11 @@ int aig_conv_forward(aig_conv_plan* pl, const aig_half* x, const aig_half* resid
   if (pl->skinny && !residual) return run_skinny(pl, x, y, FcTail{});
   if (pl->tmapA_ptr != x) {
     const int rc = encode_A(pl, x);
+    if (rc != AIG_OK) return rc;
+  }
+  pl->staged = pl->is_fc && !residual && pl->BK == 64 && pl->MS == 1 && pl->NT >= 64 && pl->prm.tw == kTileM && pl->d.out_c % 8 == 0;
+  if (pl->staged && (pl->tmapFc_ptr != y || pl->tmapFc_f32 != pl->out_f32)) {
+    const int rc = encode_fc_output(pl, y);
     if (rc != AIG_OK) return rc;
   }
   pl->prm.residual = (const __half*)residual;

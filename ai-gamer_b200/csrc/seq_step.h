@@ -35,7 +35,7 @@ int seq_step_fused_run(SeqStepFused* s, const aig_half* emb, const aig_half* fea
                        aig_half* logits, float* out_f32, bool after_encoder);
 int seq_step_fused_reset(SeqStepFused* s);
 
-// The end of the full-sequence forward in one launch (elementwise.cu): row LayerNorm, FC (weights [c][n_out], two-step
+// The end of the full-sequence forward in one launch (elementwise.cu): row LayerNorm, FC (weights [n_out][c], two-step
 // rounding), sigmoid on the first n_sigmoid outputs and tanh on the rest, as fp16 and fp32.
 bool seq_tail_supported(int c, int n_out);
 int seq_tail_forward(aig_ctx* ctx, const aig_half* x, const float* gamma, const float* beta, const aig_half* fc_w, const aig_half* fc_b, aig_half* out_half,

@@ -30,6 +30,7 @@ struct aig_seq {
   uint8_t* params = nullptr;  // device copy of the blob, every array 256-byte aligned
   aig_half *lstm_w = nullptr, *wq = nullptr, *wk = nullptr, *wv = nullptr, *wo = nullptr, *fcw = nullptr, *fcb = nullptr;
   float *ln_g = nullptr, *ln_b = nullptr;
+  aig_half* fcw_t = nullptr;  // fcw as [n_out][hidden], for seq_tail_forward
   aig_half *y = nullptr, *a = nullptr, *n = nullptr, *logits = nullptr;  // [B][T][.] work buffers
   aig_half *h_state = nullptr, *c_state = nullptr;                        // [layers][B][hid]
   float* out_f32 = nullptr;
@@ -90,7 +91,8 @@ int seq_create_with_bridge(aig_ctx* ctx, const aig_seq_config* cfg, int features
        cudaMalloc(&m->out_f32, rows * c.n_out * 4) != cudaSuccess || cudaMalloc(&m->h_state, state * 2) != cudaSuccess ||
        cudaMalloc(&m->c_state, state * 2) != cudaSuccess || cudaMemset(m->h_state, 0, state * 2) != cudaSuccess ||
        cudaMemset(m->c_state, 0, state * 2) != cudaSuccess ||
-       cudaMalloc(&m->params, aig_seq_param_bytes(&c) + 16 * 256) != cudaSuccess))
+       cudaMalloc(&m->params, aig_seq_param_bytes(&c) + 16 * 256) != cudaSuccess ||
+       cudaMalloc(&m->fcw_t, E * c.n_out * 2) != cudaSuccess))
     rc = AIG_ERR_CUDA;
   if (rc == AIG_OK && fused) rc = seq_step_fused_create(ctx, sc, &m->fused);
   if (rc != AIG_OK) {
@@ -124,7 +126,7 @@ int aig_seq_destroy(aig_seq* m) {
   seq_step_fused_destroy(m->fused);
   aig_conv_plan_destroy(m->fc_full);
   aig_conv_plan_destroy(m->fc_step);
-  void* bufs[] = {m->params, m->y, m->a, m->n, m->logits, m->out_f32, m->h_state, m->c_state};
+  void* bufs[] = {m->params, m->y, m->a, m->n, m->logits, m->out_f32, m->h_state, m->c_state, m->fcw_t};
   for (void* b : bufs) cudaFree(b);
   delete m;
   return AIG_OK;
@@ -148,6 +150,11 @@ int aig_seq_load_memory(aig_seq* m, const void* blob, size_t bytes) {
     src_off += sizes[i];
     dst_off = align256(dst_off + sizes[i]);
   }
+  std::vector<aig_half> turned(E * c.n_out);
+  const uint8_t* fcw_host = (const uint8_t*)blob + src_off - sizes[8] - sizes[7];
+  for (size_t k = 0; k < E; ++k)
+    for (int o = 0; o < c.n_out; ++o) memcpy(&turned[o * E + k], fcw_host + (k * c.n_out + o) * 2, 2);
+  SEQ_OK(m, aig_memcpy(m->ctx, m->fcw_t, turned.data(), turned.size() * 2));
   SEQ_OK(m, aig_ctx_sync(m->ctx));  // the caller may free the blob now
   SEQ_OK(m, aig_lstm_plan_set_weights(m->lstm_full, m->lstm_w));
   if (!m->fused) SEQ_OK(m, aig_lstm_plan_set_weights(m->lstm_step, m->lstm_w));
@@ -162,7 +169,7 @@ int aig_seq_load_memory(aig_seq* m, const void* blob, size_t bytes) {
 static int seq_tail(aig_seq* m, aig_conv_plan* fc, int rows) {
   const aig_seq_config& c = m->cfg;
   if (seq_tail_supported(c.hidden, c.n_out)) {
-    SEQ_OK(m, seq_tail_forward(m->ctx, m->a, m->ln_g, m->ln_b, m->fcw, m->fcb, m->logits, m->out_f32, rows, c.hidden, c.n_out, c.n_sigmoid, 1e-5f));
+    SEQ_OK(m, seq_tail_forward(m->ctx, m->a, m->ln_g, m->ln_b, m->fcw_t, m->fcb, m->logits, m->out_f32, rows, c.hidden, c.n_out, c.n_sigmoid, 1e-5f));
     return AIG_OK;
   }
   SEQ_OK(m, aig_layernorm_rows_forward(m->ctx, m->n, m->a, m->ln_g, m->ln_b, rows, c.hidden, 1e-5f));
