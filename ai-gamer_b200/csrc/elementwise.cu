@@ -650,15 +650,16 @@ __global__ void cnn_head_kernel(const __half* x, const __half* __restrict__ w1, 
 
 // Row LayerNorm, FC, sigmoid / tanh of the sequence head.  As separate launches (row LayerNorm, a GEMM of one 32-wide
 // column tile, two in-place activations, a conversion) 8192 rows of 512 took 28 us, three times through memory, and 111
-// rows of 256 took 22 us, all launches.  A warp takes 16 rows: they stay in registers in the layout of mma.sync's A operand
-// (a lane has 16-byte pieces of two rows), the row sums are two shuffles, the product with the few output columns is
+// rows of 256 took 22 us, all launches.  A warp takes 16 rows in the layout of mma.sync's A operand
+// (a lane has 16-byte pieces of two rows; the second and third pass over them find them in L1), the row sums are two shuffles, the product with the few output columns is
 // three to four mma tiles.  Bound by the one read of x; the weights come K-major from the head's own copy (turning them
 // here, per CTA, was 12 of 20 us).
-constexpr int kTailBlocks = 16, kTailTiles = 4, kTailWarps = 4;
+constexpr int kTailMaxC = 512, kTailTiles = 4, kTailWarps = 4;
 __global__ void __launch_bounds__(kTailWarps * 32) seq_tail_kernel(const __half* x, const float* __restrict__ gamma, const float* __restrict__ beta,
                                                                    const __half* __restrict__ fcw, const __half* __restrict__ fcb, __half* out_h, float* out_f,
                                                                    int rows, int C, int n_out, int n_sig, float eps) {
   extern __shared__ __align__(16) uint8_t tail_smem[];
+  __shared__ float s_bias[8 * kTailTiles];
   const int stride = C + 8;                                       // halfs: rows of the weights on different banks
   float* s_g = reinterpret_cast<float*>(tail_smem);               // gamma, beta
   float* s_b = s_g + C;
@@ -673,41 +674,40 @@ __global__ void __launch_bounds__(kTailWarps * 32) seq_tail_kernel(const __half*
     const int o = i / (C / 8), k = i - o * (C / 8);
     *reinterpret_cast<uint4*>(s_w + o * stride + k * 8) = __ldg(reinterpret_cast<const uint4*>(fcw) + i);
   }
-  for (int i = tid; i < (tiles * 8 - n_out) * C; i += blockDim.x) s_w[(n_out + i / C) * stride + i % C] = __float2half(0.f);
+  for (int o = n_out; o < tiles * 8; ++o)
+    for (int k = tid * 8; k < C; k += blockDim.x * 8) *reinterpret_cast<uint4*>(s_w + o * stride + k) = make_uint4(0, 0, 0, 0);
+  if (tid < n_out) s_bias[tid] = __half2float(fcb[tid]);
   griddep_launch_dependents();
   griddep_wait();
   __syncthreads();
   for (int r0 = (blockIdx.x * kTailWarps + (tid >> 5)) * 16; r0 < rows; r0 += gridDim.x * kTailWarps * 16) {
-    uint4 v[2][kTailBlocks];
+    const uint4* src[2];
     float mu[2], rstd[2];
 #pragma unroll
     for (int h = 0; h < 2; ++h) {
-      const int r = min(r0 + g + 8 * h, rows - 1);
-      const uint4* src = reinterpret_cast<const uint4*>(x + (size_t)r * C) + q;
-#pragma unroll
-      for (int kb = 0; kb < kTailBlocks; ++kb) v[h][kb] = kb < nb ? src[kb * 4] : make_uint4(0, 0, 0, 0);
-    }
-#pragma unroll
-    for (int h = 0; h < 2; ++h) {
+      src[h] = reinterpret_cast<const uint4*>(x + (size_t)min(r0 + g + 8 * h, rows - 1) * C) + q;
       float s = 0.f, ss = 0.f;
-#pragma unroll
-      for (int kb = 0; kb < kTailBlocks; ++kb)
+#pragma unroll 8
+      for (int kb = 0; kb < nb; ++kb) {
+        const uint4 v = src[h][kb * 4];
 #pragma unroll
         for (int e = 0; e < 4; ++e) {
-          const float2 f = __half22float2(reinterpret_cast<const __half2*>(&v[h][kb])[e]);
+          const float2 f = __half22float2(reinterpret_cast<const __half2*>(&v)[e]);
           s += f.x + f.y;
         }
+      }
       s += __shfl_xor_sync(0xffffffffu, s, 1);
       s += __shfl_xor_sync(0xffffffffu, s, 2);
       mu[h] = s / (float)C;
+#pragma unroll 8
+      for (int kb = 0; kb < nb; ++kb) {
+        const uint4 v = src[h][kb * 4];
 #pragma unroll
-      for (int kb = 0; kb < kTailBlocks; ++kb)
-        if (kb < nb)
-#pragma unroll
-          for (int e = 0; e < 4; ++e) {
-            const float2 f = __half22float2(reinterpret_cast<const __half2*>(&v[h][kb])[e]);
-            ss += (f.x - mu[h]) * (f.x - mu[h]) + (f.y - mu[h]) * (f.y - mu[h]);
-          }
+        for (int e = 0; e < 4; ++e) {
+          const float2 f = __half22float2(reinterpret_cast<const __half2*>(&v)[e]);
+          ss += (f.x - mu[h]) * (f.x - mu[h]) + (f.y - mu[h]) * (f.y - mu[h]);
+        }
+      }
       ss += __shfl_xor_sync(0xffffffffu, ss, 1);
       ss += __shfl_xor_sync(0xffffffffu, ss, 2);
       rstd[h] = rsqrtf(ss / (float)C + eps);
@@ -715,9 +715,9 @@ __global__ void __launch_bounds__(kTailWarps * 32) seq_tail_kernel(const __half*
     float acc[kTailTiles][4];
 #pragma unroll
     for (int t = 0; t < kTailTiles; ++t) acc[t][0] = acc[t][1] = acc[t][2] = acc[t][3] = 0.f;
-#pragma unroll
-    for (int kb = 0; kb < kTailBlocks; ++kb) {
-      if (kb >= nb) break;
+#pragma unroll 2
+    for (int kb = 0; kb < nb; ++kb) {
+      const uint4 v[2] = {src[0][kb * 4], src[1][kb * 4]};
       const int k0 = kb * 32 + q * 8;
       float gm[8], bt[8];
 #pragma unroll
@@ -730,7 +730,7 @@ __global__ void __launch_bounds__(kTailWarps * 32) seq_tail_kernel(const __half*
       for (int h = 0; h < 2; ++h)
 #pragma unroll
         for (int e = 0; e < 4; ++e) {
-          const float2 f = __half22float2(reinterpret_cast<const __half2*>(&v[h][kb])[e]);
+          const float2 f = __half22float2(reinterpret_cast<const __half2*>(&v[h])[e]);
           const __half2 n = __floats2half2_rn((f.x - mu[h]) * rstd[h] * gm[2 * e] + bt[2 * e], (f.y - mu[h]) * rstd[h] * gm[2 * e + 1] + bt[2 * e + 1]);
           a[h][e] = *reinterpret_cast<const uint32_t*>(&n);
         }
@@ -754,7 +754,7 @@ __global__ void __launch_bounds__(kTailWarps * 32) seq_tail_kernel(const __half*
         const int r = r0 + g + 8 * (e >> 1), o = t * 8 + 2 * q + (e & 1);
         if (t >= tiles || r >= rows || o >= n_out) continue;
         const float s = __half2float(__float2half(acc[t][e]));                  // FCLayer: GEMM result stored as half,
-        const float y = __half2float(__float2half(s + __half2float(fcb[o])));   // then bias added and stored again
+        const float y = __half2float(__float2half(s + s_bias[o]));              // then bias added and stored again
         const __half hv = __float2half(o < n_sig ? 1.0f / (1.0f + expf(-y)) : tanhf(y));
         out_h[(size_t)r * n_out + o] = hv;
         out_f[(size_t)r * n_out + o] = __half2float(hv);
@@ -764,7 +764,7 @@ __global__ void __launch_bounds__(kTailWarps * 32) seq_tail_kernel(const __half*
 
 }  // namespace
 
-bool seq_tail_supported(int c, int n_out) { return c % 32 == 0 && c <= 32 * kTailBlocks && n_out >= 1 && n_out <= 8 * kTailTiles; }
+bool seq_tail_supported(int c, int n_out) { return c % 32 == 0 && c <= kTailMaxC && n_out >= 1 && n_out <= 8 * kTailTiles; }
 int seq_tail_forward(aig_ctx* ctx, const aig_half* x, const float* gamma, const float* beta, const aig_half* fc_w, const aig_half* fc_b, aig_half* out_half,
                      float* out_f32, int rows, int c, int n_out, int n_sigmoid, float eps) {
   DeviceGuard guard(ctx->device);

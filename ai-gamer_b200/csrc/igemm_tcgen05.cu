@@ -466,30 +466,40 @@ __device__ __forceinline__ void epi_generic_cols(uint32_t t_addr, int col_lo, in
   }
 }
 
-// One 32-column step of a staged tile: affine (or the two roundings of an FC layer), activation, fp16 or fp32.
+// One 32-column step of a staged tile.  F32: affine, fp32; TWO: the two roundings of an FC layer, fp16; else affine and
+// activation, fp16.
+template <bool F32, bool TWO, int ACT>
 __device__ __forceinline__ void fc_stage_step(uint32_t t_addr, const IgemmParams& p, int n0, uint32_t stage, int row) {
   uint32_t r[32];
   tmem_ld_32x32(t_addr, r);
   tmem_ld_wait();
 #pragma unroll
-  for (int c4 = 0; c4 < 8; ++c4) {  // four columns
-    // (scale and shift are padded to whole tiles)
-    const float4 sc = __ldg(reinterpret_cast<const float4*>(p.scale + n0) + c4), sf = __ldg(reinterpret_cast<const float4*>(p.shift + n0) + c4);
-    const float s4[4] = {sc.x, sc.y, sc.z, sc.w}, f4[4] = {sf.x, sf.y, sf.z, sf.w};
-    float v[4];
+  for (int c = 0; c < 4; ++c) {  // eight columns (scale and shift are padded to whole tiles)
+    float s8[8], f8[8], v[8];
 #pragma unroll
-    for (int e = 0; e < 4; ++e) {
-      const float a = __uint_as_float(r[c4 * 4 + e]);
-      v[e] = p.two_step ? __half2float(__float2half(__half2float(__float2half(a)) + f4[e])) : a * s4[e] + f4[e];
+    for (int e = 0; e < 8; e += 4) {
+      if constexpr (!TWO) *reinterpret_cast<float4*>(s8 + e) = __ldg(reinterpret_cast<const float4*>(p.scale + n0 + c * 8 + e));
+      *reinterpret_cast<float4*>(f8 + e) = __ldg(reinterpret_cast<const float4*>(p.shift + n0 + c * 8 + e));
     }
-    if (p.y32) {
-      asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(stage + (uint32_t)row * 128u + (uint32_t)((c4 ^ (row & 7)) << 4)), "r"(__float_as_uint(v[0])),
-                   "r"(__float_as_uint(v[1])), "r"(__float_as_uint(v[2])), "r"(__float_as_uint(v[3])) : "memory");
+#pragma unroll
+    for (int e = 0; e < 8; ++e) {
+      const float a = __uint_as_float(r[c * 8 + e]);
+      if constexpr (TWO) v[e] = __half2float(__float2half(a)) + f8[e];
+      else v[e] = act_ct<ACT>(a * s8[e] + f8[e], p.slope);
+    }
+    if constexpr (F32) {
+#pragma unroll
+      for (int h = 0; h < 2; ++h)
+        asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(stage + (uint32_t)row * 128u + (uint32_t)(((2 * c + h) ^ (row & 7)) << 4)),
+                     "r"(__float_as_uint(v[4 * h])), "r"(__float_as_uint(v[4 * h + 1])), "r"(__float_as_uint(v[4 * h + 2])), "r"(__float_as_uint(v[4 * h + 3]))
+                     : "memory");
     } else {
-      const __half2 lo = __floats2half2_rn(act_apply_fast(v[0], p.act, p.slope), act_apply_fast(v[1], p.act, p.slope));
-      const __half2 hi = __floats2half2_rn(act_apply_fast(v[2], p.act, p.slope), act_apply_fast(v[3], p.act, p.slope));
-      asm volatile("st.shared.v2.b32 [%0], {%1, %2};" ::"r"(stage + (uint32_t)row * 64u + (uint32_t)((((c4 >> 1) ^ ((row >> 1) & 3)) << 4) + (c4 & 1) * 8)),
-                   "r"(*reinterpret_cast<const uint32_t*>(&lo)), "r"(*reinterpret_cast<const uint32_t*>(&hi)) : "memory");
+      uint4 o;
+      __half2* oh = reinterpret_cast<__half2*>(&o);
+#pragma unroll
+      for (int e = 0; e < 4; ++e) oh[e] = __floats2half2_rn(v[2 * e], v[2 * e + 1]);
+      asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(stage + (uint32_t)row * 64u + (uint32_t)((c ^ ((row >> 1) & 3)) << 4)), "r"(o.x), "r"(o.y),
+                   "r"(o.z), "r"(o.w) : "memory");
     }
   }
 }
@@ -697,7 +707,13 @@ igemm_kernel(const __grid_constant__ CUtensorMap tmapA, const __grid_constant__ 
         for (int c0 = col_lo; c0 < col_hi; c0 += 32) {
           if (issuer) bulk_wait_group_read0();  // the store before this one has left the tile
           named_bar_sync(1 + team, 128);
-          fc_stage_step(tmem_base + (uint32_t)(acc * NT + c0) + ((uint32_t)(q * 32) << 16), p, nb + c0, stage, row_in_tile);
+          const uint32_t t_addr = tmem_base + (uint32_t)(acc * NT + c0) + ((uint32_t)(q * 32) << 16);
+          if (p.y32) fc_stage_step<true, false, AIG_ACT_NONE>(t_addr, p, nb + c0, stage, row_in_tile);
+          else if (p.two_step && p.act == AIG_ACT_NONE) fc_stage_step<false, true, AIG_ACT_NONE>(t_addr, p, nb + c0, stage, row_in_tile);
+          else if (p.act == AIG_ACT_RELU) fc_stage_step<false, false, AIG_ACT_RELU>(t_addr, p, nb + c0, stage, row_in_tile);
+          else if (p.act == AIG_ACT_SWISH) fc_stage_step<false, false, AIG_ACT_SWISH>(t_addr, p, nb + c0, stage, row_in_tile);
+          else if (p.act == AIG_ACT_LEAKY) fc_stage_step<false, false, AIG_ACT_LEAKY>(t_addr, p, nb + c0, stage, row_in_tile);
+          else fc_stage_step<false, false, AIG_ACT_NONE>(t_addr, p, nb + c0, stage, row_in_tile);
           fence_proxy_async_smem();
           named_bar_sync(1 + team, 128);
           if (issuer) {
@@ -2367,7 +2383,7 @@ int aig_conv_forward(aig_conv_plan* pl, const aig_half* x, const aig_half* resid
     const int rc = encode_A(pl, x);
     if (rc != AIG_OK) return rc;
   }
-  pl->staged = pl->is_fc && !residual && pl->BK == 64 && pl->MS == 1 && pl->NT >= 64 && pl->prm.tw == kTileM && pl->d.out_c % 8 == 0;
+  pl->staged = pl->is_fc && !residual && pl->BK == 64 && pl->MS == 1 && pl->NT >= 64 && pl->prm.tw == kTileM && pl->d.out_c % 8 == 0 && !(pl->d.two_step && pl->d.act != AIG_ACT_NONE);
   if (pl->staged && (pl->tmapFc_ptr != y || pl->tmapFc_f32 != pl->out_f32)) {
     const int rc = encode_fc_output(pl, y);
     if (rc != AIG_OK) return rc;

@@ -1,4 +1,4 @@
-// skinny_fc.cu -- y = x . W^T for few rows of x (at most 128), W K-major as the FC plans keep it.
+// skinny_fc.cu -- y = x . W^T for few rows of x (at most 64), W K-major as the FC plans keep it.
 //
 // With few rows the product reads its weights once and does next to nothing with them, so what counts is how many SMs
 // stream them and how much each has in flight.  The tiled GEMM gives such a layer N / 64 CTAs that walk K alone: 36864 ->
@@ -29,7 +29,7 @@ __device__ __forceinline__ float round_half(float v) { return __half2float(__flo
 // NT = tiles of eight rows of x
 template <int NT>
 __global__ void __launch_bounds__(kThreads, NT <= 4 ? 2 : 1) skinny_fc_kernel(const SkinnyFc p, int share) {
-  constexpr int U = NT <= 1 ? 8 : (NT <= 2 ? 6 : (NT <= 4 ? 4 : (NT <= 8 ? 2 : 1)));  // blocks of K in flight
+  constexpr int U = NT <= 1 ? 8 : (NT <= 2 ? 6 : (NT <= 4 ? 4 : 2));  // blocks of K in flight
   __shared__ float red[kWarps / 2][16][NT * 8 + 1];
   __shared__ float sum[16 * NT * 8];
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, q = lane & 3;
@@ -142,8 +142,7 @@ int skinny_fc_forward(aig_ctx* ctx, const SkinnyFc& p) {
   if (tiles <= 1) e = launch<1>(ctx, p, ctas);
   else if (tiles <= 2) e = launch<2>(ctx, p, ctas);
   else if (tiles <= 4) e = launch<4>(ctx, p, ctas);
-  else if (tiles <= 8) e = launch<8>(ctx, p, ctas);
-  else e = launch<16>(ctx, p, ctas);
+  else e = launch<8>(ctx, p, ctas);
   AIG_CUDA_OK(ctx, e);
   return AIG_OK;
 }

@@ -22,9 +22,9 @@ struct SkinnyFc {
   float* y32;
   FcTail tail;
 };
-// Rows up to which an FC plan takes it.  Against the tiled GEMM at K = 1024, N = 1024: 6.2 us for 64 rows and 9.3 for 128,
-// the GEMM 9.9 and (144 rows) 12.3.
-constexpr int kSkinnyRows = 128;
+// Rows up to which an FC plan takes it: 6.2 us for 64 rows at K = 1024, N = 1024, 8.7 for 111 rows at K = 256, N = 768, where
+// the tiled GEMM takes 7.3.
+constexpr int kSkinnyRows = 64;
 int skinny_fc_forward(aig_ctx* ctx, const SkinnyFc& p);
 
 // igemm_tcgen05.cu:
