@@ -1916,6 +1916,27 @@ bool pconv_choose_tile(aig_ctx* ctx, aig_conv_plan* pl, const PconvNtOption* opt
   // all of its traffic
   const bool small = ceil_div_ll(total_q, kTileM) * 4 <= ctx->sm_count && !f_nt;
   q.dist_n = 0;
+  // M tiles for less than one wave (batches in between): a CTA's time is the fetch of its weights and patches, about 37 B/clk,
+  // and narrower N tiles share the weights out over the idle SMs at the price of a patch per N tile.  The tiling with the
+  // least time by that count, main tiles first and the four times shorter shortcut tiles after them, where it is at least
+  // a tenth better than the widest.  32 frames of 144x256: RESULT3
+  int spread = -1;
+  const long long m1 = ceil_div_ll(total_q, kTileM);
+  if (!small && !f_nt && m1 <= ctx->sm_count) {
+    double least = 0.0;
+    for (int o = 0; o < n_opts; ++o) {
+      const int NT = opts[o].NT, dense_kb = q.taps * q.cblocks, mains = std::min(opts[o].n_tiles, opts[o].sparse_tile0), shorts = opts[o].n_tiles - mains;
+      const double patch = (double)q.cblocks * region_rows_of(kTileM) * 128.0, mma = NT == 64 ? 49.0 : (NT == 128 ? 65.0 : 128.0);
+      auto item = [&](double kb) { return std::max(kb * 4.0 * mma, (kb * NT * 128.0 + patch) / 37.0) + 3000.0; };
+      const double main_clk = item(dense_kb), short_clk = shorts ? item((double)q.taps * q.sub_cblocks) : 0.0;
+      const double rounds = (double)ceil_div_ll(m1 * mains, ctx->sm_count);
+      const double clk = std::max(rounds * main_clk, (double)m1 * (mains * main_clk + shorts * short_clk) / ctx->sm_count);
+      if (o == 0 || clk < (spread < 0 ? 0.9 : 1.0) * least) {
+        if (o) spread = o;
+        least = clk;
+      }
+    }
+  }
   // epilogue warps: 16 (two teams) measured 5-20 % slower than 8 on every layer of the encoder, the register
   // cap of a 640-thread CTA costs more than the extra warps hide; tuning builds can still select it
   int ew = 8;
@@ -1924,14 +1945,16 @@ bool pconv_choose_tile(aig_ctx* ctx, aig_conv_plan* pl, const PconvNtOption* opt
 #endif
   pl->pc_EW = ew;
   for (int oo = 0; oo < n_opts && best < 0; ++oo) {
-    const int o = small ? n_opts - 1 - oo : oo;
+    const int o = small ? n_opts - 1 - oo : (spread >= 0 ? (oo == 0 ? spread : oo - 1) : oo);
     const int NT = opts[o].NT, wblock = NT * 128;
     const int dense_kb = q.taps * q.cblocks;
     const int kPconvBudget = pconv_budget(ew, NT == 64, pl->res_tiles);
     if (f_nt && NT != f_nt) continue;
-    if (!small && NT == 64 && o > 0) continue;  // the 64-wide tiling of a wider layer is for the small regime only
+    const bool spread_this = spread >= 0 && oo == 0;
+    if (!small && !spread_this && NT == 64 && o > 0) continue;  // the 64-wide tiling of a wider layer is for those two regimes only
     int ms_top = 256 / NT < 1 ? 1 : 256 / NT;
-    if (small) {
+    q.dist_n = 0;
+    if (small || spread_this) {
       ms_top = 1;
       q.dist_n = opts[o].n_tiles > 1 ? 1 : 0;
     }
@@ -2027,7 +2050,8 @@ bool pconv_choose_tile(aig_ctx* ctx, aig_conv_plan* pl, const PconvNtOption* opt
   }
   // a launch with a main and a (sparse) shortcut N tile whose M tiles do not fill the SMs evenly: the (M tile,
   // N tile) pairs become the work items, assigned to the CTAs longest first
-  bool lpt = !pl->pc_pair && !q.dist_n && q.n_tiles == 2 && q.sparse_tile0 == 1 && q.m_tiles % ctx->sm_count != 0;
+  bool lpt = !pl->pc_pair && (q.dist_n ? spread >= 0 && best_opt == spread && q.sparse_tile0 < q.n_tiles
+                                       : q.n_tiles == 2 && q.sparse_tile0 == 1 && q.m_tiles % ctx->sm_count != 0);
 #ifdef AIG_TUNING
   if (const char* e = getenv("AIG_PCONV_NODIST2")) if (atoi(e)) lpt = false;
 #endif
@@ -2056,8 +2080,10 @@ bool pconv_choose_tile(aig_ctx* ctx, aig_conv_plan* pl, const PconvNtOption* opt
       load[best_c] += w;
       lists[best_c].push_back(item);
     };
-    for (int m = 0; m < q.m_tiles; ++m) place(2 * m, w_main);       // item = m_tile * n_tiles + n_tile
-    for (int m = 0; m < q.m_tiles; ++m) place(2 * m + 1, w_short);
+    for (int m = 0; m < q.m_tiles; ++m)                             // item = m_tile * n_tiles + n_tile
+      for (int n = 0; n < q.sparse_tile0; ++n) place(m * q.n_tiles + n, w_main);
+    for (int m = 0; m < q.m_tiles; ++m)
+      for (int n = q.sparse_tile0; n < q.n_tiles; ++n) place(m * q.n_tiles + n, w_short);
     std::vector<int> tab(G + 1);
     int off = G + 1;
     for (int c = 0; c < G; ++c) {
