@@ -682,40 +682,52 @@ __global__ void __launch_bounds__(kTailWarps * 32) seq_tail_kernel(const __half*
   __syncthreads();
   for (int r0 = (blockIdx.x * kTailWarps + (tid >> 5)) * 16; r0 < rows; r0 += gridDim.x * kTailWarps * 16) {
     const uint4* src[2];
-    float mu[2], rstd[2];
+    float mu[2], rstd[2], s[2] = {0.f, 0.f}, ss[2] = {0.f, 0.f};
+#pragma unroll
+    for (int h = 0; h < 2; ++h) src[h] = reinterpret_cast<const uint4*>(x + (size_t)min(r0 + g + 8 * h, rows - 1) * C) + q;
+    for (int kb0 = 0; kb0 < nb; kb0 += 8) {  // (the only pass that waits for memory: sixteen loads in flight)
+      uint4 v[2][8];
+#pragma unroll
+      for (int u = 0; u < 8; ++u)
+#pragma unroll
+        for (int h = 0; h < 2; ++h) v[h][u] = kb0 + u < nb ? src[h][(kb0 + u) * 4] : make_uint4(0, 0, 0, 0);
+#pragma unroll
+      for (int u = 0; u < 8; ++u)
+#pragma unroll
+        for (int h = 0; h < 2; ++h)
+#pragma unroll
+          for (int e = 0; e < 4; ++e) {
+            const float2 f = __half22float2(reinterpret_cast<const __half2*>(&v[h][u])[e]);
+            s[h] += f.x + f.y;
+          }
+    }
 #pragma unroll
     for (int h = 0; h < 2; ++h) {
-      src[h] = reinterpret_cast<const uint4*>(x + (size_t)min(r0 + g + 8 * h, rows - 1) * C) + q;
-      float s = 0.f, ss = 0.f;
-#pragma unroll 8
-      for (int kb = 0; kb < nb; ++kb) {
+      s[h] += __shfl_xor_sync(0xffffffffu, s[h], 1);
+      s[h] += __shfl_xor_sync(0xffffffffu, s[h], 2);
+      mu[h] = s[h] / (float)C;
+    }
+#pragma unroll 4
+    for (int kb = 0; kb < nb; ++kb)
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
         const uint4 v = src[h][kb * 4];
 #pragma unroll
         for (int e = 0; e < 4; ++e) {
           const float2 f = __half22float2(reinterpret_cast<const __half2*>(&v)[e]);
-          s += f.x + f.y;
+          ss[h] += (f.x - mu[h]) * (f.x - mu[h]) + (f.y - mu[h]) * (f.y - mu[h]);
         }
       }
-      s += __shfl_xor_sync(0xffffffffu, s, 1);
-      s += __shfl_xor_sync(0xffffffffu, s, 2);
-      mu[h] = s / (float)C;
-#pragma unroll 8
-      for (int kb = 0; kb < nb; ++kb) {
-        const uint4 v = src[h][kb * 4];
 #pragma unroll
-        for (int e = 0; e < 4; ++e) {
-          const float2 f = __half22float2(reinterpret_cast<const __half2*>(&v)[e]);
-          ss += (f.x - mu[h]) * (f.x - mu[h]) + (f.y - mu[h]) * (f.y - mu[h]);
-        }
-      }
-      ss += __shfl_xor_sync(0xffffffffu, ss, 1);
-      ss += __shfl_xor_sync(0xffffffffu, ss, 2);
-      rstd[h] = rsqrtf(ss / (float)C + eps);
+    for (int h = 0; h < 2; ++h) {
+      ss[h] += __shfl_xor_sync(0xffffffffu, ss[h], 1);
+      ss[h] += __shfl_xor_sync(0xffffffffu, ss[h], 2);
+      rstd[h] = rsqrtf(ss[h] / (float)C + eps);
     }
     float acc[kTailTiles][4];
 #pragma unroll
     for (int t = 0; t < kTailTiles; ++t) acc[t][0] = acc[t][1] = acc[t][2] = acc[t][3] = 0.f;
-#pragma unroll 2
+#pragma unroll 4
     for (int kb = 0; kb < nb; ++kb) {
       const uint4 v[2] = {src[0][kb * 4], src[1][kb * 4]};
       const int k0 = kb * 32 + q * 8;

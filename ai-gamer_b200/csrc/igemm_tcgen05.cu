@@ -1919,7 +1919,8 @@ bool pconv_choose_tile(aig_ctx* ctx, aig_conv_plan* pl, const PconvNtOption* opt
   // M tiles for less than one wave (batches in between): a CTA's time is the fetch of its weights and patches, about 37 B/clk,
   // and narrower N tiles share the weights out over the idle SMs at the price of a patch per N tile.  The tiling with the
   // least time by that count, main tiles first and the four times shorter shortcut tiles after them, where it is at least
-  // a tenth better than the widest.  32 frames of 144x256: RESULT3
+  // a tenth better than the widest.  32 frames of 144x256: third block 24.5 + 29.0 -> 21.2 + 20.9 us; 128 frames: fourth block
+  // 34.0 + 27.4 -> 29.7 + 24.7.
   int spread = -1;
   const long long m1 = ceil_div_ll(total_q, kTileM);
   if (!small && !f_nt && m1 <= ctx->sm_count) {
