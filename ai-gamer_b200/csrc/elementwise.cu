@@ -650,21 +650,24 @@ __global__ void cnn_head_kernel(const __half* x, const __half* __restrict__ w1, 
 
 // Row LayerNorm, FC, sigmoid / tanh of the sequence head.  As separate launches (row LayerNorm, a GEMM of one 32-wide
 // column tile, two in-place activations, a conversion) 8192 rows of 512 took 28 us, three times through memory, and 111
-// rows of 256 took 22 us, all launches.  A warp takes 16 rows in the layout of mma.sync's A operand
-// (a lane has 16-byte pieces of two rows; the second and third pass over them find them in L1), the row sums are two shuffles, the product with the few output columns is
-// three to four mma tiles.  Bound by the one read of x; the weights come K-major from the head's own copy (turning them
-// here, per CTA, was 12 of 20 us).
-constexpr int kTailMaxC = 512, kTailTiles = 4, kTailWarps = 4;
-__global__ void __launch_bounds__(kTailWarps * 32) seq_tail_kernel(const __half* x, const float* __restrict__ gamma, const float* __restrict__ beta,
+// rows of 256 took 22 us, all launches.  A pair of warps takes 16 rows in the layout of mma.sync's A operand, half of the
+// columns each: a lane's pieces of its two rows then stay in registers from the one read to the product (a warp alone spills
+// them or reads them three times).  Row sums are two shuffles and one exchange between the pair, the product with the few
+// output columns is three to four mma tiles, the pair's halves added at the end.  Bound by the latency of that one read; the
+// weights come K-major from the head's own copy (turning them here, per CTA, was 12 of 20 us).
+constexpr int kTailMaxC = 512, kTailTiles = 4, kTailPairs = 4, kTailThreads = 2 * kTailPairs * 32, kTailBlocks = kTailMaxC / 64;
+__global__ void __launch_bounds__(kTailThreads) seq_tail_kernel(const __half* x, const float* __restrict__ gamma, const float* __restrict__ beta,
                                                                    const __half* __restrict__ fcw, const __half* __restrict__ fcb, __half* out_h, float* out_f,
                                                                    int rows, int C, int n_out, int n_sig, float eps) {
   extern __shared__ __align__(16) uint8_t tail_smem[];
-  __shared__ float s_bias[8 * kTailTiles];
+  __shared__ float s_bias[8 * kTailTiles], s_part[2][2][kTailPairs * 16], s_acc[kTailPairs][kTailTiles * 4][32];
   const int stride = C + 8;                                       // halfs: rows of the weights on different banks
   float* s_g = reinterpret_cast<float*>(tail_smem);               // gamma, beta
   float* s_b = s_g + C;
   __half* s_w = reinterpret_cast<__half*>(s_b + C);               // [tiles * 8][C]
   const int tid = threadIdx.x, lane = tid & 31, g = lane >> 2, q = lane & 3, nb = C / 32, tiles = (n_out + 7) / 8;
+  const int pair = (tid >> 5) % kTailPairs, side = (tid >> 5) / kTailPairs;
+  const int first = side * ((nb + 1) / 2), mine = side ? nb / 2 : (nb + 1) / 2;  // blocks of 32 columns
   for (int i = tid; i < C; i += blockDim.x) {
     s_g[i] = gamma[i];
     s_b[i] = beta[i];
@@ -680,57 +683,49 @@ __global__ void __launch_bounds__(kTailWarps * 32) seq_tail_kernel(const __half*
   griddep_launch_dependents();
   griddep_wait();
   __syncthreads();
-  for (int r0 = (blockIdx.x * kTailWarps + (tid >> 5)) * 16; r0 < rows; r0 += gridDim.x * kTailWarps * 16) {
-    const uint4* src[2];
-    float mu[2], rstd[2], s[2] = {0.f, 0.f}, ss[2] = {0.f, 0.f};
-#pragma unroll
-    for (int h = 0; h < 2; ++h) src[h] = reinterpret_cast<const uint4*>(x + (size_t)min(r0 + g + 8 * h, rows - 1) * C) + q;
-    for (int kb0 = 0; kb0 < nb; kb0 += 8) {  // (the only pass that waits for memory: sixteen loads in flight)
-      uint4 v[2][8];
-#pragma unroll
-      for (int u = 0; u < 8; ++u)
-#pragma unroll
-        for (int h = 0; h < 2; ++h) v[h][u] = kb0 + u < nb ? src[h][(kb0 + u) * 4] : make_uint4(0, 0, 0, 0);
-#pragma unroll
-      for (int u = 0; u < 8; ++u)
-#pragma unroll
-        for (int h = 0; h < 2; ++h)
-#pragma unroll
-          for (int e = 0; e < 4; ++e) {
-            const float2 f = __half22float2(reinterpret_cast<const __half2*>(&v[h][u])[e]);
-            s[h] += f.x + f.y;
-          }
-    }
+  for (int block0 = blockIdx.x * kTailPairs * 16; block0 < rows; block0 += gridDim.x * kTailPairs * 16) {
+    const int r0 = block0 + pair * 16;  // (rows past the end: the last row's, not stored)
+    uint4 v[2][kTailBlocks];
+    float mu[2], rstd[2];
 #pragma unroll
     for (int h = 0; h < 2; ++h) {
-      s[h] += __shfl_xor_sync(0xffffffffu, s[h], 1);
-      s[h] += __shfl_xor_sync(0xffffffffu, s[h], 2);
-      mu[h] = s[h] / (float)C;
+      const uint4* src = reinterpret_cast<const uint4*>(x + (size_t)min(r0 + g + 8 * h, rows - 1) * C) + first * 4 + q;
+#pragma unroll
+      for (int kb = 0; kb < kTailBlocks; ++kb) v[h][kb] = kb < mine ? src[kb * 4] : make_uint4(0, 0, 0, 0);
     }
-#pragma unroll 4
-    for (int kb = 0; kb < nb; ++kb)
+#pragma unroll
+    for (int pass = 0; pass < 2; ++pass) {  // the mean, then the variance about it
 #pragma unroll
       for (int h = 0; h < 2; ++h) {
-        const uint4 v = src[h][kb * 4];
+        float s = 0.f;
 #pragma unroll
-        for (int e = 0; e < 4; ++e) {
-          const float2 f = __half22float2(reinterpret_cast<const __half2*>(&v)[e]);
-          ss[h] += (f.x - mu[h]) * (f.x - mu[h]) + (f.y - mu[h]) * (f.y - mu[h]);
-        }
+        for (int kb = 0; kb < kTailBlocks; ++kb)
+          if (kb < mine)
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+              const float2 f = __half22float2(reinterpret_cast<const __half2*>(&v[h][kb])[e]);
+              s += pass ? (f.x - mu[h]) * (f.x - mu[h]) + (f.y - mu[h]) * (f.y - mu[h]) : f.x + f.y;
+            }
+        s += __shfl_xor_sync(0xffffffffu, s, 1);
+        s += __shfl_xor_sync(0xffffffffu, s, 2);
+        if (q == 0) s_part[pass][side][pair * 16 + g + 8 * h] = s;
       }
+      __syncthreads();
 #pragma unroll
-    for (int h = 0; h < 2; ++h) {
-      ss[h] += __shfl_xor_sync(0xffffffffu, ss[h], 1);
-      ss[h] += __shfl_xor_sync(0xffffffffu, ss[h], 2);
-      rstd[h] = rsqrtf(ss[h] / (float)C + eps);
+      for (int h = 0; h < 2; ++h) {
+        const int r = pair * 16 + g + 8 * h;
+        const float m = (s_part[pass][0][r] + s_part[pass][1][r]) / (float)C;
+        if (pass == 0) mu[h] = m;
+        else rstd[h] = rsqrtf(m + eps);
+      }
     }
     float acc[kTailTiles][4];
 #pragma unroll
     for (int t = 0; t < kTailTiles; ++t) acc[t][0] = acc[t][1] = acc[t][2] = acc[t][3] = 0.f;
-#pragma unroll 4
-    for (int kb = 0; kb < nb; ++kb) {
-      const uint4 v[2] = {src[0][kb * 4], src[1][kb * 4]};
-      const int k0 = kb * 32 + q * 8;
+#pragma unroll
+    for (int kb = 0; kb < kTailBlocks; ++kb) {
+      if (kb >= mine) break;
+      const int k0 = (first + kb) * 32 + q * 8;
       float gm[8], bt[8];
 #pragma unroll
       for (int e = 0; e < 8; e += 4) {
@@ -742,7 +737,7 @@ __global__ void __launch_bounds__(kTailWarps * 32) seq_tail_kernel(const __half*
       for (int h = 0; h < 2; ++h)
 #pragma unroll
         for (int e = 0; e < 4; ++e) {
-          const float2 f = __half22float2(reinterpret_cast<const __half2*>(&v[h])[e]);
+          const float2 f = __half22float2(reinterpret_cast<const __half2*>(&v[h][kb])[e]);
           const __half2 n = __floats2half2_rn((f.x - mu[h]) * rstd[h] * gm[2 * e] + bt[2 * e], (f.y - mu[h]) * rstd[h] * gm[2 * e + 1] + bt[2 * e + 1]);
           a[h][e] = *reinterpret_cast<const uint32_t*>(&n);
         }
@@ -759,14 +754,21 @@ __global__ void __launch_bounds__(kTailWarps * 32) seq_tail_kernel(const __half*
                      : "r"(a[0][2]), "r"(a[1][2]), "r"(a[0][3]), "r"(a[1][3]), "r"(w.z), "r"(w.w));
       }
     }
+    if (side)
+#pragma unroll
+      for (int t = 0; t < kTailTiles; ++t)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) s_acc[pair][t * 4 + e][lane] = acc[t][e];
+    __syncthreads();
+    if (side) continue;  // (the next rows' barriers keep s_acc until this side has read it)
 #pragma unroll
     for (int t = 0; t < kTailTiles; ++t)
 #pragma unroll
       for (int e = 0; e < 4; ++e) {
         const int r = r0 + g + 8 * (e >> 1), o = t * 8 + 2 * q + (e & 1);
         if (t >= tiles || r >= rows || o >= n_out) continue;
-        const float s = __half2float(__float2half(acc[t][e]));                  // FCLayer: GEMM result stored as half,
-        const float y = __half2float(__float2half(s + s_bias[o]));              // then bias added and stored again
+        const float s = __half2float(__float2half(acc[t][e] + s_acc[pair][t * 4 + e][lane]));  // FCLayer: GEMM result stored as half,
+        const float y = __half2float(__float2half(s + s_bias[o]));  // then bias added and stored again
         const __half hv = __float2half(o < n_sig ? 1.0f / (1.0f + expf(-y)) : tanhf(y));
         out_h[(size_t)r * n_out + o] = hv;
         out_f[(size_t)r * n_out + o] = __half2float(hv);
@@ -781,8 +783,8 @@ int seq_tail_forward(aig_ctx* ctx, const aig_half* x, const float* gamma, const 
                      float* out_f32, int rows, int c, int n_out, int n_sigmoid, float eps) {
   DeviceGuard guard(ctx->device);
   const size_t smem = (size_t)c * 8 + (size_t)(n_out + 7) / 8 * 8 * (c + 8) * 2;
-  const int grid = std::min((rows + 16 * kTailWarps - 1) / (16 * kTailWarps), 2 * ctx->sm_count);
-  AIG_CUDA_OK(ctx, launch_pdl(seq_tail_kernel, dim3(grid), dim3(kTailWarps * 32), smem, ctx->stream, (const __half*)x, gamma, beta, (const __half*)fc_w,
+  const int grid = std::min((rows + 16 * kTailPairs - 1) / (16 * kTailPairs), 2 * ctx->sm_count);
+  AIG_CUDA_OK(ctx, launch_pdl(seq_tail_kernel, dim3(grid), dim3(kTailThreads), smem, ctx->stream, (const __half*)x, gamma, beta, (const __half*)fc_w,
                               (const __half*)fc_b, (__half*)out_half, out_f32, rows, c, n_out, n_sigmoid, eps));
   return AIG_OK;
 }
