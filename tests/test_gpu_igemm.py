@@ -426,6 +426,49 @@ def test_padded_position_layout_between_down_sampling_and_conv1(env, B, C, H, W,
 
 
 @gpu
+@pytest.mark.parametrize("B,C,H,W,K", [(296, 64, 6, 6, 256), (297, 128, 6, 6, 256),      # 37 and 38 M tiles: last of the few, first of the spread
+                                       (1184, 64, 6, 6, 128), (1185, 64, 6, 6, 128),     # 148 and 149: a full wave, one more than that
+                                       (20, 64, 32, 48, 128), (100, 128, 16, 16, 256), (500, 256, 6, 6, 512), (61, 256, 10, 14, 512)])
+def test_down_sampling_and_conv1_with_fewer_m_tiles_than_sms(env, B, C, H, W, K):
+    """M tiles for less than one wave: N tilings spread over the SMs, against the oracle, from the channels-last and from
+    the padded position layout (other M tiles, so possibly another order of the channel groups)."""
+    U = env
+    import torch
+
+    c, pk = U.ctx(), U.pkg()
+    x = h(RNG.standard_normal((B, C, H, W)))
+    w0, b0 = PL.he_normal(RNG, (K, C, 4, 4)), h(RNG.uniform(-0.2, 0.2, K))
+    ws, bs = PL.he_normal(RNG, (K, C, 2, 2)), h(RNG.uniform(-0.2, 0.2, K))
+    w1, b1 = PL.he_normal(RNG, (K, K, 3, 3)), h(RNG.uniform(-0.2, 0.2, K))
+    bn, bn1 = PL.bn_params(RNG, K, trivial=False), PL.bn_params(RNG, K, trivial=False)
+    keep = [U.dev(a) for a in (w0, b0, ws, bs, w1, b1)] + [U.dev(q) for q in bn] + [U.dev(q) for q in bn1]
+    down = pk.ResDownPlan(c, B, C, H, W, K, act=pk.ACT_SWISH)
+    _, Ho, Wo = down.out_dims()
+    down.set_weights(keep[0], keep[1], keep[6:10], keep[2], keep[3], eps=1e-6)
+    conv = pk.ConvPlan(c, B, K, Ho, Wo, K, 3, 1, 1, act=pk.ACT_SWISH)
+    conv.set_weights(keep[4], keep[5], bn=keep[10:14])
+    ds = torch.zeros(pk.lib().aig_s2d_elems(B, H, W, C), dtype=torch.float16, device="cuda")
+    c.call("aig_nhwc_to_s2d", U.p(U.dev(U.nhwc(x))), U.p(ds), B, H, W, C)
+    n, rows = B * Ho * Wo * K, pk.padded_rows(B, Ho, Wo, 1)
+    got = []
+    for padded in (False, True):
+        m, s = (torch.zeros(rows * K if padded else n, dtype=torch.float16, device="cuda") for _ in range(2))
+        y = torch.full((n,), 7.0, dtype=torch.float16, device="cuda")
+        down.set_output_padded(padded)
+        conv.set_input_padded(padded)
+        down.forward(ds, m, s)
+        conv.forward(m, y, residual=s)
+        c.sync()
+        got.append(U.host(y))
+    main = O.activate(O.batchnorm(O.conv2d(x, w0, b0, 2, 1), *bn), 2, 0.01)
+    want = O.activate(O.add(O.batchnorm(O.conv2d(main, w1, b1, 1, 1), *bn1), O.conv2d(x, ws, bs, 2, 0)), 2, 0.01)
+    for y in got:
+        assert U.scaled_err(U.nchw(y.reshape(B, Ho, Wo, K)), want) < 8e-3
+    down.close()
+    conv.close()
+
+
+@gpu
 def test_fused_downsampling_refuses_unsupported_channel_counts(env):
     """Channel counts the space-to-depth GEMM cannot tile are refused with a clear status (callers then
     use the two separate convolutions)."""
