@@ -58,19 +58,13 @@ struct IgemmParams {
 // with 16 bytes each, and with the scalar affine loads the epilogue was three times as long as the tile's loads and MMAs:
 // 8192 x 512 -> 2048 in fp32 (67 MB) took 49 us.
 constexpr int kFcStage = 128 * 128;
-//
-// PAIR: two CTAs of a cluster take neighbouring M tiles and half of the weight rows each, as in pconv_kernel's pairs: 32 KB
-// a stage instead of 48.  That leaves room for a second staging tile per team, so that a store's read of one overlaps the
-// next step into the other; the epilogue bounds these products, and the smaller fetch alone gave nothing (128 sequences of
-// 64 through two LSTM layers, 8192 x 512 -> 2048 each: 380 us single, 383 pairs with one staging tile, 376 with two).
-template <int NT, int BK, int MS, bool STAGED = false, bool PAIR = false>
+template <int NT, int BK, int MS, bool STAGED = false>
 struct IgemmCfg {
   static constexpr int kSubBytes = kTileM * BK * 2;
   static constexpr int kABytes = MS * kSubBytes;
-  static constexpr int kBBytes = (PAIR ? NT / 2 : NT) * BK * 2;
+  static constexpr int kBBytes = NT * BK * 2;
   static constexpr int kStageBytes = kABytes + kBBytes;
-  static constexpr int kStageTiles = PAIR ? 2 : 1;  // staging tiles per team
-  static constexpr int kStaging = STAGED ? 2 * kStageTiles * kFcStage : 0;
+  static constexpr int kStaging = STAGED ? 2 * kFcStage : 0;
   static constexpr int kStagesRaw = (STAGED ? 227 * 1024 - 4096 - kStaging : kSmemBudget) / kStageBytes;
   static constexpr int kStages = kStagesRaw > 8 ? 8 : kStagesRaw;
   static constexpr int kTmemCols = 2 * MS * NT < 32 ? 32 : 2 * MS * NT;
@@ -510,12 +504,10 @@ __device__ __forceinline__ void fc_stage_step(uint32_t t_addr, const IgemmParams
   }
 }
 
-template <int NT, int BK, int MS, bool STAGED, bool PAIR = false>
+template <int NT, int BK, int MS, bool STAGED>
 __global__ void __launch_bounds__(kNumThreads, 1)
 igemm_kernel(const __grid_constant__ CUtensorMap tmapA, const __grid_constant__ CUtensorMap tmapB, const __grid_constant__ CUtensorMap tmapY, const IgemmParams p) {
-  static_assert(!PAIR || (STAGED && MS == 1 && BK == 64), "pair kernel: FC products with staged output");
-  using Cfg = IgemmCfg<NT, BK, MS, STAGED, PAIR>;
-  const int rank = PAIR ? (int)cluster_ctarank() : 0;
+  using Cfg = IgemmCfg<NT, BK, MS, STAGED>;
   constexpr int kStages = Cfg::kStages;
   extern __shared__ uint8_t smem_raw[];
   const uint32_t raw = smem_u32(smem_raw);
@@ -543,7 +535,7 @@ igemm_kernel(const __grid_constant__ CUtensorMap tmapA, const __grid_constant__ 
     }
     for (int a = 0; a < 2; ++a) {
       mbar_init(bar_tfull + 8 * a, 1);
-      mbar_init(bar_tempty + 8 * a, PAIR ? 16 : 8);  // (pair: both CTAs' epilogue warps arrive at the first CTA's)
+      mbar_init(bar_tempty + 8 * a, 8);
     }
     *s_abort = 0;
     fence_mbar_init();
@@ -551,13 +543,8 @@ igemm_kernel(const __grid_constant__ CUtensorMap tmapA, const __grid_constant__ 
     tma_prefetch_desc(&tmapB);
   }
   if (warp == 1) {
-    if constexpr (PAIR) {
-      tmem_alloc_pair(smem_u32(s_tmem), Cfg::kTmemCols);
-      tmem_relinquish_pair();
-    } else {
-      tmem_alloc(smem_u32(s_tmem), Cfg::kTmemCols);
-      tmem_relinquish();
-    }
+    tmem_alloc(smem_u32(s_tmem), Cfg::kTmemCols);
+    tmem_relinquish();
   }
   griddep_wait();  // weights and affine may be new as well as the activations (a training step's update)
   if (p.n_tiles == 1) {
@@ -568,18 +555,10 @@ igemm_kernel(const __grid_constant__ CUtensorMap tmapA, const __grid_constant__ 
   }
   tc_fence_before();
   __syncthreads();
-  if constexpr (PAIR) cluster_sync_all();  // both CTAs' barriers are initialised and their TMEM allocated before anything crosses
   tc_fence_after();
   const uint32_t tmem_base = *s_tmem;
-  // barriers the pair's loads count on and its epilogues arrive at: the first CTA's (cluster-window addresses)
-  const uint32_t full_first = PAIR ? mapa_shared(bar_full, 0) : bar_full;
-  const uint32_t tempty_first = PAIR ? mapa_shared(bar_tempty, 0) : bar_tempty;
-  auto wait = [&](uint32_t bar, uint32_t parity, int code) {
-    return PAIR ? mbar_wait_bounded_cl(bar, parity, s_abort, p.gerr, code) : mbar_wait_bounded(bar, parity, s_abort, p.gerr, code);
-  };
-  // (pair: tile numbers count pairs of M tiles; an odd last one's partner runs on rows past the end, zero-filled and not stored)
-  const int total_tiles = (PAIR ? (p.m_super + 1) / 2 : p.m_super) * p.n_tiles;
-  const int tile0 = PAIR ? blockIdx.x / 2 : blockIdx.x, tile_step = PAIR ? gridDim.x / 2 : gridDim.x;
+
+  const int total_tiles = p.m_super * p.n_tiles;
 
   if (warp == 0) {
     // ------------------------------------------------------------------ TMA producer
@@ -589,20 +568,8 @@ igemm_kernel(const __grid_constant__ CUtensorMap tmapA, const __grid_constant__ 
       int stage = 0;
       uint32_t phase = 0;
       bool ok = true;
-      for (int tile = tile0; tile < total_tiles && ok; tile += tile_step) {
-        const int n_tile = tile % p.n_tiles, m_sup = PAIR ? tile / p.n_tiles * 2 + rank : tile / p.n_tiles;
-        if constexpr (PAIR) {  // (both operands are plain matrices)
-          for (int kb = 0; kb < p.num_kb; ++kb) {
-            if (!wait(bar_empty + 8 * stage, phase ^ 1u, 101)) { ok = false; break; }
-            if (leader) {
-              if (rank == 0) mbar_expect_tx(bar_full + 8 * stage, 2u * Cfg::kStageBytes);
-              tma_load_2d_pair(sB + stage * Cfg::kBBytes, &tmapB, full_first + 8 * stage, kb * BK, n_tile * NT + rank * (NT / 2));
-              tma_load_2d_pair(sA + stage * Cfg::kABytes, &tmapA, full_first + 8 * stage, kb * BK, m_sup * kTileM);
-            }
-            if (++stage == kStages) { stage = 0; phase ^= 1u; }
-          }
-          continue;
-        }
+      for (int tile = blockIdx.x; tile < total_tiles && ok; tile += gridDim.x) {
+        const int n_tile = tile % p.n_tiles, m_sup = tile / p.n_tiles;
         int seg_n[MS * kMaxSegs], seg_z[MS * kMaxSegs], seg_y[MS * kMaxSegs], seg_x[MS * kMaxSegs];
         const int nseg = MS * p.segs;
         {
@@ -679,29 +646,21 @@ igemm_kernel(const __grid_constant__ CUtensorMap tmapA, const __grid_constant__ 
     }
   } else if (warp == 1) {
     // ------------------------------------------------------------------ MMA issuer
-    if (!PAIR || rank == 0) {  // (pair: the first CTA's warp issues for both)
-      constexpr uint32_t idesc = umma_idesc_f16(PAIR ? 2 * kTileM : kTileM, NT);
+    {
+      constexpr uint32_t idesc = umma_idesc_f16(kTileM, NT);
       const bool leader = elect_one();
-      auto commit = [&](uint32_t bar) {
-        if constexpr (PAIR) {
-          umma_commit_pair(bar);
-          umma_commit_pair(mapa_shared(bar, 1));
-        } else {
-          umma_commit(bar);
-        }
-      };
       int stage = 0;
       uint32_t phase = 0;
       int it = 0;
       bool ok = true;
-      for (int tile = tile0; tile < total_tiles && ok; tile += tile_step, ++it) {
+      for (int tile = blockIdx.x; tile < total_tiles && ok; tile += gridDim.x, ++it) {
         const int acc = it & 1;
         const uint32_t acc_phase = (uint32_t)(it >> 1) & 1u;
-        if (!wait(bar_tempty + 8 * acc, acc_phase ^ 1u, 201)) { ok = false; break; }
+        if (!mbar_wait_bounded(bar_tempty + 8 * acc, acc_phase ^ 1u, s_abort, p.gerr, 201)) { ok = false; break; }
         tc_fence_after();
         const uint32_t d_tmem = tmem_base + (uint32_t)(acc * MS * NT);
         for (int kb = 0; kb < p.num_kb; ++kb) {
-          if (!wait(bar_full + 8 * stage, phase, 202)) { ok = false; break; }
+          if (!mbar_wait_bounded(bar_full + 8 * stage, phase, s_abort, p.gerr, 202)) { ok = false; break; }
           const uint32_t a0 = sA + stage * Cfg::kABytes, b0 = sB + stage * Cfg::kBBytes;
           const uint32_t a_lo = umma_desc_lo(a0), b_lo = umma_desc_lo(b0);
           const uint32_t first = kb != 0 ? 1u : 0u;
@@ -709,18 +668,13 @@ igemm_kernel(const __grid_constant__ CUtensorMap tmapA, const __grid_constant__ 
           for (int sub = 0; sub < MS; ++sub) {
 #pragma unroll
             for (int k = 0; k < BK / 16; ++k)
-              if (leader) {
-                if constexpr (PAIR)
-                  umma_f16_ss_lo_pair(d_tmem, a_lo + (uint32_t)((k * 32) >> 4), b_lo + (uint32_t)((k * 32) >> 4), umma_desc_hi(BK * 2), idesc, k == 0 ? first : 1u);
-                else
-                  umma_f16_ss_lo(d_tmem + (uint32_t)(sub * NT), a_lo + (uint32_t)((sub * Cfg::kSubBytes + k * 32) >> 4),
-                                 b_lo + (uint32_t)((k * 32) >> 4), umma_desc_hi(BK * 2), idesc, k == 0 ? first : 1u);
-              }
+              if (leader) umma_f16_ss_lo(d_tmem + (uint32_t)(sub * NT), a_lo + (uint32_t)((sub * Cfg::kSubBytes + k * 32) >> 4),
+                             b_lo + (uint32_t)((k * 32) >> 4), umma_desc_hi(BK * 2), idesc, k == 0 ? first : 1u);
           }
-          if (leader) commit(bar_empty + 8 * stage);  // frees the smem stage once these MMAs have read it
+          if (leader) umma_commit(bar_empty + 8 * stage);  // frees the smem stage once these MMAs have read it
           if (++stage == kStages) { stage = 0; phase ^= 1u; }
         }
-        if (ok && leader) commit(bar_tfull + 8 * acc);
+        if (ok && leader) umma_commit(bar_tfull + 8 * acc);
       }
     }
   } else {
@@ -733,8 +687,8 @@ igemm_kernel(const __grid_constant__ CUtensorMap tmapA, const __grid_constant__ 
     const bool fast = (p.out_c & 7) == 0 && !p.two_step && !p.y32;
     int it = 0;
     bool ok = true;
-    for (int tile = tile0; tile < total_tiles && ok; tile += tile_step, ++it) {
-      const int n_tile = tile % p.n_tiles, m_sup = PAIR ? tile / p.n_tiles * 2 + rank : tile / p.n_tiles;
+    for (int tile = blockIdx.x; tile < total_tiles && ok; tile += gridDim.x, ++it) {
+      const int n_tile = tile % p.n_tiles, m_sup = tile / p.n_tiles;
       const int acc = it & 1;
       const uint32_t acc_phase = (uint32_t)(it >> 1) & 1u;
       // scale/shift: staged in shared memory when there is a single N tile, else read from global
@@ -744,18 +698,14 @@ igemm_kernel(const __grid_constant__ CUtensorMap tmapA, const __grid_constant__ 
       if constexpr (STAGED) {
         // the four warps of a team go on together: their steps meet at named barriers
         const int team = (warp - 2) >> 2;
-        ok = named_bar_and(1 + team, 128, wait(bar_tfull + 8 * acc, acc_phase, 301));
+        ok = named_bar_and(1 + team, 128, mbar_wait_bounded(bar_tfull + 8 * acc, acc_phase, s_abort, p.gerr, 301));
         if (!ok) break;
         tc_fence_after();
-        const uint32_t stage0 = base + kStages * Cfg::kStageBytes + (uint32_t)(team * Cfg::kStageTiles * kFcStage);
+        const uint32_t stage = base + kStages * Cfg::kStageBytes + (uint32_t)(team * kFcStage);
         const bool issuer = ((warp - 2) & 3) == 0 && lane == 0;
 #pragma unroll 1
         for (int c0 = col_lo; c0 < col_hi; c0 += 32) {
-          const uint32_t stage = stage0 + (PAIR ? (uint32_t)(((c0 - col_lo) >> 5) & 1) * kFcStage : 0u);
-          if (issuer) {  // the last store from this staging tile has left it
-            if constexpr (PAIR) asm volatile("cp.async.bulk.wait_group.read 1;" ::: "memory");
-            else bulk_wait_group_read0();
-          }
+          if (issuer) bulk_wait_group_read0();  // the store before this one has left the tile
           named_bar_sync(1 + team, 128);
           const uint32_t t_addr = tmem_base + (uint32_t)(acc * NT + c0) + ((uint32_t)(q * 32) << 16);
           if (p.y32) fc_stage_step<true, false, AIG_ACT_NONE>(t_addr, p, nb + c0, stage, row_in_tile);
@@ -766,17 +716,14 @@ igemm_kernel(const __grid_constant__ CUtensorMap tmapA, const __grid_constant__ 
           else fc_stage_step<false, false, AIG_ACT_NONE>(t_addr, p, nb + c0, stage, row_in_tile);
           fence_proxy_async_smem();
           named_bar_sync(1 + team, 128);
-          if (issuer && (!PAIR || m_sup < p.m_super)) {
+          if (issuer) {
             tma_store_2d(&tmapY, stage, nb + c0, m_sup * kTileM);
             bulk_commit_group();
           }
         }
         tc_fence_before();
         __syncwarp();
-        if (lane == 0) {
-          if constexpr (PAIR) mbar_arrive_cluster(tempty_first + 8 * acc);
-          else mbar_arrive(bar_tempty + 8 * acc);
-        }
+        if (lane == 0) mbar_arrive(bar_tempty + 8 * acc);
         continue;
       }
       if (!mbar_wait_bounded(bar_tfull + 8 * acc, acc_phase, s_abort, p.gerr, 301)) { ok = false; break; }
@@ -825,11 +772,9 @@ igemm_kernel(const __grid_constant__ CUtensorMap tmapA, const __grid_constant__ 
   }
   tc_fence_before();
   __syncthreads();
-  if constexpr (PAIR) cluster_sync_all();  // neither CTA frees TMEM or exits while the other may still read it or arrive at its barriers
   if (warp == 1) {
     tc_fence_after();
-    if constexpr (PAIR) tmem_dealloc_pair(tmem_base, Cfg::kTmemCols);
-    else tmem_dealloc(tmem_base, Cfg::kTmemCols);
+    tmem_dealloc(tmem_base, Cfg::kTmemCols);
   }
 }
 
@@ -1574,9 +1519,6 @@ struct aig_conv_plan {
   CUtensorMap tmapFc{};                        // the output for that
   const void* tmapFc_ptr = nullptr;
   bool tmapFc_f32 = false;
-  int pair_clusters = 0;                       // > 0: staged forwards run as this many CTA pairs at most (see IgemmCfg, PAIR)
-  CUtensorMap tmapA2{}, tmapB2{};              // operands for that
-  const void* tmapA2_ptr = nullptr;
   bool skinny = false;                         // FC plans of few rows: see skinny_fc.cu
   int BK = 64, NT = 64, MS = 1, Kpad = 0, taps = 1, Ktot = 0;
   IgemmParams prm{};
@@ -1622,53 +1564,6 @@ int launch_igemm(aig_conv_plan* pl) {
   return AIG_OK;
 }
 
-cudaLaunchConfig_t fc_pair_config(aig_ctx* ctx, int grid, cudaLaunchAttribute (&attr)[2]) {
-  attr[0].id = cudaLaunchAttributeClusterDimension;
-  attr[0].val.clusterDim.x = 2;
-  attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
-  attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr[1].val.programmaticStreamSerializationAllowed = 1;
-  cudaLaunchConfig_t cfg{};
-  cfg.gridDim = dim3((unsigned)grid);
-  cfg.blockDim = dim3(kNumThreads);
-  cfg.dynamicSmemBytes = IgemmCfg<256, 64, 1, true, true>::kSmemBytes;
-  cfg.stream = ctx->stream;
-  cfg.attrs = attr;
-  cfg.numAttrs = 2;
-  return cfg;
-}
-int launch_fc_pair(aig_conv_plan* pl) {
-  cudaLaunchAttribute attr[2];
-  const long long tiles = (long long)(pl->prm.m_super + 1) / 2 * pl->prm.n_tiles;
-  const cudaLaunchConfig_t cfg = fc_pair_config(pl->ctx, 2 * (int)std::min<long long>(tiles, pl->pair_clusters), attr);
-  AIG_CUDA_OK(pl->ctx, cudaLaunchKernelEx(&cfg, igemm_kernel<256, 64, 1, true, true>, pl->tmapA2, pl->tmapB2, pl->tmapFc, pl->prm));
-  return AIG_OK;
-}
-// A K-major matrix of `rows` rows, box 64 columns x 128 rows (both operands of a CTA of a pair).
-int encode_pair_operand(aig_conv_plan* pl, CUtensorMap* map, const void* x, int rows) {
-  EncodeTiledFn enc = get_encode_fn();
-  if (!enc) return aig_fail(pl->ctx, AIG_ERR_CUDA, "cuTensorMapEncodeTiled entry point not available");
-  const cuuint64_t dims[2] = {(cuuint64_t)pl->Ktot, (cuuint64_t)rows}, strides[1] = {(cuuint64_t)pl->Ktot * 2};
-  const cuuint32_t box[2] = {64u, 128u}, estr[2] = {1, 1};
-  const CUresult r = enc(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, const_cast<void*>(x), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
-                         CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-  if (r != CUDA_SUCCESS) return aig_fail(pl->ctx, AIG_ERR_CUDA, "cuTensorMapEncodeTiled(pair operand) failed: %d", (int)r);
-  return AIG_OK;
-}
-// Pairs where they fill the GPU: with fewer tiles the single CTAs spread further.
-int choose_fc_pair(aig_conv_plan* pl) {
-  aig_ctx* ctx = pl->ctx;
-  if (!pl->is_fc || pl->BK != 64 || pl->NT != 256 || pl->MS != 1) return AIG_OK;
-  if ((long long)pl->prm.m_super * pl->prm.n_tiles < ctx->sm_count) return AIG_OK;
-  AIG_CUDA_OK(ctx, cudaFuncSetAttribute(igemm_kernel<256, 64, 1, true, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, IgemmCfg<256, 64, 1, true, true>::kSmemBytes));
-  cudaLaunchAttribute attr[2];
-  const cudaLaunchConfig_t cfg = fc_pair_config(ctx, ctx->sm_count & ~1, attr);
-  int n = 0;
-  AIG_CUDA_OK(ctx, cudaOccupancyMaxActiveClusters(&n, igemm_kernel<256, 64, 1, true, true>, &cfg));
-  pl->pair_clusters = n;
-  return n > 0 ? encode_pair_operand(pl, &pl->tmapB2, pl->w_packed, pl->Kpad) : AIG_OK;
-}
-
 template <int NT, int MS>
 int dispatch_bk(aig_conv_plan* pl) {
   switch (pl->BK) {
@@ -1680,7 +1575,6 @@ int dispatch_bk(aig_conv_plan* pl) {
 }
 
 int dispatch(aig_conv_plan* pl) {
-  if (pl->staged && pl->pair_clusters) return launch_fc_pair(pl);
   if (pl->staged) {
     switch (pl->NT) {
       case 64: return launch_igemm<64, 64, 1, true>(pl);
@@ -1833,8 +1727,7 @@ int plan_finish(aig_ctx* ctx, aig_conv_plan* pl) {
   AIG_CUDA_OK(ctx, cudaMalloc(&pl->shift, pl->Kpad * sizeof(float)));
   p.scale = pl->scale;
   p.shift = pl->shift;
-  const int rc = encode_B(pl);
-  return rc == AIG_OK ? choose_fc_pair(pl) : rc;
+  return encode_B(pl);
 }
 
 int pconv_refresh_affine(aig_conv_plan* pl);
@@ -2518,11 +2411,6 @@ int aig_conv_forward(aig_conv_plan* pl, const aig_half* x, const aig_half* resid
     if (rc != AIG_OK) return rc;
   }
   pl->staged = pl->is_fc && !residual && pl->BK == 64 && pl->MS == 1 && pl->NT >= 64 && pl->prm.tw == kTileM && pl->d.out_c % 8 == 0 && !(pl->d.two_step && pl->d.act != AIG_ACT_NONE);
-  if (pl->staged && pl->pair_clusters && pl->tmapA2_ptr != x) {
-    const int rc = encode_pair_operand(pl, &pl->tmapA2, x, pl->d.in_w);
-    if (rc != AIG_OK) return rc;
-    pl->tmapA2_ptr = x;
-  }
   if (pl->staged && (pl->tmapFc_ptr != y || pl->tmapFc_f32 != pl->out_f32)) {
     const int rc = encode_fc_output(pl, y);
     if (rc != AIG_OK) return rc;

@@ -141,13 +141,6 @@ def test_fc_two_step(env, rows, inC, outC):
 
 
 @gpu
-@pytest.mark.parametrize("rows,inC,outC", [(2400, 80, 2048), (2432, 512, 2040), (2433, 64, 2048), (9473, 144, 264), (18880, 1024, 136)])
-def test_fc_two_step_cta_pairs(env, rows, inC, outC):
-    """A full wave of 256-wide tiles and more: CTA pairs, with odd M tiles, K tails and ragged N tiles."""
-    test_fc_two_step(env, rows, inC, outC)
-
-
-@gpu
 def test_fc_fused_per_activation_bn_relu(env):
     """FC -> BatchNorm(per activation) -> ReLU as NN.cpp:45-47 chains them."""
     U = env
