@@ -365,12 +365,13 @@ struct aig_mha_plan {
   aig_conv_plan *sq = nullptr, *sk = nullptr, *sv = nullptr, *so = nullptr;       // streaming (rows B)
   __half *qkv = nullptr, *ctxbuf = nullptr;                                        // [B][T][3E], [B][T][E]; a step's q, k, v are [B][E] each in qkv
   __half *kcache = nullptr, *vcache = nullptr;                                     // [B][window][E]
-  float2* rope = nullptr;
+  float2* rope = nullptr;  // two tables [T][kD/2]: the kept one, and the one that captures make
   CUtensorMap mq{}, mk{}, mv{};
   bool weights_set = false;
   int stream_start = -1;  // first position appended since the last reset
   int ring = 0;           // slots in the ring cache
-  int rope_pos0 = -1;     // first position of the table in `rope` (-1: none)
+  bool rope_kept = false; // the first of the two tables in `rope` is made, for positions from rope_pos0 on
+  int rope_pos0 = 0;
 };
 
 namespace {
@@ -426,7 +427,7 @@ int aig_mha_plan_create(aig_ctx* ctx, int batch, int seq_len, int embed, int hea
   if (rc == AIG_OK && (cudaMalloc(&pl->qkv, 3 * n * 2) != cudaSuccess || cudaMalloc(&pl->ctxbuf, n * 2) != cudaSuccess ||
                        cudaMalloc(&pl->kcache, (size_t)batch * pl->ring * embed * 2) != cudaSuccess ||
                        cudaMalloc(&pl->vcache, (size_t)batch * pl->ring * embed * 2) != cudaSuccess ||
-                       cudaMalloc(&pl->rope, (size_t)seq_len * (kD / 2) * sizeof(float2)) != cudaSuccess))
+                       cudaMalloc(&pl->rope, (size_t)2 * seq_len * (kD / 2) * sizeof(float2)) != cudaSuccess))
     rc = aig_fail(ctx, AIG_ERR_CUDA, "mha plan: device allocation failed");
   const int nk = seq_len <= 64 ? 64 : 128;
   if (rc == AIG_OK) rc = encode_qkv(pl, &pl->mq, pl->qkv, kQRows);
@@ -487,16 +488,23 @@ int aig_mha_forward(aig_mha_plan* pl, const aig_half* x, aig_half* y, int pos0) 
   prm.gerr = ctx->d_err;
   prm.rope = nullptr;
   if (pl->rope_base > 0.f) {
-    // the table of these positions is kept (a capture records its making: the graph may run before anything else does)
+    // The table of the last positions is kept.  A capture records the making of a table of its own behind the kept one:
+    // a replay, at whatever time, then neither finds the kept table changed nor changes it.
     cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;
     AIG_CUDA_OK(ctx, cudaStreamIsCapturing(ctx->stream, &capturing));
+    const bool captured = capturing != cudaStreamCaptureStatusNone;
     const int n = pl->T * (kD / 2);
-    if (pl->rope_pos0 != pos0 || capturing != cudaStreamCaptureStatusNone) {
-      pl->rope_pos0 = capturing == cudaStreamCaptureStatusNone ? pos0 : -1;
-      rope_table_kernel<<<ceil_div(n, 128), 128, 0, ctx->stream>>>(pl->rope, pl->T, kD / 2, kD, pl->rope_base, pos0);
+    float2* table = captured ? pl->rope + n : pl->rope;
+    if (captured || !pl->rope_kept || pl->rope_pos0 != pos0) {
+      if (!captured) pl->rope_kept = false;
+      rope_table_kernel<<<ceil_div(n, 128), 128, 0, ctx->stream>>>(table, pl->T, kD / 2, kD, pl->rope_base, pos0);
       AIG_LAUNCH_OK(ctx);
+      if (!captured) {
+        pl->rope_kept = true;
+        pl->rope_pos0 = pos0;
+      }
     }
-    prm.rope = pl->rope;
+    prm.rope = table;
   }
   rc = pl->T <= 64 ? launch_attention<64>(pl, prm) : launch_attention<128>(pl, prm);
   if (rc != AIG_OK) return rc;

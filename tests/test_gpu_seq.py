@@ -166,3 +166,43 @@ def test_mha_streaming_ring_cache_equals_windowed_full_sequence(env):
     c.sync()
     assert U.scaled_err(U.host(y).reshape(B, E), want[:, 0]) < 1e-2
     plan.close()
+
+
+@gpu
+@pytest.mark.parametrize("T", [16, 100])   # both tile kernels
+def test_mha_rotation_beside_a_replayed_capture(env, T):
+    """A captured forward of some positions, replayed between eager forwards of others: each call rotates by its own
+    positions, whatever ran before it."""
+    U = env
+    import torch
+
+    c, pk = U.ctx(), U.pkg()
+    B, E, Hh = 2, 128, 2
+    rng = np.random.default_rng(T)
+    plan = pk.MhaPlan(c, B, T, E, Hh, rope_base=10000.0)
+    plan.set_weights(*[U.dev(PL.xavier_uniform(rng, (E, E), E, E)) for _ in range(4)])
+    x = U.dev(h(rng.standard_normal((B, T, E))))
+    y = torch.zeros(B * T * E, dtype=torch.float16, device="cuda")
+    yg = torch.zeros_like(y)
+
+    def eager(pos0):
+        plan.forward(x, y, pos0=pos0)
+        c.sync()
+        return U.host(y).copy()
+
+    at = {pos0: eager(pos0) for pos0 in (-1, 0, 5)}
+    assert not np.array_equal(at[0], at[5])     # the rounding of the rotated halves differs
+    assert np.array_equal(eager(-1), at[-1])    # the plan's first forward had made its table
+    c.graph_begin()
+    plan.forward(x, yg, pos0=5)
+    g = c.graph_end()
+    for replays in range(3):
+        assert np.array_equal(eager(0), at[0]), "eager forward after %d replays" % replays
+        yg.zero_()
+        torch.cuda.synchronize()
+        c.graph_launch(g)
+        c.sync()
+        assert np.array_equal(U.host(yg), at[5])
+        assert np.array_equal(eager(0), at[0]), "eager forward after a replay"
+    pk.lib().aig_graph_destroy(g)
+    plan.close()
