@@ -35,6 +35,13 @@ int afail(aig_agent* a, int code, const std::string& msg) {
   a->err = msg;
   return code;
 }
+// the encoder's launches in them hold parameters by value: as in the encoder, a parameter load drops them
+void drop_graphs(aig_agent* a) {
+  for (aig_graph*& g : a->graphs) {
+    aig_graph_destroy(g);
+    g = nullptr;
+  }
+}
 }  // namespace
 
 extern "C" {
@@ -73,7 +80,7 @@ int aig_agent_create(aig_ctx* ctx, const aig_cnn_config* ccfg, const aig_seq_con
 int aig_agent_destroy(aig_agent* a) {
   if (!a) return AIG_OK;
   if (a->ctx) aig_ctx_sync(a->ctx);
-  for (aig_graph* g : a->graphs) aig_graph_destroy(g);
+  drop_graphs(a);
   aig_cnn_destroy(a->cnn);
   aig_seq_destroy(a->seq);
   aig_conv_plan_destroy(a->bridge);
@@ -92,6 +99,7 @@ int aig_agent_load_memory(aig_agent* a, const void* blob, size_t bytes) {
   if (bytes != aig_agent_param_bytes(&a->ccfg, &a->scfg)) return afail(a, AIG_ERR_IO, "agent parameter blob size mismatch");
   const uint8_t* p = (const uint8_t*)blob;
   const size_t n_cnn = aig_cnn_checkpoint_bytes(&a->ccfg), n_w = (size_t)a->feat * a->scfg.in_c * 2, n_b = (size_t)a->scfg.in_c * 2;
+  drop_graphs(a);
   int rc = aig_cnn_load_memory(a->cnn, p, n_cnn);
   if (rc != AIG_OK) return afail(a, rc, aig_cnn_last_error(a->cnn));
   if ((rc = aig_memcpy(a->ctx, a->bw, p + n_cnn, n_w)) != AIG_OK || (rc = aig_memcpy(a->ctx, a->bb, p + n_cnn + n_w, n_b)) != AIG_OK ||

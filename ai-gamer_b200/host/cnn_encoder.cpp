@@ -108,6 +108,7 @@ struct aig_cnn {
 };
 
 static void cnn_staging_free(CnnStaging& st);
+static void cnn_drop_graphs(aig_cnn* m);
 
 namespace {
 
@@ -335,7 +336,7 @@ int aig_cnn_create(aig_ctx* ctx, const aig_cnn_config* cfg, aig_cnn** out) {
 int aig_cnn_destroy(aig_cnn* m) {
   if (!m) return AIG_OK;
   if (m->ctx) aig_ctx_sync(m->ctx);
-  for (aig_graph* g : m->graphs) aig_graph_destroy(g);
+  cnn_drop_graphs(m);
   if (m->copy_stream) {
     cudaStreamSynchronize(m->copy_stream);
     cudaStreamDestroy(m->copy_stream);
@@ -387,6 +388,7 @@ int aig_cnn_load_memory(aig_cnn* m, const void* blob, size_t bytes) {
   if (wh[0] != c.width || wh[1] != c.height)
     return fail(m, AIG_ERR_IO, "checkpoint resolution " + std::to_string(wh[0]) + "x" + std::to_string(wh[1]) +
                                    " does not match the network input");
+  cnn_drop_graphs(m);
   m->params.used = 0;
   ConvP cv;
   BnP bn;
@@ -544,6 +546,15 @@ double aig_cnn_site_flops(aig_cnn* m, int i) { return (m && i >= 0 && i < (int)m
 double aig_cnn_site_bytes(aig_cnn* m, int i) { return (m && i >= 0 && i < (int)m->sites.size()) ? m->sites[i].bytes : 0.0; }
 
 }  // extern "C"
+
+// Captured launches hold some of the parameters by value (scale and shift of the first layer and of the stride-1 layers,
+// the mask's bias): a parameter load drops them.  One that is still running is freed when it ends.
+static void cnn_drop_graphs(aig_cnn* m) {
+  for (aig_graph*& g : m->graphs) {
+    aig_graph_destroy(g);
+    g = nullptr;
+  }
+}
 
 // Same, replayed as one CUDA graph (captured on first use for this input pointer and frame format).
 static int cnn_forward_graph_impl(aig_cnn* m, const uint8_t* bgra_dev, bool planar) {

@@ -36,7 +36,9 @@ const char* aig_cnn_last_error(aig_cnn* m);
 /* Size in bytes of the checkpoint this network reads. */
 size_t aig_cnn_checkpoint_bytes(const aig_cnn_config* cfg);
 /* NN::NN, checkpoint part (NN.cpp:13-20,67-75): header int32 width,height then every layer's
- * LoadParameters payload in construction order.  `blob` is host memory. */
+ * LoadParameters payload in construction order.  `blob` is host memory.  May be called again: later calls of
+ * every entry point use the new parameters (a graph that the caller has captured holds some of the old ones and
+ * has to be captured again). */
 int aig_cnn_load_memory(aig_cnn* m, const void* blob, size_t bytes);
 int aig_cnn_load_file(aig_cnn* m, const char* path);
 /* NN::Forward (NN.cpp:93-100) preceded by the frame preprocessing (Infer.cpp:103,109) on BGRA
@@ -136,7 +138,7 @@ int aig_agent_create(aig_ctx* ctx, const aig_cnn_config* cnn, const aig_seq_conf
 int aig_agent_destroy(aig_agent* a);
 const char* aig_agent_last_error(aig_agent* a);
 size_t aig_agent_param_bytes(const aig_cnn_config* cnn, const aig_seq_config* seq);
-/* Blob: encoder checkpoint, bridge FC (half W[feat][in_c], half b[in_c]), sequence head blob. */
+/* Blob: encoder checkpoint, bridge FC (half W[feat][in_c], half b[in_c]), sequence head blob.  May be called again. */
 int aig_agent_load_memory(aig_agent* a, const void* blob, size_t bytes);
 int aig_agent_step(aig_agent* a, const uint8_t* bgra_dev);
 int aig_agent_step_host(aig_agent* a, const uint8_t* bgra_host, float* out_host);

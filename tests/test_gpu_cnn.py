@@ -281,3 +281,43 @@ def test_small_batches_in_one_launch(env, monkeypatch, B, H, W, widths, act):
         enc.close()
     for i, (a, b) in enumerate(zip(*got)):
         assert U.scaled_err(b, a) < 6e-3, "result %d: %.4f" % (i, U.scaled_err(b, a))   # other summation orders, then a few fp16 roundings
+
+
+@gpu
+@pytest.mark.parametrize("B,chain", [(2, True), (40, False)])
+def test_second_parameter_load(env, monkeypatch, B, chain):
+    """Parameters loaded a second time take effect in full in graph replays of buffers that have been used before, in
+    both frame formats, and in the pipelined host steps."""
+    U = env
+    import torch
+
+    c, pk = U.ctx(), U.pkg()
+    monkeypatch.setenv("AIG_CNN_NO_CHAIN", "0" if chain else "1")
+    H, W, widths = 32, 64, (32, 64, 128)
+    blobs = [PL.serialize_cnn_checkpoint(PL.make_cnn_params(s, widths=widths, trivial=False), W, H) for s in (1, 2)]
+    frames = PL.make_frames(5, B, H, W)
+    d_bgra = U.dev(frames)
+    d_rgb = U.dev(np.ascontiguousarray(frames[..., [2, 1, 0]].transpose(0, 3, 1, 2)))
+    pinned, out = torch.from_numpy(frames).pin_memory(), torch.empty((B, 18), dtype=torch.float32).pin_memory()
+    enc = pk.CnnEncoder(c, B, H, W, widths=widths)
+    assert (enc.kernel_launches == 2) == chain
+    seen = []
+    for blob in (blobs[0], blobs[1], blobs[0]):
+        enc.load_bytes(blob)
+        enc.forward(d_bgra)
+        c.sync()
+        want = U.host(enc.outputs_f32()).copy()
+        seen.append(want)
+        enc.forward(d_bgra, graph=True)
+        c.sync()
+        assert np.array_equal(U.host(enc.outputs_f32()), want)
+        enc.forward_rgb(d_rgb, graph=True)
+        c.sync()
+        assert np.array_equal(U.host(enc.outputs_f32()), want)
+        for slot in (0, 1):
+            out.zero_()
+            enc.submit_host(slot, pinned, out)
+            enc.wait(slot)
+            assert np.array_equal(out.numpy(), want)
+    assert np.array_equal(seen[0], seen[2]) and not np.array_equal(seen[0], seen[1])
+    enc.close()

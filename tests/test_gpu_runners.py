@@ -201,3 +201,51 @@ def test_whole_sequences_tail_shapes(env, B, T, d, heads, n_out):
     assert U.rel_err(got, want.astype(np.float32), 0.2).max() < TOL
     assert np.abs(other - got).max() < 8e-3   # rotary attention depends on distances only; the angles round differently
     head.close()
+
+
+def _nontrivial_agent_params(seed, widths, d, heads):
+    p = PL.make_agent_params(seed, widths=widths, d=d, layers=2, heads=heads)
+    p["cnn"] = PL.make_cnn_params(seed, widths=widths, trivial=False)   # scale and shift that differ from load to load
+    return p
+
+
+@gpu
+@pytest.mark.parametrize("B,unfused", [(2, "0"), (6, "0"), (2, "1")])   # step as one captured graph, and as the encoder's graph and launches of its own
+def test_agent_second_parameter_load(env, monkeypatch, B, unfused):
+    """Parameters loaded a second time take effect in full on input buffers that have been used before."""
+    U = env
+    import torch
+
+    U.pkg()
+    from ai_gamer_b200 import runners as R
+
+    monkeypatch.setenv("AIG_SEQ_NO_FUSED_STEP", unfused)
+    H, W, widths, d, heads, window = 32, 64, (32, 64), 128, 2, 8
+    blobs = [PL.serialize_agent_params(_nontrivial_agent_params(s, widths, d, heads), W, H) for s in (3, 4)]
+    frames = PL.make_frames(9, B, H, W)
+    dev, pinned = U.dev(frames), torch.from_numpy(frames).pin_memory()
+
+    def run(agent):
+        agent.reset()
+        agent.step(dev)
+        a = U.host(agent.outputs_f32()).copy()
+        out = torch.empty((B, 18), dtype=torch.float32).pin_memory()
+        agent.step_host(pinned, out)
+        return a, out.numpy().copy()
+
+    def make():
+        return R.Agent(U.ctx(), B, H, W, widths=widths, d=d, layers=2, heads=heads, window=window)
+
+    want = []
+    for blob in blobs:
+        fresh = make()
+        fresh.load_bytes(blob)
+        want.append(run(fresh))
+        fresh.close()
+    assert not np.array_equal(want[0][0], want[1][0])
+    agent = make()
+    for i in (0, 1, 0):
+        agent.load_bytes(blobs[i])
+        for got, w in zip(run(agent), want[i]):
+            assert np.array_equal(got, w), "load of blob %d" % i
+    agent.close()
