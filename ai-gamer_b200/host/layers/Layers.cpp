@@ -10,6 +10,7 @@
 #include <string.h>
 
 #include <iostream>
+#include <memory>
 
 namespace {
 
@@ -542,7 +543,7 @@ void MultiHeadAttentionLayer::SaveParameters(std::ofstream& file, unsigned char*
 }
 
 // ------------------------------------------------------------------------------------------ NN
-// The network's inference as six launches: first convolution with BatchNorm and ReLU, the three residual blocks as one
+// NN::UseFusedInference: the network's inference as six launches: first convolution with BatchNorm and ReLU, the three residual blocks as one
 // chain, and the four FC layers with what follows them.  The layers one after another are 59 launches of 3 to 20 us with
 // a change of layout around every convolution (a 144x256 frame: 672 us, of them 318 in the first FC layer; 118 now).
 // BatchNorm is folded into the convolutions (one rounding where the layers make three); the FC layers round as the layers do.
@@ -717,16 +718,18 @@ NN::NN(cudnnHandle_t cudnnHandle, cublasHandle_t cublasHandle, int w, int h, boo
     }
     cudaFreeHost(buffer);
   }
-  if (!train) {
-    fused_ = new Inference(cudnn_, layers_);
-    if (fused_->create(inWidth_, inHeight_)) {
-      fused_->takeParameters();
-    } else {
-      cudaGetLastError();
-      delete fused_;
-      fused_ = nullptr;
-    }
+}
+bool NN::UseFusedInference() {
+  if (fused_ || batchSize_ != 1) return fused_ != nullptr;
+  fused_ = new Inference(cudnn_, layers_);
+  if (fused_->create(inWidth_, inHeight_)) {
+    fused_->takeParameters();
+  } else {
+    cudaGetLastError();
+    delete fused_;
+    fused_ = nullptr;
   }
+  return fused_ != nullptr;
 }
 NN::~NN() {
   delete fused_;
@@ -744,11 +747,14 @@ extern "C" {
 static thread_local std::string g_layers_error;
 const char* aig_layers_last_error() { return g_layers_error.c_str(); }
 
-// new NN(handle, handle, w, h, /*train*/false, ckpt_path): the reference's own network through the layer classes
+// new NN(handle, handle, w, h, /*train*/false, ckpt_path): the reference's own network through the layer classes, in its
+// fused launches: behind the opaque handle nobody reads or writes the layers
 int aig_refnn_create(aig_ctx* ctx, int w, int h, const char* ckpt_path, void** out) {
   if (!ctx || !ckpt_path || !out) return AIG_ERR_INVALID;
   try {
-    *out = new NN(ctx, ctx, w, h, false, ckpt_path);
+    std::unique_ptr<NN> nn(new NN(ctx, ctx, w, h, false, ckpt_path));
+    nn->UseFusedInference();
+    *out = nn.release();
     return AIG_OK;
   } catch (const std::exception& e) {
     g_layers_error = e.what();

@@ -291,14 +291,19 @@ class Dropout final : public Layer {
 
 // NN.h / NN.cpp:11-100: the network the reference builds (Conv k2 s2 + BN + ReLU, three ResConv blocks, three
 // FC+BN+ReLU, FC(16), Sigmoid(14)).  The checkpoint path is an argument instead of a fixed drive letter.
-// At inference (train = false) Forward runs the network as six fused launches made from the layers' parameters instead of
-// the 59 of the layers one after another; the layers stay and can be called one by one.  Parameters that change through
-// LoadParameters or SyncWeights are noticed; a caller that writes a BatchNorm's device arrays itself calls its SyncWeights.
+// Forward calls the layers one after another (59 launches): their buffers hold their outputs afterwards, and what a caller
+// has written to a BatchNorm's device arrays counts.
+// After UseFusedInference (train = false) Forward runs the network as six fused launches made from the layers' parameters
+// (a 144x256 frame: 672 -> 118 us).  The layers stay and can be called one by one, but Forward writes no layer's buffer
+// except the last FC's, which it returns, and it notices parameters that change through LoadParameters or SyncWeights
+// only: a caller that writes a BatchNorm's device arrays itself then calls its SyncWeights.  False: the fused launches do
+// not cover the network's size, and Forward stays as it was.
 class NN {
  public:
   NN(cudnnHandle_t cudnnHandle, cublasHandle_t cublasHandle, int w, int h, bool train, const std::string& ckptFile);
   ~NN();
   __half* Forward(__half* data);
+  bool UseFusedInference();
   cudnnHandle_t cudnn_;
   cublasHandle_t cublas_;
   std::vector<Layer*> layers_;
@@ -307,7 +312,7 @@ class NN {
 
  private:
   struct Inference;
-  Inference* fused_ = nullptr;  // null where the fused launches do not cover the frame size
+  Inference* fused_ = nullptr;  // from UseFusedInference on
 };
 
 // The context used by layers whose reference constructors take no handle (Swish, LeakyReLU, Sigmoid, LayerNorm):

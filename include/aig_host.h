@@ -174,7 +174,8 @@ const aig_half* aig_c3d_features(aig_c3d* m);   /* [batch][widths[n_layers]*4] p
  * The reference's own network through the C++ layer classes (ai-gamer_b200/host/layers/Layers.h, the
  * reference-compatible `Layer` subclasses and `NN`): new NN(handle, handle, w, h, train=false) with the
  * checkpoint path as an argument (NN.cpp:11-91), NN::Forward on one planar fp16 frame [3][h][w]
- * (NN.cpp:93-100).  C hooks for tests and other languages; C++ callers use the classes directly. */
+ * (NN.cpp:93-100).  C hooks for tests and other languages; C++ callers use the classes directly.  The handle is
+ * opaque, and the network behind it runs in its fused launches where they cover its size (NN::UseFusedInference). */
 int aig_refnn_create(aig_ctx* ctx, int w, int h, const char* ckpt_path, void** out);
 int aig_refnn_forward(void* nn, aig_half* x_nchw_dev, const aig_half** out_dev);
 int aig_refnn_input_size(void* nn, int* w, int* h);

@@ -308,3 +308,20 @@ def test_reference_network_sizes(env, H, W):
     # the oracle itself up to 4e-3 from exact arithmetic at these sizes
     got = U.host(got).astype(np.float32)
     assert (np.abs(got - want) / np.maximum(1.0, np.abs(want))).max() < 8e-3
+
+
+@gpu
+def test_nn_class_in_a_cpp_program(env, tmp_path):
+    """NN::Forward of the C++ class: the layers' own results and buffers, parameters as they stand on the device."""
+    import subprocess
+
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    cuda = os.environ.get("CUDA_HOME", "/usr/local/cuda")
+    lib = os.path.join(root, "ai-gamer_b200")
+    ckpt, exe = tmp_path / "n.ckpt", tmp_path / "nn_class_test"
+    ckpt.write_bytes(PL.serialize_refnn_checkpoint(PL.make_refnn_params(31, 64, 48)))
+    subprocess.run(["g++", "-std=c++17", os.path.join(root, "tests", "nn_class_test.cpp"), "-o", str(exe), "-I" + os.path.join(root, "include"),
+                    "-I" + os.path.join(lib, "host", "layers"), "-I" + os.path.join(cuda, "include"), "-L" + lib, "-laig_b200",
+                    "-Wl,-rpath," + lib, "-L" + os.path.join(cuda, "lib64"), "-lcudart"], check=True)
+    done = subprocess.run([str(exe), str(ckpt)], capture_output=True, text=True, timeout=120)
+    assert done.returncode == 0, done.stdout + done.stderr
