@@ -16,8 +16,10 @@
 
 #include <algorithm>
 #include <condition_variable>
+#include <exception>
 #include <mutex>
 #include <string>
+#include <system_error>
 #include <thread>
 #include <vector>
 
@@ -41,6 +43,27 @@ int rfail(aig_recording* r, int code, const std::string& msg) {
   r->err = msg;
   return code;
 }
+
+// The threads that read pieces, and what they share with the one that issues the copies.  Whichever way a scope that
+// holds them is left, none of them runs on.
+struct Readers {
+  std::mutex mu;
+  std::condition_variable cv;
+  long long next = 0, issued = 0;   // next piece to read; pieces whose copy has been issued
+  bool stop = false;
+  std::vector<std::thread> threads;
+
+  void finish() {
+    {
+      std::lock_guard<std::mutex> lk(mu);
+      stop = true;
+    }
+    cv.notify_all();
+    for (std::thread& t : threads) t.join();
+    threads.clear();
+  }
+  ~Readers() { finish(); }
+};
 }  // namespace
 
 extern "C" {
@@ -120,6 +143,8 @@ int aig_recording_targets(const uint16_t* key_states, const int32_t* mouse_dxdy,
   return AIG_OK;
 }
 
+}  // extern "C"
+
 // Offline inference over records [first, first + count): batches of the encoder's batch size as planar RGB (the bytes
 // of the file, untouched), two batches in flight; in the last one the frames past `count` are whatever the slot held,
 // their outputs are dropped.  out_host [count][n_out] fp32 (host memory).  n_out is the encoder's.
@@ -129,13 +154,7 @@ int aig_recording_targets(const uint16_t* key_states, const int32_t* mouse_dxdy,
 // So the file is read by several threads, in pieces of about 1 MB that go to the GPU as they come (the first batch
 // starts after one piece's read, not one batch's), through a pinned ring that the encoder keeps.  600 frames of
 // 256x144 in batches of 256: 42 ms before, 3.4 after.
-int aig_cnn_infer_recording(aig_cnn* m, aig_recording* r, long long first, long long count, int batch, int n_out, float* out_host) {
-  if (!m || !r || !out_host || batch <= 0 || n_out <= 0 || count < 0) return AIG_ERR_INVALID;
-  if (first < 0 || first + count > r->n_records) return rfail(r, AIG_ERR_INVALID, "record range outside the file");
-  const aig_cnn_config& c = cnn_config(m);
-  if (batch != c.batch || n_out != c.n_out || r->width != c.width || r->height != c.height)
-    return rfail(r, AIG_ERR_INVALID, "the encoder's batch, outputs or frame size differ from the call's");
-  if (count == 0) return AIG_OK;
+static int infer_recording(aig_cnn* m, aig_recording* r, long long first, long long count, int batch, int n_out, float* out_host) {
   // pieces: whole frames, none of them across two batches
   const int per_piece = (int)std::min<size_t>(std::max<size_t>(1, kPieceBytes / r->frame_bytes), (size_t)batch);
   const int per_batch = (batch + per_piece - 1) / per_piece;
@@ -151,11 +170,7 @@ int aig_cnn_infer_recording(aig_cnn* m, aig_recording* r, long long first, long 
   cudaGetDevice(&device);
 
   // piece i goes through ring slot i % slots: read once the copy of piece i - slots has left it, copied in order
-  std::mutex mu;
-  std::condition_variable cv;
-  long long next = 0, issued = 0;        // next piece to read; pieces whose copy has been issued
   std::vector<char> ready(n_pieces, 0);
-  bool stop = false;
   const int fd = fileno(r->f);
   auto piece_frames = [&](long long i, long long* lo) {
     const long long b = i / per_batch, k = i % per_batch;
@@ -163,40 +178,49 @@ int aig_cnn_infer_recording(aig_cnn* m, aig_recording* r, long long first, long 
     const long long end = std::min(std::min(*lo + per_piece, (b + 1) * batch), count);
     return (int)(end - *lo);
   };
+  auto read_piece = [&](long long i) {  // (the copy of piece i - slots has been issued)
+    bool ok = i < slots || cudaEventSynchronize(st->copied[i % slots]) == cudaSuccess;
+    long long lo;
+    const int n = piece_frames(i, &lo);
+    uint8_t* dst = st->ring + (size_t)(i % slots) * st->piece_bytes;
+    for (int k = 0; k < n && ok; ++k) {
+      const off_t at = (off_t)(kHeaderBytes + (first + lo + k) * (long long)r->stride + kRecordHeader);
+      size_t got = 0;
+      while (got < r->frame_bytes) {
+        const ssize_t x = pread(fd, dst + (size_t)k * r->frame_bytes + got, r->frame_bytes - got, at + (off_t)got);
+        if (x <= 0) break;
+        got += (size_t)x;
+      }
+      ok = got == r->frame_bytes;
+    }
+    return ok;
+  };
+  Readers rd;  // (declared after all that its threads use)
   auto reader = [&]() {
     cudaSetDevice(device);
     for (;;) {
       long long i;
       {
-        std::unique_lock<std::mutex> lk(mu);
-        if (stop || next == n_pieces) return;
-        i = next++;
-        cv.wait(lk, [&] { return stop || issued > i - slots; });
-        if (stop) return;
+        std::unique_lock<std::mutex> lk(rd.mu);
+        if (rd.stop || rd.next == n_pieces) return;
+        i = rd.next++;
+        rd.cv.wait(lk, [&] { return rd.stop || rd.issued > i - slots; });
+        if (rd.stop) return;
       }
-      bool ok = i < slots || cudaEventSynchronize(st->copied[i % slots]) == cudaSuccess;
-      long long lo;
-      const int n = piece_frames(i, &lo);
-      uint8_t* dst = st->ring + (size_t)(i % slots) * st->piece_bytes;
-      for (int k = 0; k < n && ok; ++k) {
-        const off_t at = (off_t)(kHeaderBytes + (first + lo + k) * (long long)r->stride + kRecordHeader);
-        size_t got = 0;
-        while (got < r->frame_bytes) {
-          const ssize_t x = pread(fd, dst + (size_t)k * r->frame_bytes + got, r->frame_bytes - got, at + (off_t)got);
-          if (x <= 0) break;
-          got += (size_t)x;
-        }
-        ok = got == r->frame_bytes;
-      }
-      std::lock_guard<std::mutex> lk(mu);
+      const bool ok = read_piece(i);
+      std::lock_guard<std::mutex> lk(rd.mu);
       ready[i] = ok ? 1 : 2;
-      cv.notify_all();
+      rd.cv.notify_all();
     }
   };
-  // a core copies about 8 GB/s out of the page cache and PCIe takes 52: eight readers keep ahead of it
+  // a core copies about 8 GB/s out of the page cache and PCIe takes 52: eight readers keep ahead of it.  Where the host
+  // gives fewer threads, those read; where it gives none, this one does.
   const long long n_readers = std::min<long long>(n_pieces, std::min(8u, std::max(1u, std::thread::hardware_concurrency())));
-  std::vector<std::thread> readers;
-  for (long long i = 0; i < n_readers; ++i) readers.emplace_back(reader);
+  rd.threads.reserve((size_t)n_readers);
+  try {
+    for (long long i = 0; i < n_readers; ++i) rd.threads.emplace_back(reader);
+  } catch (const std::system_error&) {
+  }
 
   auto collect = [&](long long b) {
     const int s = (int)(b & 1);
@@ -210,9 +234,11 @@ int aig_cnn_infer_recording(aig_cnn* m, aig_recording* r, long long first, long 
   for (long long i = 0; i < n_pieces && rc == AIG_OK; ++i) {
     const long long b = i / per_batch;
     const int s = (int)(b & 1);
-    {
-      std::unique_lock<std::mutex> lk(mu);
-      cv.wait(lk, [&] { return ready[i] != 0; });
+    if (rd.threads.empty()) {
+      io_ok = read_piece(i);
+    } else {
+      std::unique_lock<std::mutex> lk(rd.mu);
+      rd.cv.wait(lk, [&] { return ready[i] != 0; });
       io_ok = ready[i] == 1;
     }
     if (!io_ok) break;
@@ -223,9 +249,9 @@ int aig_cnn_infer_recording(aig_cnn* m, aig_recording* r, long long first, long 
       rc = cnn_stream_copy(m, s, (size_t)(lo - b * batch) * r->frame_bytes, st->ring + (size_t)(i % slots) * st->piece_bytes,
                            (size_t)n * r->frame_bytes, st->copied[i % slots]);
     {
-      std::lock_guard<std::mutex> lk(mu);
-      issued = i + 1;
-      cv.notify_all();
+      std::lock_guard<std::mutex> lk(rd.mu);
+      rd.issued = i + 1;
+      rd.cv.notify_all();
     }
     if (rc == AIG_OK && (i + 1 == n_pieces || (i + 1) % per_batch == 0)) {
       // the slot's output buffer is free once the batch before the last has been taken from it
@@ -233,16 +259,29 @@ int aig_cnn_infer_recording(aig_cnn* m, aig_recording* r, long long first, long 
       if (rc == AIG_OK) rc = cnn_stream_submit(m, s, st->out[s], true);
     }
   }
-  {
-    std::lock_guard<std::mutex> lk(mu);
-    stop = true;
-    cv.notify_all();
-  }
-  for (std::thread& t : readers) t.join();
+  rd.finish();
   for (long long b = (n_batches >= 2 ? n_batches - 2 : 0); b < n_batches && rc == AIG_OK && io_ok; ++b) rc = collect(b);
   if (rc == AIG_OK && io_ok) return AIG_OK;
   cnn_stream_drain(m);  // the ring and the output buffers are not in use any more
   return rc != AIG_OK ? rfail(r, rc, aig_cnn_last_error(m)) : rfail(r, AIG_ERR_IO, "short read of a frame");
 }
 
-}  // extern "C"
+extern "C" int aig_cnn_infer_recording(aig_cnn* m, aig_recording* r, long long first, long long count, int batch, int n_out, float* out_host) {
+  if (!m || !r || !out_host || batch <= 0 || n_out <= 0 || count < 0) return AIG_ERR_INVALID;
+  try {
+    if (first < 0 || first + count > r->n_records) return rfail(r, AIG_ERR_INVALID, "record range outside the file");
+    const aig_cnn_config& c = cnn_config(m);
+    if (batch != c.batch || n_out != c.n_out || r->width != c.width || r->height != c.height)
+      return rfail(r, AIG_ERR_INVALID, "the encoder's batch, outputs or frame size differ from the call's");
+    return count == 0 ? AIG_OK : infer_recording(m, r, first, count, batch, n_out, out_host);
+  } catch (const std::exception&) {
+    // host memory or threads ran out; the threads have ended, and copies that were issued end here
+    try {
+      cnn_stream_drain(m);
+      r->err = "out of host memory or threads";
+    } catch (const std::exception&) {
+      r->err.clear();
+    }
+    return AIG_ERR_IO;
+  }
+}

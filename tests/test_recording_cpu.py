@@ -76,3 +76,18 @@ def test_byte_normalisation_by_reciprocal_is_exact():
     recip = np.float32(1.0) / np.float32(255.0)
     assert recip.view(np.uint32) == 0x3B808081
     assert np.array_equal(by_div.view(np.uint16), (v * recip).astype(np.float16).view(np.uint16))
+
+
+def test_inference_where_the_host_refuses_threads_or_memory(tmp_path):
+    """aig_cnn_infer_recording returns a status, and right outputs with it, whatever number of reader threads can be
+    started and whichever allocation fails; nothing leaves the C entry point as an exception."""
+    import subprocess
+
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    host = os.path.join(root, "ai-gamer_b200", "host")
+    exe = tmp_path / "recording_threads_test"
+    subprocess.run(["g++", "-std=c++17", "-O1", "-rdynamic", os.path.join(root, "tests", "recording_threads_test.cpp"), os.path.join(host, "recording.cpp"),
+                    "-o", str(exe), "-I" + os.path.join(root, "include"), "-I" + host,
+                    "-I" + os.path.join(os.environ.get("CUDA_HOME", "/usr/local/cuda"), "include"), "-pthread", "-ldl"], check=True)
+    done = subprocess.run([str(exe), str(tmp_path / "r.rec")], capture_output=True, text=True, timeout=120)
+    assert done.returncode == 0, "status %d\n%s%s" % (done.returncode, done.stdout, done.stderr)
