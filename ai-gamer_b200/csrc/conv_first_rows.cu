@@ -29,6 +29,7 @@
 #include "conv_first_rows.h"
 
 #include "aig_common.cuh"
+#include "conv_first_words.h"
 
 namespace {
 
@@ -62,6 +63,7 @@ struct RowsParams {
   float slope;
   float scale[kN], shift[kN];
   const uint8_t* frames;   // clips: planar fp16
+  uintptr_t end;           // address behind them
   const uint4* wimg;       // RowsCfg::kSmemB bytes, the shared-memory image of the weights
   int* gerr;
 };
@@ -110,34 +112,11 @@ __device__ __forceinline__ float act_rows(float v, float slope) {
   return v;
 }
 
-// eight halves of a row starting at any element, `n` of them in the row (zero beyond), by aligned 32-bit words; a word
-// that holds a needed half may hold one past the tensor's end as well
-__device__ __forceinline__ uint4 load_halfs8(const __half* src, int n) {
-  const uintptr_t a = reinterpret_cast<uintptr_t>(src);
-  const uint32_t* w = reinterpret_cast<const uint32_t*>(a & ~(uintptr_t)3);
-  const int odd = (int)(a >> 1) & 1;
-  uint32_t v[5];
-#pragma unroll
-  for (int k = 0; k < 5; ++k) v[k] = 2 * k - odd < n && (k < 4 || odd) ? __ldg(w + k) : 0u;
-  uint4 o;
-  uint32_t* p = reinterpret_cast<uint32_t*>(&o);
-#pragma unroll
-  for (int k = 0; k < 4; ++k) {
-    p[k] = odd ? __funnelshift_r(v[k], v[k + 1], 16) : v[k];
-    if (2 * k >= n) p[k] = 0u;
-    else if (2 * k + 1 >= n) p[k] &= 0xFFFFu;
-  }
-  return o;
-}
-// four bytes likewise
-__device__ __forceinline__ uint32_t load_bytes4(const uint8_t* src, int n) {
-  const uintptr_t a = reinterpret_cast<uintptr_t>(src);
-  const uint32_t* w = reinterpret_cast<const uint32_t*>(a & ~(uintptr_t)3);
-  const int off = (int)(a & 3);
-  const uint32_t lo = __ldg(w), hi = off + n > 4 ? __ldg(w + 1) : 0u;
-  const uint32_t v = __funnelshift_r(lo, hi, off * 8);
-  return n < 4 ? v & ((1u << (8 * n)) - 1u) : v;
-}
+struct GlobalLoads {
+  __device__ __forceinline__ uint32_t word(uintptr_t a) const { return __ldg(reinterpret_cast<const uint32_t*>(a)); }
+  __device__ __forceinline__ uint32_t half(uintptr_t a) const { return __ldg(reinterpret_cast<const uint16_t*>(a)); }
+  __device__ __forceinline__ uint32_t byte(uintptr_t a) const { return __ldg(reinterpret_cast<const uint8_t*>(a)); }
+};
 
 template <int ACT, bool CLIP>
 __global__ void __launch_bounds__(kThreads, RowsCfg<CLIP>::kCtas)
@@ -323,10 +302,17 @@ conv_first_rows_kernel(const __grid_constant__ CUtensorMap tmapY, const __grid_c
           const int rr = idx / segs, seg = idx - rr * segs, c = rr / kColRows, r = rr - c * kColRows, row = 2 * y - 1 + r;
           if (row < 0 || row >= p.H) continue;
           const __half* src = reinterpret_cast<const __half*>(p.frames) + (size_t)n * 3 * plane + ((size_t)(d0 + c) * p.H + row) * p.W + 8 * seg;
-          uint4 v[3];
+          uint32_t v[3][4];
+          if (whole) {
 #pragma unroll
-          for (int ch = 0; ch < 3; ++ch) v[ch] = whole ? __ldg(reinterpret_cast<const uint4*>(src + ch * plane)) : load_halfs8(src + ch * plane, p.W - 8 * seg);
-          const uint32_t *pr = reinterpret_cast<const uint32_t*>(&v[0]), *pg = reinterpret_cast<const uint32_t*>(&v[1]), *pb = reinterpret_cast<const uint32_t*>(&v[2]);
+            for (int ch = 0; ch < 3; ++ch) {
+              const uint4 q = __ldg(reinterpret_cast<const uint4*>(src + ch * plane));
+              v[ch][0] = q.x; v[ch][1] = q.y; v[ch][2] = q.z; v[ch][3] = q.w;
+            }
+          } else {
+            row_halfs8x3(reinterpret_cast<uintptr_t>(src), plane * sizeof(__half), p.W - 8 * seg, p.end, GlobalLoads(), v);
+          }
+          const uint32_t *pr = v[0], *pg = v[1], *pb = v[2];
           uint2* d = reinterpret_cast<uint2*>(sm + kOffRing + (size_t)(((col + c) & (kColumns - 1)) * kColRows + r) * kPitch) + 8 * seg + 1;
 #pragma unroll
           for (int k = 0; k < 4; ++k) {
@@ -364,7 +350,9 @@ conv_first_rows_kernel(const __grid_constant__ CUtensorMap tmapY, const __grid_c
 #pragma unroll
           for (int k = 0; k < 4; ++k) px[k] = k < left ? pixel_bgra(__ldg(s + k)) : make_uint2(0, 0);
         } else {
-          const uint32_t r = load_bytes4(frame + off, left), g = load_bytes4(frame + plane + off, left), b = load_bytes4(frame + 2 * plane + off, left);
+          uint32_t v[3];
+          row_bytes4x3(reinterpret_cast<uintptr_t>(frame + off), plane, left, p.end, GlobalLoads(), v);
+          const uint32_t r = v[0], g = v[1], b = v[2];
           px[0] = pixel_rgb(r, g, b, 0x7540u);
           px[1] = pixel_rgb(r, g, b, 0x7541u);
           px[2] = pixel_rgb(r, g, b, 0x7542u);
@@ -592,6 +580,8 @@ static int rows_forward(ConvFirstRows* t, const void* x, __half* y) {
     if (rc != AIG_OK) return rc;
   }
   t->prm.frames = static_cast<const uint8_t*>(x);
+  const size_t pixels = (size_t)t->g.batch * t->g.D * t->g.H * t->g.W;
+  t->prm.end = reinterpret_cast<uintptr_t>(x) + pixels * (CLIP ? 3 * sizeof(__half) : t->prm.planar ? 3 : 4);
   switch (t->g.act) {
     case AIG_ACT_RELU: return rows_launch<AIG_ACT_RELU, CLIP>(t);
     case AIG_ACT_SWISH: return rows_launch<AIG_ACT_SWISH, CLIP>(t);
