@@ -18,6 +18,7 @@ struct aig_ctx {
   bool own_stream = false;
   int* d_err = nullptr;   // device error word written by kernels whose bounded waits expire
   int* h_err = nullptr;   // pinned mirror
+  bool dependent_launches = true;  // launches may start under their predecessors' tails (AIG_NO_PDL=1 at creation: none does)
   std::string last_error;
 };
 
@@ -75,17 +76,22 @@ static inline long long ceil_div_ll(long long a, long long b) { return (a + b - 
 // Device helpers
 #ifdef __CUDACC__
 
-// Launch that may start under its predecessor's tail (the kernel calls griddep_wait before it touches what others write)
+// Attribute of a launch that may start under its predecessor's tail (the kernel calls griddep_wait before it touches what
+// others write)
+static inline cudaLaunchAttribute pdl_attribute(const aig_ctx* ctx) {
+  cudaLaunchAttribute a{};
+  a.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  a.val.programmaticStreamSerializationAllowed = ctx->dependent_launches ? 1 : 0;
+  return a;
+}
 template <class... P, class... A>
-static inline cudaError_t launch_pdl(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, A&&... args) {
+static inline cudaError_t launch_pdl(const aig_ctx* ctx, void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, A&&... args) {
   cudaLaunchConfig_t cfg{};
   cfg.gridDim = grid;
   cfg.blockDim = block;
   cfg.dynamicSmemBytes = smem;
-  cfg.stream = stream;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.stream = ctx->stream;
+  cudaLaunchAttribute attr[1] = {pdl_attribute(ctx)};
   cfg.attrs = attr;
   cfg.numAttrs = 1;
   return cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);

@@ -1,5 +1,6 @@
 // ctx.cu -- context, error reporting, CUDA-graph capture, host-side output decisions.
 #include <stdarg.h>
+#include <stdlib.h>
 
 #include "aig_common.cuh"
 
@@ -66,6 +67,7 @@ int aig_ctx_create(aig_ctx** out, int device) {
     return AIG_ERR_CUDA;
   }
   ctx->own_stream = true;
+  if (const char* e = getenv("AIG_NO_PDL")) ctx->dependent_launches = !atoi(e);
   *out = ctx;
   return AIG_OK;
 }

@@ -784,7 +784,7 @@ int seq_tail_forward(aig_ctx* ctx, const aig_half* x, const float* gamma, const 
   DeviceGuard guard(ctx->device);
   const size_t smem = (size_t)c * 8 + (size_t)(n_out + 7) / 8 * 8 * (c + 8) * 2;
   const int grid = std::min((rows + 16 * kTailPairs - 1) / (16 * kTailPairs), 2 * ctx->sm_count);
-  AIG_CUDA_OK(ctx, launch_pdl(seq_tail_kernel, dim3(grid), dim3(kTailThreads), smem, ctx->stream, (const __half*)x, gamma, beta, (const __half*)fc_w,
+  AIG_CUDA_OK(ctx, launch_pdl(ctx, seq_tail_kernel, dim3(grid), dim3(kTailThreads), smem, (const __half*)x, gamma, beta, (const __half*)fc_w,
                               (const __half*)fc_b, (__half*)out_half, out_f32, rows, c, n_out, n_sigmoid, eps));
   return AIG_OK;
 }
@@ -1065,8 +1065,7 @@ int aig_adaptive_avgpool3d_ndhwc(aig_ctx* ctx, const aig_half* x, aig_half* y, i
     attr[0].id = cudaLaunchAttributeClusterDimension;
     attr[0].val.clusterDim.x = ctas;
     attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
-    attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[1].val.programmaticStreamSerializationAllowed = 1;
+    attr[1] = pdl_attribute(ctx);
     cfg.attrs = attr;
     cfg.numAttrs = 2;
     AIG_CUDA_OK(ctx, cudaLaunchKernelEx(&cfg, adaptive_avgpool3d_vec_kernel, (const __half*)x, (__half*)y, batch, d, h, w, c, ph, pw));
@@ -1083,7 +1082,7 @@ int aig_fc_head_forward(aig_ctx* ctx, const aig_half* x, const aig_half* w_in_ou
   AIG_REQUIRE(ctx, x && w_in_out && out_half && rows >= 0 && in_c > 0 && n_out > 0 && n_sigmoid >= 0 && n_sigmoid <= n_out && in_c <= 12288,
               "aig_fc_head_forward: bad arguments");
   if (rows == 0) return AIG_OK;
-  AIG_CUDA_OK(ctx, launch_pdl(fc_head_kernel, dim3(rows), dim3(256), in_c * sizeof(float), ctx->stream, (const __half*)x, (const __half*)w_in_out,
+  AIG_CUDA_OK(ctx, launch_pdl(ctx, fc_head_kernel, dim3(rows), dim3(256), in_c * sizeof(float), (const __half*)x, (const __half*)w_in_out,
                               (const __half*)bias, (__half*)out_half, out_f32, in_c, n_out, n_sigmoid));
   return AIG_OK;
 }

@@ -1543,7 +1543,6 @@ struct aig_conv_plan {
   bool pc_pair = false;                        // CTA pairs (clusters of two, tcgen05 cta_group::2): see pconv_kernel, PAIR
   bool pc_wres = false;
   int pc_in_h = 0, pc_in_w = 0, pc_in_c = 0;  // extents of the tensor the patch rows are read from
-  bool pc_pdl = true;                          // launch with programmatic stream serialization (AIG_NO_PDL=1 turns it off)
   bool is_down = false;                        // fused down-sampling pair (main k4 s2 p1 + shortcut k2 s2 p0)
   bool in_padded = false;                      // input and residual arrive in the padded position layout
   bool res_tiles = false;                      // ... and the residual is delivered by TMA into two 8 KB tiles of shared memory
@@ -1560,7 +1559,7 @@ int launch_igemm(aig_conv_plan* pl) {
     AIG_CUDA_OK(ctx, cudaFuncSetAttribute(igemm_kernel<NT, BK, MS, STAGED>, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::kSmemBytes));
     attr_set[ctx->device & 63] = true;
   }
-  AIG_CUDA_OK(ctx, launch_pdl(igemm_kernel<NT, BK, MS, STAGED>, dim3(pl->grid), dim3(kNumThreads), Cfg::kSmemBytes, ctx->stream, pl->tmapA, pl->tmapB, pl->tmapFc, pl->prm));
+  AIG_CUDA_OK(ctx, launch_pdl(ctx, igemm_kernel<NT, BK, MS, STAGED>, dim3(pl->grid), dim3(kNumThreads), Cfg::kSmemBytes, pl->tmapA, pl->tmapB, pl->tmapFc, pl->prm));
   return AIG_OK;
 }
 
@@ -1787,8 +1786,7 @@ int launch_pconv(aig_conv_plan* pl) {
   cfg.dynamicSmemBytes = (size_t)pl->pc_smem;
   cfg.stream = ctx->stream;
   cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr[0].val.programmaticStreamSerializationAllowed = pl->pc_pdl ? 1 : 0;
+  attr[0] = pdl_attribute(ctx);
   cfg.attrs = attr;
   cfg.numAttrs = 1;
   AIG_CUDA_OK(ctx, cudaLaunchKernelEx(&cfg, pconv_kernel<NT, MS, WRES, EW>, pl->tmapP, pl->tmapPT, pl->tmapBp, pl->tmapY[0], pl->tmapY[1], pl->pp));
@@ -1810,8 +1808,7 @@ int launch_pconv_pair256(aig_conv_plan* pl) {
   cfg.dynamicSmemBytes = (size_t)pl->pc_smem;
   cfg.stream = ctx->stream;
   cudaLaunchAttribute attr[2];
-  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr[0].val.programmaticStreamSerializationAllowed = pl->pc_pdl ? 1 : 0;
+  attr[0] = pdl_attribute(ctx);
   attr[1].id = cudaLaunchAttributeClusterDimension;
   attr[1].val.clusterDim.x = 2;
   attr[1].val.clusterDim.y = 1;
@@ -2022,7 +2019,6 @@ bool pconv_choose_tile(aig_ctx* ctx, aig_conv_plan* pl, const PconvNtOption* opt
 #ifdef AIG_TUNING
   if (const char* e = getenv("AIG_PCONV_DIRECT")) if (atoi(e)) q.direct_store = 1;  // (the staging tiles stay allocated)
 #endif
-  if (const char* e = getenv("AIG_NO_PDL")) pl->pc_pdl = !atoi(e);
   pl->pc_NT = NT;
   pl->pc_MS = best_ms;
   pl->pc_wres = best_res;

@@ -302,8 +302,7 @@ int recurrent_config(aig_ctx* ctx, const LstmLaunch& l, int batch, cudaLaunchCon
   attr[0].id = cudaLaunchAttributeClusterDimension;
   attr[0].val.clusterDim.x = l.cluster;
   attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
-  attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr[1].val.programmaticStreamSerializationAllowed = 1;
+  attr[1] = pdl_attribute(ctx);
   *cfg = cudaLaunchConfig_t{};
   cfg->gridDim = dim3(ceil_div(batch, G * kSeqs) * l.cluster);
   cfg->blockDim = dim3(lstm_threads(G));

@@ -653,8 +653,7 @@ cudaLaunchConfig_t chain_config(const ResChain* c, int clusters, cudaLaunchAttri
   attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
   attr[1].id = cudaLaunchAttributeCooperative;
   attr[1].val.cooperative = 1;
-  attr[2].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr[2].val.programmaticStreamSerializationAllowed = 1;
+  attr[2] = pdl_attribute(c->ctx);
   cudaLaunchConfig_t cfg{};
   cfg.gridDim = dim3(clusters * kCluster);
   cfg.blockDim = dim3(kThreads);

@@ -742,8 +742,7 @@ int seq_step_fused_run(SeqStepFused* s, const aig_half* emb, const aig_half* fea
   cudaLaunchAttribute attr[2];
   attr[0].id = cudaLaunchAttributeCooperative;
   attr[0].val.cooperative = 1;
-  attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr[1].val.programmaticStreamSerializationAllowed = 1;
+  attr[1] = pdl_attribute(ctx);
   cfg.attrs = attr;
   cfg.numAttrs = after_encoder ? 2 : 1;
   AIG_CUDA_OK(ctx, cudaLaunchKernelEx(&cfg, step_kernel(s->cfg.batch), p));

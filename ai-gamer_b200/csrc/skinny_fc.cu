@@ -121,8 +121,7 @@ cudaError_t launch(aig_ctx* ctx, const SkinnyFc& p, int ctas) {
   attr[0].id = cudaLaunchAttributeClusterDimension;
   attr[0].val.clusterDim.x = ctas;
   attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
-  attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr[1].val.programmaticStreamSerializationAllowed = 1;
+  attr[1] = pdl_attribute(ctx);
   cfg.attrs = attr;
   cfg.numAttrs = 2;
   const int nkb = (p.in_c + 31) / 32;

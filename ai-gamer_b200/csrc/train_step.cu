@@ -316,7 +316,7 @@ int aig_loss_gradient(aig_ctx* ctx, aig_half* grad, const aig_half* pred, const 
   AIG_ENTER(ctx);
   AIG_REQUIRE(ctx, grad && pred && targets && n >= 0, "aig_loss_gradient: bad arguments");
   if (n == 0) return AIG_OK;
-  AIG_CUDA_OK(ctx, launch_pdl(loss_gradient_kernel, dim3(blocks_for(ctx, n)), dim3(kThreads), 0, ctx->stream, (__half*)grad, (const __half*)pred,
+  AIG_CUDA_OK(ctx, launch_pdl(ctx, loss_gradient_kernel, dim3(blocks_for(ctx, n)), dim3(kThreads), 0, (__half*)grad, (const __half*)pred,
                               (const __half*)targets, n));
   return AIG_OK;
 }
@@ -632,7 +632,7 @@ int aig_fc_adamw_update(aig_ctx* ctx, aig_conv_plan* forward_plan, int in_c, int
   a.r2 = (float)(1.0 / a.c2);
   const bool vec = out_c % 8 == 0 && (((uintptr_t)weights | (uintptr_t)grad_w | (uintptr_t)m_w | (uintptr_t)v_w) & 15) == 0;
   const dim3 grid((out_c + kAdamTile - 1) / kAdamTile, (in_c + kAdamTile - 1) / kAdamTile + 1);
-  AIG_CUDA_OK(ctx, launch_pdl(vec ? adamw_f16_fc_kernel<true> : adamw_f16_fc_kernel<false>, grid, dim3(256), 0, ctx->stream, a));
+  AIG_CUDA_OK(ctx, launch_pdl(ctx, vec ? adamw_f16_fc_kernel<true> : adamw_f16_fc_kernel<false>, grid, dim3(256), 0, a));
   return AIG_OK;
 }
 
@@ -651,7 +651,7 @@ int aig_fc_backward(aig_fc_backward_plan* pl, const aig_half* x, const aig_half*
   int rc = AIG_OK;
   if (grad_w && pl->batch <= kWgMaxBatch) {
     const bool aligned = (((uintptr_t)x | (uintptr_t)grad | (uintptr_t)grad_w) & 15) == 0;
-    AIG_CUDA_OK(ctx, launch_pdl(fc_wgrad_small_kernel, dim3((pl->out_c + kWgTile - 1) / kWgTile, (pl->in_c + kWgTile - 1) / kWgTile), dim3(128), 0, ctx->stream,
+    AIG_CUDA_OK(ctx, launch_pdl(ctx, fc_wgrad_small_kernel, dim3((pl->out_c + kWgTile - 1) / kWgTile, (pl->in_c + kWgTile - 1) / kWgTile), dim3(128), 0,
                                 (const __half*)x, (const __half*)grad, (__half*)grad_w, (__half*)grad_b, pl->batch, pl->in_c, pl->out_c,
                                 aligned && pl->in_c % 8 == 0 ? 1 : 0, aligned && pl->out_c % 8 == 0 ? 1 : 0));
   } else if (grad_w) {
