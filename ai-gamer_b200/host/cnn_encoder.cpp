@@ -325,7 +325,17 @@ int aig_cnn_create(aig_ctx* ctx, const aig_cnn_config* cfg, aig_cnn** out) {
       in = b.y;
     }
     if (ok && (rc = res_chain_create(ctx, rb, h * w, cl, c.n_out, &m->chain)) != AIG_OK) return bail(rc);
-    if (m->chain) m->launches_per_forward = 2;
+    if (m->chain) {
+      // the launches that a forward makes: the blocks' and the head's sites become one
+      m->launches_per_forward = 2;
+      aig_cnn::Site all{"res_chain_and_head", 0.0, 0.0};
+      for (size_t i = 1; i < m->sites.size(); ++i) {
+        all.flops += m->sites[i].flops;
+        all.bytes += m->sites[i].bytes;
+      }
+      m->sites.resize(1);
+      m->sites.push_back(all);
+    }
   }
   m->params.cap = aig_cnn_checkpoint_bytes(&c) + 256 * (16 + 32 * (size_t)c.n_blocks);
   if (cudaMalloc(reinterpret_cast<void**>(&m->params.base), m->params.cap) != cudaSuccess) return bail(AIG_ERR_CUDA);
@@ -457,10 +467,12 @@ static int cnn_forward_impl(aig_cnn* m, const uint8_t* bgra_dev, bool planar) {
   if (planar) CNN_OK(m, aig_conv0_forward_rgb_planar(m->conv0, bgra_dev, m->act0));
   else CNN_OK(m, aig_conv0_forward_bgra(m->conv0, bgra_dev, m->act0));
   tick();
-  if (m->chain && !prof) {
+  if (m->chain) {
     const int hw = m->bh.back() * m->bw.back();
     CNN_OK(m, res_chain_forward(m->chain, ResChainHead{m->sa_w, m->fcw, m->fcb, m->sa_b, m->feat, m->logits, m->out_f32, hw, c.widths[c.n_blocks],
                                                        c.n_out, c.n_sigmoid}));
+    tick();
+    if (prof) ++m->prof_steps;
     return AIG_OK;
   }
   const aig_half* x = m->act0;

@@ -73,7 +73,8 @@ int aig_cnn_kernel_launches(aig_cnn* m);
 /* Per-launch device timing of aig_cnn_forward (eager path) with CUDA events on the context stream:
  * begin() arms it for up to max_steps forwards; end() synchronises and writes the mean milliseconds
  * of every launch site (aig_cnn_site_count of them, in launch order).  site_flops/site_bytes are the
- * algorithmic 2*MAC and bytes of one launch, the numerators of the roofline figures. */
+ * algorithmic 2*MAC and bytes of one launch, the numerators of the roofline figures.  Small batches run the residual
+ * blocks and the head as one launch, which is one site; AIG_CNN_NO_CHAIN=1 gives an encoder launches of their own. */
 int aig_cnn_profile_begin(aig_cnn* m, int max_steps);
 int aig_cnn_profile_end(aig_cnn* m, double* mean_ms, int capacity, int* steps);
 int aig_cnn_site_count(aig_cnn* m);

@@ -321,3 +321,33 @@ def test_second_parameter_load(env, monkeypatch, B, chain):
             assert np.array_equal(out.numpy(), want)
     assert np.array_equal(seen[0], seen[2]) and not np.array_equal(seen[0], seen[1])
     enc.close()
+
+
+@gpu
+@pytest.mark.parametrize("B,H,W,widths", [(2, 48, 80, (32, 64, 128)), (300, 32, 64, (32, 64))])
+def test_profile_times_the_launches_of_a_forward(env, B, H, W, widths):
+    """Per-launch timing covers the launches that a forward makes, in one launch for the residual blocks or one each, and
+    leaves the results as they are."""
+    U = env
+    c, pk = U.ctx(), U.pkg()
+    enc = pk.CnnEncoder(c, B, H, W, widths=widths)
+    enc.load_bytes(PL.serialize_cnn_checkpoint(PL.make_cnn_params(8, widths=widths, trivial=False), W, H))
+    frames = U.dev(PL.make_frames(3, B, H, W))
+    enc.forward(frames)
+    c.sync()
+    want = U.host(enc.outputs_f32()).copy()
+    enc.profile_begin(4)
+    for _ in range(4):
+        enc.forward(frames)
+        c.sync()
+        assert np.array_equal(U.host(enc.outputs_f32()), want)
+    sites, steps = enc.profile_end()
+    assert steps == 4 and len(sites) == enc.kernel_launches and all(0.0 < ms < 50.0 for _, ms, _, _ in sites)
+    h, w = (H + 1) // 2, (W + 1) // 2
+    flops = 2.0 * B * h * w * widths[0] * 75
+    for ci, co in zip(widths, widths[1:]):
+        h, w = h // 2, w // 2
+        flops += 2.0 * B * h * w * co * (ci * 20 + co * 9)
+    flops += 2.0 * B * widths[-1] * 18
+    assert abs(sum(f for _, _, f, _ in sites) / flops - 1.0) < 1e-9
+    enc.close()
