@@ -19,13 +19,17 @@
 // every input row is read and converted once per CTA (twice at range borders).
 // Conversion: half(float(u8) / 255.0f) as the reference computes it; float(u8) * fl(1/255) rounds to the same
 // half for all 256 byte values, so the division is a multiplication here.
-// Frames whose rows are not whole 16-byte pieces are loaded by aligned 32-bit words, four pixels at a time.
+// Frames whose rows are not whole 16-byte pieces are loaded by aligned 32-bit words, four pixels at a time.  Wider rows than
+// the 256 pixels of a row buffer go to the gather kernel (conv_first_tc.cu), which has no such limit and is slower.
 //
 // CLIP: the first layer of the clip encoder (ConvLayer3D, 3 -> 32 channels, 3x3x3, stride 1x2x2, pad 1) from planar fp16
 // clips in the same way: pixel x lies at half-unit x + 1, so output pixel x reads units x, x+1 (pixels 2x-1 .. 2x+2, the
 // last with zero weights) and each of the nine (depth, row) pairs is one instruction.  Tiles run along the depth first: a
-// column of three input rows joins the ring per tile, so every input row is loaded once or, at odd rows, twice.  Bound by
-// HBM (16 clips of 8x144x256: 28 MB in, 75 MB out); the per-tap gather that this replaces took 69 us there.
+// column of three input rows joins the ring per tile, so every input row is loaded once or, at odd rows, twice.
+// 16 clips of 8x144x256 (28 MB in, 75 MB out: 16 us at the copy bandwidth) take 45 us, 69 with the per-tap gather that this
+// replaces.  No unit is near its peak (L1 39 %, issue slots 35 %, DRAM 15 %): the loaders wait for their global loads, with
+// two CTAs on an SM.  An infinity or NaN in pixel 2x + 2 times its zero weights would make output pixel x NaN: a pixel whose
+// first sum is NaN is summed again over its own window.
 #include "conv_first_rows.h"
 
 #include "aig_common.cuh"
@@ -117,6 +121,21 @@ struct GlobalLoads {
   __device__ __forceinline__ uint32_t half(uintptr_t a) const { return __ldg(reinterpret_cast<const uint16_t*>(a)); }
   __device__ __forceinline__ uint32_t byte(uintptr_t a) const { return __ldg(reinterpret_cast<const uint8_t*>(a)); }
 };
+
+// The 32 sums of one output pixel of a clip (x[n], depth z, row y, column x) over its window alone; wimg: the weights' image.
+__device__ __noinline__ void clip_pixel_sums(const __half* clips, const uint8_t* wimg, int D, int H, int W, int n, int z, int y, int x, float* sums) {
+  for (int k = 0; k < kN; ++k) sums[k] = 0.f;
+  for (int m = 0; m < 9; ++m)
+    for (int t = 0; t < 3; ++t) {
+      const int d = z - 1 + m / 3, row = 2 * y - 1 + m % 3, col = 2 * x - 1 + t;
+      if (d < 0 || d >= D || row < 0 || row >= H || col < 0 || col >= W) continue;
+      for (int ch = 0; ch < 3; ++ch) {
+        const float v = __half2float(clips[(((size_t)(n * 3 + ch) * D + d) * H + row) * W + col]);
+        const uint8_t* w = wimg + (m * 2 + (t >> 1)) * kN * 16 + (4 * (t & 1) + ch) * 2;
+        for (int k = 0; k < kN; ++k) sums[k] = fmaf(v, __half2float(*reinterpret_cast<const __half*>(w + k * 16)), sums[k]);
+      }
+    }
+}
 
 template <int ACT, bool CLIP>
 __global__ void __launch_bounds__(kThreads, RowsCfg<CLIP>::kCtas)
@@ -247,6 +266,12 @@ conv_first_rows_kernel(const __grid_constant__ CUtensorMap tmapY, const __grid_c
         tc_fence_before();
         __syncwarp();
         if (lane == 0) mbar_arrive(bar_tempty + 8 * acc);
+        if (CLIP && x < p.Wo && isnan(__uint_as_float(r[0]))) {
+          float sums[kN];
+          clip_pixel_sums(reinterpret_cast<const __half*>(p.frames), sm + kOffB, p.D, p.H, p.W, n, z, y, x, sums);
+#pragma unroll
+          for (int k = 0; k < kN; ++k) r[k] = __float_as_uint(sums[k]);
+        }
         if (x < p.Wo) {
           const uint32_t dst = sOut + (uint32_t)buf * kOutBytes + (uint32_t)slot * 64u;
 #pragma unroll

@@ -561,3 +561,35 @@ def test_first_clip_layer(env, B, D, H, W):
     c.sync()
     assert np.abs(U.host(y).astype(np.float32).transpose(0, 4, 1, 2, 3) - want).max() < 6e-3
     plan.close()
+
+
+@gpu
+@pytest.mark.parametrize("B,D,H,W", [(2, 3, 20, 256), (3, 2, 17, 101)])
+def test_first_clip_layer_infinities_and_nan(env, B, D, H, W):
+    """An infinity or NaN in a clip reaches the output pixels whose window holds it and no others (in even and odd
+    columns: the row kernel multiplies the pixel behind every window by zero weights)."""
+    U = env
+    import torch
+
+    c, pk = U.ctx(), U.pkg()
+    rng = np.random.default_rng(W)
+    w, b = h(rng.standard_normal((32, 3, 3, 3, 3)) * 0.2), h(rng.uniform(-0.2, 0.2, 32))
+    x = h(rng.random((B, 3, D, H, W)))
+    for i, (row, col) in enumerate([(0, 0), (1, 2), (4, 15), (7, 16), (8, W - 1), (9, W - 2), (12, 64), (13, 63), (H - 1, 40), (H - 1, 41)]):
+        x[i % B, i % 3, (i // 2) % D, row, col] = (np.inf, -np.inf, np.nan)[i % 3]
+    want = torch.nn.functional.conv3d(torch.from_numpy(x.astype(np.float64)), torch.from_numpy(w.astype(np.float64)),
+                                      torch.from_numpy(b.astype(np.float64)), (1, 2, 2), 1)
+    want = torch.nn.functional.leaky_relu(want, 0.01).numpy()
+    plan = pk.Conv0Plan(c, B, H, W, 32, 3, 2, 1, act=pk.ACT_LEAKY, slope=0.01, in_d=D, kd=3, sd=1, pd=1)
+    plan.set_weights(U.dev(w), U.dev(b))
+    _, Ho, Wo = plan.out_dims()
+    y = torch.full((B, D, Ho, Wo, 32), 7.0, dtype=torch.float16, device="cuda")
+    plan.forward_nchw(U.dev(x), y)
+    c.sync()
+    got = U.host(y).astype(np.float64).transpose(0, 4, 1, 2, 3)
+    plan.close()
+    assert np.isnan(want).any() and np.isinf(want).any()
+    assert np.array_equal(np.isnan(got), np.isnan(want))
+    assert np.array_equal(np.where(np.isinf(got), got, 0.0), np.where(np.isinf(want), want, 0.0))
+    ok = np.isfinite(want)
+    assert np.abs(got[ok] - want[ok]).max() < 6e-3
