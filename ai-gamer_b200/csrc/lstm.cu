@@ -17,7 +17,7 @@
 // takes 1.7 us up to 112 sequences (1.2 at H = 256).  Of a step's 3300 clk the 32 MMAs take 1400, the gate functions 560,
 // issue and delivery of the copies 1070 (about 20 B/clk of distributed shared memory).  Above 112 sequences (16 in each
 // of the seven clusters of 16 CTAs that fit the device) a cluster takes two groups of 16, each with its own epilogue
-// warps, so that one group's MMAs run under the other's gates and delivery.
+// warps, so that one group's MMAs run under the other's gates and delivery (1.9 us a step at 128 sequences).
 // Gate order i,f,g,o; blob layout: per layer W then R, then per layer bW [and bR]  (the library's
 // blob is opaque in the reference: LSTMLayer.cpp:29-35,139-146; this layout is this library's
 // definition, stated in the header).

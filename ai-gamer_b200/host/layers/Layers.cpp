@@ -545,7 +545,7 @@ void MultiHeadAttentionLayer::SaveParameters(std::ofstream& file, unsigned char*
 // ------------------------------------------------------------------------------------------ NN
 // NN::UseFusedInference: the network's inference as six launches: first convolution with BatchNorm and ReLU, the three residual blocks as one
 // chain, and the four FC layers with what follows them.  The layers one after another are 59 launches of 3 to 20 us with
-// a change of layout around every convolution (a 144x256 frame: 672 us, of them 318 in the first FC layer; 118 now).
+// a change of layout around every convolution (a 144x256 frame: 280 us a forward; 84 in these launches).
 // BatchNorm is folded into the convolutions (one rounding where the layers make three); the FC layers round as the layers do.
 struct NN::Inference {
   struct Block {

@@ -294,7 +294,7 @@ class Dropout final : public Layer {
 // Forward calls the layers one after another (59 launches): their buffers hold their outputs afterwards, and what a caller
 // has written to a BatchNorm's device arrays counts.
 // After UseFusedInference (train = false) Forward runs the network as six fused launches made from the layers' parameters
-// (a 144x256 frame: 672 -> 118 us).  The layers stay and can be called one by one, but Forward writes no layer's buffer
+// (a 144x256 frame: 280 -> 84 us).  The layers stay and can be called one by one, but Forward writes no layer's buffer
 // except the last FC's, which it returns, and it notices parameters that change through LoadParameters or SyncWeights
 // only: a caller that writes a BatchNorm's device arrays itself then calls its SyncWeights.  False: the fused launches do
 // not cover the network's size, and Forward stays as it was.

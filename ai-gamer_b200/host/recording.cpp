@@ -153,7 +153,8 @@ int aig_recording_targets(const uint16_t* key_states, const int32_t* mouse_dxdy,
 // the page cache in about 4 ms, and allocating and freeing pinned memory for two batches took longer than all of it.
 // So the file is read by several threads, in pieces of about 1 MB that go to the GPU as they come (the first batch
 // starts after one piece's read, not one batch's), through a pinned ring that the encoder keeps.  600 frames of
-// 256x144 in batches of 256: 42 ms before, 3.4 after.
+// 256x144 in batches of 256: 42 ms before, 3.3 after; an encoder's first call, which allocates the ring and captures the
+// two slots' graphs, takes 22 to 25.
 static int infer_recording(aig_cnn* m, aig_recording* r, long long first, long long count, int batch, int n_out, float* out_host) {
   // pieces: whole frames, none of them across two batches
   const int per_piece = (int)std::min<size_t>(std::max<size_t>(1, kPieceBytes / r->frame_bytes), (size_t)batch);

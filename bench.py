@@ -515,7 +515,7 @@ def leg_agent_batched(env, full):
     return {"value": env.world * B / (ms * 1e-3), "unit": "frames/s", "sequences_per_gpu": B, "steps": K,
             **{k: res[k] for k in ("ms_per_step", "ms_per_step_min", "ms_per_step_max", "repeats", "timed_s")}, "clocks": res["clocks"],
             "l2": "inputs rotate over %d frame batches (%.0f MB > 126 MB L2)" % (n_rot, n_rot * B * HEIGHT * WIDTH * 4 / 1e6),
-            "roofline": {"bound": "tensor", "kernel": "whole step (encoder graph + bridge FC + sequence-head step launches)", **fracs(whole, env.peaks)}}
+            "roofline": {"bound": "tensor", "kernel": "whole step (encoder, bridge FC and sequence-head step as one graph)", **fracs(whole, env.peaks)}}
 
 
 def streaming_latency(env, n_frames):

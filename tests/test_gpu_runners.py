@@ -8,7 +8,7 @@ from oracle import oracle as O
 from oracle import pipelines as PL
 
 gpu = pytest.mark.gpu
-TOL = 2e-2  # relative tolerance on the outputs (fp16 compute), see the north-star statement
+TOL = 2e-2  # relative tolerance on the outputs (fp16 compute)
 
 
 @pytest.fixture(scope="module")
