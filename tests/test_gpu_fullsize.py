@@ -168,10 +168,12 @@ def test_sequence_head_full_size(env):
 
 
 @gpu
-def test_sequence_head_streaming_128_sequences_ring_wraps(env):
-    """The batched streaming step (128 sequences, the per-operator path) for 80 steps over a 64-slot ring
-    cache: equal to the oracle's sliding-window forward on two of the sequences, before and after the wrap."""
+@pytest.mark.parametrize("unfused", ["0", "1"])   # the one-kernel step, and the launches per operator
+def test_sequence_head_streaming_128_sequences_ring_wraps(env, monkeypatch, unfused):
+    """The batched streaming step (128 sequences) for 80 steps over a 64-slot ring cache: equal to the oracle's
+    sliding-window forward on two of the sequences, before and after the wrap."""
     U = env
+    monkeypatch.setenv("AIG_SEQ_NO_FUSED_STEP", unfused)
     U.pkg()
     from ai_gamer_b200 import runners as R
 
@@ -199,7 +201,7 @@ def test_streaming_agent_full_geometry(env):
     """The whole agent at its configuration (Infer.cpp:96-114 loop body): full 144x256 encoder -> FC 256->512
     -> 2 x LSTM-512 with carried state -> 8 x 64 attention over a 64-slot ring -> LayerNorm -> FC, one frame
     per call for 80 frames at batch 1 (the one-kernel step), so the ring wraps; then 128 sequences per call
-    (the batched path) for a few frames with the oracle on the first and the last sequence."""
+    for a few frames with the oracle on the first and the last sequence."""
     U = env
     import torch
 

@@ -28,9 +28,10 @@ def _seq_head(U, batch, seq_len, d, heads, window):
 
 
 @gpu
-@pytest.mark.parametrize("B", [4, 6, 1])   # up to 4 sequences stream through the one-kernel step, more through the per-operator launches
-def test_sequence_head_full_and_streaming(env, B):
+@pytest.mark.parametrize("B,unfused", [(4, "0"), (6, "0"), (1, "0"), (6, "1")])   # the one-kernel step, and the launches per operator
+def test_sequence_head_full_and_streaming(env, monkeypatch, B, unfused):
     U = env
+    monkeypatch.setenv("AIG_SEQ_NO_FUSED_STEP", unfused)
     U.pkg()
     T, d, heads = 16, 128, 2
     p = PL.make_seq_params(5, d=d, hid=d, layers=2, heads=heads)

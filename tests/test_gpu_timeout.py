@@ -55,7 +55,7 @@ def test_expired_wait_reports_timeout_and_the_context_stays_usable(env):
 
 @gpu
 def test_streaming_step_keeps_working_after_a_reported_timeout(env):
-    """The one-kernel streaming step keeps its grid-barrier state per launch, so an error reported between two
+    """The one-kernel streaming step starts its grid barrier from zero in every launch, so an error reported between two
     steps (here: from the self-test kernel on the same context) does not disturb the steps that follow."""
     U = env
     from oracle import pipelines as PL
