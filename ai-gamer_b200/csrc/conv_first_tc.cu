@@ -643,8 +643,10 @@ int launch_tc(ConvFirstTc* t, const void* x, bool bgra, __half* y) {
     AIG_CUDA_OK(ctx, cudaFuncSetAttribute(conv_first_tc_kernel<KD, KHW, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)t->smem));
     conv_first_tc_kernel<KD, KHW, true><<<t->grid, kThreads, t->smem, ctx->stream>>>(x, y, reinterpret_cast<const uint4*>(t->wimg), t->prm);
   } else {
+    TcParams prm = t->prm;
+    prm.pair = prm.pair && ((uintptr_t)x & 3) == 0;  // an fp16 tensor may start at any half, a pair's load may not
     AIG_CUDA_OK(ctx, cudaFuncSetAttribute(conv_first_tc_kernel<KD, KHW, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)t->smem));
-    conv_first_tc_kernel<KD, KHW, false><<<t->grid, kThreads, t->smem, ctx->stream>>>(x, y, reinterpret_cast<const uint4*>(t->wimg), t->prm);
+    conv_first_tc_kernel<KD, KHW, false><<<t->grid, kThreads, t->smem, ctx->stream>>>(x, y, reinterpret_cast<const uint4*>(t->wimg), prm);
   }
   AIG_LAUNCH_OK(ctx);
   return AIG_OK;

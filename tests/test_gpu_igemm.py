@@ -593,3 +593,29 @@ def test_first_clip_layer_infinities_and_nan(env, B, D, H, W):
     assert np.array_equal(np.where(np.isinf(got), got, 0.0), np.where(np.isinf(want), want, 0.0))
     ok = np.isfinite(want)
     assert np.abs(got[ok] - want[ok]).max() < 6e-3
+
+
+@gpu
+@pytest.mark.parametrize("B,D,H,W", [(1, 4, 12, 20), (2, 3, 9, 64), (1, 2, 10, 23), (1, 2, 6, 300), (1, 2, 5, 301)])
+@pytest.mark.parametrize("offset", [0, 1, 4])
+def test_first_clip_layer_by_the_gather(env, offset, B, D, H, W):
+    """The per-tap gather of the 3-D first layer, which takes rows beyond 256 pixels and clips that start off a 16-byte
+    boundary: column pairs at a whole word, single halves elsewhere, rows shorter than a warp to longer than the row
+    kernel's."""
+    U = env
+    import torch
+
+    c, pk = U.ctx(), U.pkg()
+    rng = np.random.default_rng(W)
+    x, w, b = PL.make_clips(W, B, D, H, W), PL.he_normal(rng, (32, 3, 3, 3, 3)), h(rng.uniform(-0.2, 0.2, 32))
+    want = O.leaky_relu(O.conv3d(x, w, b, 1, 2, 1, 1), 0.01)
+    plan = pk.Conv0Plan(c, B, H, W, 32, 3, 2, 1, act=pk.ACT_LEAKY, slope=0.01, in_d=D, kd=3, sd=1, pd=1)
+    plan.set_weights(U.dev(w), U.dev(b))
+    room = torch.zeros(x.size + 8, dtype=torch.float16, device="cuda")
+    room[offset:offset + x.size] = U.dev(x).flatten()
+    y = torch.full((want.size,), 7.0, dtype=torch.float16, device="cuda")
+    torch.cuda.synchronize()
+    plan.forward_nchw(room[offset:], y)
+    c.sync()
+    assert U.scaled_err(U.nchw(U.host(y).reshape(B, *want.shape[2:], 32)), want) < 4e-3
+    plan.close()
