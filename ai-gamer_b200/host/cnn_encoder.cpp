@@ -154,6 +154,11 @@ struct Reader {
   }
 };
 
+int checkpoint_size_error(aig_cnn* m, long long bytes) {
+  return fail(m, AIG_ERR_IO, "checkpoint size " + std::to_string(bytes) + " does not match the network (" +
+                                 std::to_string(aig_cnn_checkpoint_bytes(&m->cfg)) + " bytes expected)");
+}
+
 bool read_conv(aig_cnn* m, Reader& rd, ConvP& c, size_t nw, size_t nb, cudaStream_t s) {
   c.nw = nw;
   c.nb = nb;
@@ -388,9 +393,7 @@ const char* aig_cnn_last_error(aig_cnn* m) { return m ? m->err.c_str() : "null m
 int aig_cnn_load_memory(aig_cnn* m, const void* blob, size_t bytes) {
   if (!m || !blob) return AIG_ERR_INVALID;
   const aig_cnn_config& c = m->cfg;
-  if (bytes != aig_cnn_checkpoint_bytes(&c))
-    return fail(m, AIG_ERR_IO, "checkpoint size " + std::to_string(bytes) + " does not match the network (" +
-                                   std::to_string(aig_cnn_checkpoint_bytes(&c)) + " bytes expected)");
+  if (bytes != aig_cnn_checkpoint_bytes(&c)) return checkpoint_size_error(m, (long long)bytes);
   cudaStream_t s = (cudaStream_t)aig_ctx_stream(m->ctx);
   Reader rd{(const uint8_t*)blob, bytes};
   int32_t wh[2];
@@ -441,7 +444,8 @@ int aig_cnn_load_file(aig_cnn* m, const char* path) {
   if (!m || !path) return AIG_ERR_INVALID;
   std::ifstream f(path, std::ios::binary | std::ios::ate);
   if (!f.is_open()) return fail(m, AIG_ERR_IO, std::string("cannot open ") + path);
-  const std::streamsize n = f.tellg();
+  const std::streamsize n = f.tellg();  // (a directory opens too, and has an absurd one)
+  if (n != (std::streamsize)aig_cnn_checkpoint_bytes(&m->cfg)) return checkpoint_size_error(m, n);
   f.seekg(0);
   std::vector<char> buf((size_t)n);
   if (!f.read(buf.data(), n)) return fail(m, AIG_ERR_IO, std::string("cannot read ") + path);

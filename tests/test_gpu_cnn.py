@@ -351,3 +351,21 @@ def test_profile_times_the_launches_of_a_forward(env, B, H, W, widths):
     flops += 2.0 * B * widths[-1] * 18
     assert abs(sum(f for _, _, f, _ in sites) / flops - 1.0) < 1e-9
     enc.close()
+
+
+@gpu
+def test_checkpoint_files(env, tmp_path):
+    """A checkpoint from a file; a file of another size, a directory and a missing file are errors, not exceptions."""
+    U = env
+    c, pk = U.ctx(), U.pkg()
+    enc = pk.CnnEncoder(c, 1, 32, 64, widths=(32, 64))
+    blob = PL.serialize_cnn_checkpoint(PL.make_cnn_params(3, widths=(32, 64)), 64, 32)
+    (tmp_path / "whole").write_bytes(blob)
+    (tmp_path / "short").write_bytes(blob[:-2])
+    for name, text in (("short", "does not match"), (".", "does not match"), ("missing", "cannot open")):
+        with pytest.raises(pk.AigError, match=text):
+            enc.load_file(str(tmp_path / name))
+    enc.load_file(str(tmp_path / "whole"))
+    enc.forward(U.dev(PL.make_frames(1, 1, 32, 64)))
+    c.sync()
+    enc.close()
