@@ -11,13 +11,18 @@
 //      within each quad of lanes, keep the cell state in registers (rounded to fp16 every step, like the library's cy
 //      tensor) and write h_t as fp16, and
 //    - one bulk copy per CTA of the cluster delivers its 32 units of h_t, already in the operand's layout.
-// With so few columns an MMA instruction costs what its issue costs: 41 to 48 clk with R in shared memory, 33 in TMEM.
-// What bounds a step is this chain's latency.  Sharing the sequences' h through global memory, with a step barrier over
-// all CTAs on a global counter, took 4.06 us a step at H = 512 and 128 sequences (3.66 at 3 sequences, H = 256); this
-// takes 1.7 us up to 112 sequences (1.2 at H = 256).  Of a step's 3300 clk the 32 MMAs take 1400, the gate functions 560,
-// issue and delivery of the copies 1070 (about 20 B/clk of distributed shared memory).  Above 112 sequences (16 in each
-// of the seven clusters of 16 CTAs that fit the device) a cluster takes two groups of 16, each with its own epilogue
-// warps, so that one group's MMAs run under the other's gates and delivery (1.9 us a step at 128 sequences).
+// What bounds a step is this chain's latency.  Of its 2550 clk (H = 512, 16 sequences; clock64) the 32 MMAs take 560, the
+// gate functions 560, issue and delivery of the copies 1270 (about 20 B/clk of distributed shared memory come into an SM);
+// with the MMAs in a loop of four it was 3240, 1160 of them the loop.  More sequences than the clusters of one group of 16 hold
+// (seven of 16 CTAs fit the device) share clusters in groups of 16, each with its own issuer and epilogue warps, so that
+// one group's MMAs run under the other's gates and delivery.  Up to eight sequences deliver half of the rows.
+//
+// (3)  Two layers run side by side in one launch where their clusters fit the device together (lstm_pair_kernel): the
+// second layer's clusters multiply W.x_t themselves, a step or two behind, W beside R in TMEM (what does not fit, in
+// shared memory).  That takes out half of the dependent steps and the second layer's projection, whose 4H fp32 values
+// per step and sequence went through memory.  Whole sequence head, before and after, us: 128 sequences of 64 at H = 512
+// (three groups a cluster and two) 380 and 260, 16 sequences 279 and 161, 64 sequences 521 and 214, 3 of 37 at H = 256
+// 132 and 76.
 // Gate order i,f,g,o; blob layout: per layer W then R, then per layer bW [and bR]  (the library's
 // blob is opaque in the reference: LSTMLayer.cpp:29-35,139-146; this layout is this library's
 // definition, stated in the header).
@@ -31,8 +36,13 @@ namespace {
 constexpr int kUnits = 32;        // hidden units per CTA: 128 gate rows, UMMA's M
 constexpr int kGateRows = 4 * kUnits;
 constexpr int kSeqs = 16;         // sequences of a group: UMMA's N
-__host__ __device__ constexpr int lstm_threads(int groups) { return 32 + 128 * groups; }  // MMA warp, four epilogue warps per group
-constexpr int kColR = 64;         // first TMEM column of R (two values of K each); the accumulator is below
+__host__ __device__ constexpr int lstm_threads(int groups) { return 32 * 5 * groups; }  // per group an MMA issuer and four epilogue warps
+__host__ __device__ constexpr int pair_threads(int ga, int gb) {  // and a warp that passes h_t on, or two for W . x_t
+  return lstm_threads(ga) + 32 > lstm_threads(gb) + 64 ? lstm_threads(ga) + 32 : lstm_threads(gb) + 64;
+}
+// TMEM columns: the groups' accumulators, [two sets of accumulators of W . x_t,] R (two values of K each) [, W]
+constexpr int kColX = 32;
+__host__ __device__ constexpr int col_r(bool second) { return second ? kColX + 4 * kSeqs : 48; }
 
 struct LstmParams {
   int T, B, H, ctas;              // ctas: CTAs of the cluster that have units (the rest of a power of two only wait)
@@ -46,22 +56,77 @@ struct LstmParams {
   __half *hT, *cT;                // [B][H] final state (may be null; may be the initial state's memory)
   int* gerr;
 };
+// Two layers in one launch: the first `a_clusters` clusters run layer a, the rest layer b (see lstm_pair_kernel).
+struct LstmPairParams {
+  LstmParams a, b;
+  int a_clusters, clusters;
+  const __half* W;                // layer b's input matrix [4][H][H]
+  const float* bias;              // and the sum of its biases [4H]
+  __half* xs;                     // h_t of layer a: [T][groups][2][H/8][8 sequences][8 units]
+  unsigned int* counters;         // [groups] parts of h_t written so far by layer a's CTAs, then clusters done
+};
 
 // own shared memory -> a cluster CTA's, the bytes counted on that CTA's barrier
 __device__ __forceinline__ void bulk_to_cluster(uint32_t dst, uint32_t src, uint32_t bytes, uint32_t bar) {
   asm volatile("cp.async.bulk.shared::cluster.shared::cta.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(dst), "r"(src), "r"(bytes), "r"(bar)
                : "memory");
 }
-// D[tmem] (+)= A[tmem] * B[smem].  B: K-major without swizzle, 8-row x 16-byte core matrices, `lbo` bytes between
-// neighbours along K, 128 along N; b_lo = plain_lo(address, lbo).
+__device__ __forceinline__ void bulk_load(uint32_t dst, const void* src, uint32_t bytes, uint32_t bar) {
+  asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(dst), "l"(src), "r"(bytes), "r"(bar)
+               : "memory");
+}
+__device__ __forceinline__ unsigned int ld_acquire_gpu(const unsigned int* p) {
+  unsigned int v;
+  asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
+  return v;
+}
+__device__ __forceinline__ void red_release_gpu_add(unsigned int* p, unsigned int v) {
+  asm volatile("red.release.gpu.global.add.u32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
+}
+__device__ __forceinline__ void fence_proxy_async_global() { asm volatile("fence.proxy.async.global;" ::: "memory"); }
+// Operands in shared memory: K-major without swizzle, core matrices of 8 rows x 16 bytes, `lbo` bytes between neighbours
+// along K, `sbo` along the rows.
 __device__ __forceinline__ uint32_t plain_lo(uint32_t saddr, uint32_t lbo) { return ((saddr & 0x3FFFFu) >> 4) | (lbo >> 4) << 16; }
-__device__ __forceinline__ void umma_f16_ts(uint32_t d_tmem, uint32_t a_tmem, uint32_t b_lo, uint32_t idesc, uint32_t accumulate) {
+__device__ __forceinline__ constexpr uint32_t plain_hi(uint32_t sbo) { return (sbo >> 4) | (1u << 14); }
+// D[tmem] (+)= A[tmem] * B[smem]
+__device__ __forceinline__ void umma_f16_ts(uint32_t d_tmem, uint32_t a_tmem, uint32_t b_lo, uint32_t b_hi, uint32_t idesc, uint32_t accumulate) {
   asm volatile(
       "{\n\t.reg .pred p;\n\t.reg .b64 db;\n\t"
       "mov.b64 db, {%2, %3};\n\t"
       "setp.ne.b32 p, %5, 0;\n\t"
       "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], db, %4, p;\n\t}"
-      ::"r"(d_tmem), "r"(a_tmem), "r"(b_lo), "r"((128u >> 4) | (1u << 14)), "r"(idesc), "r"(accumulate)
+      ::"r"(d_tmem), "r"(a_tmem), "r"(b_lo), "r"(b_hi), "r"(idesc), "r"(accumulate)
+      : "memory");
+}
+// N instructions in a row, one step of K (16) each: every iteration of a loop of them costs its branch and the way of the
+// loop's values to the uniform registers, about 75 clk, beside 20 per instruction
+template <int N>
+__device__ __forceinline__ void umma_ts_steps(bool leader, uint32_t d_tmem, uint32_t a_tmem, uint32_t b_lo, uint32_t b_units, uint32_t b_hi, uint32_t idesc,
+                                              uint32_t accumulate_first) {
+#pragma unroll
+  for (int k = 0; k < N; ++k)
+    if (leader) umma_f16_ts(d_tmem, a_tmem + k * 8, b_lo + (k >> 1) * b_units + (k & 1) * 16, b_hi, idesc, k == 0 ? accumulate_first : 1u);
+}
+// D[tmem] = A[tmem] * B[smem], `steps` (a multiple of 4) of K; b_units: from 32 units of B to the next, in 16 bytes
+__device__ __forceinline__ void umma_ts_product(bool leader, uint32_t d_tmem, uint32_t a_tmem, uint32_t b_lo, uint32_t b_units, uint32_t b_hi, uint32_t idesc,
+                                                int steps) {
+  if (steps == 32) {
+    umma_ts_steps<32>(leader, d_tmem, a_tmem, b_lo, b_units, b_hi, idesc, 0u);
+    return;
+  }
+  int k = 0;
+  for (; k + 16 <= steps; k += 16) umma_ts_steps<16>(leader, d_tmem, a_tmem + k * 8, b_lo + (k >> 1) * b_units, b_units, b_hi, idesc, k != 0 ? 1u : 0u);
+  for (; k < steps; k += 4) umma_ts_steps<4>(leader, d_tmem, a_tmem + k * 8, b_lo + (k >> 1) * b_units, b_units, b_hi, idesc, k != 0 ? 1u : 0u);
+}
+// D[tmem] += A[smem] * B[smem]
+__device__ __forceinline__ void umma_f16_ss_plain(uint32_t d_tmem, uint32_t a_lo, uint32_t a_hi, uint32_t b_lo, uint32_t b_hi, uint32_t idesc) {
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t.reg .b64 da, db;\n\t"
+      "mov.b64 da, {%1, %2};\n\t"
+      "mov.b64 db, {%3, %4};\n\t"
+      "setp.ne.b32 p, %5, 0;\n\t"
+      "tcgen05.mma.cta_group::1.kind::f16 [%0], da, db, %5, p;\n\t}"
+      ::"r"(d_tmem), "r"(a_lo), "r"(a_hi), "r"(b_lo), "r"(b_hi), "r"(idesc)
       : "memory");
 }
 __device__ __forceinline__ void tmem_st_32x32(uint32_t taddr, const uint32_t (&r)[32]) {
@@ -116,32 +181,58 @@ __device__ __forceinline__ void transpose_quad(float (&x)[4], int lane) {
   }
 }
 
-// G = groups of 16 sequences per cluster: 1 or 2.
-template <int G>
-__global__ void __launch_bounds__(lstm_threads(G), 1) lstm_recurrent_kernel(const LstmParams p) {
-  constexpr int NB = kSeqs, kThreads = lstm_threads(G);
-  constexpr int kBlock = NB * kUnits * 2;      // one CTA's units of a group: 4 chunks of 8 units, each NB rows x 16 bytes
+// What a cluster does: a layer by itself, or one of two layers that run side by side.
+enum LstmRole { kAlone, kFirst, kSecond };
+
+// Shared memory of a CTA, bytes from its start.
+struct LstmSmem {
+  int h_bytes, group_bytes;       // per group: h of all units [2] (a block per CTA), this CTA's part of h_t [2]
+  int w, x, bars, end;            // second layer: W's columns that TMEM has no room for; layer a's steps [kXStages][groups]; barriers
+};
+constexpr int kXStages = 3;
+// K of the second layer's W in TMEM: what the accumulators and R leave
+__host__ __device__ constexpr int w_tmem_k(int H) { return H <= 512 - col_r(true) ? H : 2 * (512 - col_r(true) - H / 2); }
+__host__ __device__ constexpr LstmSmem lstm_smem(int H, int groups, bool second) {
+  LstmSmem l{};
+  l.h_bytes = kSeqs * H * 2;
+  l.group_bytes = 2 * (l.h_bytes + kSeqs * kUnits * 2);
+  l.w = groups * l.group_bytes;
+  l.x = l.w + (second ? (H - w_tmem_k(H)) * kGateRows * 2 : 0);
+  l.bars = l.x + (second ? kXStages * groups * l.h_bytes : 0);
+  l.end = l.bars + 8 * (6 * groups + 2 * kXStages + 4) + 16;
+  return l;
+}
+
+// G = groups of 16 sequences per cluster.
+template <int G, int ROLE>
+__device__ __forceinline__ void recurrence(const LstmParams& p, const LstmPairParams* pp, int cluster) {
+  constexpr int NB = kSeqs;
+  constexpr int kBlock = NB * kUnits * 2;      // one CTA's units of a group: [2 x 8 sequences][4 chunks of 8 units], 8 rows x 16 bytes each
   extern __shared__ uint8_t smem_raw[];
   const uint32_t raw = smem_u32(smem_raw), base = (raw + 1023u) & ~1023u;
   uint8_t* sm = smem_raw + (base - raw);
-  const int h_bytes = NB * p.H * 2;
-  const uint32_t tmem_cols = p.H > 384 ? 512u : 256u;        // accumulators, R
-  // per group: h of all units [2] (chunks of 8 units, each NB rows x 16 bytes), then this CTA's part of h_t [2]
-  const int group_bytes = 2 * (h_bytes + kBlock);
-  uint64_t* bars = reinterpret_cast<uint64_t*>(sm + G * group_bytes);
+  const LstmSmem lay = lstm_smem(p.H, G, ROLE == kSecond);
+  const int h_bytes = lay.h_bytes, group_bytes = lay.group_bytes;
+  const uint32_t tmem_cols = ROLE != kAlone ? 512u : (p.H > 384 ? 512u : 256u);  // accumulators, R [, W]
+  uint64_t* bars = reinterpret_cast<uint64_t*>(sm + lay.bars);
   const uint32_t bar0 = smem_u32(bars);                      // per group: h arrived [2], accumulator ready, accumulator drained
-  uint32_t* s_tmem = reinterpret_cast<uint32_t*>(bars + 4 * G);
+  const uint32_t bar_part = bar0 + 32 * G;                   // first layer, per group: part of h_t written, taken
+  const uint32_t bar_xfull = bar_part + 16 * G, bar_xempty = bar_xfull + 8 * kXStages;  // second layer: x_t there, used,
+  const uint32_t bar_xready = bar_xempty + 8 * kXStages, bar_xdrained = bar_xready + 16;  // W . x_t ready, drained
+  uint32_t* s_tmem = reinterpret_cast<uint32_t*>(bars + 6 * G + 2 * kXStages + 4);
   volatile int* s_abort = reinterpret_cast<volatile int*>(s_tmem + 1);
 
   const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;  // (uniform for the compiler)
   const int rank = (int)cluster_ctarank();
-  uint32_t n_ctarank;
-  asm volatile("mov.u32 %0, %%cluster_nctarank;" : "=r"(n_ctarank));
-  const int row0 = (int)(blockIdx.x / n_ctarank) * (G * NB), unit0 = rank * kUnits;
+  const int group0 = cluster * G, row0 = group0 * NB, unit0 = rank * kUnits, n_groups = (p.B + NB - 1) / NB;
+  const int groups = min(G, n_groups - group0);
   const bool working = rank < p.ctas;
+  constexpr uint32_t kColR = col_r(ROLE == kSecond);
 
   if (threadIdx.x == 0) {
     for (int i = 0; i < 4 * G; ++i) mbar_init(bar0 + 8 * i, i % 4 == 3 ? 4 : 1);
+    for (int i = 0; i < 2 * G + 2 * kXStages + 2; ++i) mbar_init(bar_part + 8 * i, 1);
+    for (int i = 0; i < 2; ++i) mbar_init(bar_xdrained + 8 * i, 4 * groups);
     *s_abort = 0;
     fence_mbar_init();
   }
@@ -154,23 +245,32 @@ __global__ void __launch_bounds__(lstm_threads(G), 1) lstm_recurrent_kernel(cons
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *s_tmem;
-  if (working && warp >= 1 && warp <= 4) {
-    // R to TMEM: lane = row = unit * 4 + gate
+  [[maybe_unused]] const uint32_t colW = kColR + (uint32_t)p.H / 2;
+  // R to TMEM: lane = row = unit * 4 + gate.  W likewise, its last columns to shared memory.
+  const auto load_rows = [&](const __half* m, uint32_t col, int k_tmem) {
     const int q = warp & 3;
-    const uint4* src = reinterpret_cast<const uint4*>(p.R + ((size_t)(lane & 3) * p.H + unit0 + q * 8 + (lane >> 2)) * p.H);
+    const uint4* src = reinterpret_cast<const uint4*>(m + ((size_t)(lane & 3) * p.H + unit0 + q * 8 + (lane >> 2)) * p.H);
     for (int k = 0; k < p.H / 64; ++k) {
       uint4 v[8];
 #pragma unroll
       for (int i = 0; i < 8; ++i) v[i] = __ldg(src + k * 8 + i);
-      tmem_st_32x32(tmem_base + kColR + k * 32 + ((uint32_t)(q * 32) << 16), reinterpret_cast<const uint32_t (&)[32]>(v));
+      if (k * 64 < k_tmem) {
+        tmem_st_32x32(tmem_base + col + k * 32 + ((uint32_t)(q * 32) << 16), reinterpret_cast<const uint32_t (&)[32]>(v));
+      } else if (ROLE == kSecond) {
+#pragma unroll
+        for (int i = 0; i < 8; ++i) reinterpret_cast<uint4*>(sm + lay.w)[((k * 64 - k_tmem) / 8 + i) * kGateRows + q * 32 + lane] = v[i];
+      }
     }
     asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
-  }
-  griddep_wait();  // (R is what the plan was given at load time; the rest comes from the launches before this one)
+  };
+  constexpr int kWWarp = G == 1 ? G : G + 4;
+  if (working && warp >= G && warp < G + 4) load_rows(p.R, kColR, p.H);
+  if (ROLE == kSecond && working && warp >= kWWarp && warp < kWWarp + 4) load_rows(pp->W, colW, w_tmem_k(p.H));
+  griddep_wait();  // (the weights are what the plan was given at load time; the rest comes from the launches before this one)
   if (working) {
     // h_{-1}, as step -1 would have delivered it (buffer 1)
-    for (int i = threadIdx.x; i < G * h_bytes / 16; i += kThreads) {
-      const int g = i / (h_bytes / 16), k = i - g * (h_bytes / 16), chunk = k / NB, b = row0 + g * NB + k % NB;
+    for (int i = threadIdx.x; i < G * h_bytes / 16; i += blockDim.x) {
+      const int g = i / (h_bytes / 16), k = i - g * (h_bytes / 16), chunk = (k >> 6) * 4 + (k >> 3 & 3), b = row0 + g * NB + (k >> 5 & 1) * 8 + (k & 7);
       uint4 v = make_uint4(0, 0, 0, 0);
       if (p.h0 && b < p.B) v = *reinterpret_cast<const uint4*>(p.h0 + (size_t)b * p.H + chunk * 8);
       reinterpret_cast<uint4*>(sm + g * group_bytes + h_bytes)[k] = v;
@@ -181,61 +281,146 @@ __global__ void __launch_bounds__(lstm_threads(G), 1) lstm_recurrent_kernel(cons
   cluster_sync_all();  // barriers and R are there, and every CTA has read the initial h
   tc_fence_after();
 
-  if (working && warp == 0) {
-    // ------------------------------------------------------------------ MMA issuer
-    // (all lanes run the loop with identical values, one elected lane issues: see elect_one)
-    constexpr uint32_t idesc = umma_idesc_f16(kGateRows, NB);
-    const bool leader = elect_one();
-    bool ok = true;
-    for (int t = 0; t < p.T && ok; ++t) {
-      const uint32_t prev = (uint32_t)(t + 1) & 1u;  // buffer of h_{t-1}
-#pragma unroll
-      for (int g = 0; g < G; ++g) {
-        const uint32_t bar_h = bar0 + 32 * g;
-        if (row0 + g * NB >= p.B) break;  // (no sequence in this group)
-        if (leader && t + 1 < p.T) mbar_expect_tx(bar_h + 8 * (t & 1), (uint32_t)h_bytes);
-        if (t > 0) ok = ok && mbar_wait_bounded_cl(bar_h + 8 * prev, (uint32_t)((t - 1) >> 1) & 1u, s_abort, p.gerr, 404) &&
-                        mbar_wait_bounded(bar_h + 24, (uint32_t)(t - 1) & 1u, s_abort, p.gerr, 403);
-        if (!ok) break;
+  if (working && warp < G) {
+    // ------------------------------------------------------------------ MMA issuer of a group
+    // (all lanes run the loop with identical values, one elected lane issues: see elect_one.  A warp per group: one warp
+    // for all of them left the tensor pipe idle for 200 clk between two groups, and waited for them in one order.)
+    if (warp < groups) {
+      constexpr uint32_t idesc = umma_idesc_f16(kGateRows, NB);
+      const bool leader = elect_one();
+      const uint32_t bar_h = bar0 + 32 * warp, d = tmem_base + warp * NB;
+      const uint32_t part_bytes = p.B - row0 - warp * NB > NB / 2 ? kBlock : kBlock / 2;
+      for (int t = 0; t < p.T; ++t) {
+        const uint32_t prev = (uint32_t)(t + 1) & 1u;  // buffer of h_{t-1}
+        if (leader && t + 1 < p.T) mbar_expect_tx(bar_h + 8 * (t & 1), p.ctas * part_bytes);
+        if (t > 0 && !(mbar_wait_bounded_cl(bar_h + 8 * prev, (uint32_t)((t - 1) >> 1) & 1u, s_abort, p.gerr, 404) &&
+                       mbar_wait_bounded(bar_h + 24, (uint32_t)(t - 1) & 1u, s_abort, p.gerr, 403)))
+          break;
         tc_fence_after();
-        const uint32_t h = plain_lo(base + g * group_bytes + prev * h_bytes, NB * 16);
-#pragma unroll 4
-        for (int k = 0; k < p.H / 16; ++k)
-          if (leader) umma_f16_ts(tmem_base + g * NB, tmem_base + kColR + k * 8, h + (uint32_t)(k * 2 * NB), idesc, k != 0 ? 1u : 0u);
+        const uint32_t h = plain_lo(base + warp * group_bytes + prev * h_bytes, 128);
+        umma_ts_product(leader, d, tmem_base + kColR, h, kBlock / 16, plain_hi(512), idesc, p.H / 16);
         if (leader) umma_commit(bar_h + 16);
       }
     }
-  } else if (working && row0 + ((warp - 1) >> 2) * NB < p.B) {
+  } else if (ROLE == kSecond && working && warp == 5 * G) {
+    // ------------------------------------------------------------------ W . x_t of all groups at once, a step or more ahead
+    const uint32_t idesc = groups == 2 ? umma_idesc_f16(kGateRows, 2 * NB) : umma_idesc_f16(kGateRows, NB), x_hi = plain_hi(p.H * 16);
+    const uint32_t w = plain_lo(base + lay.w, kGateRows * 16);
+    const int k_tmem = w_tmem_k(p.H);
+    const bool leader = elect_one();
+    for (int t = 0; t < p.T; ++t) {
+      const int stage = t % kXStages;
+      if (!mbar_wait_bounded(bar_xfull + 8 * stage, (uint32_t)(t / kXStages) & 1u, s_abort, p.gerr, 406) ||
+          !mbar_wait_bounded(bar_xdrained + 8 * (t & 1), (uint32_t)((t >> 1) + 1) & 1u, s_abort, p.gerr, 411))
+        break;
+      tc_fence_after();
+      const uint32_t d = tmem_base + kColX + (t & 1) * 2 * NB, x = plain_lo(base + lay.x + stage * G * h_bytes, 128);
+      umma_ts_product(leader, d, tmem_base + colW, x, 32, x_hi, idesc, k_tmem / 16);
+#pragma unroll 4
+      for (int k = k_tmem / 16; k < p.H / 16; ++k)
+        if (leader) umma_f16_ss_plain(d, w + (k - k_tmem / 16) * 2 * kGateRows, plain_hi(128), x + k * 16, x_hi, idesc);
+      if (leader) umma_commit(bar_xempty + 8 * stage);
+      if (leader) umma_commit(bar_xready + 8 * (t & 1));
+    }
+  } else if (ROLE == kSecond && working && warp == 5 * G + 1) {
+    // ------------------------------------------------------------------ layer a's steps to shared memory
+    if (elect_one()) {
+      bool ok = true;
+      for (int t = 0; t < p.T && ok; ++t) {
+        const int stage = t % kXStages;
+        const uint32_t full = bar_xfull + 8 * stage;
+        ok = mbar_wait_bounded(bar_xempty + 8 * stage, (uint32_t)(t / kXStages + 1) & 1u, s_abort, p.gerr, 407);
+        if (!ok) break;
+        mbar_expect_tx(full, (uint32_t)(groups * h_bytes));
+        for (int g = 0; g < groups; ++g) {
+          const unsigned int target = (unsigned int)p.ctas * (unsigned int)(t + 1);
+          const unsigned int* counter = pp->counters + group0 + g;
+          if (ld_acquire_gpu(counter) < target) {
+            const long long t0 = clock64();
+            while (ok && ld_acquire_gpu(counter) < target) {
+              if (*s_abort) ok = false;
+              else if (clock64() - t0 > AIG_WAIT_CYCLES) {
+                *s_abort = 1;
+                atomicCAS(p.gerr, 0, 408);
+                ok = false;
+              } else __nanosleep(40);
+            }
+          }
+          if (!ok) break;
+          fence_proxy_async_global();  // written with ordinary stores, read by the bulk copy
+          bulk_load(base + lay.x + (stage * G + g) * h_bytes, pp->xs + ((size_t)t * n_groups + group0 + g) * NB * p.H, (uint32_t)h_bytes, full);
+        }
+      }
+    }
+    __syncwarp();
+  } else if (ROLE == kFirst && working && warp == 5 * G) {
+    // ------------------------------------------------------------------ this CTA's part of h_t to the second layer
+    // (a warp of its own: the release waits for the stores)
+    const uint4* stage = reinterpret_cast<const uint4*>(sm + 2 * h_bytes);
+    __half* dst = pp->xs + (size_t)group0 * NB * p.H + (unit0 + lane) * 8;
+    bool ok = true;
+    for (int t = 0; t < p.T && ok; ++t) {
+      for (int g = 0; g < groups && ok; ++g) {
+        const uint32_t bar = bar_part + 16 * g;
+        ok = __all_sync(0xffffffffu, mbar_wait_bounded(bar, (uint32_t)t & 1u, s_abort, p.gerr, 409));
+        if (!ok) break;
+        const uint4* src = stage + (g * group_bytes + (t & 1) * kBlock) / 16 + lane;
+        const uint4 v0 = src[0], v1 = src[32];
+        __syncwarp();
+        if (lane == 0) mbar_arrive(bar + 8);
+        __half* d = dst + ((size_t)t * n_groups + g) * NB * p.H;
+        *reinterpret_cast<uint4*>(d) = v0;
+        *reinterpret_cast<uint4*>(d + NB / 2 * p.H) = v1;
+      }
+      // one release for all groups: it waits for the stores to land, about 1500 clk
+      fence_proxy_async_global();
+      __syncwarp();
+      if (ok && lane < groups) red_release_gpu_add(pp->counters + group0 + lane, 1u);
+    }
+  } else if (working && warp < 5 * G && (warp - G) >> 2 < groups) {
     // ------------------------------------------------------------------ gates: one thread per gate row
-    const int group = (warp - 1) >> 2, w4 = (warp - 1) & 3, q = warp & 3, tid = w4 * 32 + lane, seq0 = row0 + group * NB;
+    const int group = (warp - G) >> 2, w4 = (warp - G) & 3, q = warp & 3, tid = w4 * 32 + lane, seq0 = row0 + group * NB;
     const uint32_t sH = base + group * group_bytes, bar_h = bar0 + 32 * group;
+    const int n_seq = p.B - seq0;
+    const uint32_t part_bytes = n_seq > NB / 2 ? kBlock : kBlock / 2;
     uint8_t* stage = sm + group * group_bytes + 2 * h_bytes;
     const int gate = lane & 3, unit = q * 8 + (lane >> 2);
     // sigmoid(x), or 2*sigmoid(2x) - 1 on the lanes of the g gate
     const float in_scale = gate == 2 ? 2.0f : 1.0f, out_scale = in_scale, out_shift = gate == 2 ? -1.0f : 0.0f;
-    const float* gsrc = p.gx + (size_t)gate * p.H + unit0 + unit;
+    const float* gsrc = ROLE == kSecond ? pp->bias + (size_t)gate * p.H + unit0 + unit : p.gx + (size_t)gate * p.H + unit0 + unit;
     float c[NB / 4], gx[NB];
 #pragma unroll
     for (int j = 0; j < NB / 4; ++j) {  // this lane's cells: its unit of sequences gate, gate + 4, ...
       const int b = seq0 + 4 * j + gate;
       c[j] = p.c0 && b < p.B ? __half2float(p.c0[(size_t)b * p.H + unit0 + unit]) : 0.f;
     }
+    const float bias = ROLE == kSecond ? __ldg(gsrc) : 0.f;
+    if (ROLE != kSecond) {
 #pragma unroll
-    for (int n = 0; n < NB; ++n) gx[n] = seq0 + n < p.B ? __ldg(gsrc + (size_t)(seq0 + n) * p.gx_sB) : 0.f;
+      for (int n = 0; n < NB; ++n) gx[n] = seq0 + n < p.B ? __ldg(gsrc + (size_t)(seq0 + n) * p.gx_sB) : 0.f;
+    }
     const uint32_t t_addr = tmem_base + group * NB + ((uint32_t)(q * 32) << 16);
     bool ok = true;
     for (int t = 0; t < p.T && ok; ++t) {
-      ok = mbar_wait_bounded(bar_h + 16, (uint32_t)t & 1u, s_abort, p.gerr, 405);
+      // (what is there early comes before the wait for R . h)
+      if (ROLE == kFirst && t > 0) ok = mbar_wait_bounded(bar_part + 16 * group + 8, (uint32_t)(t - 1) & 1u, s_abort, p.gerr, 410);
+      if (ROLE == kSecond) ok = mbar_wait_bounded(bar_xready + 8 * (t & 1), (uint32_t)(t >> 1) & 1u, s_abort, p.gerr, 412);
+      ok = mbar_wait_bounded(bar_h + 16, (uint32_t)t & 1u, s_abort, p.gerr, 405) && ok;
       tc_fence_after();
       uint32_t r[NB];
       tmem_ld_32x16(t_addr, r);
+      if (ROLE == kSecond) tmem_ld_32x16(tmem_base + kColX + ((t & 1) * 2 + group) * NB + ((uint32_t)(q * 32) << 16), reinterpret_cast<uint32_t (&)[NB]>(gx));
       tmem_ld_wait();
       tc_fence_before();
       __syncwarp();
       if (lane == 0) mbar_arrive(bar_h + 24);
-      __half* st = reinterpret_cast<__half*>(stage + (t & 1) * kBlock);
+      if (ROLE == kSecond) {
+        if (lane == 0) mbar_arrive(bar_xdrained + 8 * (t & 1));
 #pragma unroll
-      for (int j = 0; j < NB / 4; ++j) {
+        for (int n = 0; n < NB; ++n) gx[n] += bias;
+      }
+      __half* st = reinterpret_cast<__half*>(stage + (t & 1) * kBlock);
+      auto cells = [&](int j) {  // sequences 4j .. 4j + 3
         float x[4];
 #pragma unroll
         for (int k = 0; k < 4; ++k) x[k] = fmaf(sigmoid_fast(in_scale * (__uint_as_float(r[4 * j + k]) + gx[4 * j + k])), out_scale, out_shift);
@@ -244,28 +429,38 @@ __global__ void __launch_bounds__(lstm_threads(G), 1) lstm_recurrent_kernel(cons
         if (p.clip > 0.f) cn = fminf(p.clip, fmaxf(-p.clip, cn));
         c[j] = __half2float(__float2half(cn));
         const int n = 4 * j + gate;
-        st[(q * NB + n) * 8 + (lane >> 2)] = __float2half(x[3] * tanh_fast(c[j]));
+        st[((n >> 3) * 4 + q) * 64 + (n & 7) * 8 + (lane >> 2)] = __float2half(x[3] * tanh_fast(c[j]));
+      };
+      if (n_seq > 8) {  // (without branches in between: they interleave)
+        cells(0);
+        cells(1);
+        cells(2);
+        cells(3);
+      } else {
+        cells(0);
+        if (n_seq > 4) cells(1);
       }
       fence_proxy_async_smem();
       ok = epilogue_and(group, ok);
       if (!ok) break;
+      if (ROLE == kFirst && tid == 0) mbar_arrive(bar_part + 16 * group);
       // (four warps issue: the copies of one warp's lanes go out one after another)
       const int dst = (lane << 2) | w4;
       if (t + 1 < p.T && dst < p.ctas)
-        bulk_to_cluster(mapa_shared(sH + (uint32_t)((t & 1) * h_bytes + rank * kBlock), (uint32_t)dst), smem_u32(st), kBlock,
+        bulk_to_cluster(mapa_shared(sH + (uint32_t)((t & 1) * h_bytes + rank * kBlock), (uint32_t)dst), smem_u32(st), part_bytes,
                         mapa_shared(bar_h + 8 * (t & 1), (uint32_t)dst));
       // under the delivery: this step's h to memory (16 bytes of a sequence per thread), the next step's projection
-      if (t + 1 < p.T) {
+      if (ROLE != kSecond && t + 1 < p.T) {
         const float* g1 = gsrc + (size_t)(t + 1) * p.gx_sT;
 #pragma unroll
         for (int n = 0; n < NB; ++n)
           if (seq0 + n < p.B) gx[n] = __ldg(g1 + (size_t)(seq0 + n) * p.gx_sB);
       }
       if (tid < 4 * NB) {
-        const int chunk = tid / NB, b = seq0 + tid % NB;
+        const int chunk = tid >> 3 & 3, b = seq0 + (tid >> 5) * 8 + (tid & 7);
+        const uint4 v = reinterpret_cast<const uint4*>(st)[tid];
         if (b < p.B) {
-          const uint4 v = reinterpret_cast<const uint4*>(st)[tid];
-          *reinterpret_cast<uint4*>(p.y + (size_t)t * p.y_sT + (size_t)b * p.y_sB + unit0 + chunk * 8) = v;
+          if (ROLE != kFirst) *reinterpret_cast<uint4*>(p.y + (size_t)t * p.y_sT + (size_t)b * p.y_sB + unit0 + chunk * 8) = v;
           if (t == p.T - 1 && p.hT) *reinterpret_cast<uint4*>(p.hT + (size_t)b * p.H + unit0 + chunk * 8) = v;
         }
       }
@@ -290,29 +485,81 @@ __global__ void __launch_bounds__(lstm_threads(G), 1) lstm_recurrent_kernel(cons
   }
 }
 
+// One layer.  G = groups of 16 sequences per cluster: 1 or 2.
+template <int G>
+__global__ void __launch_bounds__(lstm_threads(G), 1) lstm_recurrent_kernel(const LstmParams p) {
+  uint32_t n_ctarank;
+  asm volatile("mov.u32 %0, %%cluster_nctarank;" : "=r"(n_ctarank));
+  recurrence<G, kAlone>(p, nullptr, (int)(blockIdx.x / n_ctarank));
+}
+
+// Two layers: clusters of the first do what lstm_recurrent_kernel does and write each h_t where the bulk copies of the
+// second layer's clusters find it as an operand; those run a step or two behind and multiply W . x_t themselves.
+template <int GA, int GB>
+__global__ void __launch_bounds__(pair_threads(GA, GB), 1) lstm_pair_kernel(const __grid_constant__ LstmPairParams pp) {
+  uint32_t n_ctarank;
+  asm volatile("mov.u32 %0, %%cluster_nctarank;" : "=r"(n_ctarank));
+  const int cluster = (int)(blockIdx.x / n_ctarank);
+  if (cluster < pp.a_clusters) recurrence<GA, kFirst>(pp.a, &pp, cluster);
+  else recurrence<GB, kSecond>(pp.b, &pp, cluster - pp.a_clusters);
+  // The last cluster to end (all counting is over then) leaves the counters as it found them, also after a wait that ran out.
+  if (cluster_ctarank() == 0 && threadIdx.x == 0) {
+    const int n_groups = (pp.a.B + kSeqs - 1) / kSeqs;
+    unsigned int done;
+    asm volatile("atom.acq_rel.gpu.global.add.u32 %0, [%1], 1;" : "=r"(done) : "l"(pp.counters + n_groups) : "memory");
+    if (done + 1 == (unsigned int)pp.clusters)
+      for (int i = 0; i <= n_groups; ++i) pp.counters[i] = 0u;
+  }
+}
+
 // Shape of a recurrence launch.
 struct LstmLaunch {
   int groups = 1, ctas = 0, cluster = 0;
   size_t smem = 0;
+  // two layers side by side: groups per cluster of the first and the second (0: one layer after the other)
+  int pair_a = 0, pair_b = 0;
+  size_t pair_smem = 0;
 };
-size_t recurrent_smem(int H, int groups) { return (size_t)groups * (2 * kSeqs * (H + kUnits) * 2 + 32) + 64 + 1024; }
+// (a CTA's shared memory keeps more of them off its SM than TMEM has columns for: one that waits there for another cluster's
+// TMEM would make its own cluster wait, too)
+size_t recurrent_smem(int H, int groups) {
+  const size_t n = (size_t)lstm_smem(H, groups, false).end + 1024, least = (H > 384 ? 116 : 77) * 1024;
+  return n < least ? least : n;
+}
+// (more than half of an SM's: a CTA takes all TMEM columns, so that a second one on its SM could not start)
+size_t pair_smem(int H, int ga, int gb) {
+  size_t n = lstm_smem(H, ga, false).end;
+  if (n < (size_t)lstm_smem(H, gb, true).end) n = lstm_smem(H, gb, true).end;
+  return (n < 116 * 1024 ? 116 * 1024 : n) + 1024;
+}
 
-template <int G>
-int recurrent_config(aig_ctx* ctx, const LstmLaunch& l, int batch, cudaLaunchConfig_t* cfg, cudaLaunchAttribute (&attr)[2]) {
+int cluster_config(aig_ctx* ctx, const void* kernel, int cluster, int clusters, int threads, size_t smem, bool cooperative, cudaLaunchConfig_t* cfg,
+                   cudaLaunchAttribute (&attr)[3]) {
   attr[0].id = cudaLaunchAttributeClusterDimension;
-  attr[0].val.clusterDim.x = l.cluster;
+  attr[0].val.clusterDim.x = cluster;
   attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
   attr[1] = pdl_attribute(ctx);
+  attr[2].id = cudaLaunchAttributeCooperative;
+  attr[2].val.cooperative = 1;
   *cfg = cudaLaunchConfig_t{};
-  cfg->gridDim = dim3(ceil_div(batch, G * kSeqs) * l.cluster);
-  cfg->blockDim = dim3(lstm_threads(G));
-  cfg->dynamicSmemBytes = l.smem;
+  cfg->gridDim = dim3(clusters * cluster);
+  cfg->blockDim = dim3(threads);
+  cfg->dynamicSmemBytes = smem;
   cfg->stream = ctx->stream;
   cfg->attrs = attr;
-  cfg->numAttrs = 2;
-  AIG_CUDA_OK(ctx, cudaFuncSetAttribute(lstm_recurrent_kernel<G>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)l.smem));
-  AIG_CUDA_OK(ctx, cudaFuncSetAttribute(lstm_recurrent_kernel<G>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+  cfg->numAttrs = cooperative ? 3 : 2;
+  AIG_CUDA_OK(ctx, cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  AIG_CUDA_OK(ctx, cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
   return AIG_OK;
+}
+template <int G>
+int recurrent_config(aig_ctx* ctx, const LstmLaunch& l, int batch, cudaLaunchConfig_t* cfg, cudaLaunchAttribute (&attr)[3]) {
+  return cluster_config(ctx, (const void*)lstm_recurrent_kernel<G>, l.cluster, ceil_div(batch, G * kSeqs), lstm_threads(G), l.smem, false, cfg, attr);
+}
+template <int GA, int GB>
+int pair_config(aig_ctx* ctx, const LstmLaunch& l, int batch, cudaLaunchConfig_t* cfg, cudaLaunchAttribute (&attr)[3]) {
+  return cluster_config(ctx, (const void*)lstm_pair_kernel<GA, GB>, l.cluster, ceil_div(batch, GA * kSeqs) + ceil_div(batch, GB * kSeqs),
+                        pair_threads(GA, GB), l.pair_smem, true, cfg, attr);
 }
 
 // One group of sequences per cluster, or two where the clusters of one group would not all run at once.
@@ -323,7 +570,7 @@ int recurrent_shape(aig_ctx* ctx, int H, int batch, LstmLaunch* l) {
   l->groups = 1;
   l->smem = recurrent_smem(H, 1);
   cudaLaunchConfig_t cfg;
-  cudaLaunchAttribute attr[2];
+  cudaLaunchAttribute attr[3];
   int rc = recurrent_config<1>(ctx, *l, batch, &cfg, attr), n = 0;
   if (rc != AIG_OK) return rc;
   AIG_CUDA_OK(ctx, cudaOccupancyMaxActiveClusters(&n, lstm_recurrent_kernel<1>, &cfg));
@@ -335,10 +582,33 @@ int recurrent_shape(aig_ctx* ctx, int H, int batch, LstmLaunch* l) {
   return AIG_OK;
 }
 
+// The fewest groups per cluster with which the clusters of both layers run at once.
+template <int GA, int GB>
+int try_pair(aig_ctx* ctx, int H, int batch, LstmLaunch* l) {
+  if (l->pair_a) return AIG_OK;
+  LstmLaunch t = *l;
+  t.pair_a = GA;
+  t.pair_b = GB;
+  t.pair_smem = pair_smem(H, GA, GB);
+  cudaLaunchConfig_t cfg;
+  cudaLaunchAttribute attr[3];
+  int rc = pair_config<GA, GB>(ctx, t, batch, &cfg, attr), n = 0;
+  if (rc != AIG_OK) return rc;
+  AIG_CUDA_OK(ctx, cudaOccupancyMaxActiveClusters(&n, lstm_pair_kernel<GA, GB>, &cfg));
+  if ((int)cfg.gridDim.x <= n * t.cluster) *l = t;
+  return AIG_OK;
+}
+int pair_shape(aig_ctx* ctx, int H, int batch, LstmLaunch* l) {
+  int rc = try_pair<1, 1>(ctx, H, batch, l);
+  if (rc == AIG_OK) rc = try_pair<2, 2>(ctx, H, batch, l);
+  if (rc == AIG_OK) rc = try_pair<3, 2>(ctx, H, batch, l);
+  return rc;
+}
+
 template <int G>
 int launch_recurrent(aig_ctx* ctx, const LstmLaunch& l, const LstmParams& prm) {
   cudaLaunchConfig_t cfg;
-  cudaLaunchAttribute attr[2];
+  cudaLaunchAttribute attr[3];
   const int rc = recurrent_config<G>(ctx, l, prm.B, &cfg, attr);
   if (rc != AIG_OK) return rc;
   AIG_CUDA_OK(ctx, cudaLaunchKernelEx(&cfg, lstm_recurrent_kernel<G>, prm));
@@ -348,6 +618,23 @@ int run_recurrent(aig_ctx* ctx, const LstmLaunch& l, LstmParams prm) {
   prm.ctas = l.ctas;
   prm.gerr = ctx->d_err;
   return l.groups == 1 ? launch_recurrent<1>(ctx, l, prm) : launch_recurrent<2>(ctx, l, prm);
+}
+template <int GA, int GB>
+int launch_pair(aig_ctx* ctx, const LstmLaunch& l, LstmPairParams& pp) {
+  cudaLaunchConfig_t cfg;
+  cudaLaunchAttribute attr[3];
+  const int rc = pair_config<GA, GB>(ctx, l, pp.a.B, &cfg, attr);
+  if (rc != AIG_OK) return rc;
+  pp.a_clusters = ceil_div(pp.a.B, GA * kSeqs);
+  pp.clusters = (int)cfg.gridDim.x / l.cluster;
+  AIG_CUDA_OK(ctx, cudaLaunchKernelEx(&cfg, lstm_pair_kernel<GA, GB>, pp));
+  return AIG_OK;
+}
+int run_pair(aig_ctx* ctx, const LstmLaunch& l, LstmPairParams pp) {
+  pp.a.ctas = pp.b.ctas = l.ctas;
+  pp.a.gerr = pp.b.gerr = ctx->d_err;
+  if (l.pair_a == 1) return launch_pair<1, 1>(ctx, l, pp);
+  return l.pair_a == 2 ? launch_pair<2, 2>(ctx, l, pp) : launch_pair<3, 2>(ctx, l, pp);
 }
 
 }  // namespace
@@ -363,6 +650,8 @@ struct aig_lstm_plan {
   std::vector<aig_conv_plan*> proj;     // hoisted input projection per layer
   float* gx = nullptr;                  // [T*B][4H] fp32 scratch
   __half* mid = nullptr;                // intermediate layer outputs (same layout as y)
+  __half* xs = nullptr;                 // layers in pairs: the first one's outputs as the second one's operands
+  unsigned int* counters = nullptr;     // and how far they are
 };
 
 extern "C" {
@@ -388,6 +677,7 @@ int aig_lstm_plan_create(aig_ctx* ctx, int seq_len, int layers, int hidden, int 
   pl->T = seq_len; pl->L = layers; pl->H = hidden; pl->B = batch; pl->in_c = in_c;
   pl->clip = clip; pl->double_bias = double_bias != 0; pl->batch_major = batch_major != 0;
   int rc = recurrent_shape(ctx, hidden, batch, &pl->shape);
+  if (rc == AIG_OK && layers > 1) rc = pair_shape(ctx, hidden, batch, &pl->shape);
   if (rc != AIG_OK) {
     delete pl;
     return rc;
@@ -417,6 +707,11 @@ int aig_lstm_plan_create(aig_ctx* ctx, int seq_len, int layers, int hidden, int 
   const size_t seq = (size_t)seq_len * batch;
   if (rc == AIG_OK && (cudaMalloc(&pl->gx, seq * 4 * hidden * sizeof(float)) != cudaSuccess || cudaMalloc(&pl->mid, seq * hidden * sizeof(__half)) != cudaSuccess))
     rc = aig_fail(ctx, AIG_ERR_CUDA, "lstm plan: device allocation failed");
+  const size_t groups = ceil_div(batch, kSeqs), words = (groups + 1) * sizeof(unsigned int);
+  if (rc == AIG_OK && pl->shape.pair_a &&
+      (cudaMalloc(&pl->xs, groups * kSeqs * seq_len * hidden * sizeof(__half)) != cudaSuccess || cudaMalloc(&pl->counters, words) != cudaSuccess ||
+       cudaMemsetAsync(pl->counters, 0, words, ctx->stream) != cudaSuccess))
+    rc = aig_fail(ctx, AIG_ERR_CUDA, "lstm plan: device allocation failed");
   if (rc != AIG_OK) {
     aig_lstm_plan_destroy(pl);
     return rc;
@@ -432,6 +727,8 @@ int aig_lstm_plan_destroy(aig_lstm_plan* pl) {
   for (aig_conv_plan* fp : pl->proj) aig_conv_plan_destroy(fp);
   cudaFree(pl->gx);
   cudaFree(pl->mid);
+  cudaFree(pl->xs);
+  cudaFree(pl->counters);
   delete pl;
   return AIG_OK;
 }
@@ -462,13 +759,7 @@ int aig_lstm_forward(aig_lstm_plan* pl, const aig_half* x, aig_half* y, aig_half
   AIG_REQUIRE(ctx, !use_state || h_state, "lstm forward: use_state needs the state tensors");
   const int T = pl->T, B = pl->B, H = pl->H;
   const long long sT = pl->batch_major ? H : (long long)B * H, sB = pl->batch_major ? (long long)T * H : H;
-  const __half* in = (const __half*)x;
-  for (int l = 0; l < pl->L; ++l) {
-    // a middle layer may read and write `mid`: its input is fully consumed by the hoisted projection
-    // before the recurrence starts overwriting it
-    __half* out = (l == pl->L - 1) ? (__half*)y : pl->mid;
-    int rc = aig_conv_forward(pl->proj[l], (const aig_half*)in, nullptr, (aig_half*)pl->gx);
-    if (rc != AIG_OK) return rc;
+  auto layer = [&](int l) {
     LstmParams prm{};
     prm.T = T; prm.B = B; prm.H = H;
     prm.clip = pl->clip;
@@ -477,13 +768,37 @@ int aig_lstm_forward(aig_lstm_plan* pl, const aig_half* x, aig_half* y, aig_half
     // the projection's rows follow x's memory order
     prm.gx_sT = pl->batch_major ? (long long)4 * H : (long long)B * 4 * H;
     prm.gx_sB = pl->batch_major ? (long long)T * 4 * H : (long long)4 * H;
-    prm.y = out; prm.y_sT = sT; prm.y_sB = sB;
+    // a middle layer may read and write `mid`: its input is fully consumed by the hoisted projection
+    // before the recurrence starts overwriting it
+    prm.y = (l == pl->L - 1) ? (__half*)y : pl->mid;
+    prm.y_sT = sT; prm.y_sB = sB;
     prm.h0 = use_state ? (const __half*)h_state + (size_t)l * B * H : nullptr;
     prm.c0 = use_state ? (const __half*)c_state + (size_t)l * B * H : nullptr;
     prm.hT = h_state ? (__half*)h_state + (size_t)l * B * H : nullptr;
     prm.cT = c_state ? (__half*)c_state + (size_t)l * B * H : nullptr;
-    if ((rc = run_recurrent(ctx, pl->shape, prm)) != AIG_OK) return rc;
-    in = out;
+    return prm;
+  };
+  const __half* in = (const __half*)x;
+  for (int l = 0; l < pl->L;) {
+    int rc = aig_conv_forward(pl->proj[l], (const aig_half*)in, nullptr, (aig_half*)pl->gx);
+    if (rc != AIG_OK) return rc;
+    const LstmParams first = layer(l++);
+    in = first.y;
+    if (pl->shape.pair_a && l < pl->L) {
+      LstmPairParams pp{};
+      pp.a = first;
+      pp.b = layer(l);
+      pp.W = pl->blob + pl->w_off[l];
+      pp.bias = fc_plan_shift_buffer(pl->proj[l]);
+      pp.xs = pl->xs;
+      pp.counters = pl->counters;
+      in = pp.b.y;
+      ++l;
+      rc = run_pair(ctx, pl->shape, pp);
+    } else {
+      rc = run_recurrent(ctx, pl->shape, first);
+    }
+    if (rc != AIG_OK) return rc;
   }
   return AIG_OK;
 }

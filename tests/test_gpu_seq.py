@@ -76,6 +76,45 @@ def test_lstm_matches_oracle(env, T, B, I, H, L, clip, dbl):
 
 
 @gpu
+@pytest.mark.parametrize("T,B,H,L", [
+    (1, 1, 64, 2),                                       # a single step, one CTA pair of layers
+    (5, 8, 192, 2), (5, 9, 192, 2),                      # half and whole rows delivered; six CTAs in a cluster of eight
+    (4, 4, 448, 3), (4, 5, 448, 3),                      # the first and second quad of sequences; a third layer by itself
+    (5, 16, 512, 2), (5, 17, 512, 2),                    # W partly in shared memory; a second group
+    (4, 48, 512, 2), (4, 49, 512, 2),                    # one group per cluster, two
+    (4, 112, 512, 4), (4, 113, 512, 2), (4, 128, 512, 2), (4, 129, 512, 2),  # three and two; beyond: one layer after the other
+])
+def test_lstm_layers_side_by_side(env, T, B, H, L):
+    U = env
+    import torch
+
+    c = U.ctx()
+    pk = U.pkg()
+    rng = np.random.default_rng(B * 1000 + H)
+    blob = PL.make_lstm_blob(rng, 32, H, L, True, 1.0)
+    blob[-4 * H:] = h(rng.uniform(-0.2, 0.2, 4 * H))
+    x = h(rng.standard_normal((T, B, 32)))
+    plan = pk.LstmPlan(c, T, L, H, B, 32, clip=5.0, double_bias=True)
+    plan.set_weights(U.dev(blob))
+    dy = torch.zeros(T * B * H, dtype=torch.float16, device="cuda")
+    dx = U.dev(x)
+    runs = []
+    for _ in range(2):  # the counters between the layers are as before after a run
+        dy.zero_()
+        torch.cuda.synchronize()
+        plan.forward(dx, dy)
+        c.sync()
+        runs.append(U.host(dy).reshape(T, B, H))
+    assert np.array_equal(runs[0], runs[1])
+    # sequences are independent of each other: the oracle on the first and last ones of the groups
+    pick = sorted({0, B - 1, min(B - 1, 15), min(B - 1, 16), min(B - 1, 47), min(B - 1, 48)})
+    want = O.lstm(np.ascontiguousarray(x[:, pick]), blob, H, L, 5.0, True)
+    # as test_lstm_matches_oracle: fp16 state over a few steps and layers
+    assert np.abs(runs[0][:, pick].astype(np.float32) - want.astype(np.float32)).max() < 6e-3
+    plan.close()
+
+
+@gpu
 def test_lstm_batch_major_and_step_by_step(env):
     U = env
     import torch
