@@ -11,8 +11,11 @@
 //    fetched as in the patch-resident kernel: one run of rows per 64 channels, every filter tap a row offset into it;
 //  - a stage's barrier counts only the CTAs that had jobs in it, and a CTA without further jobs leaves, so that the
 //    next launch finds room while the last, small stages run.
-// Bound by the latency of the nine stages at batch 1, by the fetch of weights and patches (about 35 B/clk per SM) from
-// batch 6 on.
+// Bound by the latency of the nine stages at batch 1 (about 9500 clk each: 1200 to hear of the stage before, 1700 for the
+// first patch, 2050 for nine blocks of K, 2000 for the exchange of partial sums, 900 to finish the rows, 1250 for the stores
+// to be seen; clock64), by the tensor pipe's rate with 64 columns (50 clk an instruction, shared-memory reads) from batch 6
+// on.  Before the second MMA issuer, the second set of epilogue warps and the third and fourth patch buffer: 11000 a stage;
+// 19 frames of 107x189 82 us, now 66.
 #include "res_chain.h"
 
 #include <limits.h>
@@ -22,7 +25,7 @@
 
 namespace {
 
-constexpr int kThreads = 256;       // patch producer, MMA issuer, weight producer, TMEM owner, four epilogue warps
+constexpr int kThreads = 384;       // patch producer, MMA issuer, weight producer, second issuer and TMEM owner, eight epilogue warps
 constexpr int kCluster = 4;
 constexpr int kTileM = 128, kTileN = 64;
 constexpr int kWBlock = kTileN * 128;
@@ -31,8 +34,10 @@ constexpr int kAcc = 4;             // accumulator buffers of two times 64 TMEM 
 constexpr int kAccCols = 2 * kTileN;
 constexpr int kPartBytes = kTileM * kTileN * 4;
 constexpr int kMaxRing = 12;
+constexpr int kMaxBufs = 4;
 constexpr int kStageBytes = 2560;
 constexpr int kEpi0 = 128;          // first epilogue thread
+constexpr int kEpi = kThreads - kEpi0;
 // Tiles of the first stage up to which the chain is the faster way.  Measured per frame batch, chain / per-layer launches:
 // 144x256 x 1 (19 tiles) 66 / 86 us, x 6 (113) 78 / 92, 180x320 x 6 (175) 94 / 104, 107x189 x 19 (192) 92 / 102; beyond, the
 // per-layer kernels' wider tiles win: 107x189 x 32 (324) 121 / 114, 144x256 x 19 (357) 120 / 114.
@@ -44,6 +49,7 @@ struct Walk {                       // what the loops over jobs and K need of a 
   int sparse0, sub;                 // first column tile of a shortcut whose K is one space-to-depth position per tap
   int split;                        // CTAs per job: 1, 2 or 4
   int boxes, box_rows;
+  int bufs, buf_bytes;              // patch buffers: as many of this stage's patches as the room for two of the largest holds
 };
 struct Stage : Walk {
   int RP, Ho, Wo, rows;             // flattened position space of the stage (rows = batch * RP * P)
@@ -83,16 +89,16 @@ __device__ __forceinline__ void bulk_to_cluster(uint32_t dst, uint32_t src, uint
   asm volatile("cp.async.bulk.shared::cluster.shared::cta.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(dst), "r"(src), "r"(bytes), "r"(bar)
                : "memory");
 }
-// the four epilogue warps meet; true if all of them say so
+// the epilogue warps meet; true if all of them say so
 __device__ __forceinline__ bool epilogue_and(bool v) {
   uint32_t r;
   asm volatile(
       "{\n\t.reg .pred p, q;\n\t"
       "setp.ne.u32 q, %1, 0;\n\t"
-      "bar.red.and.pred p, 1, 128, q;\n\t"
+      "bar.red.and.pred p, 1, %2, q;\n\t"
       "selp.u32 %0, 1, 0, p;\n\t}"
       : "=r"(r)
-      : "r"(v ? 1u : 0u)
+      : "r"(v ? 1u : 0u), "n"(kEpi)
       : "memory");
   return r != 0;
 }
@@ -118,7 +124,7 @@ __device__ __forceinline__ Walk uniform_walk(const Stage& s) {
   w.P = uniform(s.P); w.pad = uniform(s.pad); w.n_tiles = uniform(s.n_tiles); w.jobs = uniform(s.jobs);
   w.taps = uniform(s.taps); w.kw = uniform(s.kw); w.cblocks = uniform(s.cblocks);
   w.sparse0 = uniform(s.sparse0); w.sub = uniform(s.sub); w.split = uniform(s.split);
-  w.boxes = uniform(s.boxes); w.box_rows = uniform(s.box_rows);
+  w.boxes = uniform(s.boxes); w.box_rows = uniform(s.box_rows); w.bufs = uniform(s.bufs); w.buf_bytes = uniform(s.buf_bytes);
   return w;
 }
 
@@ -170,16 +176,15 @@ __device__ __forceinline__ RowDst row_dst(const Stage& s, int q) {
   else if (!s.padded) r.row = ((size_t)n * s.Ho + yy) * s.Wo + vc;
   return r;
 }
-// Sixteen columns of it: affine, residual, activation, store.  aff: scale[64], shift[64] of the job's columns.
+// Eight columns of it: affine, residual, activation, store.  aff: scale[64], shift[64] of the job's columns.
 template <int ACT>
-__device__ __forceinline__ void finish16(const float* aff, int c, const float (&v)[16], bool res, const uint4 (&rv)[2], const RowDst& r, __half* dst,
-                                         float slope) {
-  const __half2* rh = reinterpret_cast<const __half2*>(rv);
-  uint4 o[2];
-  __half2* oh = reinterpret_cast<__half2*>(o);
+__device__ __forceinline__ void finish8(const float* aff, const float (&v)[8], bool res, const uint4& rv, const RowDst& r, __half* dst, float slope) {
+  const __half2* rh = reinterpret_cast<const __half2*>(&rv);
+  uint4 o;
+  __half2* oh = reinterpret_cast<__half2*>(&o);
 #pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    const float4 a = *reinterpret_cast<const float4*>(aff + c + 4 * i), b = *reinterpret_cast<const float4*>(aff + kTileN + c + 4 * i);
+  for (int i = 0; i < 2; ++i) {
+    const float4 a = *reinterpret_cast<const float4*>(aff + 4 * i), b = *reinterpret_cast<const float4*>(aff + kTileN + 4 * i);
     float2 x = make_float2(fmaf(v[4 * i], a.x, b.x), fmaf(v[4 * i + 1], a.y, b.y));
     float2 y = make_float2(fmaf(v[4 * i + 2], a.z, b.z), fmaf(v[4 * i + 3], a.w, b.w));
     if (res) {
@@ -190,18 +195,15 @@ __device__ __forceinline__ void finish16(const float* aff, int c, const float (&
     oh[2 * i] = __floats2half2_rn(act_apply_fast(x.x, ACT, slope), act_apply_fast(x.y, ACT, slope));
     oh[2 * i + 1] = __floats2half2_rn(act_apply_fast(y.x, ACT, slope), act_apply_fast(y.y, ACT, slope));
   }
-  if (!r.valid) o[0] = o[1] = make_uint4(0, 0, 0, 0);
-  if (r.store) {
-    reinterpret_cast<uint4*>(dst)[0] = o[0];
-    reinterpret_cast<uint4*>(dst)[1] = o[1];
-  }
+  if (!r.valid) o = make_uint4(0, 0, 0, 0);
+  if (r.store) *reinterpret_cast<uint4*>(dst) = o;
 }
-// Groups of sixteen columns [g0, g0 + N) of one row.
+// N groups of eight columns of one row, the first at aff and dst.
 template <int N>
-__device__ __forceinline__ void finish_row(int act, const float* aff, int g0, const float (&v)[N][16], bool res, const uint4 (&rv)[N][2], const RowDst& r,
-                                           __half* dst, float slope) {
-#define AIG_FINISH(ACT)   \
-  _Pragma("unroll") for (int g = 0; g < N; ++g) finish16<ACT>(aff, (g0 + g) * 16, v[g], res, rv[g], r, dst + (g0 + g) * 16, slope)
+__device__ __forceinline__ void finish_row(int act, const float* aff, const float (&v)[N][8], bool res, const uint4* rv, const RowDst& r, __half* dst,
+                                           float slope) {
+#define AIG_FINISH(ACT) \
+  _Pragma("unroll") for (int g = 0; g < N; ++g) finish8<ACT>(aff + 8 * g, v[g], res, rv[g], r, dst + 8 * g, slope)
   switch (act) {
     case AIG_ACT_RELU: AIG_FINISH(AIG_ACT_RELU); break;
     case AIG_ACT_SWISH: AIG_FINISH(AIG_ACT_SWISH); break;
@@ -210,67 +212,54 @@ __device__ __forceinline__ void finish_row(int act, const float* aff, int g0, co
   }
 #undef AIG_FINISH
 }
-template <int N>
-__device__ __forceinline__ void load_residual(const __half* src, int g0, bool on, uint4 (&rv)[N][2]) {
-#pragma unroll
-  for (int g = 0; g < N; ++g) {
-    rv[g][0] = rv[g][1] = make_uint4(0, 0, 0, 0);
-    if (on) {
-      rv[g][0] = __ldcg(reinterpret_cast<const uint4*>(src + (g0 + g) * 16));
-      rv[g][1] = __ldcg(reinterpret_cast<const uint4*>(src + (g0 + g) * 16) + 1);
-    }
-  }
-}
-// Partial sums of a split job in shared memory: rows of 64 floats, 16-byte chunk c of row r at this place, so that the
-// writers (a lane per row, one chunk at a time) and the readers (two or four lanes per row, 16 columns each) both meet
-// eight different bank groups.
-__device__ __forceinline__ int part_slot(int row, int c) { return (((c >> 2) | ((c & 3) << 2)) ^ (row & 7)) << 4; }
-__device__ __forceinline__ int part_row(int i) { return (i & ~7) | ((i & 1) << 2) | ((i >> 1) & 3); }
-template <int S>
-__device__ __forceinline__ void sum_parts(const uint8_t* part, int row, int g0, float (&v)[S == 4 ? 1 : 2][16]) {
+// Partial sums of a split job in shared memory: [half of the columns][share of K][R rows][128 bytes], 16-byte chunk c of
+// row r at this place of it, so that the writers (a lane per row, one chunk at a time) and the readers (two or four
+// neighbouring lanes per row) both meet eight different bank groups.
+__device__ __forceinline__ int part_slot(int row, int c) { return row * 128 + ((c ^ (row & 7)) << 4); }
+// 8 N columns of row `row`, from chunk c0 of its half on.
+template <int S, int N>
+__device__ __forceinline__ void sum_parts(const uint8_t* part, int half, int row, int c0, float (&v)[N][8]) {
   constexpr int R = kTileM / S;
+  float4 x[S][2 * N];
 #pragma unroll
-  for (int g = 0; g < (S == 4 ? 1 : 2); ++g) {
-    float4 x[S][4];
+  for (int k = 0; k < S; ++k)
 #pragma unroll
-    for (int k = 0; k < S; ++k)
+    for (int c = 0; c < 2 * N; ++c) x[k][c] = *reinterpret_cast<const float4*>(part + (half * S + k) * R * 128 + part_slot(row, c0 + c));
 #pragma unroll
-      for (int c = 0; c < 4; ++c) x[k][c] = *reinterpret_cast<const float4*>(part + (size_t)(k * R + row) * 256 + part_slot(row, (g0 + g) * 4 + c));
+  for (int c = 0; c < 2 * N; ++c) {
+    float4 s = x[0][c];
 #pragma unroll
-    for (int c = 0; c < 4; ++c) {
-      float4 s = x[0][c];
-#pragma unroll
-      for (int k = 1; k < S; ++k) {
-        s.x += x[k][c].x;
-        s.y += x[k][c].y;
-        s.z += x[k][c].z;
-        s.w += x[k][c].w;
-      }
-      v[g][4 * c] = s.x;
-      v[g][4 * c + 1] = s.y;
-      v[g][4 * c + 2] = s.z;
-      v[g][4 * c + 3] = s.w;
+    for (int k = 1; k < S; ++k) {
+      s.x += x[k][c].x;
+      s.y += x[k][c].y;
+      s.z += x[k][c].z;
+      s.w += x[k][c].w;
     }
+    float* o = v[c >> 1] + 4 * (c & 1);
+    o[0] = s.x;
+    o[1] = s.y;
+    o[2] = s.z;
+    o[3] = s.w;
   }
 }
 
-// Mask attention, pool, FC and outputs of one frame by the four epilogue warps (the arithmetic of cnn_head_kernel).
+// Mask attention, pool, FC and outputs of one frame by the epilogue warps (the arithmetic of cnn_head_kernel).
 // sx: [HW][C] in shared memory; w: the FC's weights, the mask's, the FC's bias, there already.
 __device__ void head_frame(const ResChainHead& h, const __half* x, int b, __half* sx, const __half* w, float* s_mask, float* s_pool, int tid) {
   const int warp = tid >> 5, lane = tid & 31, HW = h.hw, C = h.c, nvec = HW * C / 8;
   const uint4* xb = reinterpret_cast<const uint4*>(x + (size_t)b * HW * C);
-  for (int i0 = tid; i0 < nvec; i0 += 128 * 8) {
-    uint4 v[8];
+  for (int i0 = tid; i0 < nvec; i0 += kEpi * 4) {
+    uint4 v[4];
 #pragma unroll
-    for (int u = 0; u < 8; ++u) v[u] = i0 + u * 128 < nvec ? __ldcg(xb + i0 + u * 128) : make_uint4(0, 0, 0, 0);
+    for (int u = 0; u < 4; ++u) v[u] = i0 + u * kEpi < nvec ? __ldcg(xb + i0 + u * kEpi) : make_uint4(0, 0, 0, 0);
 #pragma unroll
-    for (int u = 0; u < 8; ++u)
-      if (i0 + u * 128 < nvec) reinterpret_cast<uint4*>(sx)[i0 + u * 128] = v[u];
+    for (int u = 0; u < 4; ++u)
+      if (i0 + u * kEpi < nvec) reinterpret_cast<uint4*>(sx)[i0 + u * kEpi] = v[u];
   }
-  named_bar_sync(1, 128);
+  named_bar_sync(1, kEpi);
   const __half* w1 = w + C * h.n_out;
-  constexpr int kAtOnce = 8;
-  for (int p0 = warp; p0 < HW; p0 += 4 * kAtOnce) {
+  constexpr int kAtOnce = 4, kWarps = kEpi / 32;
+  for (int p0 = warp; p0 < HW; p0 += kWarps * kAtOnce) {
     float s[kAtOnce];
 #pragma unroll
     for (int u = 0; u < kAtOnce; ++u) s[u] = 0.f;
@@ -279,7 +268,7 @@ __device__ void head_frame(const ResChainHead& h, const __half* x, int b, __half
       const __half2* wh = reinterpret_cast<const __half2*>(&wv);
 #pragma unroll
       for (int u = 0; u < kAtOnce; ++u) {
-        const uint4 xv = p0 + 4 * u < HW ? *reinterpret_cast<const uint4*>(sx + (p0 + 4 * u) * C + c) : make_uint4(0, 0, 0, 0);
+        const uint4 xv = p0 + kWarps * u < HW ? *reinterpret_cast<const uint4*>(sx + (p0 + kWarps * u) * C + c) : make_uint4(0, 0, 0, 0);
         const __half2* xh = reinterpret_cast<const __half2*>(&xv);
 #pragma unroll
         for (int e = 0; e < 4; ++e) {
@@ -296,10 +285,10 @@ __device__ void head_frame(const ResChainHead& h, const __half* x, int b, __half
     float mine = s[0];
 #pragma unroll
     for (int u = 1; u < kAtOnce; ++u) mine = lane == u ? s[u] : mine;
-    if (lane < kAtOnce && p0 + 4 * lane < HW) s_mask[p0 + 4 * lane] = 1.0f / (1.0f + expf(-(mine + h.mask_b)));
+    if (lane < kAtOnce && p0 + kWarps * lane < HW) s_mask[p0 + kWarps * lane] = 1.0f / (1.0f + expf(-(mine + h.mask_b)));
   }
-  named_bar_sync(1, 128);
-  for (int c = tid * 2; c < C; c += 256) {
+  named_bar_sync(1, kEpi);
+  for (int c = tid * 2; c < C; c += 2 * kEpi) {
     float s0 = 0.f, s1 = 0.f;
 #pragma unroll 16
     for (int p = 0; p < HW; ++p) {
@@ -313,17 +302,18 @@ __device__ void head_frame(const ResChainHead& h, const __half* x, int b, __half
     s_pool[c] = __low2float(f);
     s_pool[c + 1] = __high2float(f);
   }
-  named_bar_sync(1, 128);
-  for (int o = tid >> 2; o < (h.n_out + 31) / 32 * 32; o += 32) {  // four lanes an output
+  named_bar_sync(1, kEpi);
+  for (int o = tid >> 3; o < (h.n_out + 31) / 32 * 32; o += 32) {  // eight lanes an output
     const bool on = o < h.n_out;
     float acc = 0.f;
     if (on) {
 #pragma unroll 16
-      for (int c = tid & 3; c < C; c += 4) acc = fmaf(s_pool[c], __half2float(w[(size_t)c * h.n_out + o]), acc);
+      for (int c = tid & 7; c < C; c += 8) acc = fmaf(s_pool[c], __half2float(w[(size_t)c * h.n_out + o]), acc);
     }
     acc += __shfl_xor_sync(0xffffffffu, acc, 1);
     acc += __shfl_xor_sync(0xffffffffu, acc, 2);
-    if (on && (tid & 3) == 0) {
+    acc += __shfl_xor_sync(0xffffffffu, acc, 4);
+    if (on && (tid & 7) == 0) {
       const float t = __half2float(__float2half(acc));
       const float y = __half2float(__float2half(t + __half2float(w1[C + o])));
       const __half v = o < h.n_sigmoid ? __float2half(1.0f / (1.0f + expf(-y))) : __float2half(tanhf(y));
@@ -331,7 +321,7 @@ __device__ void head_frame(const ResChainHead& h, const __half* x, int b, __half
       h.out_f32[(size_t)b * h.n_out + o] = __half2float(v);
     }
   }
-  named_bar_sync(1, 128);
+  named_bar_sync(1, kEpi);
 }
 
 __global__ void __launch_bounds__(kThreads, 1) res_chain_kernel(const __grid_constant__ ChainMaps maps, const __grid_constant__ ChainParams p) {
@@ -346,11 +336,11 @@ __global__ void __launch_bounds__(kThreads, 1) res_chain_kernel(const __grid_con
   const Stage* st = reinterpret_cast<const Stage*>(s_aff + 256);
   __half* s_head = reinterpret_cast<__half*>(sm + 2 * p.patch_bytes + p.ring * kWBlock + 2 * kPartBytes + 1024 + kStageBytes);  // the head's weights
   uint64_t* bars = reinterpret_cast<uint64_t*>(reinterpret_cast<uint8_t*>(s_head) + p.head_bytes);
-  const uint32_t bar_pfull = smem_u32(bars), bar_pempty = bar_pfull + 16, bar_tfull = bar_pfull + 32, bar_tempty = bar_tfull + 8 * kAcc;
+  const uint32_t bar_pfull = smem_u32(bars), bar_pempty = bar_pfull + 8 * kMaxBufs, bar_tfull = bar_pempty + 8 * kMaxBufs, bar_tempty = bar_tfull + 8 * kAcc;
   const uint32_t bar_wfull = bar_tempty + 8 * kAcc, bar_wempty = bar_wfull + 8 * kMaxRing;
   const uint32_t bar_part = bar_wempty + 8 * kMaxRing;  // partial sums of a split job have arrived
   const uint32_t bar_free = bar_part + 8;               // [2]: the other CTAs of a job split in two / four have read theirs
-  uint32_t* s_tmem = reinterpret_cast<uint32_t*>(bars + 4 + 2 * kAcc + 2 * kMaxRing + 3);
+  uint32_t* s_tmem = reinterpret_cast<uint32_t*>(bars + 2 * kMaxBufs + 2 * kAcc + 2 * kMaxRing + 3);
   volatile int* s_abort = reinterpret_cast<volatile int*>(s_tmem + 1);
 
   const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
@@ -359,17 +349,17 @@ __global__ void __launch_bounds__(kThreads, 1) res_chain_kernel(const __grid_con
   for (int i = threadIdx.x; i < (int)(sizeof(Stage) / 8) * p.n_stages; i += kThreads)
     const_cast<uint64_t*>(reinterpret_cast<const uint64_t*>(st))[i] = reinterpret_cast<const uint64_t*>(p.st)[i];
   if (threadIdx.x == 0) {
-    for (int i = 0; i < 2; ++i) {
+    for (int i = 0; i < kMaxBufs; ++i) {
       mbar_init(bar_pfull + 8 * i, 1);
-      mbar_init(bar_pempty + 8 * i, 1);
+      mbar_init(bar_pempty + 8 * i, 2);
     }
     for (int i = 0; i < kAcc; ++i) {
-      mbar_init(bar_tfull + 8 * i, 1);
-      mbar_init(bar_tempty + 8 * i, 4);
+      mbar_init(bar_tfull + 8 * i, 2);
+      mbar_init(bar_tempty + 8 * i, kEpi / 32);
     }
     for (int i = 0; i < p.ring; ++i) {
       mbar_init(bar_wfull + 8 * i, 1);
-      mbar_init(bar_wempty + 8 * i, 1);
+      mbar_init(bar_wempty + 8 * i, 2);
     }
     mbar_init(bar_part, 1);
     mbar_init(bar_free, 2);
@@ -398,8 +388,7 @@ __global__ void __launch_bounds__(kThreads, 1) res_chain_kernel(const __grid_con
   if (warp == 0) {
     // ------------------------------------------------------------------ patch producer
     const bool leader = elect_one();
-    int buf = 0;
-    uint32_t ph = 0;
+    uint32_t ph = 0;  // a bit per buffer
     bool ok = true;
     griddep_wait();
     for (int si = 0; si < p.n_stages && ok; ++si) {
@@ -411,6 +400,7 @@ __global__ void __launch_bounds__(kThreads, 1) res_chain_kernel(const __grid_con
         if (!ok) break;
         fence_proxy_async_global();  // written with ordinary stores, read by the TMA unit
       }
+      int buf = 0;  // (every MMA of the stage before has been done: its buffers are free, however large they were)
       for (int job = it.job; job < s.jobs && ok; job += it.step) {
         const int n_tile = job % s.n_tiles, m_tile = job / s.n_tiles;
         const KRange k = k_range(s, n_tile, it.part);
@@ -418,13 +408,14 @@ __global__ void __launch_bounds__(kThreads, 1) res_chain_kernel(const __grid_con
         for (int u = k.lo; u < k.hi; ++u) {
           int cb, t0, t1;
           unit_of(s, k, u, cb, t0, t1);
-          if (!mbar_wait_bounded(bar_pempty + 8 * buf, ph ^ 1u, s_abort, p.gerr, 801)) { ok = false; break; }
+          if (!mbar_wait_bounded(bar_pempty + 8 * buf, (ph >> buf & 1u) ^ 1u, s_abort, p.gerr, 801)) { ok = false; break; }
           if (leader) {
             mbar_expect_tx(bar_pfull + 8 * buf, (uint32_t)(s.boxes * s.box_rows * 128));
             for (int b = 0; b < s.boxes; ++b)
-              tma_load_2d(sPatch + buf * p.patch_bytes + b * s.box_rows * 128, &maps.a[si], bar_pfull + 8 * buf, cb * 64, row0 + b * s.box_rows);
+              tma_load_2d(sPatch + buf * s.buf_bytes + b * s.box_rows * 128, &maps.a[si], bar_pfull + 8 * buf, cb * 64, row0 + b * s.box_rows);
           }
-          if (++buf == 2) { buf = 0; ph ^= 1u; }
+          ph ^= 1u << buf;
+          if (++buf == s.bufs) buf = 0;
         }
       }
     }
@@ -454,42 +445,48 @@ __global__ void __launch_bounds__(kThreads, 1) res_chain_kernel(const __grid_con
         }
       }
     }
-  } else if (warp == 1) {
-    // ------------------------------------------------------------------ MMA issuer (all lanes run it, one issues: see elect_one)
-    // Every second instruction goes to a second accumulator that the epilogue adds: into one and the same they took 84 to
-    // 93 clk each, twice what an N = 64 instruction takes.
+  } else if (warp == 1 || warp == 3) {
+    // ------------------------------------------------------------------ MMA issuers (all lanes run it, one issues: see elect_one)
+    // Two warps issue every second instruction each, into an accumulator of its own (the epilogue adds them): a block of K
+    // costs one warp 300 to 340 clk, the wait for its weights 75 and every instruction 38 of them, where the tensor pipe needs
+    // 210 for its four instructions.
     constexpr uint32_t idesc = umma_idesc_f16(kTileM, kTileN);
     const bool leader = elect_one();
-    int buf = 0, slot = 0, acc = 0;
-    uint32_t pph = 0, wph = 0, aph = 0;
+    const int mine = warp >> 1;
+    int slot = 0, acc = 0;
+    uint32_t pph = 0, wph = 0, aph = 0;  // pph: a bit per buffer
     bool ok = true;
     for (int si = 0; si < p.n_stages && ok; ++si) {
       const Walk s = uniform_walk(st[si]);
       const JobIter it = jobs_of(s, p.clusters, cluster, rank);
+      int buf = 0;
       for (int job = it.job; job < s.jobs && ok; job += it.step) {
         const KRange k = k_range(s, job % s.n_tiles, it.part);
         if (!mbar_wait_bounded(bar_tempty + 8 * acc, aph ^ 1u, s_abort, p.gerr, 803)) { ok = false; break; }
         tc_fence_after();
-        const uint32_t d = tmem_base + (uint32_t)(acc * kAccCols);
+        const uint32_t d = tmem_base + (uint32_t)(acc * kAccCols + mine * kTileN);
         uint32_t first = 0;
         for (int u = k.lo; u < k.hi && ok; ++u) {
           int cb, t0, t1;
           unit_of(s, k, u, cb, t0, t1);
-          if (!mbar_wait_bounded(bar_pfull + 8 * buf, pph, s_abort, p.gerr, 804)) { ok = false; break; }
-          int fr = t0 / s.kw, fs = t0 - fr * s.kw;
+          if (!mbar_wait_bounded(bar_pfull + 8 * buf, pph >> buf & 1u, s_abort, p.gerr, 804)) { ok = false; break; }
+          int fs = t0 % s.kw;
+          uint32_t a_lo = umma_desc_lo(sPatch + buf * s.buf_bytes) + (uint32_t)(t0 / s.kw * s.P + fs) * 8u + mine * 2u;
           for (int tap = t0; tap < t1; ++tap) {
             if (!mbar_wait_bounded(bar_wfull + 8 * slot, wph, s_abort, p.gerr, 805)) { ok = false; break; }
-            const uint32_t a_lo = umma_desc_lo(sPatch + buf * p.patch_bytes + (uint32_t)(fr * s.P + fs) * 128u), b_lo = umma_desc_lo(sW + slot * kWBlock);
+            const uint32_t b_lo = umma_desc_lo(sW + slot * kWBlock) + mine * 2u;
 #pragma unroll
-            for (int kk = 0; kk < 4; ++kk)
-              if (leader) umma_f16_ss_lo(d + (uint32_t)((kk & 1) * kTileN), a_lo + (uint32_t)(kk * 2), b_lo + (uint32_t)(kk * 2), umma_desc_hi(128), idesc, kk < 2 ? first : 1u);
+            for (int kk = 0; kk < 2; ++kk)
+              if (leader) umma_f16_ss_lo(d, a_lo + (uint32_t)(kk * 4), b_lo + (uint32_t)(kk * 4), umma_desc_hi(128), idesc, kk == 0 ? first : 1u);
             first = 1u;
             if (leader) umma_commit(bar_wempty + 8 * slot);
             if (++slot == p.ring) { slot = 0; wph ^= 1u; }
-            if (++fs == s.kw) { fs = 0; ++fr; }
+            a_lo += 8u;
+            if (++fs == s.kw) { fs = 0; a_lo += (uint32_t)(s.P - s.kw) * 8u; }
           }
           if (ok && leader) umma_commit(bar_pempty + 8 * buf);
-          if (++buf == 2) { buf = 0; pph ^= 1u; }
+          pph ^= 1u << buf;
+          if (++buf == s.bufs) buf = 0;
         }
         if (ok && leader) umma_commit(bar_tfull + 8 * acc);
         if (++acc == kAcc) { acc = 0; aph ^= 1u; }
@@ -497,16 +494,16 @@ __global__ void __launch_bounds__(kThreads, 1) res_chain_kernel(const __grid_con
     }
   } else if (warp >= 4) {
     // ------------------------------------------------------------------ epilogue
-    const int tid = threadIdx.x - kEpi0, q4 = warp & 3;
+    const int tid = threadIdx.x - kEpi0, q4 = warp & 3, half = tid >> 7, tl = tid & 127;
     int acc = 0, split_jobs = 0, free_jobs[2] = {0, 0}, jobs = 0;
     uint32_t aph = 0;
     bool ok = true;
     const bool with_head = p.head.hw > 0;
     if (with_head && (int)blockIdx.x < p.batch) {
       const int n_fc = p.head.c * p.head.n_out;
-      for (int i = tid; i < n_fc / 8; i += 128) reinterpret_cast<uint4*>(s_head)[i] = __ldg(reinterpret_cast<const uint4*>(p.head.fc_w) + i);
-      for (int i = tid; i < p.head.c; i += 128) s_head[n_fc + i] = reinterpret_cast<const __half*>(p.head.mask_w)[i];
-      for (int i = tid; i < p.head.n_out; i += 128) s_head[n_fc + p.head.c + i] = p.head.fc_b ? reinterpret_cast<const __half*>(p.head.fc_b)[i] : __float2half(0.f);
+      for (int i = tid; i < n_fc / 8; i += kEpi) reinterpret_cast<uint4*>(s_head)[i] = __ldg(reinterpret_cast<const uint4*>(p.head.fc_w) + i);
+      for (int i = tid; i < p.head.c; i += kEpi) s_head[n_fc + i] = reinterpret_cast<const __half*>(p.head.mask_w)[i];
+      for (int i = tid; i < p.head.n_out; i += kEpi) s_head[n_fc + p.head.c + i] = p.head.fc_b ? reinterpret_cast<const __half*>(p.head.fc_b)[i] : __float2half(0.f);
     }
     for (int si = 0; si < p.n_stages && ok; ++si) {
       const Stage s = st[si];
@@ -514,82 +511,78 @@ __global__ void __launch_bounds__(kThreads, 1) res_chain_kernel(const __grid_con
       if (it.job >= s.jobs) continue;
       const int S = s.split, R = kTileM / S, which = S == 4 ? 1 : 0, rank0 = rank - it.part;
       const bool res = s.res != nullptr;
-      // the row this thread finishes: its TMEM lane, or (in a split job, 128 / R threads a row) one of this CTA's share
-      const int row = S == 1 ? tid : it.part * R + part_row(tid / S), g0 = S == 1 ? 0 : (tid % S) * (S == 4 ? 1 : 2);
+      // what this thread finishes: 32 columns of its TMEM lane or, in a split job, S neighbouring threads share 32 columns of
+      // one of this CTA's rows
+      const int lrow = S == 1 ? tl : tl / S, row = (S == 1 ? 0 : it.part * R) + lrow, part_cols = 32 / S, c0 = half * 32 + tl % S * part_cols;
       if (res) {  // residual rows come from the stage before
         if (tid == 0) ok = wait_stage(counters + si - 1, (unsigned int)st[si - 1].arrivals, s_abort, p.gerr, 840 + si);
         ok = epilogue_and(ok);
       }
-      for (int job = it.job; job < s.jobs && ok; job += it.step, ++jobs) {
+      // (after a wait that ran out a warp goes on with the rest, whose waits return at once, so that all warps meet at every barrier)
+      for (int job = it.job; job < s.jobs; job += it.step, ++jobs) {
         const int n_tile = job % s.n_tiles, m_tile = job / s.n_tiles, col0 = n_tile * kTileN;
         const bool second = col0 >= s.c_split;
         const int ch0 = second ? col0 - s.c_split : col0, act = second ? s.act1 : s.act0;
         // everything that does not depend on the accumulator, while it is being computed
         float* aff = s_aff + (jobs & 1) * 128;
-        aff[tid] = tid < kTileN ? __ldg(s.scale + col0 + tid) : __ldg(s.shift + col0 + tid - kTileN);
+        if (tid < 2 * kTileN) aff[tid] = tid < kTileN ? __ldg(s.scale + col0 + tid) : __ldg(s.shift + col0 + tid - kTileN);
         const RowDst rd = row_dst(s, m_tile * kTileM + row);
-        __half* dst = (second ? s.y1 : s.y0) + rd.row * s.co + ch0;
-        const __half* rsrc = s.res + (size_t)(m_tile * kTileM + row) * s.co + ch0;
-        uint4 rv[4][2];
-        if (S == 1) {
-          load_residual(rsrc, 0, res && rd.valid, rv);
-        } else {
-          uint4 (&r2)[2][2] = reinterpret_cast<uint4 (&)[2][2]>(rv);
-          if (S == 4) load_residual(rsrc, g0, res && rd.valid, reinterpret_cast<uint4 (&)[1][2]>(rv));
-          else load_residual(rsrc, g0, res && rd.valid, r2);
-        }
-        ok = mbar_wait_bounded(bar_tfull + 8 * acc, aph, s_abort, p.gerr, 806);
+        __half* dst = (second ? s.y1 : s.y0) + rd.row * s.co + ch0 + c0;
+        uint4 rv[4];
+#pragma unroll
+        for (int g = 0; g < 4; ++g)
+          rv[g] = res && rd.valid && g * 8 < part_cols ? __ldcg(reinterpret_cast<const uint4*>(s.res + (size_t)(m_tile * kTileM + row) * s.co + ch0 + c0) + g)
+                                                       : make_uint4(0, 0, 0, 0);
+        named_bar_sync(1, kEpi);  // scale and shift are there
+        ok = mbar_wait_bounded(bar_tfull + 8 * acc, aph, s_abort, p.gerr, 806) && ok;
         if (S > 1 && job != it.job) ok = ok && mbar_wait_bounded_cl(bar_free + 8 * which, (uint32_t)(free_jobs[which] - 1) & 1u, s_abort, p.gerr, 807);
-        ok = epilogue_and(ok);
-        if (!ok) break;
         tc_fence_after();
-        const uint32_t t_addr = tmem_base + (uint32_t)(acc * kAccCols) + ((uint32_t)(q4 * 32) << 16);
-        float v[4][16];
+        const uint32_t t_addr = tmem_base + (uint32_t)(acc * kAccCols + half * 32) + ((uint32_t)(q4 * 32) << 16);
+        float v[4][8];
+        uint32_t w[32];
+        tmem_ld_32x32(t_addr, reinterpret_cast<uint32_t (&)[32]>(v));
+        tmem_ld_32x32(t_addr + kTileN, w);
+        tmem_ld_wait();
 #pragma unroll
-        for (int h = 0; h < 2; ++h) {
-          uint32_t w[32];
-          tmem_ld_32x32(t_addr + 32 * h, reinterpret_cast<uint32_t (&)[32]>(v[2 * h]));
-          tmem_ld_32x32(t_addr + kTileN + 32 * h, w);
-          tmem_ld_wait();
-#pragma unroll
-          for (int i = 0; i < 32; ++i) v[2 * h + (i >> 4)][i & 15] += __uint_as_float(w[i]);
-        }
+        for (int i = 0; i < 32; ++i) v[i >> 3][i & 7] += __uint_as_float(w[i]);
         tc_fence_before();
         __syncwarp();
         if (lane == 0) mbar_arrive(bar_tempty + 8 * acc);
         if (S == 1) {
-          finish_row<4>(act, aff, 0, v, res, rv, rd, dst, p.slope);
+          finish_row<4>(act, aff + c0, v, res, rv, rd, dst, p.slope);
         } else {
           // this warp's 32 rows go to the CTA that finishes them
-          const int target = q4 * 32 / R, lrow = q4 * 32 % R + lane;
-          uint8_t* mine = sent + (size_t)(q4 * 32 + lane) * 256;
+          const int target = q4 * 32 / R, r0 = q4 * 32 % R, block = (half * S + it.part) * R * 128;
+          uint8_t* mine = target == it.part ? part + block + r0 * 128 : sent + (half * 4 + q4) * 4096;
 #pragma unroll
-          for (int c = 0; c < 16; ++c)
-            *reinterpret_cast<float4*>(mine + part_slot(lrow, c)) = make_float4(v[c >> 2][(c & 3) * 4], v[c >> 2][(c & 3) * 4 + 1], v[c >> 2][(c & 3) * 4 + 2], v[c >> 2][(c & 3) * 4 + 3]);
+          for (int c = 0; c < 8; ++c)
+            *reinterpret_cast<float4*>(mine + part_slot(lane, c)) = make_float4(v[c >> 1][(c & 1) * 4], v[c >> 1][(c & 1) * 4 + 1], v[c >> 1][(c & 1) * 4 + 2], v[c >> 1][(c & 1) * 4 + 3]);
           fence_proxy_async_smem();
           __syncwarp();
-          if (lane == 0)
-            bulk_to_cluster(mapa_shared(sPart, (uint32_t)(rank0 + target)) + (uint32_t)((it.part * R + q4 * 32 % R) * 256), smem_u32(sent) + q4 * 8192, 8192,
+          if (lane == 0 && target != it.part)
+            bulk_to_cluster(mapa_shared(sPart, (uint32_t)(rank0 + target)) + (uint32_t)(block + r0 * 128), smem_u32(mine), 4096,
                             mapa_shared(bar_part, (uint32_t)(rank0 + target)));
-          if (tid == 0) mbar_expect_tx(bar_part, kPartBytes);
-          ok = mbar_wait_bounded_cl(bar_part, (uint32_t)split_jobs & 1u, s_abort, p.gerr, 808);
+          if (tid == 0) mbar_expect_tx(bar_part, kPartBytes - kPartBytes / S);
+          ok = mbar_wait_bounded_cl(bar_part, (uint32_t)split_jobs & 1u, s_abort, p.gerr, 808) && ok;
           ++split_jobs;
-          if (S == 4) sum_parts<4>(part, part_row(tid / 4), g0, reinterpret_cast<float (&)[1][16]>(v));
-          else sum_parts<2>(part, part_row(tid / 2), g0, reinterpret_cast<float (&)[2][16]>(v));
-          ok = epilogue_and(ok);  // (all have read)
-          if (!ok) break;
+          named_bar_sync(1, kEpi);  // this CTA's own share is there as well
+          float (&v2)[2][8] = reinterpret_cast<float (&)[2][8]>(v);
+          float (&v1)[1][8] = reinterpret_cast<float (&)[1][8]>(v);
+          if (S == 4) sum_parts<4, 1>(part, half, lrow, tl % 4 * 2, v1);
+          else sum_parts<2, 2>(part, half, lrow, tl % 2 * 4, v2);
           if (job + it.step < s.jobs) {  // (between stages the stage barrier says as much; the arrival waits for all this thread has in flight)
+            named_bar_sync(1, kEpi);  // all have read
             if (tid < S) mbar_arrive_cluster(mapa_shared(bar_free + 8 * which, (uint32_t)(rank0 + tid)));
             ++free_jobs[which];
           }
-          if (S == 4) finish_row<1>(act, aff, g0, reinterpret_cast<float (&)[1][16]>(v), res, reinterpret_cast<uint4 (&)[1][2]>(rv), rd, dst, p.slope);
-          else finish_row<2>(act, aff, g0, reinterpret_cast<float (&)[2][16]>(v), res, reinterpret_cast<uint4 (&)[2][2]>(rv), rd, dst, p.slope);
+          if (S == 4) finish_row<1>(act, aff + c0, v1, res, rv, rd, dst, p.slope);
+          else finish_row<2>(act, aff + c0, v2, res, rv, rd, dst, p.slope);
         }
         if (++acc == kAcc) { acc = 0; aph ^= 1u; }
       }
-      if (!ok) break;
       fence_proxy_async_global();  // the next stage's TMA loads read these rows
-      named_bar_sync(1, 128);
+      ok = epilogue_and(ok);
+      if (!ok) break;
       if (tid == 0) red_release_gpu_add(counters + si, 1u);
     }
     if (ok && with_head && (int)blockIdx.x < p.batch) {
@@ -713,6 +706,12 @@ int res_chain_create(aig_ctx* ctx, const std::vector<ResChainBlock>& blocks, int
       p.slope = v.slope;
     }
   p.patch_bytes = (patch_rows * 128 + 1023) / 1024 * 1024;
+  for (int i = 0; i < p.n_stages; ++i) {
+    Stage& s = p.st[i];
+    s.buf_bytes = (s.boxes * s.box_rows * 128 + 1023) / 1024 * 1024;
+    s.bufs = 2 * p.patch_bytes / s.buf_bytes;
+    if (s.bufs > kMaxBufs) s.bufs = kMaxBufs;
+  }
   p.head_bytes = ((n_out + 1) * c_last + n_out) * 2;
   p.head_bytes = (p.head_bytes + 127) / 128 * 128;
   const int fixed = 1024 + 2 * kPartBytes + 1024 + kStageBytes + p.head_bytes + 512;
