@@ -294,7 +294,7 @@ conv_first_rows_kernel(const __grid_constant__ CUtensorMap tmapY, const __grid_c
       if (*s_abort) break;                        // uniform: every thread reads the flag after the same barrier
       if (tid_e == 0) {
         const uint32_t src = sOut + (uint32_t)buf * kOutBytes;
-        if (p.s2d) tma_store_5d(&tmapY, src, 0, 0, 0, (y + 1) & 1, n * p.Hb + ((y + 1) >> 1));
+        if (p.s2d) tma_store_5d(&tmapY, src, 0, 0, 0, (y + 1) & 1, (CLIP ? z * p.batch + n : n) * p.Hb + ((y + 1) >> 1));
         else tma_store_4d(&tmapY, src, 0, 0, y, CLIP ? n * p.D + z : n);
         bulk_commit();
       }
@@ -561,9 +561,9 @@ static int rows_encode_output(ConvFirstRows* t, __half* y) {
   const ConvFirstGeom& g = t->g;
   CUresult r;
   if (t->prm.s2d) {
-    // blocks [n][hb][wb][sy][sx][c] seen as (c, sx, wb, sy, n*hb): one output row = sub-row sy of block row hb,
-    // pixels in (wb, sx) order = x + 1
-    cuuint64_t dims[5] = {(cuuint64_t)kN, 2, (cuuint64_t)t->Wb, 2, (cuuint64_t)g.batch * t->Hb};
+    // blocks [n][hb][wb][sy][sx][c] (clips: [d][n][hb]...) seen as (c, sx, wb, sy, n*hb): one output row = sub-row sy of
+    // block row hb, pixels in (wb, sx) order = x + 1
+    cuuint64_t dims[5] = {(cuuint64_t)kN, 2, (cuuint64_t)t->Wb, 2, (cuuint64_t)g.batch * g.D * t->Hb};
     cuuint64_t strides[4] = {(cuuint64_t)kN * 2, (cuuint64_t)4 * kN * 2, (cuuint64_t)2 * kN * 2, (cuuint64_t)t->Wb * 4 * kN * 2};
     cuuint32_t box[5] = {(cuuint32_t)kN, 2, (cuuint32_t)t->Wb, 1, 1};
     cuuint32_t es[5] = {1, 1, 1, 1, 1};

@@ -223,7 +223,9 @@ conv_first_tc_kernel(const void* __restrict__ xin, __half* __restrict__ y, const
       if (p.s2d && valid) {
         const int ow = (int)(px % g.Wo);
         const long long t = px / g.Wo;
-        const int oh = (int)(t % g.Ho), n = (int)(t / g.Ho);
+        const int oh = (int)(t % g.Ho);
+        int n = (int)(t / g.Ho);
+        if (g.Do > 1) n = n % g.Do * g.batch + n / g.Do;  // clips: [d][n][Hb][Wb][4][K]
         const int by = (oh + 1) >> 1, bx = (ow + 1) >> 1, sp = ((oh + 1) & 1) * 2 + ((ow + 1) & 1);
         yrow = y + ((((size_t)n * p.Hb + by) * p.Wb + bx) * 4 + sp) * g.K;
       }
@@ -710,7 +712,6 @@ int conv_first_tc_set_weights(ConvFirstTc* t, const __half* w) {
 }
 
 int conv_first_tc_set_s2d(ConvFirstTc* t, int enable, int Hb, int Wb) {
-  if (enable && t->prm.g.Do != 1) return aig_fail(t->ctx, AIG_ERR_UNSUPPORTED, "conv0: space-to-depth output is for 2-D layers");
   t->prm.s2d = enable ? 1 : 0;
   t->prm.Hb = Hb;
   t->prm.Wb = Wb;

@@ -13,13 +13,15 @@
 
 #include "aig_b200.h"
 #include "aig_host.h"
+#include "clip_conv.h"
 
 struct aig_c3d {
   aig_ctx* ctx = nullptr;
   aig_c3d_config cfg{};
   std::string err;
   aig_conv0_plan* first = nullptr;
-  std::vector<aig_conv_plan*> convs;
+  std::vector<ClipConv*> walks;        // the layers behind the first, as far as the depth-walking kernel takes them
+  std::vector<aig_conv_plan*> convs;   // the layers after those
   aig_conv_plan* fc = nullptr;
   std::vector<aig_half*> acts;
   std::vector<int> d, h, w;
@@ -65,8 +67,21 @@ int aig_c3d_create(aig_ctx* ctx, const aig_c3d_config* cfg, aig_c3d** out) {
   int D = c.depth, H = c.height, W = c.width;
   int rc = aig_conv0_plan_create_3d(ctx, c.batch, D, H, W, c.widths[1], 3, 3, 1, 2, 1, 1, AIG_ACT_LEAKY, c.slope, &m->first);
   if (rc == AIG_OK) aig_conv0_plan_out_dims(m->first, &D, &H, &W);
+  auto geom = [&](int i, int h, int w) { return ClipConvGeom{c.batch, D, h, w, c.widths[i], c.widths[i + 1], c.slope, 0}; };  // layer i's
+  int n_walk = 0;
+  for (int h = H, w = W; rc == AIG_OK && n_walk + 1 < c.n_layers && clip_conv_supported(ctx, geom(n_walk + 1, h, w)); ++n_walk) h = (h - 1) / 2 + 1, w = (w - 1) / 2 + 1;
+  if (n_walk > 0 && !conv0_plan_set_output_clip_blocks(m->first)) n_walk = 0;
   for (int i = 0; i < c.n_layers && rc == AIG_OK; ++i) {
-    if (i > 0) {
+    if (i > 0 && i <= n_walk) {
+      ClipConvGeom g = geom(i, H, W);
+      g.out_blocks = i < n_walk;
+      ClipConv* p = nullptr;
+      rc = clip_conv_create(ctx, g, &p);
+      if (rc != AIG_OK) break;
+      m->walks.push_back(p);
+      H = (H - 1) / 2 + 1;
+      W = (W - 1) / 2 + 1;
+    } else if (i > 0) {
       aig_conv_desc d{};
       d.batch = c.batch; d.in_c = c.widths[i]; d.in_d = D; d.in_h = H; d.in_w = W; d.out_c = c.widths[i + 1];
       d.kd = d.kh = d.kw = 3; d.sd = 1; d.sh = d.sw = 2; d.pd = d.ph = d.pw = 1;
@@ -78,7 +93,8 @@ int aig_c3d_create(aig_ctx* ctx, const aig_c3d_config* cfg, aig_c3d** out) {
       aig_conv_plan_out_dims(p, &D, &H, &W);
     }
     aig_half* buf = nullptr;
-    if (cudaMalloc(reinterpret_cast<void**>(&buf), (size_t)c.batch * D * H * W * c.widths[i + 1] * 2) != cudaSuccess) rc = AIG_ERR_CUDA;
+    const size_t bytes = 2 * (i < n_walk ? clip_block_elems(c.batch, D, H, W, c.widths[i + 1]) : (size_t)c.batch * D * H * W * c.widths[i + 1]);
+    if (cudaMalloc(reinterpret_cast<void**>(&buf), bytes) != cudaSuccess || (i < n_walk && cudaMemset(buf, 0, bytes) != cudaSuccess)) rc = AIG_ERR_CUDA;
     m->acts.push_back(buf);
     m->d.push_back(D); m->h.push_back(H); m->w.push_back(W);
   }
@@ -101,6 +117,7 @@ int aig_c3d_destroy(aig_c3d* m) {
   if (!m) return AIG_OK;
   if (m->ctx) aig_ctx_sync(m->ctx);
   aig_conv0_plan_destroy(m->first);
+  for (ClipConv* p : m->walks) clip_conv_destroy(p);
   for (aig_conv_plan* p : m->convs) aig_conv_plan_destroy(p);
   aig_conv_plan_destroy(m->fc);
   for (aig_half* a : m->acts) cudaFree(a);
@@ -132,7 +149,8 @@ int aig_c3d_load_memory(aig_c3d* m, const void* blob, size_t bytes) {
     for (int j = 0; j < 6; ++j) bn[j] = (float*)take(K * 4);
     if (!w || !b || !bn[5]) return cfail(m, AIG_ERR_CUDA, aig_last_error(m->ctx));
     if (i == 0) C3D_OK(m, aig_conv0_plan_set_weights(m->first, w, b, bn[0], bn[1], bn[2], bn[3], 1e-6f));
-    else C3D_OK(m, aig_conv_plan_set_weights(m->convs[i - 1], w, b, bn[0], bn[1], bn[2], bn[3], 1e-6f));
+    else if (i <= (int)m->walks.size()) C3D_OK(m, clip_conv_set_weights(m->walks[i - 1], w, b, bn[0], bn[1], bn[2], bn[3], 1e-6f));
+    else C3D_OK(m, aig_conv_plan_set_weights(m->convs[i - 1 - m->walks.size()], w, b, bn[0], bn[1], bn[2], bn[3], 1e-6f));
   }
   const size_t feat = (size_t)c.widths[c.n_layers] * 4;
   aig_half* fw = (aig_half*)take(feat * c.n_out * 2);
@@ -152,7 +170,9 @@ int aig_c3d_forward(aig_c3d* m, const aig_half* clips) {
   if (!m->loaded) return cfail(m, AIG_ERR_INVALID, "parameters not loaded");
   const aig_c3d_config& c = m->cfg;
   C3D_OK(m, aig_conv0_forward_nchw(m->first, clips, m->acts[0]));
-  for (size_t i = 0; i < m->convs.size(); ++i) C3D_OK(m, aig_conv_forward(m->convs[i], m->acts[i], nullptr, m->acts[i + 1]));
+  const size_t nw = m->walks.size();
+  for (size_t i = 0; i < nw; ++i) C3D_OK(m, clip_conv_forward(m->walks[i], m->acts[i], m->acts[i + 1]));
+  for (size_t i = 0; i < m->convs.size(); ++i) C3D_OK(m, aig_conv_forward(m->convs[i], m->acts[nw + i], nullptr, m->acts[nw + i + 1]));
   const int L = c.n_layers - 1;
   C3D_OK(m, aig_adaptive_avgpool3d_ndhwc(m->ctx, m->acts[L], m->feat, c.batch, m->d[L], m->h[L], m->w[L], c.widths[c.n_layers], 2, 2));
   if (c.batch <= 64) {

@@ -250,3 +250,36 @@ def test_agent_second_parameter_load(env, monkeypatch, B, unfused):
         for got, w in zip(run(agent), want[i]):
             assert np.array_equal(got, w), "load of blob %d" % i
     agent.close()
+
+
+@gpu
+@pytest.mark.parametrize("B,D,H,W,offset,widths", [
+    (1, 1, 12, 16, 0, (3, 32, 64, 128)),       # a clip of one frame: only the middle depth tap
+    (3, 5, 37, 53, 0, (3, 32, 64, 128)),       # odd extents in every layer, tiles that span clips
+    (1, 11, 33, 66, 0, (3, 32, 64, 128)),      # more depths than accumulators
+    (5, 2, 18, 31, 4, (3, 32, 64, 128)),       # first layer by the gather (clips off a 16-byte boundary)
+    (1, 3, 17, 300, 0, (3, 32, 64, 128)),      # and by rows beyond 256 pixels
+    (16, 8, 70, 90, 0, (3, 32, 64, 128)),      # several tiles a CTA, runs that begin and end inside a tile
+    (2, 4, 40, 48, 0, (3, 32, 128, 32)),       # two channel shares, then a layer that the walk does not take
+    (2, 4, 40, 48, 0, (3, 32, 64, 32)),        # one share of 32 channels
+])
+def test_clip_encoder_depth_walk(env, B, D, H, W, offset, widths):
+    """The depth-walking 3-D convolution at the edges of its tiles, runs and channel shares."""
+    U = env
+    U.pkg()
+    import torch
+    from ai_gamer_b200 import runners as R
+
+    p = PL.make_conv3d_params(B + D, widths=widths, trivial=False)
+    clips = PL.make_clips(W, B, D, H, W)
+    feat, _, _ = PL.conv3d_forward(p, clips)
+    enc = R.ClipEncoder(U.ctx(), B, D, H, W, widths=widths)
+    enc.load_bytes(PL.serialize_conv3d_params(p))
+    room = torch.zeros(clips.size + 8, dtype=torch.float16, device="cuda")
+    room[offset:offset + clips.size] = U.dev(clips).flatten()
+    torch.cuda.synchronize()
+    enc.forward(room[offset:])
+    got = U.host(enc.features()).astype(np.float32)
+    # three layers of fp16 activations (2^-11 each) and the pool's own rounding, against a scale of at least the rms
+    assert U.scaled_err(got, feat.astype(np.float32)) < 4e-3
+    enc.close()
