@@ -5,7 +5,7 @@
 // output tile is staged in shared memory and each thread produces one output pixel x 32 channels.
 // Output is channels-last fp16 with bias + folded BatchNorm + activation applied.
 #include "aig_common.cuh"
-#include "clip_conv.h"
+#include "walk_conv.h"
 #include "conv_first_rows.h"
 #include "conv_first_tc.h"
 
@@ -351,4 +351,10 @@ bool conv0_plan_set_output_clip_blocks(aig_conv0_plan* pl) {
   if (!pl->tc || pl->p.kd == 1 || pl->p.K % 8 != 0) return false;
   const int Hb = clip_block_extent(pl->p.Ho), Wb = clip_block_extent(pl->p.Wo);
   return (!pl->rows || conv_first_rows_set_s2d(pl->rows, 1, Hb, Wb) == AIG_OK) && conv_first_tc_set_s2d(pl->tc, 1, Hb, Wb) == AIG_OK;
+}
+
+bool conv0_plan_set_output_row_blocks(aig_conv0_plan* pl) {
+  if (!pl->tc || pl->p.D != 1 || pl->p.kd != 1 || pl->p.K % 8 != 0) return false;
+  const int Hb = (pl->p.Ho - 2) / 2 + 2, Wb = (pl->p.Wo - 2) / 2 + 2;
+  return (!pl->rows || conv_first_rows_set_s2d(pl->rows, 1, Hb, Wb, true) == AIG_OK) && conv_first_tc_set_s2d(pl->tc, 1, Hb, Wb, true) == AIG_OK;
 }

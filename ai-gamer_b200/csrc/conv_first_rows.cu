@@ -63,6 +63,7 @@ struct RowsParams {
   int batch, D, H, W, Ho, Wo;
   int tiles;               // batch * Ho (* D)
   int s2d, Hb;             // output in space-to-depth blocks; block rows per image
+  int rows_outer;          // of them [yb][n] instead of [n][yb]
   int planar;              // 1: frames are three uint8 planes R, G, B; 0: BGRA pixels
   float slope;
   float scale[kN], shift[kN];
@@ -294,7 +295,7 @@ conv_first_rows_kernel(const __grid_constant__ CUtensorMap tmapY, const __grid_c
       if (*s_abort) break;                        // uniform: every thread reads the flag after the same barrier
       if (tid_e == 0) {
         const uint32_t src = sOut + (uint32_t)buf * kOutBytes;
-        if (p.s2d) tma_store_5d(&tmapY, src, 0, 0, 0, (y + 1) & 1, (CLIP ? z * p.batch + n : n) * p.Hb + ((y + 1) >> 1));
+        if (p.s2d) tma_store_5d(&tmapY, src, 0, 0, 0, (y + 1) & 1, p.rows_outer ? ((y + 1) >> 1) * p.batch + n : (CLIP ? z * p.batch + n : n) * p.Hb + ((y + 1) >> 1));
         else tma_store_4d(&tmapY, src, 0, 0, y, CLIP ? n * p.D + z : n);
         bulk_commit();
       }
@@ -546,9 +547,10 @@ int conv_first_rows_set_weights(ConvFirstRows* t, const __half* w) {
   return AIG_OK;
 }
 
-int conv_first_rows_set_s2d(ConvFirstRows* t, int enable, int Hb, int Wb) {
+int conv_first_rows_set_s2d(ConvFirstRows* t, int enable, int Hb, int Wb, bool rows_outer) {
   if (enable && 2 * Wb > kOutSlots) return aig_fail(t->ctx, AIG_ERR_UNSUPPORTED, "first-layer row kernel: block row too wide");
   t->prm.s2d = enable ? 1 : 0;
+  t->prm.rows_outer = rows_outer ? 1 : 0;
   t->prm.Hb = Hb;
   t->Hb = Hb;
   t->Wb = Wb;
@@ -561,7 +563,7 @@ static int rows_encode_output(ConvFirstRows* t, __half* y) {
   const ConvFirstGeom& g = t->g;
   CUresult r;
   if (t->prm.s2d) {
-    // blocks [n][hb][wb][sy][sx][c] (clips: [d][n][hb]...) seen as (c, sx, wb, sy, n*hb): one output row = sub-row sy of
+    // blocks [n][hb][wb][sy][sx][c] (or [hb][n]..., of clips [d][n][hb]...) seen as (c, sx, wb, sy, n*hb): one output row = sub-row sy of
     // block row hb, pixels in (wb, sx) order = x + 1
     cuuint64_t dims[5] = {(cuuint64_t)kN, 2, (cuuint64_t)t->Wb, 2, (cuuint64_t)g.batch * g.D * t->Hb};
     cuuint64_t strides[4] = {(cuuint64_t)kN * 2, (cuuint64_t)4 * kN * 2, (cuuint64_t)2 * kN * 2, (cuuint64_t)t->Wb * 4 * kN * 2};

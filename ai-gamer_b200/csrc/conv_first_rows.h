@@ -14,7 +14,7 @@ bool conv_first_rows_supported(const ConvFirstGeom& g);
 int conv_first_rows_create(aig_ctx* ctx, const ConvFirstGeom& g, const float* scale, const float* shift, ConvFirstRows** out);
 void conv_first_rows_destroy(ConvFirstRows* t);
 int conv_first_rows_set_weights(ConvFirstRows* t, const __half* w_kcrs);
-int conv_first_rows_set_s2d(ConvFirstRows* t, int enable, int Hb, int Wb);
+int conv_first_rows_set_s2d(ConvFirstRows* t, int enable, int Hb, int Wb, bool rows_outer = false);
 // frames: BGRA pixels [B][H][W][4] or, planar_rgb != 0, uint8 planes [B][3][H][W]; both 16-byte aligned
 int conv_first_rows_forward(ConvFirstRows* t, const uint8_t* frames, int planar_rgb, __half* y);
 // clips: planar fp16 [B][3][D][H][W], 16-byte aligned (plans with kd == 3)

@@ -27,6 +27,7 @@ struct TcParams {
   int* gerr;
   int pair;         // planar fp16 input, k3 s2 p1, even width: the gather loads column pairs (see the producers)
   int s2d, Hb, Wb;  // s2d: store into the 2x2 space-to-depth layout [n][Hb][Wb][4][K] read by a fused down-sampling block
+  int rows_outer;   // that layout with the block rows outside, [Hb][n][Wb][4][K]
 };
 
 __device__ __forceinline__ uint32_t swz(int r, int c) { return (uint32_t)(r * 128 + ((c ^ (r & 7)) << 4)); }
@@ -227,7 +228,7 @@ conv_first_tc_kernel(const void* __restrict__ xin, __half* __restrict__ y, const
         int n = (int)(t / g.Ho);
         if (g.Do > 1) n = n % g.Do * g.batch + n / g.Do;  // clips: [d][n][Hb][Wb][4][K]
         const int by = (oh + 1) >> 1, bx = (ow + 1) >> 1, sp = ((oh + 1) & 1) * 2 + ((ow + 1) & 1);
-        yrow = y + ((((size_t)n * p.Hb + by) * p.Wb + bx) * 4 + sp) * g.K;
+        yrow = y + (((p.rows_outer ? (size_t)by * g.batch + n : (size_t)n * p.Hb + by) * p.Wb + bx) * 4 + sp) * g.K;
       }
       if (!mbar_wait_bounded(bar_tfull + 8 * st, ph, s_abort, p.gerr, 604)) break;
       tc_fence_after();
@@ -480,7 +481,7 @@ conv_first_patch_kernel(const uint32_t* __restrict__ xin, __half* __restrict__ y
       size_t pix = ((size_t)n * g.Ho + oh) * g.Wo + ow;
       if (p.s2d) {
         const int sby = (oh + 1) >> 1, sbx = (ow + 1) >> 1, sp = ((oh + 1) & 1) * 2 + ((ow + 1) & 1);
-        pix = (((size_t)n * p.Hb + sby) * p.Wb + sbx) * 4 + sp;
+        pix = ((p.rows_outer ? (size_t)sby * g.batch + n : (size_t)n * p.Hb + sby) * p.Wb + sbx) * 4 + sp;
       }
       __half* yrow = y + pix * g.K;
       if (!mbar_wait_bounded(bar_tfull + 8 * st, ph, s_abort, p.gerr, 614)) break;
@@ -711,8 +712,9 @@ int conv_first_tc_set_weights(ConvFirstTc* t, const __half* w) {
   return AIG_OK;
 }
 
-int conv_first_tc_set_s2d(ConvFirstTc* t, int enable, int Hb, int Wb) {
+int conv_first_tc_set_s2d(ConvFirstTc* t, int enable, int Hb, int Wb, bool rows_outer) {
   t->prm.s2d = enable ? 1 : 0;
+  t->prm.rows_outer = rows_outer ? 1 : 0;
   t->prm.Hb = Hb;
   t->prm.Wb = Wb;
   return AIG_OK;

@@ -29,6 +29,7 @@
 #include "aig_host.h"
 #include "cnn_stream.h"
 #include "res_chain.h"
+#include "walk_conv.h"
 
 namespace {
 
@@ -66,9 +67,12 @@ struct aig_cnn {
     aig_conv_plan *c0 = nullptr, *c1 = nullptr, *sc = nullptr;
     aig_conv_plan* down = nullptr;  // main k4 s2 + shortcut k2 s2 as one launch over the space-to-depth input (replaces c0 and sc)
     aig_half *t = nullptr, *r = nullptr, *y = nullptr;
+    size_t t_elems = 0;             // of t and of r
+    WalkConv *walk_down = nullptr, *walk_c1 = nullptr;  // the block by rows (replaces down and c1)
     bool y_s2d = false;             // y is written in the space-to-depth layout the next block's fused launch reads
+    bool y_rows = false;            // and with the block rows outermost
   };
-  bool act0_s2d = false;
+  bool act0_s2d = false, act0_rows = false;
   aig_half* stage_scratch = nullptr;  // channels-last copy of a space-to-depth stage, made on request
   size_t stage_scratch_elems = 0;
   std::vector<Block> blocks;
@@ -177,6 +181,38 @@ bool read_bn(aig_cnn* m, Reader& rd, BnP& b, int c, cudaStream_t s) {
 
 }  // namespace
 
+// The first blocks by rows, as far as that kernel takes them.  Buffers are still all zero here, as its zero columns have to be.
+static int cnn_use_row_walk(aig_cnn* m) {
+  const aig_cnn_config& c = m->cfg;
+  auto geom = [&](int i) {
+    return ResWalkGeom{c.batch, i == 0 ? m->H0 : m->bh[i - 1], i == 0 ? m->W0 : m->bw[i - 1], c.widths[i], c.widths[i + 1], c.act, c.slope, RES_OUT_NHWC};
+  };
+  int n = 0;
+  while (n < c.n_blocks && m->blocks[n].down && res_walk_supported(m->ctx, geom(n))) ++n;
+  if (n == 0 || !conv0_plan_set_output_row_blocks(m->conv0)) return AIG_OK;
+  m->act0_rows = true;
+  for (int i = 0; i < n; ++i) {
+    aig_cnn::Block& b = m->blocks[i];
+    ResWalkGeom g = geom(i);
+    b.y_rows = i + 1 < n;
+    g.out = b.y_rows ? RES_OUT_ROW_BLOCKS : b.y_s2d ? RES_OUT_BLOCKS : RES_OUT_NHWC;
+    const int rc = res_walk_create(m->ctx, g, &b.walk_down, &b.walk_c1);
+    if (rc != AIG_OK) return rc;
+    aig_conv_plan_destroy(b.down);
+    aig_conv_plan_destroy(b.c1);
+    b.down = b.c1 = nullptr;
+    aig_half** bufs[2] = {&b.t, &b.r};
+    for (aig_half** p : bufs) {
+      if (b.t_elems >= res_walk_rows(g) * g.K) continue;
+      cudaFree(*p);
+      *p = nullptr;
+      const int arc = dev_alloc(m, p, res_walk_rows(g) * g.K);
+      if (arc != AIG_OK) return arc;
+    }
+  }
+  return AIG_OK;
+}
+
 extern "C" {
 
 size_t aig_cnn_checkpoint_bytes(const aig_cnn_config* c) {
@@ -269,6 +305,7 @@ int aig_cnn_create(aig_ctx* ctx, const aig_cnn_config* cfg, aig_cnn** out) {
       if (aig_conv_plan_set_input_padded(b.c1, 1) == AIG_OK) n = (size_t)aig_conv_padded_rows(c.batch, oh, ow, 1) * co;
       else aig_resdown_plan_set_output_padded(b.down, 0);
     }
+    b.t_elems = n;
     if (dev_alloc(m, &b.t, n) != AIG_OK || dev_alloc(m, &b.r, n) != AIG_OK) return bail(AIG_ERR_CUDA);
     m->blocks.push_back(b);
     m->bh.push_back(oh);
@@ -342,6 +379,7 @@ int aig_cnn_create(aig_ctx* ctx, const aig_cnn_config* cfg, aig_cnn** out) {
       m->sites.push_back(all);
     }
   }
+  if (!m->chain && (rc = cnn_use_row_walk(m)) != AIG_OK) return bail(rc);
   m->params.cap = aig_cnn_checkpoint_bytes(&c) + 256 * (16 + 32 * (size_t)c.n_blocks);
   if (cudaMalloc(reinterpret_cast<void**>(&m->params.base), m->params.cap) != cudaSuccess) return bail(AIG_ERR_CUDA);
   *out = m;
@@ -370,6 +408,8 @@ int aig_cnn_destroy(aig_cnn* m) {
     aig_conv_plan_destroy(b.c1);
     aig_conv_plan_destroy(b.sc);
     aig_conv_plan_destroy(b.down);
+    walk_conv_destroy(b.walk_down);
+    walk_conv_destroy(b.walk_c1);
     cudaFree(b.t);
     cudaFree(b.r);
     cudaFree(b.y);
@@ -418,6 +458,11 @@ int aig_cnn_load_memory(aig_cnn* m, const void* blob, size_t bytes) {
         !read_conv(m, rd, c1, (size_t)co * co * 9, co, s) || !read_bn(m, rd, b1, co, s) ||
         !read_conv(m, rd, sc, (size_t)co * ci * 4, co, s))
       return fail(m, AIG_ERR_IO, io);
+    if (m->blocks[i].walk_down) {
+      CNN_OK(m, res_walk_set_down(m->blocks[i].walk_down, c0.w, c0.b, b0.a[0], b0.a[1], b0.a[2], b0.a[3], eps, sc.w, sc.b));
+      CNN_OK(m, res_walk_set_conv1(m->blocks[i].walk_c1, c1.w, c1.b, b1.a[0], b1.a[1], b1.a[2], b1.a[3], eps));
+      continue;
+    }
     if (m->blocks[i].down) {
       CNN_OK(m, aig_resdown_plan_set_weights(m->blocks[i].down, c0.w, c0.b, b0.a[0], b0.a[1], b0.a[2], b0.a[3], eps, sc.w, sc.b));
     } else {
@@ -481,6 +526,14 @@ static int cnn_forward_impl(aig_cnn* m, const uint8_t* bgra_dev, bool planar) {
   }
   const aig_half* x = m->act0;
   for (auto& b : m->blocks) {
+    if (b.walk_down) {
+      CNN_OK(m, res_walk_down(b.walk_down, x, b.t, b.r));
+      tick();
+      CNN_OK(m, res_walk_conv1(b.walk_c1, b.t, b.r, b.y));
+      tick();
+      x = b.y;
+      continue;
+    }
     if (b.down) {
       CNN_OK(m, aig_resdown_forward(b.down, x, b.t, b.r));
       tick();
@@ -761,7 +814,8 @@ const aig_half* aig_cnn_stage_output(aig_cnn* m, int stage, int* h, int* w, int*
     if (cudaMalloc(reinterpret_cast<void**>(&m->stage_scratch), n * sizeof(aig_half)) != cudaSuccess) return nullptr;
     m->stage_scratch_elems = n;
   }
-  if (aig_s2d_to_nhwc(m->ctx, buf, m->stage_scratch, m->cfg.batch, sh, sw, sc) != AIG_OK) return nullptr;
+  const bool rows = stage == 0 ? m->act0_rows : m->blocks[stage - 1].y_rows;
+  if ((rows ? row_blocks_to_nhwc : aig_s2d_to_nhwc)(m->ctx, buf, m->stage_scratch, m->cfg.batch, sh, sw, sc) != AIG_OK) return nullptr;
   return m->stage_scratch;
 }
 

@@ -13,14 +13,14 @@
 
 #include "aig_b200.h"
 #include "aig_host.h"
-#include "clip_conv.h"
+#include "walk_conv.h"
 
 struct aig_c3d {
   aig_ctx* ctx = nullptr;
   aig_c3d_config cfg{};
   std::string err;
   aig_conv0_plan* first = nullptr;
-  std::vector<ClipConv*> walks;        // the layers behind the first, as far as the depth-walking kernel takes them
+  std::vector<WalkConv*> walks;        // the layers behind the first, as far as the depth-walking kernel takes them
   std::vector<aig_conv_plan*> convs;   // the layers after those
   aig_conv_plan* fc = nullptr;
   std::vector<aig_half*> acts;
@@ -75,7 +75,7 @@ int aig_c3d_create(aig_ctx* ctx, const aig_c3d_config* cfg, aig_c3d** out) {
     if (i > 0 && i <= n_walk) {
       ClipConvGeom g = geom(i, H, W);
       g.out_blocks = i < n_walk;
-      ClipConv* p = nullptr;
+      WalkConv* p = nullptr;
       rc = clip_conv_create(ctx, g, &p);
       if (rc != AIG_OK) break;
       m->walks.push_back(p);
@@ -117,7 +117,7 @@ int aig_c3d_destroy(aig_c3d* m) {
   if (!m) return AIG_OK;
   if (m->ctx) aig_ctx_sync(m->ctx);
   aig_conv0_plan_destroy(m->first);
-  for (ClipConv* p : m->walks) clip_conv_destroy(p);
+  for (WalkConv* p : m->walks) walk_conv_destroy(p);
   for (aig_conv_plan* p : m->convs) aig_conv_plan_destroy(p);
   aig_conv_plan_destroy(m->fc);
   for (aig_half* a : m->acts) cudaFree(a);

@@ -369,3 +369,34 @@ def test_checkpoint_files(env, tmp_path):
     enc.forward(U.dev(PL.make_frames(1, 1, 32, 64)))
     c.sync()
     enc.close()
+
+
+@gpu
+@pytest.mark.parametrize("B,H,W,widths,act", [
+    (1950, 32, 40, (32, 64, 128), "ACT_SWISH"),       # runs of one to eight rows, all the ways they follow one another in the accumulators
+    (3, 10, 12, (32, 64, 128), "ACT_RELU"),           # one tile, fewer rows than accumulators
+    (37, 67, 131, (32, 64, 128, 256), "ACT_LEAKY"),   # odd extents, a block by rows before one by patches
+    (5, 50, 322, (32, 64, 192), "ACT_SWISH"),         # rows beyond 256 pixels; one block by rows
+    (150, 20, 20, (32, 64), "ACT_NONE"),              # the last block by rows
+])
+def test_residual_blocks_by_rows(env, monkeypatch, B, H, W, widths, act):
+    """The row-walking residual blocks at the edges of their tiles and runs, every stage against the oracle on a sample."""
+    U = env
+    c, pk = U.ctx(), U.pkg()
+    monkeypatch.setenv("AIG_CNN_NO_CHAIN", "1")
+    params = PL.make_cnn_params(B + H, widths=widths, trivial=False)
+    frames = PL.make_frames(B, B, H, W)
+    pick = np.unique(np.linspace(0, B - 1, 60).astype(int))
+    enc = pk.CnnEncoder(c, B, H, W, widths=widths, act=getattr(pk, act))
+    enc.load_bytes(PL.serialize_cnn_checkpoint(params, W, H))
+    runs = []
+    for _ in range(3):
+        enc.forward(U.dev(frames))
+        c.sync()
+        runs.append([U.host(enc.stage_output(i)) for i in range(len(widths))])
+    assert all(np.array_equal(x, y) for r in runs[1:] for x, y in zip(runs[0], r))
+    stages = PL.cnn_forward(params, frames[pick], act=getattr(O, act), return_all=True)[3]
+    for i, (got, want) in enumerate(zip(runs[0], stages)):
+        err = U.scaled_err(U.nchw(got[pick]), want)
+        assert err < STAGE_TOL, "stage %d: max scaled err %.4f" % (i, err)
+    enc.close()
