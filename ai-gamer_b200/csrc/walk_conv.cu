@@ -55,6 +55,7 @@ struct Clip32 {                    // unit u: the two sub-positions of sub-row u
   }
   static constexpr int kHalo[kUnits] = {3, 1};        // largest shift of the unit, bits as above
   static constexpr bool kEqualPatches = false;        // patch buffers in pairs of the two units' sizes
+  static constexpr bool kImages = false;              // (see Conv256)
 };
 struct Clip64 {                    // unit u: sub-position u
   static constexpr int kTaps = 3, kNC = 32, kUnits = 4, kBlocks = 9, kShort = 0, kEntries = 9, kStart = 0, kEpiWarps = 4;
@@ -67,6 +68,7 @@ struct Clip64 {                    // unit u: sub-position u
   }
   static constexpr int kHalo[kUnits] = {3, 2, 1, 0};
   static constexpr bool kEqualPatches = true;         // any unit in any buffer: five fit, four would be one plane's
+  static constexpr bool kImages = false;
 };
 // k3 s1 p1 over U * 64 channels: unit u its 64 channels, weight block 3 * u + filter column
 template <int U>
@@ -74,7 +76,15 @@ struct Conv1 {
   static constexpr int kTaps = 3, kNC = 64, kUnits = U, kBlocks = 3 * U, kShort = 0, kEntries = 3 * U, kStart = 1, kEpiWarps = 16;
   __host__ __device__ static constexpr Entry entry(int e) { return Entry{e / 3, e % 3 == 2 ? 4 : e % 3, e, 0, 0, 4, MAIN, e % 3 == 0, e % 3 == 2}; }
   static constexpr int kHalo[2] = {4, 4};
-  static constexpr bool kEqualPatches = true;
+  static constexpr bool kEqualPatches = true, kImages = false;
+};
+// The same over 256 channels, 32 outputs a CTA, on images outermost ([n][y][x] with a zero column and row behind every image):
+// a tile is as many whole image rows as 128 positions hold, one of each image, with a zero row of its own before them.
+struct Conv256 {
+  static constexpr int kTaps = 3, kNC = 32, kUnits = 4, kBlocks = 12, kShort = 0, kEntries = 12, kStart = 1, kEpiWarps = 8;
+  __host__ __device__ static constexpr Entry entry(int e) { return Conv1<4>::entry(e); }
+  static constexpr int kHalo[kUnits] = {4, 4, 4, 4};
+  static constexpr bool kEqualPatches = true, kImages = true;
 };
 // k4 s2 p1 and the shortcut k2 s2 p0: over blocks, filter (2*ty + dy, 2*tx + dx) at block tap (ty, tx), sub-position (dy, dx);
 // of the shortcut's filter (ty, tx) at sub-position (1 - ty, 1 - tx).  Weight block 2 * unit + tx; the shortcut's: unit
@@ -87,7 +97,7 @@ struct Down32 {                    // unit u: the two sub-positions of sub-row u
     return Entry{u, tx, u, half, half, 2, u == 1 ? SHORT_HERE : SHORT_BEFORE, false, i == 3};
   }
   static constexpr int kHalo[kUnits] = {1, 1};
-  static constexpr bool kEqualPatches = true;
+  static constexpr bool kEqualPatches = true, kImages = false;
 };
 struct Down64 {                    // unit u: sub-position u
   static constexpr int kTaps = 2, kNC = 64, kUnits = 4, kBlocks = 8, kShort = 4, kEntries = 12, kStart = 0, kEpiWarps = 16;
@@ -97,12 +107,13 @@ struct Down64 {                    // unit u: sub-position u
     return Entry{u, 1 - (u & 1), u, 0, 0, 4, u >= 2 ? SHORT_HERE : SHORT_BEFORE, false, true};
   }
   static constexpr int kHalo[kUnits] = {1, 1, 1, 1};
-  static constexpr bool kEqualPatches = true;
+  static constexpr bool kEqualPatches = true, kImages = false;
 };
 
 struct WalkParams {
   int steps, outs_per_tile;        // input and output steps of the axis
-  int P;                           // positions of a step
+  int P, tile;                     // positions of a step, of a tile
+  uint32_t res_n, res_step;        // residual: rows from image to image and from step to step
   int img, Wb, Ho, Wo;             // positions of one image and of one of its rows; of them, rows and columns that give outputs
   int outs, parts, ctas;           // tiles * output steps, channel shares, CTAs per share
   int patches, patch_bytes[2];     // buffers; sizes of the even and the odd ones
@@ -122,6 +133,12 @@ struct WalkMaps {
   CUtensorMap u[kMaxUnits];
 };
 
+__device__ __forceinline__ void tma_load_4d(uint32_t dst, const void* desc, uint32_t bar, int c0, int c1, int c2, int c3) {
+  asm volatile(
+      "cp.async.bulk.tensor.4d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5, %6}], [%2];"
+      ::"r"(dst), "l"(reinterpret_cast<uint64_t>(desc)), "r"(bar), "r"(c0), "r"(c1), "r"(c2), "r"(c3)
+      : "memory");
+}
 __device__ __forceinline__ void bulk_load(uint32_t dst, const void* src, uint32_t bytes, uint32_t bar) {
   asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(dst), "l"(src), "r"(bytes), "r"(bar)
                : "memory");
@@ -283,6 +300,11 @@ __global__ void __launch_bounds__(walk_threads<G>(), 1) walk_conv_kernel(const _
     *s_abort = 0;
     fence_mbar_init();
   }
+  if (G::kImages) {                // the zero rows
+    for (int i = threadIdx.x; i < p.patches * 8; i += walk_threads<G>())
+      *reinterpret_cast<uint4*>(sm + kWBytes + patch_offset<G>(p, i >> 3) + (i & 7) * 16) = make_uint4(0, 0, 0, 0);
+    fence_proxy_async_smem();
+  }
   if (warp == 2) {
     tmem_alloc(smem_u32(s_tmem), kCols);
     tmem_relinquish();
@@ -311,8 +333,10 @@ __global__ void __launch_bounds__(walk_threads<G>(), 1) walk_conv_kernel(const _
         for (int u = 0; u < U; ++u) {
           if (!mbar_wait_bounded_sleepy(bar_uempty + 8 * ring.i, ring.phase ^ 1u, s_abort, p.gerr, 901)) { ok = false; break; }
           if (leader) {
-            mbar_expect_tx(bar_ufull + 8 * ring.i, (uint32_t)p.unit_rows[u] * 128u);
-            tma_load_2d(sPatch + patch_offset<G>(p, ring.i), &maps.u[u], bar_ufull + 8 * ring.i, 64 * u, f * p.P + r.t * 128 - G::kStart);
+            mbar_expect_tx(bar_ufull + 8 * ring.i, (uint32_t)(G::kImages ? p.tile : p.unit_rows[u]) * 128u);
+            const uint32_t dst = sPatch + patch_offset<G>(p, ring.i);
+            if (G::kImages) tma_load_4d(dst + 128, &maps.u[0], bar_ufull + 8 * ring.i, 64 * u, 0, f, r.t * (p.tile / p.Wb));
+            else tma_load_2d(dst, &maps.u[u], bar_ufull + 8 * ring.i, 64 * u, f * p.P + r.t * 128 - G::kStart);
           }
           ring.advance(p.patches);
         }
@@ -458,13 +482,14 @@ __global__ void __launch_bounds__(walk_threads<G>(), 1) walk_conv_kernel(const _
       for (int i = 0; i < kSlots; ++i) release(i);
     griddep_wait();                                       // the output may still be read by an earlier launch
     while (ok && r.next()) {
-      uint32_t offs[4];
+      uint32_t offs[4], res_offs[4];
       bool vs[4];
 #pragma unroll
       for (int i = 0; i < 4; ++i) {
-        const int pos = r.t * 128 + q * 32 + 8 * i + gr;
+        const int row = q * 32 + 8 * i + gr, pos = r.t * p.tile + row;
         const int n = pos / p.img, rem = pos - n * p.img, y = rem / p.Wb, x = rem - y * p.Wb;
-        vs[i] = pos < p.P && y < p.Ho && x < p.Wo;
+        vs[i] = row < p.tile && pos < p.P && y < p.Ho && x < p.Wo;
+        res_offs[i] = ((uint32_t)n * p.res_n + (uint32_t)x) * (uint32_t)(p.K / 8) + (uint32_t)(ch / 8);
         // (sub16 is the step between a block's sub-rows, half of it the one between its columns)
         offs[i] = (uint32_t)n * p.n16 + (uint32_t)(ch / 8) +
                   (p.y_blocks ? (uint32_t)((y + 1) >> 1) * p.y16 + (uint32_t)((y + 1) & 1) * p.sub16 : (uint32_t)y * p.y16) +
@@ -472,9 +497,9 @@ __global__ void __launch_bounds__(walk_threads<G>(), 1) walk_conv_kernel(const _
       }
       uint4 res[4];                                       // the residual, fetched an output ahead
       auto fetch = [&](int d) {
-        const uint4* rr = p.residual + ((size_t)d * p.P + r.t * 128 + q * 32 + gr) * (p.K / 8) + ch / 8;
+        const uint4* rr = p.residual + (size_t)d * p.res_step * (p.K / 8);
 #pragma unroll
-        for (int i = 0; i < 4; ++i) res[i] = vs[i] ? __ldg(rr + (size_t)(8 * i) * (p.K / 8)) : make_uint4(0, 0, 0, 0);
+        for (int i = 0; i < 4; ++i) res[i] = vs[i] ? __ldg(rr + res_offs[i]) : make_uint4(0, 0, 0, 0);
       };
       if constexpr (kRes) {
         const int d = r.da + (kGroups > 1 && turn != group ? 1 : 0);
@@ -561,11 +586,10 @@ __global__ void clip_pack_kernel(const __half* __restrict__ w, __half* __restric
     img[(size_t)((i >> 6) - r) * 64 + swizzled(r, k)] = used ? w[((size_t)(out * C + c) * 3 + kd) * 9 + fr * 3 + fs] : __ushort_as_half((unsigned short)0);
   }
 }
-// w [K][64 U][3][3]: row s * 64 + n is output channel n of the share with filter row 2 - s
-template <int U>
+// w [K][64 U][3][3]: row s * NC + n is output channel n of the share with filter row 2 - s
+template <class G>
 __global__ void conv1_pack_kernel(const __half* __restrict__ w, __half* __restrict__ img, int K) {
-  using G = Conv1<U>;
-  constexpr int NC = G::kNC, rows = 3 * NC;
+  constexpr int NC = G::kNC, rows = 3 * NC, U = G::kUnits;
   const int total = K / NC * G::kBlocks * rows * 64;
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < total; i += gridDim.x * blockDim.x) {
     const int k = i & 63, r = (i >> 6) % rows, b = (i >> 6) / rows % G::kBlocks, part = (i >> 6) / (rows * G::kBlocks);
@@ -573,7 +597,7 @@ __global__ void conv1_pack_kernel(const __half* __restrict__ w, __half* __restri
     img[(size_t)((i >> 6) - r) * 64 + swizzled(r, k)] = w[(size_t)(out * 64 * U + c) * 9 + (2 - r / NC) * 3 + b % 3];
   }
 }
-// w_main [K][C][4][4]: row s * 64 + n is output channel n of the share at block tap ty = 1 - s; w_short [K][C][2][2]
+// w_main [K][C][4][4]: row s * NC + n is output channel n of the share at block tap ty = 1 - s; w_short [K][C][2][2]
 template <class G>
 __global__ void down_pack_kernel(const __half* __restrict__ w_main, const __half* __restrict__ w_short, __half* __restrict__ img, int K) {
   constexpr int NC = G::kNC, C = std::is_same<G, Down32>::value ? 32 : 64, rows = G::kBlocks * 2 * NC + G::kShort * NC;  // of a share
@@ -630,7 +654,7 @@ int walk_layout(WalkParams& p) {   // fills in the patches' rows and buffers; th
 }
 
 // what walk_conv_kernel is instantiated for
-enum Variant { CLIP32, CLIP64, CONV64, CONV128, DOWN32, DOWN64 };
+enum Variant { CLIP32, CLIP64, CONV64, CONV128, CONV256, DOWN32, DOWN64 };
 template <class F>
 auto with_variant(Variant v, F&& f) {
   switch (v) {
@@ -638,6 +662,7 @@ auto with_variant(Variant v, F&& f) {
     case CLIP64: return f(Clip64());
     case CONV64: return f(Conv1<1>());
     case CONV128: return f(Conv1<2>());
+    case CONV256: return f(Conv256());
     case DOWN32: return f(Down32());
     default: return f(Down64());
   }
@@ -653,6 +678,7 @@ WalkParams clip_params(const ClipConvGeom& g) {
   p.Wb = clip_block_extent(g.W);
   p.img = clip_block_extent(g.H) * p.Wb;
   p.P = g.batch * p.img;
+  p.tile = 128;
   p.K = g.K;
   p.parts = g.K / (g.C == 32 ? Clip32::kNC : Clip64::kNC);
   const uint32_t k16 = (uint32_t)g.K / 8, Hb2 = clip_block_extent(p.Ho), Wb2 = clip_block_extent(p.Wo);
@@ -675,6 +701,8 @@ WalkParams res_params(const ResWalkGeom& g, bool down) {
   p.Wo = res_out_w(g);
   p.Wb = p.img = p.Wo + 1;         // blocks of an input row, or an image row with its zero column: as many
   p.P = g.batch * p.Wb;
+  p.tile = 128;
+  p.res_n = (uint32_t)p.Wb; p.res_step = (uint32_t)p.P;
   p.outs_per_tile = res_out_h(g);
   p.steps = down ? p.outs_per_tile + 1 : p.outs_per_tile;
   p.K = g.K;
@@ -695,6 +723,14 @@ WalkParams res_params(const ResWalkGeom& g, bool down) {
   return p;
 }
 Variant down_variant(const ResWalkGeom& g) { return g.C == 32 ? DOWN32 : DOWN64; }
+// k3 s1 p1 alone, h x w pixels
+WalkParams conv_params(const ConvWalkGeom& g) {
+  WalkParams p = res_params(ResWalkGeom{g.batch, 2 * g.h, 2 * g.w, 0, g.C, g.act, g.slope, g.out}, false);  // (a block of that output)
+  p.parts = g.C / Conv256::kNC;
+  p.tile = 128 / p.Wb * p.Wb;
+  p.res_step = (uint32_t)p.Wb; p.res_n = (uint32_t)((g.h + 1) * p.Wb);
+  return p;
+}
 Variant conv1_variant(const ResWalkGeom& g) { return g.K == 64 ? CONV64 : CONV128; }
 
 }  // namespace
@@ -722,7 +758,7 @@ static int walk_create(aig_ctx* ctx, Variant v, int in_c, const WalkParams& prm,
   c->prm = prm;
   WalkParams& p = c->prm;
   c->smem = variant_layout(v, p);
-  p.outs = ceil_div(p.P, 128) * p.outs_per_tile;
+  p.outs = ceil_div(p.P, p.tile) * p.outs_per_tile;
   p.ctas = ctx->sm_count / p.parts;
   if (p.ctas > p.outs) p.ctas = p.outs;
   const bool shortcut = v == DOWN32 || v == DOWN64;
@@ -775,8 +811,12 @@ static int walk_launch(WalkConv* c, const aig_half* x, const aig_half* residual,
       cuuint64_t strides[1] = {(cuuint64_t)c->in_c * 2};
       cuuint32_t box[2] = {64u, (cuuint32_t)p.unit_rows[u]};
       cuuint32_t es[2] = {1, 1};
-      const CUresult r = enc(&c->maps.u[u], CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, const_cast<aig_half*>(x), dims, strides, box, es, CU_TENSOR_MAP_INTERLEAVE_NONE,
-                             CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+      const cuuint64_t h1 = (cuuint64_t)p.steps + 1, w1 = (cuuint64_t)p.Wb;                     // images outermost: (channel, x, y, n)
+      cuuint64_t dims4[4] = {(cuuint64_t)c->in_c, w1, h1, (cuuint64_t)p.P / w1}, strides4[3] = {strides[0], strides[0] * w1, strides[0] * w1 * h1};
+      cuuint32_t box4[4] = {64u, (cuuint32_t)w1, 1, (cuuint32_t)(p.tile / p.Wb)}, es4[4] = {1, 1, 1, 1};
+      const bool images = c->variant == CONV256;
+      const CUresult r = enc(&c->maps.u[u], CU_TENSOR_MAP_DATA_TYPE_FLOAT16, images ? 4 : 2, const_cast<aig_half*>(x), images ? dims4 : dims,
+                             images ? strides4 : strides, images ? box4 : box, images ? es4 : es, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
       if (r != CUDA_SUCCESS) return aig_fail(ctx, AIG_ERR_CUDA, "cuTensorMapEncodeTiled(walking convolution) failed: %d", (int)r);
     }
     c->map_x = x;
@@ -853,8 +893,9 @@ int res_walk_set_down(WalkConv* c, const aig_half* w_main, const aig_half* b_mai
 }
 int res_walk_set_conv1(WalkConv* c, const aig_half* w, const aig_half* bias, const float* gamma, const float* beta, const float* mean, const float* var,
                        float eps) {
-  if (c->variant == CONV64) conv1_pack_kernel<1><<<128, 256, 0, c->ctx->stream>>>((const __half*)w, c->wimg, c->prm.K);
-  else conv1_pack_kernel<2><<<128, 256, 0, c->ctx->stream>>>((const __half*)w, c->wimg, c->prm.K);
+  if (c->variant == CONV64) conv1_pack_kernel<Conv1<1>><<<128, 256, 0, c->ctx->stream>>>((const __half*)w, c->wimg, c->prm.K);
+  else if (c->variant == CONV128) conv1_pack_kernel<Conv1<2>><<<128, 256, 0, c->ctx->stream>>>((const __half*)w, c->wimg, c->prm.K);
+  else conv1_pack_kernel<Conv256><<<256, 256, 0, c->ctx->stream>>>((const __half*)w, c->wimg, c->prm.K);
   AIG_LAUNCH_OK(c->ctx);
   c->weights_set = true;
   return walk_affine(c, 0, bias, gamma, beta, mean, var, eps);
@@ -866,6 +907,18 @@ int res_walk_down(WalkConv* down, const aig_half* x, aig_half* t, aig_half* r) {
 int res_walk_conv1(WalkConv* conv1, const aig_half* t, const aig_half* r, aig_half* y) {
   AIG_REQUIRE(conv1->ctx, r, "residual block by rows: null pointer");
   return walk_launch(conv1, t, r, y, nullptr);
+}
+bool conv_walk_supported(const aig_ctx* ctx, const ConvWalkGeom& g) {
+  if (g.C != 256 || g.batch <= 0 || g.h < 2 || g.w < 2 || g.w + 1 > 128) return false;
+  const long long rows = (long long)g.batch * (g.h + 1) * (g.w + 1);
+  if (!walk_counts_fit(rows, g.C, rows, 4 * g.C)) return false;
+  WalkParams p = conv_params(g);
+  return p.parts <= ctx->sm_count && variant_layout(CONV256, p) <= 227 * 1024;
+}
+int conv_walk_create(aig_ctx* ctx, const ConvWalkGeom& g, WalkConv** out) {
+  *out = nullptr;
+  if (!conv_walk_supported(ctx, g)) return aig_fail(ctx, AIG_ERR_UNSUPPORTED, "convolution by rows: unsupported geometry");
+  return walk_create(ctx, CONV256, g.C, conv_params(g), out);
 }
 int row_blocks_to_nhwc(aig_ctx* ctx, const aig_half* blocks, aig_half* y, int batch, int h, int w, int c) {
   DeviceGuard guard(ctx->device);

@@ -47,6 +47,16 @@ int res_walk_set_conv1(WalkConv* conv1, const aig_half* w, const aig_half* bias,
                        float eps);
 int res_walk_down(WalkConv* down, const aig_half* x, aig_half* t, aig_half* r);
 int res_walk_conv1(WalkConv* conv1, const aig_half* t, const aig_half* r, aig_half* y);
+
+// ---- its 3x3 convolution alone, 256 channels, on the padded position layout [n][h+1][w+1][256]; weights and forward as of conv1
+struct ConvWalkGeom {
+  int batch, h, w, C;
+  int act;
+  float slope;
+  ResWalkOut out;      // channels-last or blocks [n][yb][xb]
+};
+bool conv_walk_supported(const aig_ctx* ctx, const ConvWalkGeom& g);
+int conv_walk_create(aig_ctx* ctx, const ConvWalkGeom& g, WalkConv** out);
 int row_blocks_to_nhwc(aig_ctx* ctx, const aig_half* blocks, aig_half* y, int batch, int h, int w, int c);
 
 // ---- the first layer's output in the layouts above; false: its kernels cannot

@@ -68,7 +68,8 @@ struct aig_cnn {
     aig_conv_plan* down = nullptr;  // main k4 s2 + shortcut k2 s2 as one launch over the space-to-depth input (replaces c0 and sc)
     aig_half *t = nullptr, *r = nullptr, *y = nullptr;
     size_t t_elems = 0;             // of t and of r
-    WalkConv *walk_down = nullptr, *walk_c1 = nullptr;  // the block by rows (replaces down and c1)
+    WalkConv *walk_down = nullptr, *walk_c1 = nullptr;  // the block, or its second convolution alone, by rows (replaces down and c1)
+    bool padded = false;            // t and r in the padded position layout
     bool y_s2d = false;             // y is written in the space-to-depth layout the next block's fused launch reads
     bool y_rows = false;            // and with the block rows outermost
   };
@@ -189,8 +190,17 @@ static int cnn_use_row_walk(aig_cnn* m) {
   };
   int n = 0;
   while (n < c.n_blocks && m->blocks[n].down && res_walk_supported(m->ctx, geom(n))) ++n;
-  if (n == 0 || !conv0_plan_set_output_row_blocks(m->conv0)) return AIG_OK;
-  m->act0_rows = true;
+  if (n > 0 && !conv0_plan_set_output_row_blocks(m->conv0)) n = 0;
+  for (int i = n; i < c.n_blocks; ++i) {  // of the blocks after those the second convolution
+    aig_cnn::Block& b = m->blocks[i];
+    const ConvWalkGeom g{c.batch, m->bh[i], m->bw[i], c.widths[i + 1], c.act, c.slope, b.y_s2d ? RES_OUT_BLOCKS : RES_OUT_NHWC};
+    if (!b.padded || !conv_walk_supported(m->ctx, g)) continue;
+    const int rc = conv_walk_create(m->ctx, g, &b.walk_c1);
+    if (rc != AIG_OK) return rc;
+    aig_conv_plan_destroy(b.c1);
+    b.c1 = nullptr;
+  }
+  m->act0_rows = n > 0;
   for (int i = 0; i < n; ++i) {
     aig_cnn::Block& b = m->blocks[i];
     ResWalkGeom g = geom(i);
@@ -302,7 +312,7 @@ int aig_cnn_create(aig_ctx* ctx, const aig_cnn_config* cfg, aig_cnn** out) {
     // fused down-sampling launch -> 3x3 convolution: the pair passes both tensors (conv1's input and residual) in the
     // padded position layout when both plans take it, so that conv1 loads each patch as one contiguous run of rows
     if (b.down && aig_resdown_plan_set_output_padded(b.down, 1) == AIG_OK) {
-      if (aig_conv_plan_set_input_padded(b.c1, 1) == AIG_OK) n = (size_t)aig_conv_padded_rows(c.batch, oh, ow, 1) * co;
+      if (aig_conv_plan_set_input_padded(b.c1, 1) == AIG_OK) n = (size_t)aig_conv_padded_rows(c.batch, oh, ow, 1) * co, b.padded = true;
       else aig_resdown_plan_set_output_padded(b.down, 0);
     }
     b.t_elems = n;
@@ -469,7 +479,8 @@ int aig_cnn_load_memory(aig_cnn* m, const void* blob, size_t bytes) {
       CNN_OK(m, aig_conv_plan_set_weights(m->blocks[i].c0, c0.w, c0.b, b0.a[0], b0.a[1], b0.a[2], b0.a[3], eps));
       CNN_OK(m, aig_conv_plan_set_weights(m->blocks[i].sc, sc.w, sc.b, nullptr, nullptr, nullptr, nullptr, 0.f));
     }
-    CNN_OK(m, aig_conv_plan_set_weights(m->blocks[i].c1, c1.w, c1.b, b1.a[0], b1.a[1], b1.a[2], b1.a[3], eps));
+    if (m->blocks[i].walk_c1) CNN_OK(m, res_walk_set_conv1(m->blocks[i].walk_c1, c1.w, c1.b, b1.a[0], b1.a[1], b1.a[2], b1.a[3], eps));
+    else CNN_OK(m, aig_conv_plan_set_weights(m->blocks[i].c1, c1.w, c1.b, b1.a[0], b1.a[1], b1.a[2], b1.a[3], eps));
   }
   const int cl = c.widths[c.n_blocks];
   m->sa_w = (aig_half*)m->params.take((size_t)cl * 2);
@@ -543,7 +554,8 @@ static int cnn_forward_impl(aig_cnn* m, const uint8_t* bgra_dev, bool planar) {
       CNN_OK(m, aig_conv_forward(b.c0, x, nullptr, b.t));
       tick();
     }
-    CNN_OK(m, aig_conv_forward(b.c1, b.t, b.r, b.y));
+    if (b.walk_c1) CNN_OK(m, res_walk_conv1(b.walk_c1, b.t, b.r, b.y));
+    else CNN_OK(m, aig_conv_forward(b.c1, b.t, b.r, b.y));
     tick();
     x = b.y;
   }

@@ -378,6 +378,9 @@ def test_checkpoint_files(env, tmp_path):
     (37, 67, 131, (32, 64, 128, 256), "ACT_LEAKY"),   # odd extents, a block by rows before one by patches
     (5, 50, 322, (32, 64, 192), "ACT_SWISH"),         # rows beyond 256 pixels; one block by rows
     (150, 20, 20, (32, 64), "ACT_NONE"),              # the last block by rows
+    (11, 90, 131, (32, 64, 128, 256, 256), "ACT_SWISH"),  # 256 channels: whole image rows in a tile, the last one ragged
+    (40, 34, 36, (64, 256), "ACT_RELU"),              # and into the head directly
+    (3, 40, 262, (32, 256, 256), "ACT_LEAKY"),        # and a block of them before a block by patches, long rows
 ])
 def test_residual_blocks_by_rows(env, monkeypatch, B, H, W, widths, act):
     """The row-walking residual blocks at the edges of their tiles and runs, every stage against the oracle on a sample."""
