@@ -134,7 +134,7 @@ struct StepCta {
     const int nkb = (K + 31) >> 5, stride = row_stride(K);
     const uint8_t* a0 = a + g * stride + q * 16;
     const uint8_t* a1 = a0 + 8 * stride;
-    constexpr int U = 8;  // blocks in flight
+    constexpr int U = 4;  // blocks in flight
     float acc[TPW][4];
     const __half* xr[TPW];
     bool on[TPW];
@@ -340,12 +340,15 @@ __global__ void __launch_bounds__(kThreads, 1) seq_step_kernel(const StepParams 
   }
   // a K that is an odd multiple of 16 leaves half a block per row: zero, not whatever was there
   if (p.in_c % 32 != 0)
+#pragma unroll 1
     for (int i = tid; i < kRows * 8; i += kThreads)
       *reinterpret_cast<uint32_t*>(sm + p.o_w[0] + (i >> 3) * row_stride(p.in_c) + p.in_c * 2 + (i & 7) * 4) = 0u;
   if (n_bridge && p.feat % 32 != 0)
+#pragma unroll 1
     for (int i = tid; i < n_bridge * 8; i += kThreads)
       *reinterpret_cast<uint32_t*>(sm + p.o_bridge + (i >> 3) * row_stride(p.feat) + p.feat * 2 + (i & 7) * 4) = 0u;
   float* s_bias = reinterpret_cast<float*>(sm + p.o_bias);  // [L][16]
+#pragma unroll 1
   for (int i = tid; i < L * kRows; i += kThreads) {
     const int l = i / kRows, r = i % kRows;
     const size_t at = (size_t)(r >> 2) * H + unit0 + (r & 3);
@@ -358,6 +361,7 @@ __global__ void __launch_bounds__(kThreads, 1) seq_step_kernel(const StepParams 
   const int position = (int)p.words[kPosition], n_valid = min(position + 1, p.window);
   float* s_cell = reinterpret_cast<float*>(sm + p.o_cell);    // [L][B][4]
   __half* s_hid = reinterpret_cast<__half*>(sm + p.o_hid);    // [L][B][4], this step's
+#pragma unroll 1
   for (int i = tid; i < L * B * kUnits; i += kThreads) {
     const int l = i / (B * kUnits), b = i / kUnits % B, u = i % kUnits;
     s_cell[i] = __half2float(p.c_state[((size_t)l * B + b) * H + unit0 + u]);
@@ -371,6 +375,7 @@ __global__ void __launch_bounds__(kThreads, 1) seq_step_kernel(const StepParams 
   const bool item_per_cta = B * p.heads <= (int)gridDim.x;
   for (int item = item_per_cta ? blockIdx.x : blockIdx.x * kWarps + warp; item < B * p.heads; item += item_per_cta ? gridDim.x : gridDim.x * kWarps) {
     const size_t ring = (size_t)(item / p.heads) * p.window * H + (size_t)(item % p.heads) * kHeadDim;
+#pragma unroll 1
     for (int i = item_per_cta ? tid : lane; i < n_valid; i += item_per_cta ? kThreads : 32) {
       prefetch_l2(p.kcache + ring + (size_t)i * H);
       prefetch_l2(p.vcache + ring + (size_t)i * H);
@@ -380,110 +385,142 @@ __global__ void __launch_bounds__(kThreads, 1) seq_step_kernel(const StepParams 
   StepCta c{p, sm, bars, &s_abort, &s_flag, p.words + (epoch & 1u), 0u};
   float* s_pre = reinterpret_cast<float*>(sm + p.o_pre);      // [L][16][nt*8]: R.h
   const int pre_n = p.nt * 8;
-  bool ok = c.weights(0);
-  for (int l = 0; l < L && ok; ++l) {
-    c.template multiply<TPW>(sm + p.o_r[l], p.h_state + (size_t)l * B * H, H, H);
-    for (int i = tid; i < kRows * B; i += kThreads) s_pre[((size_t)l * kRows + i / B) * pre_n + i % B] = c.value(i / B, i % B);
-    __syncthreads();
-  }
-  griddep_wait();
-  // Two counters alternate between launches: each launch clears the one that its successor will use, whose last user,
-  // the launch before this one, has finished; so a launch starts from zero even after one that gave up on a barrier.
-  if (blockIdx.x == 0 && tid == 0) p.words[(epoch + 1u) & 1u] = 0u;
-
-  // ---- bridge FC: features -> embedding, rounded before and after the bias
-  if (p.features && ok) {
-    ok = c.weights(b_bridge);
-    for (int r0 = 0; r0 < n_bridge && ok; r0 += kRows) {
-      c.template multiply<TPW>(sm + p.o_bridge + r0 * row_stride(p.feat), p.features, p.feat, p.feat);
-      const int n = min(kRows, n_bridge - r0);
+  // ---- the products, one after another through the same code: the kernel runs once through everything else it has, and its
+  // time at few sequences is that of fetching instructions.  With a copy of the product per stage, eight blocks in flight and
+  // unrolled loops around it a frame of one player took 112 us, a step of 6 sequences 94.7, of 128 292; now 107, 92.8 and 281.
+  enum { kPre, kBridge, kLayer, kQkv, kOut };
+  const int bridge_tiles = p.features ? (p.bridge_rows + kRows - 1) / kRows : 0;
+  auto after_predecessor = [&]() {
+    griddep_wait();
+    // Two counters alternate between launches: each launch clears the one that its successor will use, whose last user,
+    // the launch before this one, has finished; so a launch starts from zero even after one that gave up on a barrier.
+    if (blockIdx.x == 0 && tid == 0) p.words[(epoch + 1u) & 1u] = 0u;
+  };
+  bool ok = true, waited = false;
+#pragma unroll 1
+  for (int st = 0; ok; ++st) {
+    int kind = kPre, l = st, wait = 0, K = H, stride = H;
+    const uint8_t* a = sm + p.o_r[st < L ? st : 0];
+    const __half* x = p.h_state + (size_t)st * B * H;           // R.h of every layer needs the step before only
+    if (st >= L) {
+      if (!waited) after_predecessor();
+      waited = true;
+      l = st - L;                                               // bridge FC's tile of rows
+      kind = kBridge;
+      wait = b_bridge;
+      a = sm + p.o_bridge + l * kRows * row_stride(p.feat);
+      x = p.features;
+      K = stride = p.feat;
+      if (l >= bridge_tiles) {
+        l -= bridge_tiles;                                      // LSTM layer
+        kind = kLayer;
+        wait = 2 + l;
+        a = sm + p.o_w[l < L ? l : 0];
+        x = p.h_new + (size_t)(l - 1) * B * H;
+        K = stride = H;
+        if (l == 0) {
+          x = p.features ? p.emb_out : p.emb;
+          K = stride = p.in_c;
+        } else if (l == L) {
+          kind = kQkv;
+          wait = b_qkv;
+          a = sm + p.o_qkv;
+        } else if (l > L) {
+          kind = kOut;
+          wait = b_wo;
+          a = sm + p.o_wo;
+          x = p.ctx;
+        }
+      }
+    }
+    ok = c.weights(wait);
+    if (!ok) break;
+    if (kind != kBridge || l * kRows < n_bridge) c.template multiply<TPW>(a, x, stride, K);
+    if (kind == kPre) {
+#pragma unroll 1
+      for (int i = tid; i < kRows * B; i += kThreads) s_pre[((size_t)l * kRows + i / B) * pre_n + i % B] = c.value(i / B, i % B);
+      __syncthreads();
+    } else if (kind == kBridge) {
+      // features -> embedding, rounded before and after the bias
+      const int n = min(kRows, n_bridge - l * kRows);
+#pragma unroll 1
       for (int i = tid; i < n * B; i += kThreads) {
-        const int r = i % n, b = i / n, o = bridge0 + r0 + r;
+        const int r = i % n, b = i / n, o = bridge0 + l * kRows + r;
         const float t = __half2float(__float2half(c.value(r, b)));
         p.emb_out[(size_t)b * p.in_c + o] = __float2half(t + __half2float(p.bb[o]));
       }
-      __syncthreads();
-    }
-    ok = ok && c.barrier(701);
-  }
-
-  // ---- LSTM layers
-  for (int l = 0; l < L && ok; ++l) {
-    ok = c.weights(2 + l);
-    if (!ok) break;
-    if (l == 0) c.template multiply<TPW>(sm + p.o_w[0], p.features ? p.emb_out : p.emb, p.in_c, p.in_c);
-    else c.template multiply<TPW>(sm + p.o_w[l], p.h_new + (size_t)(l - 1) * B * H, H, H);
-    // a lane per gate, four lanes per (unit, sequence)
-    for (int i = tid; i < (B * kRows + 31) / 32 * 32; i += kThreads) {
-      const int g = i & 3, cell = i >> 2, u = cell & 3, b = cell >> 2, r = g * kUnits + u;
-      const bool on = b < B;
-      float act = 0.f;
-      if (on) {
-        const float pre = s_pre[((size_t)l * kRows + r) * pre_n + b] + (c.value(r, b) + s_bias[l * kRows + r]);
-        act = sigmoidf_(g == 2 ? 2.0f * pre : pre);
-        if (g == 2) act = 2.0f * act - 1.0f;
-      }
-      const float fg = __shfl_down_sync(0xffffffffu, act, 1), gg = __shfl_down_sync(0xffffffffu, act, 2), og = __shfl_down_sync(0xffffffffu, act, 3);
-      if (on && g == 0) {
-        float cn = fg * s_cell[l * B * kUnits + cell] + act * gg;
-        if (p.clip > 0.f) cn = fminf(p.clip, fmaxf(-p.clip, cn));
-        const __half ch = __float2half(cn), hn = __float2half(og * tanhf(__half2float(ch)));
-        const size_t si = ((size_t)l * B + b) * H + unit0 + u;
-        p.c_state[si] = ch;
-        p.h_new[si] = hn;
-        s_hid[l * B * kUnits + cell] = hn;
-        if (l == L - 1) p.y[(size_t)b * H + unit0 + u] = hn;
-      }
-    }
-    ok = c.barrier(702 + l);
-  }
-
-  // ---- q, k, v
-  if (ok && (ok = c.weights(b_qkv))) {
-    c.template multiply<TPW>(sm + p.o_qkv, p.h_new + (size_t)(L - 1) * B * H, H, H);
-    for (int i = tid; i < 3 * B * kUnits; i += kThreads) {
-      const int m = i / (B * kUnits), b = i / kUnits % B, u = i % kUnits;
-      (m == 0 ? p.q : (m == 1 ? p.k : p.v))[(size_t)b * H + unit0 + u] = __float2half(c.value(m * kUnits + u, b));
-    }
-    // every CTA has read the previous hidden state by now: publish the new one
-    for (int i = tid; i < L * B * kUnits; i += kThreads) {
-      const int l = i / (B * kUnits), b = i / kUnits % B, u = i % kUnits;
-      p.h_state[((size_t)l * B + b) * H + unit0 + u] = s_hid[i];
-    }
-    ok = c.barrier(707);
-  }
-  // ---- attention
-  if (ok) {
-    // an item per warp, or per CTA where every item can have one of its own
-    float* sq = reinterpret_cast<float*>(sm + p.o_attn) + warp * kAttnFloats;
-    const int items = B * p.heads;
-    if (!item_per_cta) {
-      for (int item = blockIdx.x * kWarps + warp; item < items; item += gridDim.x * kWarps)
-        attend(p, item, position, n_valid, cs, sn, sq, nullptr, 1, 0, lane);
-    } else if ((int)blockIdx.x < items) {
-      float* part = sq + 2 * kHeadDim;
-      attend(p, blockIdx.x, position, n_valid, cs, sn, sq, part, kWarps, warp, lane);
-      __syncthreads();
-      if (tid < kHeadDim) {
-        const float* all = reinterpret_cast<float*>(sm + p.o_attn) + 2 * kHeadDim;
-        float mx = -INFINITY, sum = 0.f, acc = 0.f;
-        for (int w = 0; w < kWarps; ++w) mx = fmaxf(mx, all[w * kAttnFloats + kHeadDim]);
-        for (int w = 0; w < kWarps; ++w) {
-          const float f = expf(all[w * kAttnFloats + kHeadDim] - mx);  // (0 for a warp without a share)
-          sum = fmaf(f, all[w * kAttnFloats + kHeadDim + 1], sum);
-          acc = fmaf(f, all[w * kAttnFloats + tid], acc);
+      if (l + 1 < bridge_tiles) __syncthreads();
+      else ok = c.barrier(701);
+    } else if (kind == kLayer) {
+      // a lane per gate, four lanes per (unit, sequence)
+#pragma unroll 1
+      for (int i = tid; i < (B * kRows + 31) / 32 * 32; i += kThreads) {
+        const int g = i & 3, cell = i >> 2, u = cell & 3, b = cell >> 2, r = g * kUnits + u;
+        const bool on = b < B;
+        float act = 0.f;
+        if (on) {
+          const float pre = s_pre[((size_t)l * kRows + r) * pre_n + b] + (c.value(r, b) + s_bias[l * kRows + r]);
+          act = sigmoidf_(g == 2 ? 2.0f * pre : pre);
+          if (g == 2) act = 2.0f * act - 1.0f;
         }
-        p.ctx[(size_t)(blockIdx.x / p.heads) * H + (size_t)(blockIdx.x % p.heads) * kHeadDim + tid] = __float2half(acc / sum);
+        const float fg = __shfl_down_sync(0xffffffffu, act, 1), gg = __shfl_down_sync(0xffffffffu, act, 2), og = __shfl_down_sync(0xffffffffu, act, 3);
+        if (on && g == 0) {
+          float cn = fg * s_cell[l * B * kUnits + cell] + act * gg;
+          if (p.clip > 0.f) cn = fminf(p.clip, fmaxf(-p.clip, cn));
+          const __half ch = __float2half(cn), hn = __float2half(og * tanhf(__half2float(ch)));
+          const size_t si = ((size_t)l * B + b) * H + unit0 + u;
+          p.c_state[si] = ch;
+          p.h_new[si] = hn;
+          s_hid[l * B * kUnits + cell] = hn;
+          if (l == L - 1) p.y[(size_t)b * H + unit0 + u] = hn;
+        }
       }
+      ok = c.barrier(702 + l);
+    } else if (kind == kQkv) {
+#pragma unroll 1
+      for (int i = tid; i < 3 * B * kUnits; i += kThreads) {
+        const int m = i / (B * kUnits), b = i / kUnits % B, u = i % kUnits;
+        (m == 0 ? p.q : (m == 1 ? p.k : p.v))[(size_t)b * H + unit0 + u] = __float2half(c.value(m * kUnits + u, b));
+      }
+      // every CTA has read the previous hidden state by now: publish the new one
+#pragma unroll 1
+      for (int i = tid; i < L * B * kUnits; i += kThreads) {
+        const int k = i / (B * kUnits), b = i / kUnits % B, u = i % kUnits;
+        p.h_state[((size_t)k * B + b) * H + unit0 + u] = s_hid[i];
+      }
+      ok = c.barrier(707);
+      if (!ok) break;
+      // ---- attention: an item per warp, or per CTA where every item can have one of its own
+      float* sq = reinterpret_cast<float*>(sm + p.o_attn) + warp * kAttnFloats;
+      const int items = B * p.heads, first = item_per_cta ? blockIdx.x : blockIdx.x * kWarps + warp, step = item_per_cta ? items : gridDim.x * kWarps;
+#pragma unroll 1
+      for (int item = first; item < items; item += step)
+        attend(p, item, position, n_valid, cs, sn, sq, sq + 2 * kHeadDim, item_per_cta ? kWarps : 1, item_per_cta ? warp : 0, lane);
+      if (item_per_cta && (int)blockIdx.x < items) {
+        __syncthreads();
+        if (tid < kHeadDim) {
+          const float* all = reinterpret_cast<float*>(sm + p.o_attn) + 2 * kHeadDim;
+          float mx = -INFINITY, sum = 0.f, acc = 0.f;
+#pragma unroll 1
+          for (int w = 0; w < kWarps; ++w) mx = fmaxf(mx, all[w * kAttnFloats + kHeadDim]);
+#pragma unroll 1
+          for (int w = 0; w < kWarps; ++w) {
+            const float f = expf(all[w * kAttnFloats + kHeadDim] - mx);  // (0 for a warp without a share)
+            sum = fmaf(f, all[w * kAttnFloats + kHeadDim + 1], sum);
+            acc = fmaf(f, all[w * kAttnFloats + tid], acc);
+          }
+          p.ctx[(size_t)(blockIdx.x / p.heads) * H + (size_t)(blockIdx.x % p.heads) * kHeadDim + tid] = __float2half(acc / sum);
+        }
+      }
+      ok = c.barrier(708);
+    } else {
+#pragma unroll 1
+      for (int i = tid; i < B * kUnits; i += kThreads) p.a[(size_t)(i / kUnits) * H + unit0 + i % kUnits] = __float2half(c.value(i % kUnits, i / kUnits));
+      ok = c.barrier(709);
+      break;
     }
-    ok = c.barrier(708);
   }
-  // ---- output projection
-  if (ok && (ok = c.weights(b_wo))) {
-    c.template multiply<TPW>(sm + p.o_wo, p.ctx, H, H);
-    for (int i = tid; i < B * kUnits; i += kThreads) p.a[(size_t)(i / kUnits) * H + unit0 + i % kUnits] = __float2half(c.value(i % kUnits, i / kUnits));
-    ok = c.barrier(709);
-  }
+  if (!waited) after_predecessor();                             // (gave up before)
   // ---- per sequence: row LayerNorm (eps 1e-5; every warp for itself), FC with the two-step rounding, sigmoid / tanh
   if (ok && (ok = c.weights(b_fc))) {
     constexpr int kPairs = 512 / 64;  // half2 a lane holds at most
