@@ -22,7 +22,7 @@
 // instead of four for 64 channels: 3340 -> 2660 clk a plane (a patch takes over 2000 clk to come).
 // Frames: the 64-channel block is bound by memory (256 frames of 144x256: 302 and 226 MB, 46 and 35 us at the copy bandwidth),
 // the 128-channel one by the products (3690 and 2410 clk a row of a tile).  By the patch-resident kernels, 256 frames: 89, 75,
-// 65 and 57 us; now 51, 44, 45 and 37 (start to start of the launches).  That kernel multiplies 64 columns at a time, reads a
+// 65 and 57 us; now 51, 44, 45 and 37 (start to start of the launches); the 256-channel 3x3 convolutions 52 and 27, now 46 and 18.  That kernel multiplies 64 columns at a time, reads a
 // patch's halo rows again for every tile and, with 128 channels, streams the weights.
 #include "walk_conv.h"
 

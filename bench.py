@@ -386,7 +386,7 @@ def leg_cnn2d(env, full):
         if all(r[0] in tj for r in gemm):
             traffic = sum(tj[r[0]] for r in gemm)
     whole = FLOP_PER_FRAME * B / (ms * 1e-3) / 1e12
-    roof = {"bound": "tensor", "kernel": "pconv_kernel (tcgen05 convolution GEMM), %d launches per step, %.0f%% of the step" % (
+    roof = {"bound": "tensor", "kernel": "walk_conv_kernel and pconv_kernel (tcgen05 convolutions), %d launches per step, %.0f%% of the step" % (
                 len(gemm), 100.0 * g_ms / sum(r[1] for r in sites)),
             **fracs(achieved, env.peaks), "traffic": traffic,
             "timed_with": "one CUDA event between launches over %d steps of the same loop (%.4f ms/step with the events)" % (prof_steps, prof_ms),
