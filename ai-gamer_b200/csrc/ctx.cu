@@ -61,7 +61,7 @@ int aig_ctx_create(aig_ctx** out, int device) {
   if (cudaStreamCreateWithFlags(&ctx->stream, cudaStreamNonBlocking) != cudaSuccess ||
       cudaMalloc(&ctx->d_err, sizeof(int)) != cudaSuccess ||
       cudaMallocHost(&ctx->h_err, sizeof(int)) != cudaSuccess ||
-      cudaMemset(ctx->d_err, 0, sizeof(int)) != cudaSuccess) {
+      cudaMemsetAsync(ctx->d_err, 0, sizeof(int), ctx->stream) != cudaSuccess) {
     g_noctx_error = "context allocation failed";
     delete ctx;
     return AIG_ERR_CUDA;

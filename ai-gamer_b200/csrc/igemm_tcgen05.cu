@@ -2089,8 +2089,10 @@ bool pconv_choose_tile(aig_ctx* ctx, aig_conv_plan* pl, const PconvNtOption* opt
     }
     tab[G] = off;
     for (int c = 0; c < G; ++c) tab.insert(tab.end(), lists[c].begin(), lists[c].end());
-    if (cudaMalloc(&pl->pc_sched, tab.size() * sizeof(int)) != cudaSuccess) return false;
-    cudaMemcpy(pl->pc_sched, tab.data(), tab.size() * sizeof(int), cudaMemcpyHostToDevice);
+    // (copied in the order of the context's stream; from pageable memory, which has been read when the call returns)
+    if (cudaMalloc(&pl->pc_sched, tab.size() * sizeof(int)) != cudaSuccess ||
+        cudaMemcpyAsync(pl->pc_sched, tab.data(), tab.size() * sizeof(int), cudaMemcpyHostToDevice, ctx->stream) != cudaSuccess)
+      return false;
     q.sched = pl->pc_sched;
   }
   return true;
@@ -2131,7 +2133,7 @@ int pconv_build_tables(aig_ctx* ctx, aig_conv_plan* pl) {
   cudaFree(pl->pc_tab);
   pl->pc_tab = nullptr;
   AIG_CUDA_OK(ctx, cudaMalloc(&pl->pc_tab, tab.size() * sizeof(uint32_t)));
-  AIG_CUDA_OK(ctx, cudaMemcpy(pl->pc_tab, tab.data(), tab.size() * sizeof(uint32_t), cudaMemcpyHostToDevice));
+  AIG_CUDA_OK(ctx, cudaMemcpyAsync(pl->pc_tab, tab.data(), tab.size() * sizeof(uint32_t), cudaMemcpyHostToDevice, ctx->stream));
   q.tab = pl->pc_tab;
   q.tab_words = (int)tab.size();
   q.dbg = 0;
@@ -2275,7 +2277,7 @@ int pconv_try_plain(aig_ctx* ctx, aig_conv_plan* pl) {
   const char* ts = getenv("AIG_PCONV_TS");
   if (ts && atoi(ts)) {
     AIG_CUDA_OK(ctx, cudaMalloc(&q.ts, 128 * sizeof(long long)));
-    AIG_CUDA_OK(ctx, cudaMemset(q.ts, 0, 128 * sizeof(long long)));
+    AIG_CUDA_OK(ctx, cudaMemsetAsync(q.ts, 0, 128 * sizeof(long long), ctx->stream));
   }
 #endif
   pl->use_pconv = true;
@@ -2344,8 +2346,8 @@ int aig_conv_plan_destroy(aig_conv_plan* pl) {
 // stamps per tile, 16 tiles) and the tile shape into out[0..135].
 int aig_conv_plan_debug_timeline(aig_conv_plan* pl, long long* out) {
   if (!pl || !out || !pl->use_pconv || !pl->pp.ts) return AIG_ERR_INVALID;
+  cudaMemcpyAsync(out, pl->pp.ts, 128 * sizeof(long long), cudaMemcpyDeviceToHost, pl->ctx->stream);
   cudaStreamSynchronize(pl->ctx->stream);
-  cudaMemcpy(out, pl->pp.ts, 128 * sizeof(long long), cudaMemcpyDeviceToHost);
   out[128] = pl->pc_NT; out[129] = pl->pc_MS; out[130] = pl->pc_wres ? -1 : pl->pp.w_stages; out[131] = pl->pp.m_tiles;
   out[132] = pl->pp.patch_bufs; out[133] = pl->pp.G; out[134] = pl->pp.acc_bufs; out[135] = 0;
   return AIG_OK;
@@ -2674,7 +2676,7 @@ int aig_resdown_plan_create(aig_ctx* ctx, int batch, int in_c, int in_h, int in_
   if (n_opts == 0 || !pconv_choose_tile(ctx, pl, opts, n_opts, 2)) return bail(aig_fail(ctx, AIG_ERR_UNSUPPORTED, "resdown plan: no tile fits shared memory"));
 #ifdef AIG_TUNING
   if (const char* ts = getenv("AIG_PCONV_TS")) {
-    if (atoi(ts) && cudaMalloc(&q.ts, 128 * sizeof(long long)) == cudaSuccess) cudaMemset(q.ts, 0, 128 * sizeof(long long));
+    if (atoi(ts) && cudaMalloc(&q.ts, 128 * sizeof(long long)) == cudaSuccess) cudaMemsetAsync(q.ts, 0, 128 * sizeof(long long), ctx->stream);
   }
 #endif
   pl->pc_in_h = Hb; pl->pc_in_w = Wb; pl->pc_in_c = C4;

@@ -133,10 +133,11 @@ int fail(aig_cnn* m, int code, const std::string& msg) {
     if (e__ != cudaSuccess) return fail((m), AIG_ERR_CUDA, std::string(#expr ": ") + cudaGetErrorString(e__)); \
   } while (0)
 
+// Zeroed in the order of the context's stream: that one does not wait for the legacy stream, where cudaMemset would run.
 template <class T>
 int dev_alloc(aig_cnn* m, T** p, size_t count) {
   CNN_CUDA(m, cudaMalloc(reinterpret_cast<void**>(p), count * sizeof(T)));
-  CNN_CUDA(m, cudaMemset(*p, 0, count * sizeof(T)));
+  CNN_CUDA(m, cudaMemsetAsync(*p, 0, count * sizeof(T), (cudaStream_t)aig_ctx_stream(m->ctx)));
   return AIG_OK;
 }
 

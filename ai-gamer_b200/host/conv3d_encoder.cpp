@@ -94,7 +94,7 @@ int aig_c3d_create(aig_ctx* ctx, const aig_c3d_config* cfg, aig_c3d** out) {
     }
     aig_half* buf = nullptr;
     const size_t bytes = 2 * (i < n_walk ? clip_block_elems(c.batch, D, H, W, c.widths[i + 1]) : (size_t)c.batch * D * H * W * c.widths[i + 1]);
-    if (cudaMalloc(reinterpret_cast<void**>(&buf), bytes) != cudaSuccess || (i < n_walk && cudaMemset(buf, 0, bytes) != cudaSuccess)) rc = AIG_ERR_CUDA;
+    if (cudaMalloc(reinterpret_cast<void**>(&buf), bytes) != cudaSuccess || (i < n_walk && cudaMemsetAsync(buf, 0, bytes, (cudaStream_t)aig_ctx_stream(ctx)) != cudaSuccess)) rc = AIG_ERR_CUDA;
     m->acts.push_back(buf);
     m->d.push_back(D); m->h.push_back(H); m->w.push_back(W);
   }

@@ -85,12 +85,13 @@ int seq_create_with_bridge(aig_ctx* ctx, const aig_seq_config* cfg, int features
   if (rc == AIG_OK && !fused) rc = aig_fc_plan_create(ctx, c.batch, c.hidden, c.n_out, AIG_ACT_NONE, 0.f, 1, &m->fc_step);
   const size_t rows = (size_t)c.batch * c.seq_len, E = c.hidden;
   const size_t state = (size_t)c.layers * c.batch * E;
+  const cudaStream_t s = (cudaStream_t)aig_ctx_stream(ctx);
   if (rc == AIG_OK &&
       (cudaMalloc(&m->y, rows * E * 2) != cudaSuccess || cudaMalloc(&m->a, rows * E * 2) != cudaSuccess ||
        cudaMalloc(&m->n, rows * E * 2) != cudaSuccess || cudaMalloc(&m->logits, rows * c.n_out * 2) != cudaSuccess ||
        cudaMalloc(&m->out_f32, rows * c.n_out * 4) != cudaSuccess || cudaMalloc(&m->h_state, state * 2) != cudaSuccess ||
-       cudaMalloc(&m->c_state, state * 2) != cudaSuccess || cudaMemset(m->h_state, 0, state * 2) != cudaSuccess ||
-       cudaMemset(m->c_state, 0, state * 2) != cudaSuccess ||
+       cudaMalloc(&m->c_state, state * 2) != cudaSuccess || cudaMemsetAsync(m->h_state, 0, state * 2, s) != cudaSuccess ||
+       cudaMemsetAsync(m->c_state, 0, state * 2, s) != cudaSuccess ||
        cudaMalloc(&m->params, aig_seq_param_bytes(&c) + 16 * 256) != cudaSuccess ||
        cudaMalloc(&m->fcw_t, E * c.n_out * 2) != cudaSuccess))
     rc = AIG_ERR_CUDA;
