@@ -630,6 +630,11 @@ int launch_pair(aig_ctx* ctx, const LstmLaunch& l, LstmPairParams& pp) {
   AIG_CUDA_OK(ctx, cudaLaunchKernelEx(&cfg, lstm_pair_kernel<GA, GB>, pp));
   return AIG_OK;
 }
+// sum of a layer's biases, for a second layer (it has no projection to add them)
+__global__ void bias_sum_kernel(float* out, const __half* bw, const __half* br, int n) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i < n) out[i] = __half2float(bw[i]) + (br ? __half2float(br[i]) : 0.f);
+}
 int run_pair(aig_ctx* ctx, const LstmLaunch& l, LstmPairParams pp) {
   pp.a.ctas = pp.b.ctas = l.ctas;
   pp.a.gerr = pp.b.gerr = ctx->d_err;
@@ -647,11 +652,13 @@ struct aig_lstm_plan {
   LstmLaunch shape;
   const __half* blob = nullptr;
   std::vector<size_t> w_off, r_off, bw_off, br_off;
-  std::vector<aig_conv_plan*> proj;     // hoisted input projection per layer
+  std::vector<aig_conv_plan*> proj;     // hoisted input projection per layer; none of a pair's second layer
   float* gx = nullptr;                  // [T*B][4H] fp32 scratch
-  __half* mid = nullptr;                // intermediate layer outputs (same layout as y)
+  __half* mid = nullptr;                // outputs that a further layer or pair reads (same layout as y); null: there is none
   __half* xs = nullptr;                 // layers in pairs: the first one's outputs as the second one's operands
   unsigned int* counters = nullptr;     // and how far they are
+  float* pair_bias = nullptr;           // per pair the second layer's [4H]
+  bool second(int l) const { return shape.pair_a != 0 && (l & 1); }  // (layers 0 and 1, 2 and 3, ...)
 };
 
 extern "C" {
@@ -697,6 +704,10 @@ int aig_lstm_plan_create(aig_ctx* ctx, int seq_len, int layers, int hidden, int 
   }
   for (int l = 0; l < layers && rc == AIG_OK; ++l) {
     aig_conv_plan* fp = nullptr;
+    if (pl->second(l)) {
+      pl->proj.push_back(nullptr);
+      continue;
+    }
     rc = aig_fc_plan_create(ctx, seq_len * batch, l == 0 ? in_c : hidden, 4 * hidden, AIG_ACT_NONE, 0.f, 0, &fp);
     if (rc == AIG_OK) {
       aig_fc_plan_set_output_f32(fp, 1);
@@ -705,11 +716,14 @@ int aig_lstm_plan_create(aig_ctx* ctx, int seq_len, int layers, int hidden, int 
     }
   }
   const size_t seq = (size_t)seq_len * batch;
-  if (rc == AIG_OK && (cudaMalloc(&pl->gx, seq * 4 * hidden * sizeof(float)) != cudaSuccess || cudaMalloc(&pl->mid, seq * hidden * sizeof(__half)) != cudaSuccess))
+  const bool between = layers > (pl->shape.pair_a ? 2 : 1);
+  if (rc == AIG_OK && (cudaMalloc(&pl->gx, seq * 4 * hidden * sizeof(float)) != cudaSuccess ||
+                       (between && cudaMalloc(&pl->mid, seq * hidden * sizeof(__half)) != cudaSuccess)))
     rc = aig_fail(ctx, AIG_ERR_CUDA, "lstm plan: device allocation failed");
   const size_t groups = ceil_div(batch, kSeqs), words = (groups + 1) * sizeof(unsigned int);
   if (rc == AIG_OK && pl->shape.pair_a &&
       (cudaMalloc(&pl->xs, groups * kSeqs * seq_len * hidden * sizeof(__half)) != cudaSuccess || cudaMalloc(&pl->counters, words) != cudaSuccess ||
+       cudaMalloc(&pl->pair_bias, (size_t)(layers / 2) * 4 * hidden * sizeof(float)) != cudaSuccess ||
        cudaMemsetAsync(pl->counters, 0, words, ctx->stream) != cudaSuccess))
     rc = aig_fail(ctx, AIG_ERR_CUDA, "lstm plan: device allocation failed");
   if (rc != AIG_OK) {
@@ -729,6 +743,7 @@ int aig_lstm_plan_destroy(aig_lstm_plan* pl) {
   cudaFree(pl->mid);
   cudaFree(pl->xs);
   cudaFree(pl->counters);
+  cudaFree(pl->pair_bias);
   delete pl;
   return AIG_OK;
 }
@@ -740,6 +755,13 @@ int aig_lstm_plan_set_weights(aig_lstm_plan* pl, const aig_half* blob) {
   AIG_REQUIRE(ctx, blob != nullptr && ((uintptr_t)blob & 15) == 0, "lstm set_weights: blob must be non-null and 16-byte aligned");
   pl->blob = (const __half*)blob;
   for (int l = 0; l < pl->L; ++l) {
+    if (pl->second(l)) {
+      const int n = 4 * pl->H;
+      bias_sum_kernel<<<ceil_div(n, 128), 128, 0, ctx->stream>>>(pl->pair_bias + (size_t)(l / 2) * n, (const __half*)blob + pl->bw_off[l],
+                                                                 pl->double_bias ? (const __half*)blob + pl->br_off[l] : nullptr, n);
+      AIG_LAUNCH_OK(ctx);
+      continue;
+    }
     int rc = aig_fc_plan_set_weights_out_in(pl->proj[l], blob + pl->w_off[l], blob + pl->bw_off[l]);
     if (rc != AIG_OK) return rc;
     if (pl->double_bias && (rc = aig_fc_plan_add_bias(pl->proj[l], blob + pl->br_off[l])) != AIG_OK) return rc;
@@ -769,7 +791,7 @@ int aig_lstm_forward(aig_lstm_plan* pl, const aig_half* x, aig_half* y, aig_half
     prm.gx_sT = pl->batch_major ? (long long)4 * H : (long long)B * 4 * H;
     prm.gx_sB = pl->batch_major ? (long long)T * 4 * H : (long long)4 * H;
     // a middle layer may read and write `mid`: its input is fully consumed by the hoisted projection
-    // before the recurrence starts overwriting it
+    // before the recurrence starts overwriting it (a pair's first layer writes `xs` instead)
     prm.y = (l == pl->L - 1) ? (__half*)y : pl->mid;
     prm.y_sT = sT; prm.y_sB = sB;
     prm.h0 = use_state ? (const __half*)h_state + (size_t)l * B * H : nullptr;
@@ -789,7 +811,7 @@ int aig_lstm_forward(aig_lstm_plan* pl, const aig_half* x, aig_half* y, aig_half
       pp.a = first;
       pp.b = layer(l);
       pp.W = pl->blob + pl->w_off[l];
-      pp.bias = fc_plan_shift_buffer(pl->proj[l]);
+      pp.bias = pl->pair_bias + (size_t)(l / 2) * 4 * H;
       pp.xs = pl->xs;
       pp.counters = pl->counters;
       in = pp.b.y;
