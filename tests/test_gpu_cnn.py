@@ -403,3 +403,42 @@ def test_residual_blocks_by_rows(env, monkeypatch, B, H, W, widths, act):
         err = U.scaled_err(U.nchw(got[pick]), want)
         assert err < STAGE_TOL, "stage %d: max scaled err %.4f" % (i, err)
     enc.close()
+
+
+@gpu
+def test_blocks_by_rows_keep_infinities_in_their_windows(env, monkeypatch):
+    """Activations beyond fp16's range around one bright spot of one image: only what its windows cover becomes infinite
+    or NaN, all else keeps its bits, and so does the next forward (the kernel adds to columns that its last tile left)."""
+    U = env
+    c, pk = U.ctx(), U.pkg()
+    monkeypatch.setenv("AIG_CNN_NO_CHAIN", "1")
+    B, H, W, widths = 9, 150, 190, (32, 64, 128, 256, 256)
+    params = PL.make_cnn_params(4, widths=widths, trivial=False)
+    params["c0w"] = (params["c0w"].astype(np.float32) * 4e4).astype(np.float16)   # 255 overflows behind it, 0 and 1 do not
+    frames = np.random.default_rng(4).integers(0, 2, (B, H, W, 4), dtype=np.uint8)
+    spot = frames.copy()
+    image, rows, cols = 4, (70, 73), (90, 93)
+    spot[image, rows[0]:rows[1] + 1, cols[0]:cols[1] + 1] = 255
+    enc = pk.CnnEncoder(c, B, H, W, widths=widths)
+    enc.load_bytes(PL.serialize_cnn_checkpoint(params, W, H))
+
+    def run(f):
+        enc.forward(U.dev(f))
+        c.sync()
+        return [U.host(enc.stage_output(i)) for i in range(len(widths))] + [U.host(enc.features()), U.host(enc.outputs_f32())]
+
+    clean = run(frames)
+    assert all(np.isfinite(a.astype(np.float32)).all() for a in clean)
+    dirty = run(spot)
+    box = [rows, cols]
+    for i in range(len(widths)):
+        # k5 s2 p2, then per block k4 s2 p1 (the shortcut's window lies inside it) and k3 s1 p1
+        box = [((a - 1) // 2, (b + 2) // 2) for a, b in box] if i == 0 else [((a - 1) // 2 - 1, (b + 1) // 2 + 1) for a, b in box]
+        inside = np.zeros(clean[i].shape[:3], bool)
+        inside[image, max(box[0][0], 0):box[0][1] + 1, max(box[1][0], 0):box[1][1] + 1] = True
+        assert not inside.all() and np.array_equal(dirty[i][~inside], clean[i][~inside]), "stage %d" % i
+        assert not np.isfinite(dirty[i][inside].astype(np.float32)).all(), "stage %d" % i
+    others = np.arange(B) != image
+    assert all(np.array_equal(d[others], k[others]) for d, k in zip(dirty[len(widths):], clean[len(widths):]))
+    assert all(np.array_equal(a, b) for a, b in zip(run(frames), clean))
+    enc.close()

@@ -283,3 +283,36 @@ def test_clip_encoder_depth_walk(env, B, D, H, W, offset, widths):
     # three layers of fp16 activations (2^-11 each) and the pool's own rounding, against a scale of at least the rms
     assert U.scaled_err(got, feat.astype(np.float32)) < 4e-3
     enc.close()
+
+
+@gpu
+def test_clip_encoder_depth_walk_keeps_infinities_in_their_windows(env):
+    """An infinity and a NaN in two clips: the features that their windows reach are as finite as the oracle's, the other
+    clips keep their bits, and so does the next forward."""
+    U = env
+    U.pkg()
+    from ai_gamer_b200 import runners as R
+
+    B, D, H, W = 5, 6, 72, 104
+    p = PL.make_conv3d_params(9, trivial=False)
+    clips = PL.make_clips(9, B, D, H, W)
+    bad = clips.copy()
+    bad[1, 0, 5, 10, 12] = np.inf       # in the first of the four cells
+    bad[3, 2, 0, 60, 90] = np.nan       # in the last
+    enc = R.ClipEncoder(U.ctx(), B, D, H, W)
+    enc.load_bytes(PL.serialize_conv3d_params(p))
+
+    def run(x):
+        enc.forward(U.dev(x))
+        return U.host(enc.features()), U.host(enc.outputs_f32())
+
+    clean, dirty = run(clips), run(bad)
+    assert all(np.isfinite(a.astype(np.float32)).all() for a in clean)
+    want = np.isfinite(PL.conv3d_forward(p, bad)[0].astype(np.float32)).reshape(B, -1)
+    assert 0 < (~want[1]).sum() < want[1].size and 0 < (~want[3]).sum() < want[3].size
+    assert np.array_equal(np.isfinite(dirty[0].astype(np.float32)).reshape(B, -1), want)
+    for d, k in zip(dirty, clean):
+        assert np.array_equal(d[[0, 2, 4]], k[[0, 2, 4]])
+    assert np.array_equal(dirty[0].reshape(B, -1)[want], clean[0].reshape(B, -1)[want])
+    assert all(np.array_equal(a, b) for a, b in zip(run(clips), clean))
+    enc.close()

@@ -115,6 +115,55 @@ def test_lstm_layers_side_by_side(env, T, B, H, L):
 
 
 @gpu
+@pytest.mark.parametrize("T,B,H,L,clip,dbl,batch_major", [
+    (6, 3, 192, 2, 0.0, False, True),                       # one group a cluster, half of the rows delivered
+    (4, 70, 512, 2, 5.0, True, True),                       # two groups, the last one ragged
+    (4, 112, 512, 2, 0.0, True, True), (4, 101, 512, 3, 5.0, False, False),   # three and two; a third layer by itself
+    (2, 128, 512, 4, 5.0, True, False),                     # two pairs
+])
+def test_lstm_pairs_with_carried_state(env, T, B, H, L, clip, dbl, batch_major):
+    """Two layers in one launch that start from a state and leave one, in both layouts, with and without clip: against the
+    oracle, and a sequence in halves against the whole."""
+    U = env
+    import torch
+
+    c, pk, I = U.ctx(), U.pkg(), 32
+    rng = np.random.default_rng(B * 1000 + H + L)
+    blob = PL.make_lstm_blob(rng, I, H, L, dbl, 1.0)
+    n_bias = 4 * H * L * (2 if dbl else 1)
+    blob[-n_bias:] = h(rng.uniform(-0.2, 0.2, n_bias))      # biases of every layer
+    x = h(rng.standard_normal((T, B, I)))
+    h0, c0 = h(rng.uniform(-1, 1, (L, B, H))), h(rng.standard_normal((L, B, H)))
+    order = (1, 0, 2) if batch_major else (0, 1, 2)         # time and sequences change places
+    d_blob = U.dev(blob)
+
+    def run(pieces):
+        hs, cs, ys = U.dev(h0), U.dev(c0), []
+        for piece in pieces:
+            t = piece.shape[0]
+            plan = pk.LstmPlan(c, t, L, H, B, I, clip=clip, double_bias=dbl, batch_major=batch_major)
+            plan.set_weights(d_blob)
+            y = torch.zeros(t * B * H, dtype=torch.float16, device="cuda")
+            torch.cuda.synchronize()
+            plan.forward(U.dev(piece.transpose(order)), y, hs, cs, use_state=True)
+            c.sync()
+            ys.append(U.host(y).reshape((B, t, H) if batch_major else (t, B, H)).transpose(order))
+            plan.close()
+        return np.concatenate(ys), U.host(hs), U.host(cs)
+
+    whole = run([x])
+    for a, b in zip(whole, run([x[:T // 2], x[T // 2:]])):
+        assert np.array_equal(a, b)
+    pick = sorted({0, B - 1, min(B - 1, 15), min(B - 1, 16), min(B - 1, 47), min(B - 1, 48), min(B - 1, 64)})
+    hw, cw = np.ascontiguousarray(h0[:, pick]), np.ascontiguousarray(c0[:, pick])
+    want = O.lstm(np.ascontiguousarray(x[:, pick]), blob, H, L, clip, dbl, hw, cw, True)
+    # as test_lstm_matches_oracle for h; the cell state is a sum of a few such steps and up to four times as large
+    assert np.abs(whole[0][:, pick].astype(np.float32) - want.astype(np.float32)).max() < 6e-3
+    assert np.abs(whole[1][:, pick].astype(np.float32) - hw.astype(np.float32)).max() < 6e-3
+    assert np.abs(whole[2][:, pick].astype(np.float32) - cw.astype(np.float32)).max() < 2.4e-2
+
+
+@gpu
 def test_lstm_batch_major_and_step_by_step(env):
     U = env
     import torch
