@@ -94,6 +94,7 @@ SIGNATURES = {
     "aig_lstm_weight_count": [c_int, c_int, c_int, c_int],
     "aig_lstm_plan_create": [P, c_int, c_int, c_int, c_int, c_int, c_float, c_int, c_int, PP],
     "aig_lstm_plan_destroy": [P],
+    "aig_lstm_plan_pair_groups": [P, ctypes.POINTER(c_int), ctypes.POINTER(c_int)],
     "aig_lstm_plan_set_weights": [P, P],
     "aig_lstm_forward": [P, P, P, P, P, c_int],
     "aig_lstm_forward_noalloc": [P, P, P, P, c_int, c_int, c_int, c_int, c_float, c_int],
@@ -170,6 +171,7 @@ SIGNATURES.update({
     "aig_cnn_features": [P],
     "aig_cnn_stage_output": [P, c_int, PI, PI, PI],
     "aig_cnn_kernel_launches": [P],
+    "aig_cnn_walked_launches": [P],
     "aig_cnn_profile_begin": [P, c_int],
     "aig_cnn_profile_end": [P, ctypes.POINTER(ctypes.c_double), c_int, PI],
     "aig_cnn_site_count": [P],
@@ -248,9 +250,11 @@ SIGNATURES.update({
     "aig_c3d_forward": [P, P],
     "aig_c3d_outputs_f32": [P],
     "aig_c3d_features": [P],
+    "aig_c3d_stage_output": [P, c_int, PI, PI, PI, PI],
+    "aig_c3d_walked_layers": [P],
 })
 _RESTYPES = {"aig_compat_context": c_void_p, "aig_fc_backward_weight_storage": c_void_p, "aig_recording_last_error": ctypes.c_char_p, "aig_layer_param_bytes": c_size_t, "aig_s2d_elems": c_size_t, "aig_conv_padded_rows": ctypes.c_longlong, "aig_c3d_last_error": ctypes.c_char_p, "aig_c3d_param_bytes": c_size_t, "aig_c3d_outputs_f32": c_void_p,
-             "aig_c3d_features": c_void_p, "aig_ctx_stream": c_void_p, "aig_last_error": ctypes.c_char_p, "aig_cnn_last_error": ctypes.c_char_p,
+             "aig_c3d_features": c_void_p, "aig_c3d_stage_output": c_void_p, "aig_ctx_stream": c_void_p, "aig_last_error": ctypes.c_char_p, "aig_cnn_last_error": ctypes.c_char_p,
              "aig_cnn_checkpoint_bytes": c_size_t, "aig_cnn_outputs_half": c_void_p, "aig_cnn_outputs_f32": c_void_p,
              "aig_cnn_features": c_void_p, "aig_cnn_stage_output": c_void_p, "aig_cnn_site_name": ctypes.c_char_p,
              "aig_cnn_site_flops": ctypes.c_double, "aig_cnn_site_bytes": ctypes.c_double,
@@ -577,6 +581,10 @@ class CnnEncoder:
     def kernel_launches(self):
         return lib().aig_cnn_kernel_launches(self.handle)
 
+    @property
+    def walked_launches(self):
+        return lib().aig_cnn_walked_launches(self.handle)
+
     def profile_begin(self, max_steps):
         self.check(lib().aig_cnn_profile_begin(self.handle, max_steps))
 
@@ -608,6 +616,13 @@ class LstmPlan(_Plan):
     def set_weights(self, blob):
         self._keep = [blob]
         self.check(lib().aig_lstm_plan_set_weights(self.handle, ptr(blob)))
+
+    @property
+    def pair_groups(self):
+        """(first, second): groups of sequences a cluster of two layers that run side by side; (0, 0): one after the other."""
+        first, second = c_int(), c_int()
+        self.check(lib().aig_lstm_plan_pair_groups(self.handle, ctypes.byref(first), ctypes.byref(second)))
+        return first.value, second.value
 
     def forward(self, x, y, h_state=None, c_state=None, use_state=False):
         self.check(lib().aig_lstm_forward(self.handle, ptr(x), ptr(y), ptr(h_state), ptr(c_state), 1 if use_state else 0))

@@ -734,6 +734,13 @@ int aig_lstm_plan_create(aig_ctx* ctx, int seq_len, int layers, int hidden, int 
   return AIG_OK;
 }
 
+int aig_lstm_plan_pair_groups(const aig_lstm_plan* pl, int* first, int* second) {
+  if (!pl || !first || !second) return AIG_ERR_INVALID;
+  *first = pl->shape.pair_a;
+  *second = pl->shape.pair_b;
+  return AIG_OK;
+}
+
 int aig_lstm_plan_destroy(aig_lstm_plan* pl) {
   if (!pl) return AIG_OK;
   DeviceGuard g(pl->ctx->device);

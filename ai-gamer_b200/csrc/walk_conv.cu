@@ -632,6 +632,15 @@ __global__ void row_blocks_kernel(const uint4* __restrict__ src, uint4* __restri
   }
 }
 
+// blocks [d][n][Hb][Wb][4][c] -> [n][d][h][w][c], 8 channels per thread
+__global__ void clip_blocks_kernel(const uint4* __restrict__ src, uint4* __restrict__ dst, int batch, int d, int h, int w, int c8, int Hb, int Wb) {
+  const long long total = (long long)batch * d * h * w * c8;
+  for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (long long)gridDim.x * blockDim.x) {
+    const int c = (int)(i % c8), x = (int)(i / c8 % w), y = (int)(i / c8 / w % h), z = (int)(i / c8 / w / h % d), n = (int)(i / c8 / w / h / d);
+    dst[i] = src[((((size_t)z * batch + n) * Hb + ((y + 1) >> 1)) * Wb + ((x + 1) >> 1)) * 4 * c8 + (((y + 1) & 1) * 2 + ((x + 1) & 1)) * c8 + c];
+  }
+}
+
 typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*, const cuuint32_t*,
                                   const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
 
@@ -865,6 +874,12 @@ int clip_conv_set_weights(WalkConv* c, const aig_half* w, const aig_half* bias, 
   return walk_affine(c, 0, bias, gamma, beta, mean, var, eps);
 }
 int clip_conv_forward(WalkConv* c, const aig_half* x, aig_half* y) { return walk_launch(c, x, nullptr, y, nullptr); }
+int clip_blocks_to_ndhwc(aig_ctx* ctx, const aig_half* blocks, aig_half* y, int batch, int d, int h, int w, int c) {
+  DeviceGuard guard(ctx->device);
+  clip_blocks_kernel<<<ctx->sm_count * 8, 256, 0, ctx->stream>>>((const uint4*)blocks, (uint4*)y, batch, d, h, w, c / 8, clip_block_extent(h), clip_block_extent(w));
+  AIG_LAUNCH_OK(ctx);
+  return AIG_OK;
+}
 
 bool res_walk_supported(const aig_ctx* ctx, const ResWalkGeom& g) {
   if (!(g.C == 32 && g.K == 64) && !(g.C == 64 && g.K == 128)) return false;

@@ -26,6 +26,7 @@ int clip_conv_create(aig_ctx* ctx, const ClipConvGeom& g, WalkConv** out);
 int clip_conv_set_weights(WalkConv* c, const aig_half* w_kcx, const aig_half* bias, const float* gamma, const float* beta, const float* mean,
                           const float* var, float eps);
 int clip_conv_forward(WalkConv* c, const aig_half* x, aig_half* y);
+int clip_blocks_to_ndhwc(aig_ctx* ctx, const aig_half* blocks, aig_half* y, int batch, int d, int h, int w, int c);
 
 // ---- a residual block of the frame encoder (main k4 s2 p1, then k3 s1 p1; shortcut k2 s2 p0): along the rows
 // Input: blocks [yb][n][xb][4][c] (extents as of aig_nhwc_to_s2d, rows outermost).  Between the two launches: [y][n][x][K]

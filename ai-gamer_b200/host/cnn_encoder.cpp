@@ -808,6 +808,12 @@ const aig_half* aig_cnn_outputs_half(aig_cnn* m) { return m ? m->logits : nullpt
 const float* aig_cnn_outputs_f32(aig_cnn* m) { return m ? m->out_f32 : nullptr; }
 const aig_half* aig_cnn_features(aig_cnn* m) { return m ? m->feat : nullptr; }
 int aig_cnn_kernel_launches(aig_cnn* m) { return m ? m->launches_per_forward : 0; }
+int aig_cnn_walked_launches(aig_cnn* m) {
+  int n = 0;
+  if (m)
+    for (const auto& b : m->blocks) n += (b.walk_down != nullptr) + (b.walk_c1 != nullptr);
+  return n;
+}
 const aig_half* aig_cnn_stage_output(aig_cnn* m, int stage, int* h, int* w, int* ch) {
   if (!m || stage < 0 || stage > (int)m->blocks.size()) return nullptr;
   const int sh = stage == 0 ? m->H0 : m->bh[stage - 1], sw = stage == 0 ? m->W0 : m->bw[stage - 1], sc = m->cfg.widths[stage];

@@ -25,6 +25,8 @@ struct aig_c3d {
   aig_conv_plan* fc = nullptr;
   std::vector<aig_half*> acts;
   std::vector<int> d, h, w;
+  aig_half* stage_scratch = nullptr;   // channels-last copy of a layer's blocks, made on request
+  size_t stage_scratch_elems = 0;
   aig_half *feat = nullptr, *logits = nullptr;
   aig_half *fcw = nullptr, *fcb = nullptr;   // FC parameters as loaded ([in][out], [out])
   float* out_f32 = nullptr;
@@ -121,6 +123,7 @@ int aig_c3d_destroy(aig_c3d* m) {
   for (aig_conv_plan* p : m->convs) aig_conv_plan_destroy(p);
   aig_conv_plan_destroy(m->fc);
   for (aig_half* a : m->acts) cudaFree(a);
+  cudaFree(m->stage_scratch);
   cudaFree(m->feat); cudaFree(m->logits); cudaFree(m->out_f32); cudaFree(m->params);
   delete m;
   return AIG_OK;
@@ -187,6 +190,28 @@ int aig_c3d_forward(aig_c3d* m, const aig_half* clips) {
   return AIG_OK;
 }
 
+int aig_c3d_walked_layers(aig_c3d* m) { return m ? (int)m->walks.size() : 0; }
+const aig_half* aig_c3d_stage_output(aig_c3d* m, int layer, int* d, int* h, int* w, int* ch) {
+  if (!m || layer < 0 || layer >= m->cfg.n_layers) return nullptr;
+  const int od = m->d[layer], oh = m->h[layer], ow = m->w[layer], oc = m->cfg.widths[layer + 1];
+  if (d) *d = od;
+  if (h) *h = oh;
+  if (w) *w = ow;
+  if (ch) *ch = oc;
+  if (layer >= (int)m->walks.size()) return m->acts[layer];
+  // the layer's output lives in blocks: hand out a channels-last copy
+  const size_t n = (size_t)m->cfg.batch * od * oh * ow * oc;
+  if (m->stage_scratch_elems < n) {
+    aig_ctx_sync(m->ctx);
+    cudaFree(m->stage_scratch);
+    m->stage_scratch = nullptr;
+    m->stage_scratch_elems = 0;
+    if (cudaMalloc(reinterpret_cast<void**>(&m->stage_scratch), n * sizeof(aig_half)) != cudaSuccess) return nullptr;
+    m->stage_scratch_elems = n;
+  }
+  if (clip_blocks_to_ndhwc(m->ctx, m->acts[layer], m->stage_scratch, m->cfg.batch, od, oh, ow, oc) != AIG_OK) return nullptr;
+  return m->stage_scratch;
+}
 const float* aig_c3d_outputs_f32(aig_c3d* m) { return m ? m->out_f32 : nullptr; }
 const aig_half* aig_c3d_features(aig_c3d* m) { return m ? m->feat : nullptr; }
 

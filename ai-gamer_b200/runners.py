@@ -149,6 +149,17 @@ class ClipEncoder:
         feat = self.cfg.widths[self.cfg.n_layers] * 4
         return _device_copy(self.ctx, lib().aig_c3d_features(self.handle), (self.cfg.batch, feat), torch.float16)
 
+    def stage_output(self, layer):
+        import torch
+
+        d, h, w, c = (ctypes.c_int() for _ in range(4))
+        addr = lib().aig_c3d_stage_output(self.handle, layer, *(ctypes.byref(v) for v in (d, h, w, c)))
+        return _device_copy(self.ctx, addr, (self.cfg.batch, d.value, h.value, w.value, c.value), torch.float16)
+
+    @property
+    def walked_layers(self):
+        return lib().aig_c3d_walked_layers(self.handle)
+
     def close(self):
         if self.handle:
             lib().aig_c3d_destroy(self.handle)

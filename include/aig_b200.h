@@ -40,7 +40,8 @@ enum { AIG_ACT_NONE = 0, AIG_ACT_RELU = 1, AIG_ACT_SWISH = 2, AIG_ACT_LEAKY = 3 
 typedef struct aig_ctx aig_ctx;
 int aig_ctx_create(aig_ctx** out, int device);
 int aig_ctx_destroy(aig_ctx* ctx);
-/* Use an existing cudaStream_t (passed as void*) instead of the context's own stream. */
+/* Use an existing cudaStream_t (passed as void*) instead of the context's own stream.  Work queued on the context's own
+ * stream is waited for; between two streams of the caller's the caller keeps the order. */
 int aig_ctx_set_stream(aig_ctx* ctx, void* cuda_stream);
 void* aig_ctx_stream(aig_ctx* ctx);
 /* Synchronise the stream and report any deferred kernel error (including AIG_ERR_TIMEOUT raised by a
@@ -350,6 +351,9 @@ size_t aig_lstm_weight_count(int in_c, int hidden, int layers, int double_bias);
 int aig_lstm_plan_create(aig_ctx* ctx, int seq_len, int layers, int hidden, int batch, int in_c,
                          float clip, int double_bias, int batch_major, aig_lstm_plan** out);
 int aig_lstm_plan_destroy(aig_lstm_plan* plan);
+/* Groups of 16 sequences that a cluster of the first and of the second of two layers takes where the plan runs layers in
+ * pairs, in one launch; both 0: one layer after the other. */
+int aig_lstm_plan_pair_groups(const aig_lstm_plan* plan, int* first, int* second);
 /* LSTMLayer::LoadParameters (LSTMLayer.cpp:139-146): the blob stays where it is (device memory,
  * 16-byte aligned) and must outlive the plan's forwards. */
 int aig_lstm_plan_set_weights(aig_lstm_plan* plan, const aig_half* blob);

@@ -70,6 +70,8 @@ const aig_half* aig_cnn_features(aig_cnn* m);      /* [batch][widths[n_blocks]] 
 const aig_half* aig_cnn_stage_output(aig_cnn* m, int stage, int* h, int* w, int* c);
 /* Kernels launched by one aig_cnn_forward. */
 int aig_cnn_kernel_launches(aig_cnn* m);
+/* Of them, convolution launches of the row-walking kernel. */
+int aig_cnn_walked_launches(aig_cnn* m);
 /* Per-launch device timing of aig_cnn_forward (eager path) with CUDA events on the context stream:
  * begin() arms it for up to max_steps forwards; end() synchronises and writes the mean milliseconds
  * of every launch site (aig_cnn_site_count of them, in launch order).  site_flops/site_bytes are the
@@ -170,6 +172,10 @@ int aig_c3d_load_memory(aig_c3d* m, const void* blob, size_t bytes);
 int aig_c3d_forward(aig_c3d* m, const aig_half* clips);
 const float* aig_c3d_outputs_f32(aig_c3d* m);   /* [batch][n_out] */
 const aig_half* aig_c3d_features(aig_c3d* m);   /* [batch][widths[n_layers]*4] pooled features */
+/* Channels-last output [batch][d][h][w][c] of layer 0 .. n_layers - 1 of the last forward, for layer-wise checks. */
+const aig_half* aig_c3d_stage_output(aig_c3d* m, int layer, int* d, int* h, int* w, int* c);
+/* Layers behind the first that the depth-walking kernel runs. */
+int aig_c3d_walked_layers(aig_c3d* m);
 
 /* ---------------------------------------------------------------------------------------------
  * The reference's own network through the C++ layer classes (ai-gamer_b200/host/layers/Layers.h, the

@@ -372,18 +372,19 @@ def test_checkpoint_files(env, tmp_path):
 
 
 @gpu
-@pytest.mark.parametrize("B,H,W,widths,act", [
-    (1950, 32, 40, (32, 64, 128), "ACT_SWISH"),       # runs of one to eight rows, all the ways they follow one another in the accumulators
-    (3, 10, 12, (32, 64, 128), "ACT_RELU"),           # one tile, fewer rows than accumulators
-    (37, 67, 131, (32, 64, 128, 256), "ACT_LEAKY"),   # odd extents, a block by rows before one by patches
-    (5, 50, 322, (32, 64, 192), "ACT_SWISH"),         # rows beyond 256 pixels; one block by rows
-    (150, 20, 20, (32, 64), "ACT_NONE"),              # the last block by rows
-    (11, 90, 131, (32, 64, 128, 256, 256), "ACT_SWISH"),  # 256 channels: whole image rows in a tile, the last one ragged
-    (40, 34, 36, (64, 256), "ACT_RELU"),              # and into the head directly
-    (3, 40, 262, (32, 256, 256), "ACT_LEAKY"),        # and a block of them before a block by patches, long rows
+@pytest.mark.parametrize("B,H,W,widths,act,walked", [
+    (1950, 32, 40, (32, 64, 128), "ACT_SWISH", 4),       # runs of one to eight rows, all the ways they follow one another in the accumulators
+    (3, 10, 12, (32, 64, 128), "ACT_RELU", 2),           # one tile, fewer rows than accumulators
+    (37, 67, 131, (32, 64, 128, 256), "ACT_LEAKY", 5),   # odd extents, a block by rows before one by patches
+    (5, 50, 322, (32, 64, 192), "ACT_SWISH", 2),         # rows beyond 256 pixels; one block by rows
+    (150, 20, 20, (32, 64), "ACT_NONE", 2),              # the last block by rows
+    (11, 90, 131, (32, 64, 128, 256, 256), "ACT_SWISH", 6),  # 256 channels: whole image rows in a tile, the last one ragged
+    (40, 34, 36, (64, 256), "ACT_RELU", 1),              # and into the head directly
+    (3, 40, 262, (32, 256, 256), "ACT_LEAKY", 2),        # and a block of them before a block by patches, long rows
 ])
-def test_residual_blocks_by_rows(env, monkeypatch, B, H, W, widths, act):
-    """The row-walking residual blocks at the edges of their tiles and runs, every stage against the oracle on a sample."""
+def test_residual_blocks_by_rows(env, monkeypatch, B, H, W, widths, act, walked):
+    """The row-walking residual blocks at the edges of their tiles and runs, every stage against the oracle on a sample.
+    `walked`: launches of that kernel."""
     U = env
     c, pk = U.ctx(), U.pkg()
     monkeypatch.setenv("AIG_CNN_NO_CHAIN", "1")
@@ -391,6 +392,7 @@ def test_residual_blocks_by_rows(env, monkeypatch, B, H, W, widths, act):
     frames = PL.make_frames(B, B, H, W)
     pick = np.unique(np.linspace(0, B - 1, 60).astype(int))
     enc = pk.CnnEncoder(c, B, H, W, widths=widths, act=getattr(pk, act))
+    assert enc.walked_launches == walked
     enc.load_bytes(PL.serialize_cnn_checkpoint(params, W, H))
     runs = []
     for _ in range(3):
@@ -420,6 +422,7 @@ def test_blocks_by_rows_keep_infinities_in_their_windows(env, monkeypatch):
     image, rows, cols = 4, (70, 73), (90, 93)
     spot[image, rows[0]:rows[1] + 1, cols[0]:cols[1] + 1] = 255
     enc = pk.CnnEncoder(c, B, H, W, widths=widths)
+    assert enc.walked_launches == 6
     enc.load_bytes(PL.serialize_cnn_checkpoint(params, W, H))
 
     def run(f):

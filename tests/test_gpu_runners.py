@@ -264,7 +264,8 @@ def test_agent_second_parameter_load(env, monkeypatch, B, unfused):
     (2, 4, 40, 48, 0, (3, 32, 64, 32)),        # one share of 32 channels
 ])
 def test_clip_encoder_depth_walk(env, B, D, H, W, offset, widths):
-    """The depth-walking 3-D convolution at the edges of its tiles, runs and channel shares."""
+    """The depth-walking 3-D convolution at the edges of its tiles, runs and channel shares: every layer's output against the
+    oracle's, and the same bits from one forward to the next."""
     U = env
     U.pkg()
     import torch
@@ -272,16 +273,28 @@ def test_clip_encoder_depth_walk(env, B, D, H, W, offset, widths):
 
     p = PL.make_conv3d_params(B + D, widths=widths, trivial=False)
     clips = PL.make_clips(W, B, D, H, W)
-    feat, _, _ = PL.conv3d_forward(p, clips)
     enc = R.ClipEncoder(U.ctx(), B, D, H, W, widths=widths)
+    assert enc.walked_layers == (1 if widths == (3, 32, 128, 32) else 2)
     enc.load_bytes(PL.serialize_conv3d_params(p))
     room = torch.zeros(clips.size + 8, dtype=torch.float16, device="cuda")
     room[offset:offset + clips.size] = U.dev(clips).flatten()
     torch.cuda.synchronize()
-    enc.forward(room[offset:])
-    got = U.host(enc.features()).astype(np.float32)
-    # three layers of fp16 activations (2^-11 each) and the pool's own rounding, against a scale of at least the rms
-    assert U.scaled_err(got, feat.astype(np.float32)) < 4e-3
+    runs = []
+    for _ in range(3):
+        enc.forward(room[offset:])
+        runs.append([U.host(enc.features())] + [U.host(enc.stage_output(i)) for i in range(len(widths) - 1)])
+    assert all(np.array_equal(x, y) for r in runs[1:] for x, y in zip(runs[0], r))
+    x = clips
+    for i, L in enumerate(p["layers"]):
+        x = O.leaky_relu(O.batchnorm(O.conv3d(x, L["w"], L["b"], 1, 2, 1, 1), *L["bn"]), 0.01)
+        # element by element, against a scale of at least the rms: the oracle rounds to fp16 after the convolution, BatchNorm
+        # and activation, this once a layer (2^-11 each, up to three times the value where BatchNorm shifts it), and each
+        # layer carries on what the ones before it differ by
+        err = U.scaled_err(runs[0][1 + i], np.moveaxis(x, 1, -1))
+        assert err < (i + 1) * 4e-3, "layer %d: %.5f" % (i, err)
+    # and the pool, whose mean takes the roundings out again, adds its own
+    feat = O.adaptive_avgpool3d(x, 2, 2).astype(np.float32)
+    assert U.scaled_err(runs[0][0].astype(np.float32).reshape(feat.shape), feat) < 4e-3
     enc.close()
 
 
@@ -300,6 +313,7 @@ def test_clip_encoder_depth_walk_keeps_infinities_in_their_windows(env):
     bad[1, 0, 5, 10, 12] = np.inf       # in the first of the four cells
     bad[3, 2, 0, 60, 90] = np.nan       # in the last
     enc = R.ClipEncoder(U.ctx(), B, D, H, W)
+    assert enc.walked_layers == 2
     enc.load_bytes(PL.serialize_conv3d_params(p))
 
     def run(x):
