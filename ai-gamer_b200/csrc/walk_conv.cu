@@ -19,11 +19,13 @@
 // Clips: bound by shared-memory bandwidth.  A plane of a tile takes 1950 clk for 18 products of 10 KB of operands and 41 KB of
 // patches written (64 channels: 2470 for 36 of 7 KB and 77 KB).  16 clips of 8x144x256, the two layers: 61 and 38 us by the
 // streamed GEMM, now 28 and 31; smaller clips gain more (9 of 5x98x305, the whole encoder: 143 -> 72 us).  Five patch buffers
-// instead of four for 64 channels: 3340 -> 2660 clk a plane (a patch takes over 2000 clk to come).
-// Frames: the 64-channel block is bound by memory (256 frames of 144x256: 302 and 226 MB, 46 and 35 us at the copy bandwidth),
-// the 128-channel one by the products (3690 and 2410 clk a row of a tile).  By the patch-resident kernels, 256 frames: 89, 75,
-// 65 and 57 us; now 51, 44, 45 and 37 (start to start of the launches); the 256-channel 3x3 convolutions 52 and 27, now 46 and 18.  That kernel multiplies 64 columns at a time, reads a
-// patch's halo rows again for every tile and, with 128 channels, streams the weights.
+// instead of four for 64 channels, measured with outputs that left through a staging tile: 3340 -> 2660 clk a plane (a patch takes
+// over 2000 clk to come); without the staging 2470.
+// Frames: the 64-channel block has no unit at its peak.  256 frames of 144x256: 261 and 194 MB of DRAM traffic in 51 and 44 us,
+// 0.78 and 0.67 of the copy bandwidth; 128 frames: tensor pipe active 49 and 54 %.  The 128-channel one is bound by the products
+// (3690 and 2410 clk a row of a tile).  By the patch-resident kernels, 256 frames: 89, 75, 65 and 57 us; now 51, 44, 45 and 37
+// (start to start of the launches); the 256-channel 3x3 convolutions 52 and 27, now 46 and 18.  That kernel multiplies 64 columns
+// at a time, reads a patch's halo rows again for every tile and, with 128 channels, streams the weights.
 #include "walk_conv.h"
 
 #include <type_traits>
