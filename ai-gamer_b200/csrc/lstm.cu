@@ -20,9 +20,10 @@
 // (3)  Two layers run side by side in one launch where their clusters fit the device together (lstm_pair_kernel): the
 // second layer's clusters multiply W.x_t themselves, a step or two behind, W beside R in TMEM (what does not fit, in
 // shared memory).  That takes out half of the dependent steps and the second layer's projection, whose 4H fp32 values
-// per step and sequence went through memory.  Whole sequence head, before and after, us: 128 sequences of 64 at H = 512
-// (three groups a cluster and two) 380 and 260, 16 sequences 279 and 161, 64 sequences 521 and 214, 3 of 37 at H = 256
-// 132 and 76.
+// per step and sequence went through memory.  Whole sequence head, before and after, us, sequences of 64 steps at H = 512:
+// 16 of them 279 and 161, 64 (two groups a cluster) 519 and 212, 128 (three groups and two) 379 and 264; 3 of 37 steps at
+// H = 256 132 and 76.  (64 took longer than 128 before because two CTAs of different clusters could share an SM, of which
+// one waited for the other's TMEM: see recurrent_smem.)
 // Gate order i,f,g,o; blob layout: per layer W then R, then per layer bW [and bR]  (the library's
 // blob is opaque in the reference: LSTMLayer.cpp:29-35,139-146; this layout is this library's
 // definition, stated in the header).

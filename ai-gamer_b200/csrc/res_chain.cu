@@ -38,9 +38,11 @@ constexpr int kMaxBufs = 4;
 constexpr int kStageBytes = 2560;
 constexpr int kEpi0 = 128;          // first epilogue thread
 constexpr int kEpi = kThreads - kEpi0;
-// Tiles of the first stage up to which the chain is the faster way.  Measured per frame batch, chain / per-layer launches:
-// 144x256 x 1 (19 tiles) 66 / 86 us, x 6 (113) 78 / 92, 180x320 x 6 (175) 94 / 104, 107x189 x 19 (192) 92 / 102; beyond, the
-// per-layer kernels' wider tiles win: 107x189 x 32 (324) 121 / 114, 144x256 x 19 (357) 120 / 114.
+// Tiles of the first stage up to which the chain is the faster way.  Measured per frame batch, the whole encoder, chain / launches
+// per layer (by rows where they can be): 144x256 x 1 (19 tiles) 57 / 82 us, x 6 (113) 66 / 82, x 10 (188) 78 / 86, 180x320 x 6 (175)
+// 79 / 89, 107x189 x 19 (200) 78 / 85, 64x96 x 60 (200) 85 / 85, 360x640 x 2 (229) 90 / 106; beyond, the launches of wider tiles win:
+// 144x256 x 13 (245) 88 / 87, 107x189 x 24 (252) 84 / 87, 180x320 x 9 (262) 95 / 92, 144x256 x 16 (301) 99 / 94, 107x189 x 32 (336)
+// 100 / 94.
 constexpr long long kMaxChainTiles = 240;
 
 struct Walk {                       // what the loops over jobs and K need of a stage
@@ -731,7 +733,8 @@ int res_chain_create(aig_ctx* ctx, const std::vector<ResChainBlock>& blocks, int
   if (p.clusters < 8) return decline();
   for (int i = 0; i < p.n_stages; ++i) {
     Stage& s = p.st[i];
-    // CTAs per job: the busiest CTA's blocks of K (0.17 us each) and hand-overs (1 us a job, 2 with the exchange)
+    // CTAs per job: the busiest CTA's blocks of K (0.17 us each, measured with one MMA issuer; 0.12 with two) and hand-overs
+    // (1 us a job, 2 with the exchange)
     double best = 0.0;
     const int units = s.sub ? (s.cblocks < s.taps * s.sub ? s.cblocks : s.taps * s.sub) : s.cblocks;
     for (int split = 1; split <= kCluster && split <= units; split *= 2) {

@@ -214,7 +214,7 @@ static int infer_recording(aig_cnn* m, aig_recording* r, long long first, long l
       rd.cv.notify_all();
     }
   };
-  // a core copies about 8 GB/s out of the page cache and PCIe takes 52: eight readers keep ahead of it.  Where the host
+  // A core copies about 6 GB/s out of the page cache and PCIe takes 52: eight readers about keep up with it.  Where the host
   // gives fewer threads, those read; where it gives none, this one does.
   const long long n_readers = std::min<long long>(n_pieces, std::min(8u, std::max(1u, std::thread::hardware_concurrency())));
   rd.threads.reserve((size_t)n_readers);
