@@ -408,6 +408,23 @@ def test_residual_blocks_by_rows(env, monkeypatch, B, H, W, widths, act, walked)
 
 
 @gpu
+@pytest.mark.parametrize("B,H,W,walked", [
+    (192, 144, 256, 6), (222, 144, 256, 5), (256, 144, 256, 6), (334, 144, 256, 5),  # rows per CTA against rounds of tiles by patches
+    (16, 480, 854, 6), (32, 480, 854, 5),
+    (2, 64, 1024, 1), (2, 64, 1280, 1),                                             # rows of 65 and 81 positions in a tile of 128
+    (2, 72, 1440, 2), (2, 72, 1408, 1),                                             # the least that are taken (0.71) and the most that are not (0.695)
+])
+def test_which_convolutions_go_by_rows(env, monkeypatch, B, H, W, walked):
+    """256-channel convolutions stay with the patch-resident kernel where that was measured to be the faster one.  (Frames
+    of 1024 columns and more have no block by rows, the last block's convolution has half the width.)"""
+    U = env
+    monkeypatch.setenv("AIG_CNN_NO_CHAIN", "1")
+    enc = U.pkg().CnnEncoder(U.ctx(), B, H, W, widths=(32, 64, 128, 256, 256))
+    assert enc.walked_launches == walked
+    enc.close()
+
+
+@gpu
 def test_blocks_by_rows_keep_infinities_in_their_windows(env, monkeypatch):
     """Activations beyond fp16's range around one bright spot of one image: only what its windows cover becomes infinite
     or NaN, all else keeps its bits, and so does the next forward (the kernel adds to columns that its last tile left)."""
