@@ -380,7 +380,8 @@ def test_checkpoint_files(env, tmp_path):
     (150, 20, 20, (32, 64), "ACT_NONE", 2),              # the last block by rows
     (11, 90, 131, (32, 64, 128, 256, 256), "ACT_SWISH", 6),  # 256 channels: whole image rows in a tile, the last one ragged
     (40, 34, 36, (64, 256), "ACT_RELU", 1),              # and into the head directly
-    (3, 40, 262, (32, 256, 256), "ACT_LEAKY", 2),        # and a block of them before a block by patches, long rows
+    (3, 40, 250, (32, 256, 256), "ACT_LEAKY", 2),        # and a block of them before a block by patches, rows of half a tile
+    (3, 40, 262, (32, 256, 256), "ACT_LEAKY", 1),        # rows of a little more: the first block's stays with the patches
 ])
 def test_residual_blocks_by_rows(env, monkeypatch, B, H, W, widths, act, walked):
     """The row-walking residual blocks at the edges of their tiles and runs, every stage against the oracle on a sample.
