@@ -931,15 +931,17 @@ bool conv_walk_supported(const aig_ctx* ctx, const ConvWalkGeom& g) {
   if (!walk_counts_fit(rows, g.C, rows, 4 * g.C)) return false;
   WalkParams p = conv_params(g);
   if (p.parts > ctx->sm_count || variant_layout(CONV256, p) > 227 * 1024) return false;
-  // Against the patch-resident kernel, which takes a round of one 128-position tile per SM (30 us for the first, 41, 57, 68-80 and
-  // 85-94 us for two to five) whatever the width, while this one takes 2.0 to 2.9 us a row of a tile on a share's CTAs, however
-  // full: not where whole rows fill less than 0.7 of a tile (16 frames of 576x1024, 64 columns, 0.51: 51 us by patches, 74 by rows;
-  // 8 of 720x1280, 0.63: 41, 52; 8 of 380x672, 0.67: 21.6, 22.2; 64 of 72x1440, 0.71: 40.9, 39.0), and not where the rows per CTA
-  // are more than the rounds make up for (144x256, 192 frames, 14 rows and 2 rounds: 41.8, 41.7; 222, 16 and 2: 45.0, 47.3; 256,
-  // 18.5 and 3: 56.8, 49.4; 334, 24 and 3: 62.8, 66.7; 800 of 96x160, 24.3 and 4: 72.8, 66.8; 64 of 360x640, 27 and 4: 67.9, 74.9).
-  const long long outs = (long long)ceil_div(p.P, p.tile) * p.outs_per_tile, ctas = ctx->sm_count / p.parts;
+  // Against the patch-resident kernel, which takes a round of one 128-position tile per SM (17 to 30 us for the first, 41, 57, 68-80
+  // and 85-94 us for two to five), while this one takes 2.0 to 2.9 us a row of a tile on a share's CTAs, however full, and 11 for the
+  // launch.  Not where rows of the images side by side fill less than 0.68 of the tiles (16 frames of 576x1024, 65 of 128: 51 us by
+  // patches, 74 by rows; 8 of 720x1280, 0.63: 41, 52; 8 of 380x672, 0.67: 21.6, 22.2; one of 1400x400, 0.20: 16.8, 20.5; but 64 of
+  // 72x1440, 0.71: 40.9, 39.0), unless a CTA has two rows or so (one of 576x1024, 0.51, 2.0 rows: 17.1, 15.4); and not where the rows
+  // per CTA are more than the rounds make up for (144x256, 192 frames, 14 rows and 2 rounds: 41.8, 41.7; 222, 16 and 2: 45.0, 47.3;
+  // 256, 18.5 and 3: 56.8, 49.4; 334, 24 and 3: 62.8, 66.7; 800 of 96x160, 24.3 and 4: 72.8, 66.8; 64 of 360x640, 27 and 4: 67.9, 74.9).
+  const long long tiles = ceil_div(p.P, p.tile), outs = tiles * p.outs_per_tile, ctas = ctx->sm_count / p.parts;
   const long long rounds = ceil_div_ll(ceil_div_ll(rows, 128), ctx->sm_count);
-  return 10 * p.tile >= 7 * 128 && 10 * outs <= ctas * (40 + 53 * rounds);
+  const bool full = 100ll * p.P >= 68ll * 128 * tiles;
+  return 10 * outs <= ctas * (full ? 40 + 53 * rounds : 24);
 }
 int conv_walk_create(aig_ctx* ctx, const ConvWalkGeom& g, WalkConv** out) {
   *out = nullptr;

@@ -380,8 +380,7 @@ def test_checkpoint_files(env, tmp_path):
     (150, 20, 20, (32, 64), "ACT_NONE", 2),              # the last block by rows
     (11, 90, 131, (32, 64, 128, 256, 256), "ACT_SWISH", 6),  # 256 channels: whole image rows in a tile, the last one ragged
     (40, 34, 36, (64, 256), "ACT_RELU", 1),              # and into the head directly
-    (3, 40, 250, (32, 256, 256), "ACT_LEAKY", 2),        # and a block of them before a block by patches, rows of half a tile
-    (3, 40, 262, (32, 256, 256), "ACT_LEAKY", 1),        # rows of a little more: the first block's stays with the patches
+    (3, 40, 262, (32, 256, 256), "ACT_LEAKY", 2),        # and a block of them before a block by patches, long rows
 ])
 def test_residual_blocks_by_rows(env, monkeypatch, B, H, W, widths, act, walked):
     """The row-walking residual blocks at the edges of their tiles and runs, every stage against the oracle on a sample.
@@ -412,8 +411,9 @@ def test_residual_blocks_by_rows(env, monkeypatch, B, H, W, widths, act, walked)
 @pytest.mark.parametrize("B,H,W,walked", [
     (192, 144, 256, 6), (222, 144, 256, 5), (256, 144, 256, 6), (334, 144, 256, 5),  # rows per CTA against rounds of tiles by patches
     (16, 480, 854, 6), (32, 480, 854, 5),
-    (2, 64, 1024, 1), (2, 64, 1280, 1),                                             # rows of 65 and 81 positions in a tile of 128
-    (2, 72, 1440, 2), (2, 72, 1408, 1),                                             # the least that are taken (0.71) and the most that are not (0.695)
+    (16, 576, 1024, 1), (8, 720, 1280, 1), (8, 380, 672, 5),                        # rows of 65, 81 and twice 43 positions in a tile of 128
+    (64, 72, 1392, 2), (64, 72, 1376, 1),                                           # the least that are taken (0.688) and the most that are not (0.680)
+    (1, 1400, 400, 5), (1, 576, 1024, 2),                                           # few rows to a tile, many and few rows to a CTA
 ])
 def test_which_convolutions_go_by_rows(env, monkeypatch, B, H, W, walked):
     """256-channel convolutions stay with the patch-resident kernel where that was measured to be the faster one.  (Frames
